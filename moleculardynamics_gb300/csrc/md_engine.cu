@@ -178,7 +178,7 @@ struct md_ctx {
   // io_st; a slot is reused only after its copy completed (a stream wait,
   // not a host wait)
   int anim_every = -1, anim_next = 0, anim_frames = 0, anim_slot = 0, anim_per_block = 1;
-  float* anim_dev = nullptr;  // 2 slots of 7 floats per atom
+  float* anim_dev = nullptr;  // 2 slots of 7 floats per atom, anim_pitch(n) apart
   cudaStream_t io_st = nullptr;
   cudaEvent_t anim_ready[2] = {nullptr, nullptr}, anim_done[2] = {nullptr, nullptr};
   bool anim_busy[2] = {false, false};
@@ -695,6 +695,10 @@ md_status push_record(md_ctx* c, int t) {
   return s;
 }
 
+// Floats between the two device slots of a frame: the positions are stored as
+// float4, so the second slot has to start on a 16-byte boundary for any n.
+size_t anim_pitch(int n) { return (7 * (size_t)n + 3) & ~(size_t)3; }
+
 // One animation frame of the current state (pushAnim, common/Results.cpp:12-31).
 md_status capture_frame(md_ctx* c) {
   const size_t per = 7 * (size_t)c->n;
@@ -702,7 +706,7 @@ md_status capture_frame(md_ctx* c) {
   const int s = c->anim_slot;
   c->anim_slot ^= 1;
   if (c->anim_busy[s]) CK(cudaStreamWaitEvent(c->st, c->anim_done[s], 0), "animation");
-  float* slot = c->anim_dev + (size_t)s * per;
+  float* slot = c->anim_dev + (size_t)s * anim_pitch(c->n);
   launch_anim_pack(c->pos, c->vel, c->permuted() ? c->cl.orig : nullptr, c->n, slot, c->st);
   c->stats.launches++;
   CK(cudaEventRecord(c->anim_ready[s], c->st), "animation");
@@ -1548,7 +1552,7 @@ md_status md_set_animation(md_ctx* c, int every, int frames_hint) {
   }
   const size_t fb = sizeof(float) * 7 * (size_t)c->n;
   if (!c->anim_dev) {
-    CK(cudaMalloc(&c->anim_dev, 2 * fb), "animation");
+    CK(cudaMalloc(&c->anim_dev, 2 * sizeof(float) * anim_pitch(c->n)), "animation");
     CK(cudaStreamCreateWithFlags(&c->io_st, cudaStreamNonBlocking), "animation");
     for (int k = 0; k < 2; k++) {
       CK(cudaEventCreateWithFlags(&c->anim_ready[k], cudaEventDisableTiming), "animation");
