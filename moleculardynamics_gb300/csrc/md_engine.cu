@@ -637,7 +637,7 @@ md_status make_record(md_ctx* c, int t, double* rec16) {
   }
   CK(cudaMemsetAsync(elj, 0, sizeof(double) * 8, c->st), "record");
   if (c->cfg.use_lj) {
-    int B = c->cluster ? cluster_blocks(c->cl) : lj_blocks(c->n);
+    int B = c->cluster ? cluster_blocks(c->cl) : lj_blocks(c->n, c->mixed());
     md_status s = ensure_epart(c, 3LL * B);
     if (s != MD_OK) return s;
     if (c->cluster)

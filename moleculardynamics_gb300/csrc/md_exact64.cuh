@@ -1,0 +1,170 @@
+// Correctly rounded FP64 products, quotients and square roots by integer
+// operations.
+//
+// GB300's FP64 pipe takes 64 cycles of a scheduler for a warp-wide operation
+// (1.25 TFLOP/s measured), and a division or a square root is eight to ten of
+// them.  The integer pipes run at half to full rate, so a 53-bit product by
+// 32 x 32 -> 64 multiplies costs about 25 issue slots, and a reciprocal or a
+// square root about 45: the plain FP64 Lennard-Jones pair (one square root,
+// three quotients, a dozen products, every one rounded as the reference
+// rounds it) is evaluated here with the FP64 pipe left for the additions.
+//
+// Method: a seed of 22 bits from the FP32 approximation instruction, Newton
+// steps in fixed point (the residual N - q B or N - q^2 is exact, taken modulo
+// 2^64 once it is known to fit), and one exact test of the last residual
+// against half a unit in the last place.  Quotients and roots of 53-bit
+// numbers never lie halfway between two results, so the test is strict.
+//
+// Arguments and results are the bit patterns of positive normal doubles whose
+// results are normal (no zero, subnormal, infinity or NaN): callers screen the
+// range.  Everything but the two seeds is plain integer code, compiled for
+// the host as well.
+#pragma once
+#include <stdint.h>
+
+#include <cuda_runtime.h>
+
+namespace mdgb {
+
+constexpr uint64_t kMant52 = (1ull << 52) - 1;
+
+__host__ __device__ __forceinline__ uint64_t wide32(uint32_t a, uint32_t b) {
+  return (uint64_t)a * b;
+}
+
+// hi 2^64 + lo = a b, four 32 x 32 -> 64 multiply-adds
+__host__ __device__ __forceinline__ void mul128(uint64_t a, uint64_t b, uint64_t& hi,
+                                                uint64_t& lo) {
+  const uint32_t al = (uint32_t)a, ah = (uint32_t)(a >> 32);
+  const uint32_t bl = (uint32_t)b, bh = (uint32_t)(b >> 32);
+  const uint64_t p0 = wide32(al, bl);
+  const uint64_t p1 = wide32(al, bh) + (p0 >> 32);
+  const uint64_t p2 = wide32(ah, bl) + (uint32_t)p1;
+  hi = wide32(ah, bh) + (p1 >> 32) + (p2 >> 32);
+  lo = (p2 << 32) | (uint32_t)p0;
+}
+
+__host__ __device__ __forceinline__ uint64_t mant64(uint64_t a) {
+  return (a & kMant52) | (1ull << 52);
+}
+
+// the bits of a double from its biased exponent and its mantissa with the
+// leading one (which may have carried into 2^53)
+__host__ __device__ __forceinline__ uint64_t pack64(uint32_t exponent, uint64_t m) {
+  return m + ((uint64_t)((exponent - 1) << 20) << 32);
+}
+
+// a b
+__host__ __device__ __forceinline__ uint64_t imul64(uint64_t a, uint64_t b) {
+  uint64_t hi, lo;
+  mul128(mant64(a), mant64(b) << 11, hi, lo);  // hi in [2^51, 2^53)
+  const uint32_t big = (uint32_t)(hi >> 52);   // product of mantissas at least 2
+  if (!big) {
+    hi = (hi << 1) | (lo >> 63);
+    lo <<= 1;
+  }
+  // above half a unit, or half and odd
+  const uint64_t up = lo > (1ull << 63) - (hi & 1);
+  return pack64((uint32_t)(a >> 52) + (uint32_t)(b >> 52) - 1023 + big, hi + up);
+}
+
+// the seed y of 22 bits as a 32-bit fraction (y in [0.5, 1): the true value
+// lies in (0.5, 1], the approximation may fall just outside)
+__host__ __device__ __forceinline__ uint32_t seed_fraction(uint32_t ybits) {
+  const uint32_t b = ybits < 0x3F7FFFFFu ? ybits : 0x3F7FFFFFu;
+  return b > 0x3F000000u ? (b << 8) | 0x80000000u : 0x80000000u;
+}
+
+// 1 / b from the seed's fraction y ~ 2^32 / (mantissa of b)
+__host__ __device__ __forceinline__ uint64_t ircp64_seeded(uint64_t b, uint32_t y) {
+  const uint64_t mb = mant64(b);
+  // d = 1 - y b in units of 2^-62 (below 2^40)
+  const uint64_t pl = (uint64_t)y * (uint32_t)mb, ph = (uint64_t)y * (uint32_t)(mb >> 32);
+  const int64_t d = (int64_t)((1ull << 62) - ((ph << 10) + (pl >> 22)));
+  const int32_t y31 = (int32_t)(y >> 1);
+  // c ~ 2^105 / mb within 2^9; the exact residual 2^105 - c mb fits 63 bits
+  uint64_t c = ((uint64_t)y << 21) + (uint64_t)(((int64_t)(int32_t)(d >> 10) * y31) >> 30);
+  int64_t r = (int64_t)(0 - c * mb);
+  const int32_t q =
+      (int32_t)(((int64_t)(int32_t)(r >> 32) * y31 + (1ll << 50)) >> 51);
+  c += (uint64_t)(int64_t)q;
+  r -= (int64_t)q * (int64_t)mb;
+  const int64_t h = (int64_t)mb;
+  c += (uint64_t)(2 * r > h) - (uint64_t)(2 * r < -h);
+  return pack64(2045 - (uint32_t)(b >> 52), c);
+}
+
+// sqrt(x) from the seed's fraction y ~ 2^32 / sqrt(v), x = v 4^k, v in [1, 4);
+// sq receives the rounded square of the rounded root
+__host__ __device__ __forceinline__ uint64_t isqrt64_seeded(uint64_t x, uint32_t y,
+                                                            uint64_t& sq) {
+  const uint32_t ex = (uint32_t)(x >> 52), even = ~ex & 1;
+  const uint64_t m = mant64(x), M = m << (10 + even);  // v 2^62
+  const int32_t y31 = (int32_t)(y >> 1);
+  const uint32_t g = (uint32_t)(wide32((uint32_t)(M >> 32), y) >> 32);  // sqrt(v) 2^30
+  const int64_t d = (int64_t)((M >> 2) - wide32(g, g));
+  uint64_t c = ((uint64_t)g << 20) + (uint64_t)(((int64_t)(int32_t)(d >> 12) * y31) >> 30);
+  // c ~ sqrt(v) 2^50 within 2^9; the exact residual v 2^100 - c^2 fits 62 bits
+  int64_t r = (int64_t)((M << 38) - c * c);
+  const int32_t q =
+      (int32_t)(((int64_t)(int32_t)(r >> 32) * y31 + (1ll << 47)) >> 48);
+  c <<= 2;
+  r = (int64_t)((uint64_t)r << 4) - (int64_t)q * (int64_t)(2 * c + (uint64_t)(int64_t)q);
+  c += (uint64_t)(int64_t)q;
+  const int64_t h = (int64_t)c;
+  if (r > h) {  // (c + 1)^2 = c^2 + 2 c + 1
+    r -= 2 * h + 1;
+    c++;
+  } else if (r <= -h) {
+    r += 2 * h - 1;
+    c--;
+  }
+  const uint64_t root = pack64((ex + 1023) >> 1, c);
+  // the square is m 2^(52 + even) - r, |r| < 2^53: m less r rounded to whole
+  // units.  At the ends of the binade the unit may change: take the product.
+  if (m - ((1ull << 52) + 2) < (1ull << 52) - 4) {
+    const uint64_t t = m - (uint64_t)(r >> (52 + even));
+    const uint64_t f = (uint64_t)r & ((1ull << (52 + even)) - 1);
+    sq = pack64(ex, t - (uint64_t)(f + (t & 1) > (1ull << (51 + even))));
+  } else {
+    sq = imul64(root, root);
+  }
+  return root;
+}
+
+// a / b for a divisor known beforehand: y = divisor_fraction(b)
+__host__ __device__ __forceinline__ uint64_t idiv64_const(uint64_t a, uint64_t b, uint64_t y) {
+  const uint64_t ma = mant64(a), mb = mant64(b);
+  uint64_t t, low;  // t = 2^63 a / b, at most 2 below
+  mul128(ma << 11, y, t, low);
+  const uint32_t s = (uint32_t)(t >> 63);
+  uint64_t c = t >> (10 + s);
+  const uint64_t r = (ma << (53 - s)) - c * mb;  // in [0, 2 mb)
+  c += (uint64_t)(2 * r > mb) + (uint64_t)(2 * r > 3 * mb);
+  return pack64((uint32_t)(a >> 52) - (uint32_t)(b >> 52) + 1022 + s, c);
+}
+
+// floor(2^116 / mantissa of b), at most 2^64 - 1
+inline uint64_t divisor_fraction(uint64_t b) {
+  const unsigned __int128 q = ((unsigned __int128)1 << 116) / mant64(b);
+  return q >> 64 ? ~0ull : (uint64_t)q;
+}
+
+#ifdef __CUDACC__
+__device__ __forceinline__ uint64_t ircp64(uint64_t b) {
+  const uint32_t f = 0x3F800000u | (uint32_t)((b >> 29) & 0x7FFFFFu);
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint_as_float(f)));
+  return ircp64_seeded(b, seed_fraction(__float_as_uint(y)));
+}
+
+__device__ __forceinline__ uint64_t isqrt64(uint64_t x, uint64_t& sq) {
+  const uint32_t odd = (uint32_t)(x >> 52) & 1;  // odd biased exponent: v in [1, 2)
+  const uint32_t f = (odd ? 0x3F800000u : 0x40000000u) | (uint32_t)((x >> 29) & 0x7FFFFFu);
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint_as_float(f)));
+  return isqrt64_seeded(x, seed_fraction(__float_as_uint(y)), sq);
+}
+#endif
+
+}  // namespace mdgb

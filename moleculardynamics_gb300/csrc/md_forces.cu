@@ -1,10 +1,10 @@
 // Force kernels: Lennard-Jones (cpu/common/LennardJones.h) and the bond-order
 // many-body term (cpu/common/BondOrderFuncs.h).
 //
-// LJ, FP64 ("plain"): one thread per atom walks its compact row in the
-// reference's candidate order and evaluates every in-range pair with the
-// reference's roundings (no FMA contraction), so that forces are bit-identical
-// to the reference on the same positions and list.
+// LJ, FP64 ("plain"): a few lanes per atom evaluate its compact row with the
+// reference's roundings (integer operations in place of most of the narrow
+// FP64 pipe's) and add the pairs in the reference's candidate order, so that
+// forces are bit-identical to the reference on the same positions and list.
 // LJ, FP32 (precision form): same rows; pair arithmetic in FP32 from the FP32
 // position copy; pairs within 1e-5 of the cutoff are re-tested in FP64 so the
 // pair set equals the FP64 one; per-atom sums are FP32 chunks of 16 pairs
@@ -17,9 +17,11 @@
 //           loops over j of i's short list that lie in k's candidate row and
 //           adds k's third-body force (BondOrderFuncs.h:148-237, 339-393).
 // Lane sums are combined with warp shuffles.
-#include <type_traits>
 #include <cmath>
+#include <cstring>
+#include <type_traits>
 
+#include "md_exact64.cuh"
 #include "md_forces.h"
 #include "md_neighbor.cuh"
 #include "md_potential.cuh"
@@ -64,91 +66,279 @@ __device__ __forceinline__ void block_partial(double (&v)[NV], double* out) {
 }
 
 // ------------------------------------------------------------------ LJ FP64
+// Per species-pair constants of the exact pair (LennardJones.h:12-30): sigma^2
+// with its fraction for the division, 24 eps / sigma^2, and the energy terms.
+struct LjPairConst {
+  double sq[3], con[3], eps2[3], eshift[3];
+  uint64_t yq[3];
+};
+
+// d d, rounded; the FP64 pipe near the ends of the exponent range (0 is 0)
+__device__ __forceinline__ double sq64(double d) {
+  const uint64_t b = (uint64_t)__double_as_longlong(d) & ~(1ull << 63);
+  if ((uint32_t)(b >> 52) - 512u < 1022u) return __longlong_as_double((long long)imul64(b, b));
+  return b == 0 ? 0.0 : xmul(d, d);
+}
+
+// the FP64 instructions, out of line (see lj_terms)
+__device__ __noinline__ double3 lj_terms_far(double r2, double ijx, double ijy, double ijz,
+                                             double sq, double con) {
+  // from zero sums the additions return the products themselves
+  double3 t = make_double3(0.0, 0.0, 0.0);
+  lj_pair_exact_c(t.x, t.y, t.z, __dsqrt_rn(r2), ijx, ijy, ijz, sq, con);
+  return t;
+}
+
+// r_ij f_ij of a pair in (tx, ty, tz): LennardJones.h:12-30 with every rounding
+// of the reference.  The root, the quotients and the power chain are integer
+// operations (md_exact64.cuh); the last five operations stay on the FP64 pipe,
+// which the integers leave idle otherwise (with those in integers too the
+// 108,000-atom launch took 276 us, not 255).  Squared distances outside
+// 2^-30 .. 2^30 take lj_pair_exact_c's instructions.
+__device__ __forceinline__ void lj_terms(double r2, double ijx, double ijy, double ijz, double sq,
+                                         uint64_t yq, double con, double& tx, double& ty,
+                                         double& tz) {
+  const uint64_t rb = (uint64_t)__double_as_longlong(r2);
+  if ((uint32_t)(rb >> 52) - 993u < 60u) {
+    uint64_t d2;  // the rounded square of the rounded root
+    isqrt64(rb, d2);
+    const uint64_t dist2 = idiv64_const(d2, (uint64_t)__double_as_longlong(sq), yq);
+    const uint64_t dist4 = imul64(dist2, dist2);
+    const uint64_t dist8 = imul64(dist4, dist4);
+    const uint64_t dist14 = imul64(imul64(dist2, dist4), dist8);
+    const uint64_t inv8 = ircp64(dist8), inv14 = ircp64(dist14);
+    // 2 / dist14 is exact: one more in the exponent
+    const double s = xsub(__longlong_as_double((long long)(inv14 + (1ull << 52))),
+                          __longlong_as_double((long long)inv8));
+    const double fij = xmul(s, con);
+    tx = xmul(ijx, fij);
+    ty = xmul(ijy, fij);
+    tz = xmul(ijz, fij);
+    return;
+  }
+  const double3 t = lj_terms_far(r2, ijx, ijy, ijz, sq, con);
+  tx = t.x;
+  ty = t.y;
+  tz = t.z;
+}
+
+// (int)w of a species word (0, 1 or 2 as a double) without a conversion
+// instruction, which takes the FP64 pipe
+__device__ __forceinline__ int species64(double w) {
+  const uint32_t hi = (uint32_t)__double2hiint(w);
+  if (hi - 0x40000000u < 0x80000u) return 2;
+  if (hi - 0x3FF00000u < 0x100000u) return 1;
+  return (hi & 0x7FFFFFFFu) < 0x3FF00000u ? 0 : (int)w;
+}
+
+// x truncated to FP32 by moving the fields (tiny values to 0; NaN beyond
+// FP32's range, so that no screen rejects it)
+__device__ __forceinline__ float trunc32(double x) {
+  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+  const uint32_t e = (hi >> 20) & 0x7FFu;
+  if (e >= 1151u) return __int_as_float(0x7FC00000);
+  const uint32_t m = ((hi & 0xFFFFFu) << 3) | (lo >> 29);
+  return __uint_as_float(e < 897u ? 0u : (hi & 0x80000000u) | ((e - 896u) << 23) | m);
+}
+
+// x + img box, img in {-1, 0, 1} (the product is exact: no operation for it)
+__device__ __forceinline__ double image64(double x, int img, double box) {
+  return img == 0 ? x : xadd(x, img > 0 ? box : -box);
+}
+
+__device__ __forceinline__ bool below64(double r2, double rcutsq) {
+  // r2 >= 0: the order of the bit patterns; a NaN counts as inside, as the
+  // comparison r2 >= rcutsq is false for it
+  const uint64_t a = (uint64_t)__double_as_longlong(r2);
+  return a < (uint64_t)__double_as_longlong(rcutsq) || a > 0x7FF0000000000000ull;
+}
+
+// common/DebugCalculations.cpp:199-201 per ordered pair, restricted to the
+// force's pairs; shifted by its value at the cutoff; the virial
+__device__ __forceinline__ void lj64_energy(double r2, double ijx, double ijy, double ijz,
+                                            double tx, double ty, double tz,
+                                            const LjPairConst& c, int sel, double* ev) {
+  const double sr2 = xdiv(c.sq[sel], r2);
+  const double sr6 = xmul(xmul(sr2, sr2), sr2);
+  const double e = xmul(c.eps2[sel], xsub(xmul(sr6, sr6), sr6));
+  ev[0] += e;
+  ev[1] += e - c.eshift[sel];
+  ev[2] += 0.5 * (ijx * tx + ijy * ty + ijz * tz);
+}
+
+// One atom by one thread (a tripped skin: the full candidate row, the
+// reference's row and order, and a fresh compact row at the current
+// positions).
 template <bool ENERGY>
-__global__ void __launch_bounds__(128)
+__device__ __noinline__ void lj64_refresh(int i, const md_double4* __restrict__ pos,
+                                          double* __restrict__ f3, int ld,
+                                          uint32_t* __restrict__ list, int* __restrict__ len,
+                                          const RowWalker& w, int* skin, int cap, float rv2,
+                                          float4* __restrict__ pos_build, double rcutsq,
+                                          const LjPairConst& c, double* ev) {
+  const md_double4 pi = pos[i];
+  const int ti = species64(pi.w);
+  const double box = w.g.box;
+  const float4 pc = cur_pos(pos, (const float4*)nullptr, i);
+  double fx = 0.0, fy = 0.0, fz = 0.0;
+  int kept = 0;
+  walk_row(w, pos, i, [&](int m, int ix, int iy, int iz) {
+    const md_double4 pj = pos[m];
+    double xj = pj.x, yj = pj.y, zj = pj.z;
+    if (w.g.periodic && (ix | iy | iz)) {
+      xj = xadd(xj, (double)ix * box);
+      yj = xadd(yj, (double)iy * box);
+      zj = xadd(zj, (double)iz * box);
+    }
+    const double ijx = xsub(pi.x, xj), ijy = xsub(pi.y, yj), ijz = xsub(pi.z, zj);
+    const double r2 = norm2_exact(ijx, ijy, ijz);
+    const int tj = species64(pj.w);
+    if (below64(r2, rcutsq) && (tj == SP_NG || ti == SP_NG)) {
+      const int sel = lj_select(ti, tj);
+      double tx, ty, tz;
+      lj_terms(r2, ijx, ijy, ijz, c.sq[sel], c.yq[sel], c.con[sel], tx, ty, tz);
+      fx = xadd(fx, tx);
+      fy = xadd(fy, ty);
+      fz = xadd(fz, tz);
+      if (ENERGY) lj64_energy(r2, ijx, ijy, ijz, tx, ty, tz, c, sel, ev);
+    }
+    const float4 pm = cur_pos(pos, (const float4*)nullptr, m);
+    const float dx = pc.x - (pm.x + (float)ix * w.g.box_f);
+    const float dy = pc.y - (pm.y + (float)iy * w.g.box_f);
+    const float dz = pc.z - (pm.z + (float)iz * w.g.box_f);
+    if (dx * dx + dy * dy + dz * dz < rv2) {
+      if (kept < cap) list[(size_t)kept * ld + i] = pack_entry(m, ix, iy, iz);
+      kept++;
+    }
+  });
+  if (kept > cap) atomicOr(&skin[2], 1);
+  len[i] = kept < cap ? kept : cap;
+  pos_build[i] = pc;
+  f3[3 * i] = fx;
+  f3[3 * i + 1] = fy;
+  f3[3 * i + 2] = fz;
+}
+
+constexpr int kLj64Cap = 96;  // screened entries of a group in shared memory
+
+// G lanes of a warp per atom.  The row is read G entries at a time; an FP32
+// screen (conservative: the cutoff widened by the truncation error of the
+// coordinates) drops the entries beyond the cutoff, and the others queue in
+// shared memory in row order.  Then each lane evaluates one queued pair, and
+// three lanes add the G products of their component one after another, so the
+// sums run in the reference's order and forces are bit-identical to it for
+// every G.
+// The FP64 pipe bounds it (14 operations per pair of one lane and 4 of three
+// lanes for the sums, at 64 cycles each), then the latency of the integer
+// chains: 64 registers (8 blocks per SM) took 255 us for 108,000 atoms, 72
+// registers 259, 80 registers 267, 96 unbounded 280; one thread per atom with
+// the FP64 instructions took 1010.
+template <int G, bool ENERGY>
+__global__ void __launch_bounds__(128, 8)
     k_lj_fp64(const md_double4* __restrict__ pos, double* __restrict__ f3, int n, int ld,
               uint32_t* __restrict__ list, int* __restrict__ len, RowWalker w, int* skin,
               int parity, int cap, float rv2, float4* __restrict__ pos_build, double rcutsq,
-              Species sp, double* __restrict__ epart) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+              const __grid_constant__ LjPairConst c, double* __restrict__ epart) {
+  constexpr int kAtoms = 32 / G;  // atoms per warp
+  __shared__ uint32_t queue[128 / G][kLj64Cap];
+  __shared__ double term[4][3][32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int gl = lane & (G - 1), group = lane / G;
   double ev[3] = {0.0, 0.0, 0.0};
-  if (i < n) {
-    const md_double4 pi = pos[i];
-    const int ti = (int)pi.w;
+  const bool tripped = (skin[parity] | skin[2]) != 0;
+  const int t = blockIdx.x * 128 + tid;
+  if (t == 0) skin[parity ^ 1] = 0;  // the next step's flag starts clear
+  if (tripped) {
+    // one thread per atom; the grid holds at least n threads
+    if (t < n)
+      lj64_refresh<ENERGY>(t, pos, f3, ld, list, len, w, skin, cap, rv2, pos_build, rcutsq, c, ev);
+    if (t == 0) atomicAdd(&skin[3], 1);
+  } else {
+    const int i = (blockIdx.x * 4 + warp) * kAtoms + group;
+    const bool live = i < n;
+    const md_double4 pi = live ? pos[i] : md_double4{0, 0, 0, 0};
+    const int ti = species64(pi.w);
     const double box = w.g.box;
-    double fx = 0.0, fy = 0.0, fz = 0.0;
-    // the species-pair constants of LennardJones.h:12-30, once per thread
-    double sq[3], cn[3];
+    const float xf = trunc32(pi.x), yf = trunc32(pi.y), zf = trunc32(pi.z);
+    // screen: each coordinate is off by less than 2^-23 of itself, and a pair
+    // inside the cutoff has |x_j| <= |x_i| + rcut (+ the box, for an image)
+    const float rc2 = (float)rcutsq * 1.000001f, rc = sqrtf(rc2), bf = w.g.box_f;
+    const float off = (fmaxf(fabsf(xf), fmaxf(fabsf(yf), fabsf(zf))) + fabsf(bf) + rc) * 0x1p-20f;
+    const float thr = rc2 + off * (8.0f * rc + 16.0f * off);
+    uint32_t* q = queue[warp * kAtoms + group];
+    double acc = 0.0;  // lane gl < 3: component gl
+    const int L = live ? len[i] : 0;
+    int k0 = 0;
+    for (;;) {
+      // screen until the queue could overflow or every row of the warp ends
+      int cnt = 0;
+      while (__any_sync(0xffffffffu, k0 < L && cnt + G <= kLj64Cap)) {
+        const bool go = k0 < L && cnt + G <= kLj64Cap;
+        const int k = k0 + gl;
+        bool keep = false;
+        uint32_t e = 0;
+        if (go && k < L) {
+          e = list[(size_t)k * ld + i];
+          const md_double4 pj = pos[entry_index(e)];
+          float dx = xf - trunc32(pj.x), dy = yf - trunc32(pj.y), dz = zf - trunc32(pj.z);
+          if (e >> 26) {
+            dx -= (float)entry_img(e, 0) * bf;
+            dy -= (float)entry_img(e, 1) * bf;
+            dz -= (float)entry_img(e, 2) * bf;
+          }
+          keep = !(dx * dx + dy * dy + dz * dz > thr);
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, keep) >> (group * G) &
+                           (G == 32 ? 0xffffffffu : (1u << (G & 31)) - 1u);
+        if (keep) q[cnt + __popc(m & ((1u << gl) - 1u))] = e;
+        cnt += __popc(m);
+        if (go) k0 += G;
+      }
+      __syncwarp();
+      int most = cnt;
 #pragma unroll
-    for (int t = 0; t < 3; t++) {
-      sq[t] = lj_sigsq(sp.sig[t]);
-      cn[t] = lj_con(sp.eps[t], sq[t]);
-    }
-    auto visit = [&](int j, int ix, int iy, int iz, bool img) {
-      const md_double4 pj = pos[j];
-      double xj = pj.x, yj = pj.y, zj = pj.z;
-      if (img) {
-        xj = xadd(xj, (double)ix * box);
-        yj = xadd(yj, (double)iy * box);
-        zj = xadd(zj, (double)iz * box);
-      }
-      const double ijx = xsub(pi.x, xj), ijy = xsub(pi.y, yj), ijz = xsub(pi.z, zj);
-      const double r2 = norm2_exact(ijx, ijy, ijz);
-      if (r2 >= rcutsq) return;
-      const int tj = (int)pj.w;
-      if (tj == SP_NG || ti == SP_NG) {
-        const int sel = lj_select(ti, tj);
-        const double sig = sp.sig[sel], eps = sp.eps[sel];
-        const double sigsq = sel == 0 ? sq[0] : (sel == 1 ? sq[1] : sq[2]);
-        const double con = sel == 0 ? cn[0] : (sel == 1 ? cn[1] : cn[2]);
-        const double fij = lj_pair_exact_c(fx, fy, fz, __dsqrt_rn(r2), ijx, ijy, ijz, sigsq, con);
-        if (ENERGY) {
-          // common/DebugCalculations.cpp:199-201 per ordered pair, restricted
-          // to the force's pairs; shifted by its value at the cutoff
-          double sr2 = xdiv(xmul(sig, sig), r2);
-          double sr6 = xmul(xmul(sr2, sr2), sr2);
-          double e = xmul(xmul(2.0, eps), xsub(xmul(sr6, sr6), sr6));
-          double src2 = xdiv(xmul(sig, sig), rcutsq);
-          double src6 = xmul(xmul(src2, src2), src2);
-          ev[0] += e;
-          ev[1] += e - xmul(xmul(2.0, eps), xsub(xmul(src6, src6), src6));
-          ev[2] += 0.5 * (ijx * (ijx * fij) + ijy * (ijy * fij) + ijz * (ijz * fij));
+      for (int o = 16; o >= G; o >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
+      for (int s0 = 0; s0 < most; s0 += G) {
+        double tx = 0.0, ty = 0.0, tz = 0.0;
+        bool in = s0 + gl < cnt;
+        if (in) {
+          const uint32_t e = q[s0 + gl];
+          const md_double4 pj = pos[entry_index(e)];
+          double xj = pj.x, yj = pj.y, zj = pj.z;
+          if (e >> 26) {
+            xj = image64(xj, entry_img(e, 0), box);
+            yj = image64(yj, entry_img(e, 1), box);
+            zj = image64(zj, entry_img(e, 2), box);
+          }
+          const double ijx = xsub(pi.x, xj), ijy = xsub(pi.y, yj), ijz = xsub(pi.z, zj);
+          const double r2 = xadd(xadd(sq64(ijx), sq64(ijy)), sq64(ijz));
+          const int tj = species64(pj.w);
+          in = below64(r2, rcutsq) && (tj == SP_NG || ti == SP_NG);
+          if (in) {
+            const int sel = lj_select(ti, tj);
+            const double sq = sel == 0 ? c.sq[0] : (sel == 1 ? c.sq[1] : c.sq[2]);
+            const double con = sel == 0 ? c.con[0] : (sel == 1 ? c.con[1] : c.con[2]);
+            const uint64_t yq = sel == 0 ? c.yq[0] : (sel == 1 ? c.yq[1] : c.yq[2]);
+            lj_terms(r2, ijx, ijy, ijz, sq, yq, con, tx, ty, tz);
+            if (ENERGY) lj64_energy(r2, ijx, ijy, ijz, tx, ty, tz, c, sel, ev);
+          }
         }
-      }
-    };
-    const bool tripped = (skin[parity] | skin[2]) != 0;
-    if (!tripped) {
-      const int L = len[i];
-      for (int k = 0; k < L; k++) {
-        const uint32_t e = list[(size_t)k * ld + i];
-        visit(entry_index(e), entry_img(e, 0), entry_img(e, 1), entry_img(e, 2), (e >> 26) != 0);
-      }
-    } else {
-      // skin exceeded: walk the full candidate row (the reference's row,
-      // same order) and refresh this atom's compact row at the current
-      // positions, so that the following steps use the compact row again
-      const float4 pc = cur_pos(pos, (const float4*)nullptr, i);
-      int kept = 0;
-      walk_row(w, pos, i, [&](int m, int ix, int iy, int iz) {
-        visit(m, ix, iy, iz, w.g.periodic && (ix | iy | iz));
-        const float4 pm = cur_pos(pos, (const float4*)nullptr, m);
-        const float dx = pc.x - (pm.x + (float)ix * w.g.box_f);
-        const float dy = pc.y - (pm.y + (float)iy * w.g.box_f);
-        const float dz = pc.z - (pm.z + (float)iz * w.g.box_f);
-        if (dx * dx + dy * dy + dz * dz < rv2) {
-          if (kept < cap) list[(size_t)kept * ld + i] = pack_entry(m, ix, iy, iz);
-          kept++;
+        const unsigned m = __ballot_sync(0xffffffffu, in) >> (group * G);
+        term[warp][0][lane] = tx;
+        term[warp][1][lane] = ty;
+        term[warp][2][lane] = tz;
+        __syncwarp();
+        if (gl < 3) {
+          const double* tv = &term[warp][gl][group * G];
+#pragma unroll
+          for (int s = 0; s < G; s++)
+            if ((m >> s) & 1u) acc = xadd(acc, tv[s]);
         }
-      });
-      if (kept > cap) atomicOr(&skin[2], 1);
-      len[i] = kept < cap ? kept : cap;
-      pos_build[i] = pc;
-      if (i == 0) atomicAdd(&skin[3], 1);
+        __syncwarp();
+      }
+      if (!__any_sync(0xffffffffu, k0 < L)) break;
     }
-    if (i == 0) skin[parity ^ 1] = 0;  // the next step's flag starts clear
-    f3[3 * i] = fx;
-    f3[3 * i + 1] = fy;
-    f3[3 * i + 2] = fz;
+    if (live && gl < 3) f3[3 * i + gl] = acc;
   }
   if (ENERGY) block_partial<3>(ev, epart);
 }
@@ -941,19 +1131,54 @@ inline int nblk(long long n, int t) { return (int)((n + t - 1) / t); }
 
 }  // namespace
 
+// Lanes per atom of the FP64 LJ kernel: the most that keep the launch within
+// four warps per scheduler (n G / 32 <= 16 x 152), as every doubling costs
+// throughput (the ordered sums keep three lanes of each group) and gains
+// latency.  Measured, us per launch with 4 / 8 / 16 / 32 lanes: 864 atoms
+// - / - / 18 / 17 (205 with a thread per atom), 8,000 atoms
+// 44 / 35 / 38 / 53 (207), 108,000 atoms 255 / 270 / - / - (1010).
+static int lj64_lanes(int n) {
+  const long long room = 16LL * 152 * 32;
+  return n * 32LL <= room ? 32 : (n * 16LL <= room ? 16 : (n * 8LL <= room ? 8 : 4));
+}
+
+template <int G>
+static void launch_lj64(const ForceArgs& a, const LjPairConst& c, bool energy, cudaStream_t st) {
+  const int B = nblk((long long)a.n * G, 128);
+  if (energy)
+    k_lj_fp64<G, true><<<B, 128, 0, st>>>(a.pos, a.f3, a.n, a.ld, a.list, a.len, a.walker, a.skin,
+                                          a.parity, a.cap, a.rv2, a.pos_build, a.rcutsq, c,
+                                          a.epart);
+  else
+    k_lj_fp64<G, false><<<B, 128, 0, st>>>(a.pos, a.f3, a.n, a.ld, a.list, a.len, a.walker,
+                                           a.skin, a.parity, a.cap, a.rv2, a.pos_build, a.rcutsq,
+                                           c, nullptr);
+}
+
 void launch_lj(const ForceArgs& a, bool fp32, bool energy, cudaStream_t st) {
   const int T = 128;
   const int B = nblk(a.n, T);
   if (B == 0) return;
   if (!fp32) {
-    if (energy)
-      k_lj_fp64<true><<<B, T, 0, st>>>(a.pos, a.f3, a.n, a.ld, a.list, a.len, a.walker, a.skin,
-                                       a.parity, a.cap, a.rv2, a.pos_build, a.rcutsq, a.sp,
-                                       a.epart);
-    else
-      k_lj_fp64<false><<<B, T, 0, st>>>(a.pos, a.f3, a.n, a.ld, a.list, a.len, a.walker, a.skin,
-                                        a.parity, a.cap, a.rv2, a.pos_build, a.rcutsq, a.sp,
-                                        a.epart);
+    LjPairConst c;
+    for (int t = 0; t < 3; t++) {
+      const double sig = a.sp.sig[t], eps = a.sp.eps[t];
+      c.sq[t] = sig * sig;
+      c.con[t] = 24.0 * eps / c.sq[t];
+      c.eps2[t] = 2.0 * eps;
+      const double src2 = c.sq[t] / a.rcutsq, src6 = src2 * src2 * src2;
+      const double src12 = src6 * src6;
+      c.eshift[t] = c.eps2[t] * (src12 - src6);
+      uint64_t b;
+      memcpy(&b, &c.sq[t], sizeof(b));
+      c.yq[t] = divisor_fraction(b);
+    }
+    switch (lj64_lanes(a.n)) {
+      case 32: launch_lj64<32>(a, c, energy, st); break;
+      case 16: launch_lj64<16>(a, c, energy, st); break;
+      case 8: launch_lj64<8>(a, c, energy, st); break;
+      default: launch_lj64<4>(a, c, energy, st);
+    }
   } else if (!energy && a.tmap) {
     const int TB = nblk(a.n, kListTileAtoms);
     if (a.all_ng)
@@ -978,7 +1203,9 @@ void launch_lj(const ForceArgs& a, bool fp32, bool energy, cudaStream_t st) {
   }
 }
 
-int lj_blocks(int n) { return nblk(n, 128); }
+int lj_blocks(int n, bool fp32) {
+  return fp32 ? nblk(n, 128) : nblk((long long)n * lj64_lanes(n), 128);
+}
 int mb_blocks(int n) { return nblk(n, 4); }
 
 template <typename T, bool ENERGY>

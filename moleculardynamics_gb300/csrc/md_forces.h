@@ -55,7 +55,7 @@ struct MbArgs {
 
 void launch_lj(const ForceArgs& a, bool fp32, bool energy, cudaStream_t st);
 void launch_mb(const MbArgs& a, bool fp32, bool energy, cudaStream_t st);
-int lj_blocks(int n);
+int lj_blocks(int n, bool fp32);  // blocks of an energy launch of launch_lj
 int mb_blocks(int n);
 
 }  // namespace mdgb
