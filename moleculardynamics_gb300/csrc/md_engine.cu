@@ -144,7 +144,7 @@ struct md_ctx {
   // bond-order scratch
   uint32_t* mb_sl = nullptr;
   int* mb_slen = nullptr;
-  void *xsi = nullptr, *xsj = nullptr;
+  void *xsi = nullptr, *xsj = nullptr, *mb_fslot = nullptr;
   long long mb_elems = 0;
   // flags and reductions
   int* status = nullptr;
@@ -268,15 +268,21 @@ md_status ensure_epart(md_ctx* c, long long need) {
   return MD_OK;
 }
 
+// slots per atom of the bond-order short lists (read in 16-byte words)
+int mb_pitch(const md_ctx* c) { return (std::max(c->mb.cap, 1) + 3) & ~3; }
+
 md_status ensure_mb_scratch(md_ctx* c) {
-  long long need = (long long)c->mb.cap * (c->cfg.n_mb > 0 ? c->cfg.n_mb : 1);
+  const size_t nmb = (size_t)std::max(c->cfg.n_mb, 1);
+  const size_t es = c->mixed() ? sizeof(float) : sizeof(double);
+  if (!c->mb_fslot)
+    CK(cudaMalloc(&c->mb_fslot, 4 * es * kMbSlotCount * nmb), "mb third-body forces");
+  const long long need = (long long)mb_pitch(c) * (long long)nmb;
   if (need <= c->mb_elems && c->mb_sl) return MD_OK;
   for (void** p : {(void**)&c->mb_sl, &c->xsi, &c->xsj})
     if (*p) {
       cudaFree(*p);
       *p = nullptr;
     }
-  size_t es = sizeof(double);
   CK(cudaMalloc(&c->mb_sl, sizeof(uint32_t) * (size_t)need), "mb short list");
   CK(cudaMalloc(&c->xsi, es * (size_t)need), "mb xi");
   CK(cudaMalloc(&c->xsj, es * (size_t)need), "mb xi");
@@ -326,6 +332,8 @@ MbArgs mb_args(md_ctx* c, double* f3, int ljexist) {
   a.rcutsq = (double)c->mb_rcutsq;
   a.ljexist = ljexist;
   a.sl = c->mb_sl;
+  a.pitch = mb_pitch(c);
+  a.fslot = c->mb_fslot;
   a.slen = c->mb_slen;
   a.xsi = c->xsi;
   a.xsj = c->xsj;
@@ -1096,7 +1104,7 @@ void md_destroy(md_ctx* c) {
   for (cudaGraphExec_t x : c->gexec)
     if (x) cudaGraphExecDestroy(x);
   void* ptrs[] = {c->sur_flags, c->seq_buf, c->inv, c->sur_fx, c->sur_fs, c->rep_ranges, c->rep_buf, c->io, c->pos_alt, c->posf_alt, c->pos, c->vel, c->acc, c->b, c->c, c->f3, c->f3_tmp, c->posf, c->mb_sl,
-                  c->mb_slen, c->xsi, c->xsj, c->status, c->epart, c->dsc, c->rec,
+                  c->mb_slen, c->xsi, c->xsj, c->mb_fslot, c->status, c->epart, c->dsc, c->rec,
                   c->sc.dpart, c->sc.umax, c->sc.counts, c->sc.block_sums};
   for (void* p : ptrs)
     if (p) cudaFree(p);

@@ -165,6 +165,92 @@ __device__ __forceinline__ uint64_t isqrt64(uint64_t x, uint64_t& sq) {
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint_as_float(f)));
   return isqrt64_seeded(x, seed_fraction(__float_as_uint(y)), sq);
 }
+
+// ---- nearly rounded reciprocal, root and exponential for FP64 kernels whose
+// results carry a tolerance (the bond order): one Newton step of third order
+// from the same 22-bit seeds, so three and five FP64 operations instead of the
+// library's eight to ten; errors below 1 ulp (reciprocal, inverse root) ----
+
+// 1 / b, b positive and normal with a normal reciprocal
+__device__ __forceinline__ double rcp64(double b) {
+  const uint64_t bb = (uint64_t)__double_as_longlong(b);
+  const uint32_t f = 0x3F800000u | (uint32_t)((bb >> 29) & 0x7FFFFFu);
+  float s;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(__uint_as_float(f)));
+  const uint32_t m = seed_fraction(__float_as_uint(s)) << 1;  // below the leading one
+  const double y = __hiloint2double(
+      (int)(((2045u - (uint32_t)(bb >> 52)) << 20) | (m >> 12)), (int)(m << 20));
+  const double e = fma(-b, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+
+// 1 / sqrt(x), x positive and normal, or 0
+__device__ __forceinline__ double rsqrt64(double x) {
+  const uint64_t xb = (uint64_t)__double_as_longlong(x);
+  const uint32_t ex = (uint32_t)(xb >> 52);
+  if (ex == 0) return __longlong_as_double(0x7FF0000000000000ll);  // 0: infinity
+  const uint32_t f = ((ex & 1) ? 0x3F800000u : 0x40000000u) | (uint32_t)((xb >> 29) & 0x7FFFFFu);
+  float s;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(__uint_as_float(f)));
+  const uint32_t m = seed_fraction(__float_as_uint(s)) << 1;
+  // x = v 4^k with 1023 + k = (ex + 1023) >> 1
+  const double y = __hiloint2double(
+      (int)(((2045u - ((ex + 1023u) >> 1)) << 20) | (m >> 12)), (int)(m << 20));
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y, e * fma(0.375, e, 0.5), y);
+}
+
+// 2^(k / 64)
+static __device__ const double kExp2Table[64] = {
+    0x1.0000000000000p+0, 0x1.02c9a3e778061p+0, 0x1.059b0d3158574p+0, 0x1.0874518759bc8p+0,
+    0x1.0b5586cf9890fp+0, 0x1.0e3ec32d3d1a2p+0, 0x1.11301d0125b51p+0, 0x1.1429aaea92de0p+0,
+    0x1.172b83c7d517bp+0, 0x1.1a35beb6fcb75p+0, 0x1.1d4873168b9aap+0, 0x1.2063b88628cd6p+0,
+    0x1.2387a6e756238p+0, 0x1.26b4565e27cddp+0, 0x1.29e9df51fdee1p+0, 0x1.2d285a6e4030bp+0,
+    0x1.306fe0a31b715p+0, 0x1.33c08b26416ffp+0, 0x1.371a7373aa9cbp+0, 0x1.3a7db34e59ff7p+0,
+    0x1.3dea64c123422p+0, 0x1.4160a21f72e2ap+0, 0x1.44e086061892dp+0, 0x1.486a2b5c13cd0p+0,
+    0x1.4bfdad5362a27p+0, 0x1.4f9b2769d2ca7p+0, 0x1.5342b569d4f82p+0, 0x1.56f4736b527dap+0,
+    0x1.5ab07dd485429p+0, 0x1.5e76f15ad2148p+0, 0x1.6247eb03a5585p+0, 0x1.6623882552225p+0,
+    0x1.6a09e667f3bcdp+0, 0x1.6dfb23c651a2fp+0, 0x1.71f75e8ec5f74p+0, 0x1.75feb564267c9p+0,
+    0x1.7a11473eb0187p+0, 0x1.7e2f336cf4e62p+0, 0x1.82589994cce13p+0, 0x1.868d99b4492edp+0,
+    0x1.8ace5422aa0dbp+0, 0x1.8f1ae99157736p+0, 0x1.93737b0cdc5e5p+0, 0x1.97d829fde4e50p+0,
+    0x1.9c49182a3f090p+0, 0x1.a0c667b5de565p+0, 0x1.a5503b23e255dp+0, 0x1.a9e6b5579fdbfp+0,
+    0x1.ae89f995ad3adp+0, 0x1.b33a2b84f15fbp+0, 0x1.b7f76f2fb5e47p+0, 0x1.bcc1e904bc1d2p+0,
+    0x1.c199bdd85529cp+0, 0x1.c67f12e57d14bp+0, 0x1.cb720dcef9069p+0, 0x1.d072d4a07897cp+0,
+    0x1.d5818dcfba487p+0, 0x1.da9e603db3285p+0, 0x1.dfc97337b9b5fp+0, 0x1.e502ee78b3ff6p+0,
+    0x1.ea4afa2a490dap+0, 0x1.efa1bee615a27p+0, 0x1.f50765b6e4540p+0, 0x1.fa7c1819e90d8p+0};
+
+// x truncated to FP32 by moving the fields (a conversion instruction takes the
+// FP64 pipe): tiny values to 0; NaN beyond FP32's range
+__device__ __forceinline__ float trunc32(double x) {
+  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+  const uint32_t e = (hi >> 20) & 0x7FFu;
+  if (e >= 1151u) return __int_as_float(0x7FC00000);
+  const uint32_t m = ((hi & 0xFFFFFu) << 3) | (lo >> 29);
+  return __uint_as_float(e < 897u ? 0u : (hi & 0x80000000u) | ((e - 896u) << 23) | m);
+}
+
+// exp(x) by the table-driven method of P. T. P. Tang (ACM TOMS 15, 1989): x =
+// (64 q + k) ln 2 / 64 + r, exp(x) = 2^q 2^(k/64) (1 + r + r^2/2 + ... + r^5/120),
+// |r| < 0.0055, eight FP64 operations.  |x| is held below 700 (the bond order's
+// exponents: a result of 1e-304 stands for a smaller one).
+__device__ __forceinline__ double exp64(double x) {
+  const float xt = trunc32(x);
+  const float nf = rintf(fminf(fmaxf(xt, -700.f), 700.f) * 92.332482616893657f);
+  const int n = (int)nf;
+  // nf widened by moving the fields
+  const uint32_t u = __float_as_uint(nf);
+  const double nd = __hiloint2double(
+      n == 0 ? 0 : (int)((u & 0x80000000u) | (((u >> 3) & 0x0FFFFFFFu) + (896u << 20))),
+      (int)(u << 29));
+  double r = fma(nd, -0x1.62e42fee00000p-7, x);
+  r = fma(nd, -0x1.a39ef35793c76p-39, r);
+  if (fabsf(xt) > 700.f) r = 0.0;
+  const double p = fma(fma(fma(1.0 / 120.0, r, 1.0 / 24.0), r, 1.0 / 6.0), r, 0.5);
+  const double q = fma(p, r * r, r);
+  const double t = __ldg(&kExp2Table[n & 63]);
+  const double v = fma(t, q, t);
+  return __hiloint2double(__double2hiint(v) + ((n >> 6) << 20), __double2loint(v));
+}
 #endif
 
 }  // namespace mdgb

@@ -131,16 +131,6 @@ __device__ __forceinline__ int species64(double w) {
   return (hi & 0x7FFFFFFFu) < 0x3FF00000u ? 0 : (int)w;
 }
 
-// x truncated to FP32 by moving the fields (tiny values to 0; NaN beyond
-// FP32's range, so that no screen rejects it)
-__device__ __forceinline__ float trunc32(double x) {
-  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
-  const uint32_t e = (hi >> 20) & 0x7FFu;
-  if (e >= 1151u) return __int_as_float(0x7FC00000);
-  const uint32_t m = ((hi & 0xFFFFFu) << 3) | (lo >> 29);
-  return __uint_as_float(e < 897u ? 0u : (hi & 0x80000000u) | ((e - 896u) << 23) | m);
-}
-
 // x + img box, img in {-1, 0, 1} (the product is exact: no operation for it)
 __device__ __forceinline__ double image64(double x, int img, double box) {
   return img == 0 ? x : xadd(x, img > 0 ? box : -box);
@@ -680,7 +670,7 @@ template <typename T>
 __global__ void __launch_bounds__(128)
     k_mb_short(const md_double4* __restrict__ pos, const float4* __restrict__ posf, int n,
                int ld, const uint32_t* __restrict__ list, const int* __restrict__ len, Grid g,
-               double rcutsq, uint32_t* __restrict__ sl, int* __restrict__ slen,
+               double rcutsq, uint32_t* __restrict__ sl, int pitch, int* __restrict__ slen,
                const int* __restrict__ run_if) {
   if (run_if && *run_if == 0) return;  // the whole launch: a gated call with nothing to do
   // one warp per atom, lanes over its row: the kept entries in row order
@@ -722,245 +712,365 @@ __global__ void __launch_bounds__(128)
       }
     }
     const unsigned mask = __ballot_sync(0xffffffffu, keep);
-    if (keep) sl[(size_t)(cnt + __popc(mask & ((1u << lane) - 1u))) * n + i] = e;
+    if (keep) sl[(size_t)i * pitch + cnt + __popc(mask & ((1u << lane) - 1u))] = e;
     cnt += __popc(mask);
   }
   if (lane == 0) slen[i] = cnt;
 }
 
-// Third bodies m of the warp's atom i (pass 1): what depends on i and m
-// only, computed once per warp instead of once per pair i-j.  In FP64 with
-// the expressions of the per-pair evaluation, so the values are the same.
-constexpr int kThirdMax = 64;
-template <typename T>
-struct ThirdSm {
-  T x[kThirdMax], y[kThirdMax], z[kThirdMax];  // position at its image
-  T r[kThirdMax], ir[kThirdMax], fc[kThirdMax], dfc[kThirdMax];  // r_im, 1 / r_im (FP32)
-  T ux[kThirdMax], uy[kThirdMax], uz[kThirdMax];                // (r_i - r_m) / r_im
-  int id[kThirdMax];                                            // atom, -1 for an NG atom
-};
+// FP64: the nearly rounded forms of md_exact64.cuh; FP32: the approximation
+// instructions
+__device__ __forceinline__ double mb_rcp(double b) { return rcp64(b); }
+__device__ __forceinline__ float mb_rcp(float b) { return __fdividef(1.0f, b); }
+__device__ __forceinline__ double mb_rsqrt(double x) { return rsqrt64(x); }
+__device__ __forceinline__ float mb_rsqrt(float x) { return rsqrtf(x); }
+__device__ __forceinline__ double mb_exp(double x) { return exp64(x); }
+__device__ __forceinline__ float mb_exp(float x) { return __expf(x); }
 
-// FP32: 64 registers without spills, 8 blocks per SM instead of 7 (FP64
-// instances keep their registers: a bound there spills)
-template <typename T, bool ENERGY>
-__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : 0)
-    k_mb_pass1(const md_double4* __restrict__ pos, const float4* __restrict__ posf,
-               double* __restrict__ f3, int n, const uint32_t* __restrict__ sl,
-               const int* __restrict__ slen, Grid g, int ljexist, T* __restrict__ xsi_s,
-               T* __restrict__ xsj_s, double* __restrict__ epart,
-               double* __restrict__ eatom, const int* __restrict__ run_if) {
-  if (!ENERGY && run_if && *run_if == 0) return;
-  const int warps = blockDim.x >> 5;
-  const int i = blockIdx.x * warps + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  // FP32: hardware rsqrt for distances and their reciprocals, and the
-  // third bodies' terms staged in FP32 (FP64: exact roots and quotients)
-  constexpr bool kFast = std::is_same<T, float>::value;
-  double ev[2] = {0.0, 0.0};
-  __shared__ ThirdSm<T> third_sm[4];
-  ThirdSm<T>& TS = third_sm[(threadIdx.x >> 5) & 3];
-  if (i < n) {
-    T xi, yi, zi;
-    int ti;
-    PosT<T>::load(pos, posf, i, xi, yi, zi, ti);
-    const int S = slen[i];
-    T fx = 0, fy = 0, fz = 0;
-    const T cut_rijsq = (T)MD_CUTOFF_RIJSQ;
-    const T nanv = (T)NAN;
-    const bool staged = S <= kThirdMax && blockDim.x <= 128;  // warp-uniform
-    if (staged) {
-      for (int m = lane; m < S; m += 32) {
-        const uint32_t em = sl[(size_t)m * n + i];
-        const int mp = entry_index(em);
-        T xm, ym, zm;
-        int tm;
-        PosT<T>::load(pos, posf, mp, xm, ym, zm, tm);
-        PosT<T>::image(xm, ym, zm, em, g);
-        TS.id[m] = tm == SP_NG ? -1 : mp;
-        TS.x[m] = xm;
-        TS.y[m] = ym;
-        TS.z[m] = zm;
-        if constexpr (kFast) {
-          const float imx = xi - xm, imy = yi - ym, imz = zi - zm;
-          const float r2 = imx * imx + imy * imy + imz * imz;
-          const float irim = rsqrtf(r2), rim = r2 * irim;
-          float fci, dfci;
-          cutoff<float>(rim, fci, dfci);
-          TS.r[m] = rim;
-          TS.ir[m] = irim;
-          TS.fc[m] = fci;
-          TS.dfc[m] = dfci;
-          TS.ux[m] = imx * irim;
-          TS.uy[m] = imy * irim;
-          TS.uz[m] = imz * irim;
-        } else {
-          // the per-pair branch's expressions below, once per third body
-          const T imx = xi - xm, imy = yi - ym, imz = zi - zm;
-          const T rim = md_sqrt(imx * imx + imy * imy + imz * imz);
-          T fci, dfci;
-          cutoff<T>(rim, fci, dfci);
-          TS.r[m] = rim;
-          TS.ir[m] = fdiv<T>(1.0, rim);
-          TS.fc[m] = fci;
-          TS.dfc[m] = dfci;
-          TS.ux[m] = fdiv<T>(imx, rim);
-          TS.uy[m] = fdiv<T>(imy, rim);
-          TS.uz[m] = fdiv<T>(imz, rim);
-        }
-      }
-      __syncwarp();
-    }
-    for (int s = lane; s < S; s += 32) {
-      const uint32_t e = sl[(size_t)s * n + i];
-      const int j = entry_index(e);
-      T xj, yj, zj;
-      int tj;
-      PosT<T>::load(pos, posf, j, xj, yj, zj, tj);
-      PosT<T>::image(xj, yj, zj, e, g);
-      const size_t slot = (size_t)s * n + i;
-      const T ijx = xi - xj, ijy = yi - yj, ijz = zi - zj;
-      T rij = ijx * ijx + ijy * ijy + ijz * ijz;
-      if (tj == SP_NG || rij > cut_rijsq) {
-        xsi_s[slot] = nanv;
-        xsj_s[slot] = nanv;
-        continue;
-      }
-      rij = md_sqrt(rij);
-      // BondOrderFuncs.h:242-278 bondForces
-      T va = 0, dva = 0, vr = 0, dvr = 0, vdw, dvdw, bo = 0;
-      T dbx = 0, dby = 0, dbz = 0;
-      T fcut, dfcut;
-      cutoff<T>(fdiv<T>(rij, 10), fcut, dfcut);
-      T xs_i = nanv, xs_j = nanv;
-      if (fcut > 0) {
-        const T de = get_de<T>(ti, tj), re = get_re<T>(ti, tj), beta = get_beta<T>(ti, tj);
-        attractive<T>(va, dva, rij, de, beta, re);
-        repulsive<T>(vr, dvr, rij, de, beta, re);
-        // BondOrderFuncs.h:12-143 bondOrder1
-        const T drijx = fdiv<T>(ijx, rij), drijy = fdiv<T>(ijy, rij), drijz = fdiv<T>(ijz, rij);
-        const T E = md_exp((T)MD_LAMDA3 * (rij - re));
-        const T inv_rij = fdiv<T>(1.0f, rij), half_inv_rij = 0.5f * inv_rij;
-        T xsi = 0, xsj = 0;
-        T dxsix = 0, dxsiy = 0, dxsiz = 0, dxsjx = 0, dxsjy = 0, dxsjz = 0;
-        for (int m = 0; m < S; m++) {
-          T xm, ym, zm, rim, inv_rim, fci, dfci, drimx, drimy, drimz;
-          if (staged) {
-            const int mp = TS.id[m];
-            if (mp < 0 || mp == j) continue;
-            xm = TS.x[m];
-            ym = TS.y[m];
-            zm = TS.z[m];
-            rim = TS.r[m];
-            inv_rim = TS.ir[m];
-            fci = TS.fc[m];
-            dfci = TS.dfc[m];
-            drimx = TS.ux[m];
-            drimy = TS.uy[m];
-            drimz = TS.uz[m];
-          } else {
-            const uint32_t em = sl[(size_t)m * n + i];
-            const int mp = entry_index(em);
-            int tm;
-            PosT<T>::load(pos, posf, mp, xm, ym, zm, tm);
-            if (tm == SP_NG || mp == j) continue;
-            PosT<T>::image(xm, ym, zm, em, g);
-            const T imx = xi - xm, imy = yi - ym, imz = zi - zm;
-            rim = md_sqrt(imx * imx + imy * imy + imz * imz);
-            cutoff<T>(rim, fci, dfci);
-            drimx = fdiv<T>(imx, rim);
-            drimy = fdiv<T>(imy, rim);
-            drimz = fdiv<T>(imz, rim);
-            inv_rim = fdiv<T>(1.0f, rim);
-          }
-          const T jmx = xj - xm, jmy = yj - ym, jmz = zj - zm;
-          T rjm, inv_rjm = 0;
-          if constexpr (kFast) {  // the distance and its reciprocal from one rsqrt
-            const float r2 = (float)(jmx * jmx + jmy * jmy + jmz * jmz);
-            const float ir = rsqrtf(r2);
-            inv_rjm = ir;
-            rjm = r2 * ir;
-          } else {
-            rjm = md_sqrt(jmx * jmx + jmy * jmy + jmz * jmz);
-            inv_rjm = fdiv<T>(1.0, rjm);
-          }
-          T fcj, dfcj;
-          cutoff<T>(rjm, fcj, dfcj);
-          if (fci > 0) {
-            // d cos / d r_i = drij (1/rim - cos/rij) + drim (1/rij - cos/rim): the
-            // reference's quotient per component (BondOrderFuncs.h) in two scalars
-            const T num2 = rij * rij + rim * rim - rjm * rjm;
-            const T icos = num2 * half_inv_rij * inv_rim;
-            T gth, gpre;
-            angular1<T>(icos, gth, gpre);
-            xsi += fci * gth * E;
-            const T fE = fci * E;
-            const T cm = dfci * gth * E + fE * gpre * (inv_rij - icos * inv_rim);
-            const T cj = fE * (gpre * (inv_rim - icos * inv_rij) + gth * (T)MD_LAMDA3);
-            dxsix = fma(drimx, cm, fma(drijx, cj, dxsix));
-            dxsiy = fma(drimy, cm, fma(drijy, cj, dxsiy));
-            dxsiz = fma(drimz, cm, fma(drijz, cj, dxsiz));
-          }
-          if (fcj > 0) {
-            // d cos / d r_i = drij (1/rjm - cos/rij) - drim rim / (rij rjm)
-            const T num2 = rij * rij + rjm * rjm - rim * rim;
-            const T jcos = num2 * half_inv_rij * inv_rjm;
-            T gth, gpre;
-            angular1<T>(jcos, gth, gpre);
-            xsj += fcj * gth * E;
-            const T fE = fcj * E;
-            const T cj = fE * (gpre * (inv_rjm - jcos * inv_rij) + (T)MD_LAMDA3 * gth);
-            const T cm = -fE * gpre * rim * inv_rij * inv_rjm;
-            dxsjx = fma(drijx, cj, fma(drimx, cm, dxsjx));
-            dxsjy = fma(drijy, cj, fma(drimy, cm, dxsjy));
-            dxsjz = fma(drijz, cj, fma(drimz, cm, dxsjz));
-          }
-        }
-        xs_i = xsi;
-        xs_j = xsj;
-        const T bij = fdiv<T>(1.0f, 1.0f + xsi), pbi = fdiv<T>(1.0f, (1.0f + xsi) * (1.0f + xsi));
-        const T bji = fdiv<T>(1.0f, 1.0f + xsj), pbj = fdiv<T>(1.0f, (1.0f + xsj) * (1.0f + xsj));
-        bo = 0.5f * (bij + bji);
-        dbx = 0.5f * (pbi * dxsix + pbj * dxsjx);
-        dby = 0.5f * (pbi * dxsiy + pbj * dxsjy);
-        dbz = 0.5f * (pbi * dxsiz + pbj * dxsjz);
-        // what pass 2 needs of this pair: va E / (4 (1 + xi)^2) for either
-        // end (its force is -factor x the derivative of the angle terms)
-        xs_i = (T)0.25 * va * E * pbi;
-        xs_j = (T)0.25 * va * E * pbj;
-      }
-      xsi_s[slot] = xs_i;
-      xsj_s[slot] = xs_j;
-      vander_waals<T>(vdw, dvdw, rij, get_r0v<T>(ti, tj));
-      const T fij = dvr - bo * dva + dvdw;
-      fx += fdiv<T>(fij * ijx, rij) - dbx * va;
-      fy += fdiv<T>(fij * ijy, rij) - dby * va;
-      fz += fdiv<T>(fij * ijz, rij) - dbz * va;
-      if (ENERGY) ev[0] += (double)(0.5f * ((vr - bo * va) + vdw));
-    }
-    double sx = warp_sum((double)fx), sy = warp_sum((double)fy), sz = warp_sum((double)fz);
-    if (ENERGY && eatom) {
-      // per-atom share: sum over j of 1/2 (Vr - b Va + Vdw) (the i-sum of
-      // common/DebugCalculations.cpp:129-270 restricted to the force's pairs)
-      const double ei = warp_sum(ev[0]);
-      if (lane == 0) eatom[i] = ei;
-    }
-    if (lane == 0) {
-      if (ljexist) {
-        f3[3 * i] += sx;
-        f3[3 * i + 1] += sy;
-        f3[3 * i + 2] += sz;
-      } else {
-        f3[3 * i] = sx;
-        f3[3 * i + 1] = sy;
-        f3[3 * i + 2] = sz;
-      }
-      if (ENERGY) {
-        const md_double4 p = pos[i];
-        ev[1] = p.x * sx + p.y * sy + p.z * sz;
-      }
+// common/arvdwfc.cpp:54-59, (1 - tanh x) / 2 as 1 / (1 + e^2x) and its
+// derivative -ALFA (1 - tanh^2 x) / 2 = -2 ALFA fc (1 - fc)
+template <typename T>
+__device__ __forceinline__ void mb_cutoff(T r, T& fc, T& dfc) {
+  fc = mb_rcp((T)1.0 + mb_exp((T)(2.0f * MD_ALFA) * (r - (T)MD_R0)));
+  const T t = (T)(2.0f * MD_ALFA) * fc;
+  dfc = fma(t, fc, -t);
+}
+
+// the angular function and its derivative prefactor (angular in
+// md_potential.cuh) from one reciprocal; MD_H is 0
+template <typename T>
+__device__ __forceinline__ void mb_angular(T c, T& g, T& gpre) {
+  static_assert(MD_H == 0.0f, "cos enters as H - cos");
+  const T iq = mb_rcp(fma(c, c, (T)MD_D));
+  const T h = (T)MD_C * iq;
+  g = (T)(1.0f + MD_C / MD_D) - h;
+  gpre = (h * iq) * ((T)2.0 * c);
+}
+
+// Neighbours of the block's atom i (up to 32 of its short list), in shared
+// memory: the vector r_i - r_s, the distance, its reciprocal, the unit vector
+// and the cutoff, and as the partner j of a bond the pair terms.
+template <typename T>
+struct Nb {
+  T d[3][32], u[3][32], r[32], ir[32], fc[32], dfc[32];
+  T E[32], va[32], dva[32], dv[32], v0[32];  // pair terms: E, Va, Va', Vr' + Vdw', Vr + Vdw
+  int id[32];
+  // bit 6: not a third body of i's bonds (NG), 7: not a bond (NG, or beyond
+  // the pair cutoff); bits 0-2: in the cell below i's along x, y, z, 3-5: above
+  int flag[32];
+};
+constexpr int kNbNoThird = 64, kNbNoBond = 128;
+
+// one neighbour per thread (tid < 32)
+template <typename T, bool PAIR>
+__device__ __forceinline__ void mb_stage(Nb<T>& N, int q, uint32_t e, T xi, T yi, T zi, int ti,
+                                         const md_double4* pos, const float4* posf, const Grid& g,
+                                         const int* cell3, int i) {
+  const int j = entry_index(e);
+  T x, y, z;
+  int tj;
+  PosT<T>::load(pos, posf, j, x, y, z, tj);
+  PosT<T>::image(x, y, z, e, g);
+  const T dx = xi - x, dy = yi - y, dz = zi - z;
+  const T r2 = dx * dx + dy * dy + dz * dz;
+  const T ir = mb_rsqrt(r2), r = r2 * ir;
+  T fc, dfc;
+  mb_cutoff<T>(r, fc, dfc);
+  N.d[0][q] = dx, N.d[1][q] = dy, N.d[2][q] = dz;
+  N.u[0][q] = dx * ir, N.u[1][q] = dy * ir, N.u[2][q] = dz * ir;
+  N.r[q] = r;
+  N.ir[q] = ir;
+  N.fc[q] = fc;
+  N.dfc[q] = dfc;
+  N.id[q] = j;
+  int flag = tj == SP_NG ? kNbNoThird | kNbNoBond : 0;
+  if (r2 > (T)MD_CUTOFF_RIJSQ) flag |= kNbNoBond;
+  if (cell3) {
+    const int4 a = reinterpret_cast<const int4*>(cell3)[i],
+               b = reinterpret_cast<const int4*>(cell3)[j];
+    int s[3] = {b.x - a.x, b.y - a.y, b.z - a.z};
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      if (g.periodic && s[d] > 1) s[d] -= g.cells;
+      if (g.periodic && s[d] < -1) s[d] += g.cells;
+      flag |= s[d] < 0 ? 1 << d : (s[d] > 0 ? 8 << d : 0);
     }
   }
-  if (ENERGY) block_partial<2>(ev, epart);
+  N.flag[q] = flag;
+  if (PAIR) {
+    // common/arvdwfc.cpp:17-48 with the powers of one exponential
+    const T de = get_de<T>(ti, tj), re = get_re<T>(ti, tj), beta = get_beta<T>(ti, tj);
+    const T x1 = mb_exp(-beta * (r - re)), x2 = x1 * x1, x4 = x2 * x2;
+    const T va = MD_S * de / (MD_S - 1.0f) * x1;
+    const T vr = de / (MD_S - 1.0f) * x2 + 7.0e-8f * (x4 * x4 * x2);
+    const T eplus = mb_exp(MD_ALFAV * (r - get_r0v<T>(ti, tj)));
+    const T gmexp = MD_GM * mb_rcp(eplus);
+    const T a = eplus + gmexp, b = MD_ALFAV * (eplus - gmexp), db = MD_ALFAVSQ * a;
+    const T v = 1.0f + 50.0f * MD_GM + MD_GMSQ + 10.0f * (MD_GM - 1.0f) * b;
+    const T ia = mb_rcp(a), ia2 = ia * ia;
+    const T dvdw = -1.0e-4f * ((10.0f * (MD_GM - 1.0f) * db * a - 2.0f * b * v) * (ia2 * ia));
+    N.E[q] = mb_exp((T)MD_LAMDA3 * (r - re));
+    N.va[q] = va;
+    N.dva[q] = beta * va;
+    N.dv[q] = beta * 2.0f * vr + dvdw;
+    N.v0[q] = vr + 1.0e-4f * v * ia2;
+  }
+}
+
+// What the angle terms of a bond i-j with the third body m give: the sums of
+// the bond (x: sum of fc_im g_i, y: of its derivative along r_ij, both without
+// the factor E; xj, yj the same for the angle at j) and the coefficients of
+// the forces on m along u_im (a for the angle at i, b at j) and along
+// r_j - r_m (p, q), each still without its bond's factor.
+template <typename T>
+struct Angle {
+  T x, y, xj, yj, a, b, p, q;
+};
+template <typename T>
+__device__ __forceinline__ Angle<T> mb_angle(const Nb<T>& J, int j, const Nb<T>& M, int m) {
+  const T vx = M.d[0][m] - J.d[0][j], vy = M.d[1][m] - J.d[1][j], vz = M.d[2][m] - J.d[2][j];
+  const T rij = J.r[j], irij = J.ir[j], rim = M.r[m], irim = M.ir[m], fi = M.fc[m];
+  const T r2 = vx * vx + vy * vy + vz * vz;
+  const T irjm = mb_rsqrt(r2), rjm = r2 * irjm;
+  T fj, dfj, gi, pi, gj, pj;
+  mb_cutoff<T>(rjm, fj, dfj);
+  // cosines of the angles at i (unit vectors) and at j (projection)
+  const T ci = J.u[0][j] * M.u[0][m] + J.u[1][j] * M.u[1][m] + J.u[2][j] * M.u[2][m];
+  const T cj = fma(-rim, ci, rij) * irjm;
+  mb_angular<T>(ci, gi, pi);
+  mb_angular<T>(cj, gj, pj);
+  const T xi = fi * pi, xj = fj * pj;
+  Angle<T> A;
+  A.x = fi * gi;
+  A.y = xi * fma(-ci, irij, irim);
+  A.xj = fj * gj;
+  A.yj = xj * fma(-cj, irij, irjm);
+  A.a = fma(xi, fma(-ci, irim, irij), M.dfc[m] * gi);
+  A.p = -xi * (irij * irim);
+  A.b = -xj * (rim * irij) * irjm;
+  A.q = fma(xj, fma(-cj, irjm, irij), dfj * gj) * irjm;
+  return A;
+}
+
+constexpr int kMbPitch = 36;  // columns of a warp's coefficient table (bank-conflict-free)
+constexpr int kMbSlots = kMbSlotCount;  // third-body force slots per atom
+
+// Sum of 4 values over the warp, each value to a quarter of the lanes: value
+// ((lane >> 3) & 3) of every lane's v comes back in all lanes of that quarter
+// (6 additions; 4 values by butterflies take 20).
+__device__ __forceinline__ double quarter_sum(double v0, double v1, double v2, double v3,
+                                              int lane) {
+  const bool h = lane & 16, k = lane & 8;
+  double a = h ? v2 : v0, b = h ? v3 : v1;
+  a += __shfl_xor_sync(0xffffffffu, h ? v0 : v2, 16);
+  b += __shfl_xor_sync(0xffffffffu, h ? v1 : v3, 16);
+  double s = k ? b : a;
+  s += __shfl_xor_sync(0xffffffffu, k ? a : b, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
+// Bond-order forces of atom i, one block of four warps: BondOrderFuncs.h:12-143
+// and 242-278 (the bonds i-j with the third bodies m of i) and, where the
+// bonds' third bodies see j in their own candidate rows (the cells of the list
+// build), :148-237 (the force on m), left in m's slot of i's short list for
+// k_mb_gather.  A warp takes eight bonds at a time, four lanes to a bond, each
+// every fourth m; the angle terms of a triplet are evaluated once: their sums
+// give the bond, and the four force coefficients wait in shared memory until
+// the bond's factors are known; then lane m adds over the eight bonds.  More
+// than 32 neighbours take the triplets twice, in tiles of 32.
+//
+// The FP64 instance is bound by the FP64 pipe (77 operations per triplet), the
+// FP32 one by instruction issue.
+// SLOTS: with the engine's own rows; caller-supplied rows may lack symmetry,
+// and k_mb_pass2 evaluates their third bodies.
+template <typename T, bool ENERGY, bool SLOTS>
+__global__ void __launch_bounds__(128)
+    k_mb_bonds(const md_double4* __restrict__ pos, const float4* __restrict__ posf,
+               double* __restrict__ f3, int n, const uint32_t* __restrict__ sl, int pitch,
+               const int* __restrict__ slen, Grid g, const int* __restrict__ cell3, int ljexist,
+               T* __restrict__ wi_s, T* __restrict__ wj_s, T* __restrict__ fslot,
+               int* __restrict__ missing, double* __restrict__ epart,
+               double* __restrict__ eatom, const int* __restrict__ run_if) {
+  if (!ENERGY && run_if && *run_if == 0) return;
+  __shared__ Nb<T> NA, NB;
+  __shared__ T table[4][4][8][kMbPitch];  // warp, coefficient, bond, m
+  __shared__ T wsm[4][2][8];              // factors of the warp's bonds
+  __shared__ double fsum[4][4];
+  const int i = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int jj = lane >> 2, quad = lane & 3;
+  T xi, yi, zi;
+  int ti;
+  PosT<T>::load(pos, posf, i, xi, yi, zi, ti);
+  const int S = slen[i];
+  const uint32_t* row = sl + (size_t)i * pitch;
+  T fx = 0, fy = 0, fz = 0;
+  double energy = 0.0;
+  int miss = 0;
+  const bool once = S <= 32;
+  for (int j0 = 0; j0 < S; j0 += 32) {
+    __syncthreads();
+    if (tid < 32 && j0 + tid < S)
+      mb_stage<T, true>(NA, tid, row[j0 + tid], xi, yi, zi, ti, pos, posf, g, cell3, i);
+    __syncthreads();
+    const int j = 8 * warp + jj;  // bond of this lane in the tile
+    const bool bond = j0 + j < S && !(NA.flag[j & 31] & kNbNoBond);
+    T x = 0, y = 0, xj = 0, yj = 0;
+    auto triplets = [&](const Nb<T>& M, int m0, bool sums, bool store) {
+      const int mn = min(32, S - m0);
+      if (bond)
+        for (int m = quad; m < mn; m += 4) {
+          if (m0 + m == j0 + j) continue;
+          const Angle<T> A = mb_angle<T>(NA, j, M, m);
+          if (sums && !(M.flag[m] & kNbNoThird)) {
+            x += A.x;
+            y += A.y;
+            xj += A.xj;
+            yj += A.yj;
+          }
+          if (store) {
+            table[warp][0][jj][m] = A.a;
+            table[warp][1][jj][m] = A.b;
+            table[warp][2][jj][m] = A.p;
+            table[warp][3][jj][m] = A.q;
+          }
+        }
+    };
+    // the tile of third bodies at m0: the bonds' own tile or a second one
+    auto tile = [&](int m0) -> const Nb<T>& {
+      if (m0 == j0) return NA;
+      __syncthreads();
+      if (tid < 32 && m0 + tid < S)
+        mb_stage<T, false>(NB, tid, row[m0 + tid], xi, yi, zi, ti, pos, posf, g, cell3, i);
+      __syncthreads();
+      return NB;
+    };
+    for (int m0 = 0; m0 < S; m0 += 32) triplets(tile(m0), m0, true, once);
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) {
+      x += __shfl_xor_sync(0xffffffffu, x, o);
+      y += __shfl_xor_sync(0xffffffffu, y, o);
+      xj += __shfl_xor_sync(0xffffffffu, xj, o);
+      yj += __shfl_xor_sync(0xffffffffu, yj, o);
+    }
+    if (quad == 0 && j0 + j < S) {
+      T wi = (T)NAN, wj = (T)NAN;
+      if (bond) {
+        const T E = NA.E[j], va = NA.va[j], lam = (T)MD_LAMDA3;
+        const T bi = mb_rcp(fma(E, x, (T)1.0)), bj = mb_rcp(fma(E, xj, (T)1.0));
+        const T pi = bi * bi * E, pj = bj * bj * E;  // E / (1 + xi)^2
+        const T bo = (T)0.5 * (bi + bj);
+        const T db = (T)0.5 * (pi * fma(lam, x, y) + pj * fma(lam, xj, yj));
+        // what the third bodies need of this bond: va E / (4 (1 + xi)^2)
+        wi = (T)0.25 * va * pi;
+        wj = (T)0.25 * va * pj;
+        const T f = NA.dv[j] - bo * NA.dva[j] - va * db;
+        fx = fma(f, NA.u[0][j], fx);
+        fy = fma(f, NA.u[1][j], fy);
+        fz = fma(f, NA.u[2][j], fz);
+        if (ENERGY) energy += (double)((T)0.5 * (NA.v0[j] - bo * va));
+      }
+      wsm[warp][0][jj] = wi;
+      wsm[warp][1][jj] = wj;
+      wi_s[(size_t)i * pitch + j0 + j] = wi;
+      wj_s[(size_t)i * pitch + j0 + j] = wj;
+    }
+    __syncwarp();
+    for (int m0 = 0; m0 < S; m0 += 32) {
+      const Nb<T>& M = tile(m0);
+      if (!once) triplets(M, m0, false, true);
+      __syncwarp();
+      // lane m: coefficients of this warp's bonds along u_im (c) and r_j - r_m
+      T c = 0, cu = 0, s = 0, gx = 0, gy = 0, gz = 0;
+      const int m = lane;
+      if (m0 + m < S) {
+        const int fm = M.flag[m];
+        const int opposite = ((fm >> 3) & 7) | ((fm & 7) << 3);
+#pragma unroll 1
+        for (int b = 0; b < 8; b++) {
+          const int jb = 8 * warp + b;
+          if (j0 + jb >= S) break;
+          if (m0 + m == j0 + jb) continue;
+          // j and m on opposite sides of i's cell are no candidates of each other
+          const bool seen = SLOTS && !(NA.flag[jb] & opposite);
+          if (NA.flag[jb] & kNbNoBond) {
+            miss += seen && NA.flag[jb] & kNbNoThird;
+            continue;
+          }
+          const T wi = wsm[warp][0][b], wj = wsm[warp][1][b];
+          const T ck = fma(wi, table[warp][0][b][m], wj * table[warp][1][b][m]);
+          if (seen) {
+            const T cv = fma(wi, table[warp][2][b][m], wj * table[warp][3][b][m]);
+            c += ck;
+            s += cv;
+            gx = fma(-cv, NA.d[0][jb], gx);
+            gy = fma(-cv, NA.d[1][jb], gy);
+            gz = fma(-cv, NA.d[2][jb], gz);
+          } else {
+            cu += ck;
+          }
+        }
+        // the warp's forces on m take the place of the coefficients that this
+        // lane alone has read: x y z, c seen, c unseen
+        table[warp][0][0][m] = fma(s, M.d[0][m], gx);
+        table[warp][0][1][m] = fma(s, M.d[1][m], gy);
+        table[warp][0][2][m] = fma(s, M.d[2][m], gz);
+        table[warp][0][3][m] = c;
+        table[warp][0][4][m] = cu;
+      }
+      __syncthreads();
+      if (warp == 0 && m0 + m < S) {
+        T v[5];
+#pragma unroll
+        for (int d = 0; d < 5; d++)
+          v[d] = (table[0][0][d][m] + table[1][0][d][m]) + (table[2][0][d][m] + table[3][0][d][m]);
+        // the bond's own force: both ends of the angle's derivative along u_im
+        if (!(M.flag[m] & kNbNoThird)) {
+          const T w = (T)-2.0 * (v[3] + v[4]);
+          fx = fma(w, M.u[0][m], fx);
+          fy = fma(w, M.u[1][m], fy);
+          fz = fma(w, M.u[2][m], fz);
+        }
+        if (SLOTS && m0 + m < kMbSlots) {
+          T* o = fslot + 4 * ((size_t)i * kMbSlots + m0 + m);
+          const T ox = fma(v[3], M.u[0][m], v[0]), oy = fma(v[3], M.u[1][m], v[1]),
+                  oz = fma(v[3], M.u[2][m], v[2]);
+          o[0] = j0 ? o[0] + ox : ox;
+          o[1] = j0 ? o[1] + oy : oy;
+          o[2] = j0 ? o[2] + oz : oz;
+        }
+      }
+      __syncthreads();
+    }
+  }
+  // the force on i: quarters of each warp's lanes, then the four warps
+  const double q = quarter_sum((double)fx, (double)fy, (double)fz, energy, lane);
+  if ((lane & 7) == 0) fsum[warp][lane >> 3] = q;
+  if (SLOTS) {
+    const int mw = __reduce_add_sync(0xffffffffu, miss);
+    if (lane == 0 && mw) atomicAdd(missing, mw);
+  }
+  __syncthreads();
+  if (tid < 4) {
+    const double v = (fsum[0][tid] + fsum[1][tid]) + (fsum[2][tid] + fsum[3][tid]);
+    if (tid < 3) {
+      const size_t o = 3 * (size_t)i + tid;
+      f3[o] = ljexist ? f3[o] + v : v;
+    } else if (ENERGY) {
+      // per-atom share: sum over j of 1/2 (Vr - b Va + Vdw) (the i-sum of
+      // common/DebugCalculations.cpp:129-270 restricted to the force's pairs)
+      if (eatom) eatom[i] = v;
+      epart[2 * (size_t)i] = v;
+    }
+    if (ENERGY) {
+      const double* p = (const double*)&pos[i];
+      double w = tid < 3 ? p[tid] * v : 0.0;
+      w += __shfl_xor_sync(0xfu, w, 1);
+      w += __shfl_xor_sync(0xfu, w, 2);
+      if (tid == 0) epart[2 * (size_t)i + 1] = w;
+    }
+  }
 }
 
 // the part of pass 2 for one pair (i, j) of the warp's atom k: i at (x, y, z)
@@ -1068,63 +1178,98 @@ __device__ __forceinline__ Pass2I<T> pass2_entry(uint32_t ei, T xk, T yk, T zk,
 }
 
 // Pass 2 (BondOrderFuncs.h:148-237 bondOrder2 for every pair i-j with k as
-// third body), one entry i of k's short list per lane.  Per pair, pass 1
-// left va E / (4 (1 + xi_ij)^2) and va E / (4 (1 + xi_ji)^2) in the slot, so
-// the exponential and the two quotients of the reference's per-triplet
-// expression are not evaluated again here; NaN marks a slot pass 1 did not
-// evaluate (its va is 0: counted as missing, no force).  Each angle's
-// derivative takes the shorter equal form (test_bond_order_identities: equal
-// to 1e-13 in FP64) with one reciprocal per distance: one rsqrt in FP32, a
-// square root and a quotient in FP64.  (Spreading the (i, j) pairs of k over
-// all 32 lanes through a prefix of the row lengths was measured slower in
-// FP32, 348 against 249 us on 32,768 atoms: lanes of one i read 32 different
-// lines of the slot arrays, where lanes of neighbouring i, stored side by
-// side, share sectors.)
-// FP32: 40 registers, 12 blocks per SM instead of 10 (FP64 instances keep
-// their registers)
-template <typename T, bool ENERGY>
-__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 12 : 0)
-    k_mb_pass2(const md_double4* __restrict__ pos, const float4* __restrict__ posf,
-               double* __restrict__ f3, int n, const uint32_t* __restrict__ sl,
-               const int* __restrict__ slen, Grid g, const int* __restrict__ cell3,
+// third body) for caller-supplied rows, which may name i in k's row and not k
+// in i's: one warp per atom k, one entry i of k's short list per lane.  Per
+// pair, k_mb_bonds left va E / (4 (1 + xi_ij)^2) and va E / (4 (1 + xi_ji)^2)
+// in the slot (NaN where it evaluated none: counted as missing, no force).
+__global__ void __launch_bounds__(128)
+    k_mb_pass2(const md_double4* __restrict__ pos, double* __restrict__ f3, int n,
+               const uint32_t* __restrict__ sl, int pitch, const int* __restrict__ slen, Grid g,
                const int* __restrict__ ref_rows, int ref_nls, int ref_nlargest, double rcutsq,
-               const T* __restrict__ wi_s, const T* __restrict__ wj_s,
-               int* __restrict__ missing, double* __restrict__ epart,
-               const int* __restrict__ run_if) {
+               const double* __restrict__ wi_s, const double* __restrict__ wj_s,
+               int* __restrict__ missing) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int k = blockIdx.x * 4 + warp;
+  if (k >= n) return;
+  const md_double4 pk = pos[k];
+  const int Sk = slen[k];
+  double fx = 0, fy = 0, fz = 0;
+  int miss = 0;
+  for (int s = lane; s < Sk; s += 32) {
+    const Pass2I<double> I = pass2_entry<double>(sl[(size_t)k * pitch + s], pk.x, pk.y, pk.z, pos,
+                                                 nullptr, g);
+    const int Si = slen[I.id];
+    for (int sj = 0; sj < Si; sj++)
+      pass2_pair<double>(I, (size_t)I.id * pitch + sj, k, pk.x, pk.y, pk.z, pos, nullptr, sl, g,
+                         nullptr, ref_rows, ref_nls, ref_nlargest, rcutsq,
+                         (double)MD_CUTOFF_RIJSQ, wi_s, wj_s, fx, fy, fz, miss);
+  }
+  const double v = quarter_sum(fx, fy, fz, 0.0, lane);
+  if ((lane & 7) == 0 && lane < 24) f3[3 * (size_t)k + (lane >> 3)] += v;
+  const int m = __reduce_add_sync(0xffffffffu, miss);
+  if (lane == 0 && m) atomicAdd(missing, m);
+}
+
+// The forces on k as the third body of its neighbours' bonds (BondOrderFuncs.h:
+// 339-393): one warp per atom k, a neighbour i per lane, which finds k in i's
+// short list and takes the force k_mb_bonds left there.  Rows of the engine are
+// symmetric up to the last bit of a distance at the cutoff and the reference's
+// cells at the edge of its box; where k is missing in i's list (or beyond the
+// slots), the lane evaluates i's bonds itself.
+template <typename T, bool ENERGY>
+__global__ void __launch_bounds__(128)
+    k_mb_gather(const md_double4* __restrict__ pos, const float4* __restrict__ posf,
+                double* __restrict__ f3, int n, const uint32_t* __restrict__ sl, int pitch,
+                const int* __restrict__ slen, Grid g, const int* __restrict__ cell3,
+                double rcutsq, const T* __restrict__ wi_s, const T* __restrict__ wj_s,
+                const T* __restrict__ fslot, int* __restrict__ missing,
+                double* __restrict__ epart, const int* __restrict__ run_if) {
   if (!ENERGY && run_if && *run_if == 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int k = blockIdx.x * 4 + warp;
-  double ev[1] = {0.0};
-  if (k < n) {
-    T xk, yk, zk;
-    int tk;
-    PosT<T>::load(pos, posf, k, xk, yk, zk, tk);
-    const int Sk = slen[k];
-    const T rc2 = (T)rcutsq, cut_rijsq = (T)MD_CUTOFF_RIJSQ;
-    T fx = 0, fy = 0, fz = 0;
-    int miss = 0;
-    for (int s = lane; s < Sk; s += 32) {
-      const Pass2I<T> I = pass2_entry<T>(sl[(size_t)s * n + k], xk, yk, zk, pos, posf, g);
-      const int Si = slen[I.id];
-      for (int sj = 0; sj < Si; sj++)
-        pass2_pair<T>(I, (size_t)sj * n + I.id, k, xk, yk, zk, pos, posf, sl, g, cell3,
-                      ref_rows, ref_nls, ref_nlargest, rc2, cut_rijsq, wi_s, wj_s, fx, fy, fz,
-                      miss);
+  if (k >= n) return;
+  const int Sk = slen[k];
+  T fx = 0, fy = 0, fz = 0;
+  int miss = 0;
+  for (int s = lane; s < Sk; s += 32) {
+    const uint32_t e = sl[(size_t)k * pitch + s];
+    const int i = entry_index(e);
+    const int Si = slen[i], lim = min(Si, kMbSlots);
+    const uint4* row = reinterpret_cast<const uint4*>(sl + (size_t)i * pitch);
+    int q = -1;
+    for (int q0 = 0; q0 < lim && q < 0; q0 += 4) {  // pitch is a multiple of 4
+      const uint4 w = row[q0 >> 2];
+      if (entry_index(w.w) == k) q = q0 + 3;
+      if (entry_index(w.z) == k) q = q0 + 2;
+      if (entry_index(w.y) == k) q = q0 + 1;
+      if (entry_index(w.x) == k) q = q0;
     }
-    const double sx = warp_sum((double)fx), sy = warp_sum((double)fy), sz = warp_sum((double)fz);
-    const int m = __reduce_add_sync(0xffffffffu, miss);
-    if (lane == 0) {
-      f3[3 * k] += sx;
-      f3[3 * k + 1] += sy;
-      f3[3 * k + 2] += sz;
-      if (m) atomicAdd(missing, m);
-      if (ENERGY) {
-        const md_double4 p = pos[k];
-        ev[0] = p.x * sx + p.y * sy + p.z * sz;
-      }
+    if (q >= 0 && q < lim) {
+      const T* o = fslot + 4 * ((size_t)i * kMbSlots + q);
+      fx += o[0];
+      fy += o[1];
+      fz += o[2];
+    } else {
+      T xk, yk, zk;
+      int tk;
+      PosT<T>::load(pos, posf, k, xk, yk, zk, tk);
+      const Pass2I<T> I = pass2_entry<T>(e, xk, yk, zk, pos, posf, g);
+      for (int sj = 0; sj < Si; sj++)
+        pass2_pair<T>(I, (size_t)i * pitch + sj, k, xk, yk, zk, pos, posf, sl, g, cell3, nullptr,
+                      0, 0, (T)rcutsq, (T)MD_CUTOFF_RIJSQ, wi_s, wj_s, fx, fy, fz, miss);
     }
   }
-  if (ENERGY) block_partial<1>(ev, epart);
+  const double v = quarter_sum((double)fx, (double)fy, (double)fz, 0.0, lane);
+  const int c = lane >> 3;
+  if ((lane & 7) == 0 && c < 3) f3[3 * (size_t)k + c] += v;
+  const int m = __reduce_add_sync(0xffffffffu, miss);
+  if (lane == 0 && m) atomicAdd(missing, m);
+  if (ENERGY) {
+    double w = c < 3 ? ((const double*)&pos[k])[c] * v : 0.0;
+    w += __shfl_xor_sync(0xffffffffu, w, 8);
+    w += __shfl_xor_sync(0xffffffffu, w, 16);
+    if (lane == 0) epart[k] = w;
+  }
 }
 
 inline int nblk(long long n, int t) { return (int)((n + t - 1) / t); }
@@ -1206,40 +1351,39 @@ void launch_lj(const ForceArgs& a, bool fp32, bool energy, cudaStream_t st) {
 int lj_blocks(int n, bool fp32) {
   return fp32 ? nblk(n, 128) : nblk((long long)n * lj64_lanes(n), 128);
 }
-int mb_blocks(int n) { return nblk(n, 4); }
+int mb_blocks(int n) { return n; }
 
 template <typename T, bool ENERGY>
-static void launch_pass2(const MbArgs& a, int B, T* xsi, T* xsj, cudaStream_t st) {
-  k_mb_pass2<T, ENERGY><<<B, 128, 0, st>>>(a.pos, a.posf, a.f3, a.n, a.sl, a.slen, a.grid,
-                                           a.cell3, a.ref_rows, a.ref_nls, a.ref_nlargest,
-                                           a.rcutsq, xsi, xsj, a.missing,
-                                           ENERGY ? a.epart2 : nullptr, a.run_if);
-}
-
-template <typename T>
-static void launch_mb_t(const MbArgs& a, bool energy, cudaStream_t st) {
+static void launch_mb_t(const MbArgs& a, cudaStream_t st) {
   if (a.n <= 0) return;
-  k_mb_short<T><<<nblk(a.n, 4), 128, 0, st>>>(a.pos, a.posf, a.n, a.ld, a.list, a.len, a.grid,
-                                              a.rcutsq, a.sl, a.slen, energy ? nullptr : a.run_if);
+  const int* gate = ENERGY ? nullptr : a.run_if;
+  T *wi = (T*)a.xsi, *wj = (T*)a.xsj, *fs = (T*)a.fslot;
+  double *e1 = ENERGY ? a.epart1 : nullptr, *e2 = ENERGY ? a.epart2 : nullptr;
+  double* ea = ENERGY ? a.eatom : nullptr;
   const int B = nblk(a.n, 4);
-  T* xsi = (T*)a.xsi;
-  T* xsj = (T*)a.xsj;
-  if (energy) {
-    k_mb_pass1<T, true><<<B, 128, 0, st>>>(a.pos, a.posf, a.f3, a.n, a.sl, a.slen, a.grid,
-                                           a.ljexist, xsi, xsj, a.epart1, a.eatom, nullptr);
-    launch_pass2<T, true>(a, B, xsi, xsj, st);
-  } else {
-    k_mb_pass1<T, false><<<B, 128, 0, st>>>(a.pos, a.posf, a.f3, a.n, a.sl, a.slen, a.grid,
-                                            a.ljexist, xsi, xsj, nullptr, nullptr, a.run_if);
-    launch_pass2<T, false>(a, B, xsi, xsj, st);
+  k_mb_short<T><<<B, 128, 0, st>>>(a.pos, a.posf, a.n, a.ld, a.list, a.len, a.grid, a.rcutsq,
+                                   a.sl, a.pitch, a.slen, gate);
+  if (!a.ref_rows) {
+    k_mb_bonds<T, ENERGY, true><<<a.n, 128, 0, st>>>(a.pos, a.posf, a.f3, a.n, a.sl, a.pitch,
+                                                     a.slen, a.grid, a.cell3, a.ljexist, wi, wj,
+                                                     fs, a.missing, e1, ea, gate);
+    k_mb_gather<T, ENERGY><<<B, 128, 0, st>>>(a.pos, a.posf, a.f3, a.n, a.sl, a.pitch, a.slen,
+                                              a.grid, a.cell3, a.rcutsq, wi, wj, fs, a.missing,
+                                              e2, gate);
+  } else if constexpr (sizeof(T) == 8 && !ENERGY) {
+    k_mb_bonds<T, false, false><<<a.n, 128, 0, st>>>(a.pos, a.posf, a.f3, a.n, a.sl, a.pitch,
+                                                     a.slen, a.grid, nullptr, a.ljexist, wi, wj,
+                                                     nullptr, a.missing, nullptr, nullptr, gate);
+    k_mb_pass2<<<B, 128, 0, st>>>(a.pos, a.f3, a.n, a.sl, a.pitch, a.slen, a.grid, a.ref_rows,
+                                  a.ref_nls, a.ref_nlargest, a.rcutsq, wi, wj, a.missing);
   }
 }
 
 void launch_mb(const MbArgs& a, bool fp32, bool energy, cudaStream_t st) {
   if (fp32)
-    launch_mb_t<float>(a, energy, st);
+    energy ? launch_mb_t<float, true>(a, st) : launch_mb_t<float, false>(a, st);
   else
-    launch_mb_t<double>(a, energy, st);
+    energy ? launch_mb_t<double, true>(a, st) : launch_mb_t<double, false>(a, st);
 }
 
 }  // namespace mdgb

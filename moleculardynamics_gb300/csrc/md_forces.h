@@ -42,20 +42,24 @@ struct MbArgs {
   int ref_nlargest;
   double rcutsq;
   int ljexist;          // accumulate onto F (BondOrderFuncs.h:325-336)
-  uint32_t* sl;         // short list scratch (cap x n)
+  uint32_t* sl;         // short lists, sl[i * pitch + s] (scratch, n * pitch)
+  int pitch;            // slots per atom; a multiple of 4 unless ref_rows is set
   int* slen;
-  void* xsi;            // per (i, slot), T: pass 2's factor va E / (4 (1 + xi_ij)^2)
-  void* xsj;            // and va E / (4 (1 + xi_ji)^2), NaN where pass 1 skipped the pair
+  void* xsi;            // per (i, slot), T: the bond's factor va E / (4 (1 + xi_ij)^2)
+  void* xsj;            // and va E / (4 (1 + xi_ji)^2), NaN where there is no bond
+  void* fslot = nullptr;  // forces on third bodies, 4 T for each of an atom's kMbSlotCount
+                          // first slots (not needed with ref_rows)
   int* missing;
   const int* run_if = nullptr;  // force launches only: return at once unless *run_if != 0
-  double* epart1;       // 2 doubles per pass-1 block
-  double* epart2;       // 1 double per pass-2 block
+  double* epart1;       // energy launches: 2 doubles per atom (bonds)
+  double* epart2;       // and 1 (third bodies)
   double* eatom = nullptr;  // energy launches: per-atom energy (sum over j of half the pair)
 };
 
 void launch_lj(const ForceArgs& a, bool fp32, bool energy, cudaStream_t st);
 void launch_mb(const MbArgs& a, bool fp32, bool energy, cudaStream_t st);
 int lj_blocks(int n, bool fp32);  // blocks of an energy launch of launch_lj
-int mb_blocks(int n);
+int mb_blocks(int n);            // atoms with entries in epart1, epart2
+constexpr int kMbSlotCount = 64;
 
 }  // namespace mdgb

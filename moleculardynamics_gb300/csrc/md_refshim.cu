@@ -298,6 +298,7 @@ void mdgb_many_body_forces(const double* pos4, double* f3, int n, int nlargestsi
   a.rcutsq = rcutsq;
   a.ljexist = ljexist;
   a.sl = s.sl;
+  a.pitch = cap;
   a.slen = s.slen;
   a.xsi = s.xsi;
   a.xsj = s.xsj;

@@ -126,6 +126,7 @@ extern "C" int mdgb_many_body_forces_static(const double* d_pos4, double* d_f3, 
   a.rcutsq = rcutsq;
   a.ljexist = ljexist;
   a.sl = (uint32_t*)(base + kOffSl);
+  a.pitch = nlargestsize > 0 ? nlargestsize : 1;
   a.slen = (int*)(base + kOffSlen);
   a.xsi = base + kOffXsi;
   a.xsj = base + kOffXsj;
