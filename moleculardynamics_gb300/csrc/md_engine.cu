@@ -9,10 +9,9 @@
 //   wall hit: forces and a = F/m again (Host.cpp:168-178)
 //   record at output steps (performOutput, Host.cpp:181-185)
 // Host synchronisation happens only at list builds (the schedule needs the
-// largest speed, Host.cpp:289), after a correct in the reference's wall mode
-// (the wall flag, as the reference's CUDA host also reads it every step) and
-// at the end of md_step.  The periodic mode has no walls and no per-step
-// host round trip.
+// largest speed, Host.cpp:289) and at the end of md_step.  In the reference's
+// wall mode the forces after a wall hit are launched on every step and decided
+// on the device (the reference's CUDA host reads the flag instead).
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -23,6 +22,7 @@
 #include "../../include/mdgb.h"
 #include "md_cluster.h"
 #include "md_forces.h"
+#include "md_gear64.cuh"
 #include "md_integrate.h"
 #include "md_neighbor.cuh"
 #include "md_output.h"
@@ -67,6 +67,9 @@ int next_build(float maxnlmove, double vmax, double dt, int t) {
   return nb > 2147483647LL ? 2147483647 : (int)nb;
 }
 
+// device words of a context: [0] status, [2] missing xi, [3] a species other
+// than NG, [4], [5] wall flag of even / odd steps, [6] steps with a wall hit
+constexpr int kStatusInts = 8;
 constexpr int kKernels = 8;  // timing ids of md_kernel_time
 constexpr long long kSeqTerms = 1LL << 21;  // pair terms per chunk of an in-order record
 
@@ -189,6 +192,10 @@ struct md_ctx {
   double equi_temp = 0;
   unsigned long long equi_seed = 0, equi_draws = 0;
 
+  // the plain form with LJ only: forces and Gear update in one kernel
+  bool fused64() const {
+    return !mixed() && cfg.use_lj && !(cfg.use_mb && cfg.n_mb > 0);
+  }
   bool mixed() const { return cfg.precision == MD_PREC_MIXED; }
   bool permuted() const { return cluster && cl.built; }
   bool walls() const { return !cfg.periodic; }
@@ -304,7 +311,7 @@ ForceArgs lj_args(md_ctx* c, double* f3, double* epart) {
   a.status = c->status;
   a.walker = make_walker(c->lj);
   a.skin = c->lj.skin;
-  a.parity = c->t & 1;
+  a.sf = skin_flags(c->t);
   a.cap = c->lj.cap;
   a.rv2 = c->lj.rv2_keep;
   a.pos_build = c->lj.pos_build;
@@ -420,25 +427,31 @@ md_status mb_forces_step(md_ctx* c, double* f3) {
   return MD_OK;
 }
 
-md_status forces(md_ctx* c, double* f3, bool step = false) {
+// run_if: a device flag that the launches test (LJ by rows and bond order)
+md_status forces(md_ctx* c, double* f3, bool step = false, const int* run_if = nullptr) {
   if (c->cfg.use_lj) {
     Timed tm(c, 0);
-    if (c->cluster)
+    if (c->cluster) {
       launch_lj_cluster(cl_args(c, f3, nullptr), false, c->st);
-    else
-      launch_lj(lj_args(c, f3, nullptr), c->mixed(), false, c->st);
+    } else {
+      ForceArgs a = lj_args(c, f3, nullptr);
+      a.run_if = run_if;
+      launch_lj(a, c->mixed(), false, c->st);
+    }
     c->stats.launches++;
   }
   if (c->cfg.use_mb && c->cfg.n_mb > 0) {
     Timed tm(c, 1);
     if (step && c->sur) return mb_forces_step(c, f3);
-    launch_mb(mb_args(c, f3, c->cfg.use_lj), c->mixed(), false, c->st);
+    MbArgs a = mb_args(c, f3, c->cfg.use_lj);
+    a.run_if = run_if;
+    launch_mb(a, c->mixed(), false, c->st);
     c->stats.launches += 3;
   }
   return MD_OK;
 }
 
-GearArgs gear_args(md_ctx* c, int parity) {
+GearArgs gear_args(md_ctx* c, int step) {
   GearArgs g;
   g.pos = c->pos;
   g.vel = c->vel;
@@ -457,25 +470,25 @@ GearArgs gear_args(md_ctx* c, int parity) {
   g.pos_build = skin ? pb : nullptr;
   g.trip2 = skin ? (float)(trip * trip) : 0.f;
   if (skin && trip <= 0) g.trip2 = -1.f;  // skin too thin: always walk full rows
-  g.trip = skin ? skinf + (c->cluster ? parity % 3 : parity & 1) : nullptr;
+  g.trip = skin ? skinf + step % 3 : nullptr;
   g.status = c->status;
   g.exact = !c->mixed();
   for (int k = 0; k < 3; k++) g.inv_mass[k] = 1.0 / (double)c->sp.mass[k];
   g.npos = c->box_size;
   g.energy_loss = c->energy_loss;
   g.walls = c->walls();
-  g.wall_flag = c->wall_flag;
+  g.wall_flag = c->wall_flag + (c->t & 1);
   return g;
 }
 
 md_status check_status(md_ctx* c) {
-  int s = 0;
-  CK(cudaMemcpyAsync(&s, c->status, sizeof(int), cudaMemcpyDeviceToHost, c->st), "status");
-  int miss = 0;
-  CK(cudaMemcpyAsync(&miss, c->missing, sizeof(int), cudaMemcpyDeviceToHost, c->st), "status");
+  int h[kStatusInts] = {};
+  CK(cudaMemcpyAsync(h, c->status, sizeof(h), cudaMemcpyDeviceToHost, c->st), "status");
   CK(cudaStreamSynchronize(c->st), "step");
   CK(cudaGetLastError(), "step");
-  c->stats.missing_xi = miss;
+  const int s = h[0];
+  c->stats.missing_xi = h[2];
+  c->stats.wall_hits = h[6];
   if (s & ST_NONFINITE) return fail(c, MD_NONFINITE, "non-finite position or velocity");
   if (s & ST_CELL_OVERFLOW) return fail(c, MD_CELL_OVERFLOW, "cell grid out of range");
   if (s & ST_TMA_TIMEOUT) return fail(c, MD_TIMEOUT, "a TMA transfer did not complete in time");
@@ -558,11 +571,11 @@ md_status rebuild(md_ctx* c, int t) {
   }
   if (c->cfg.use_lj && (c->lj_next == t || both)) {
     if (c->lj.skin) {
-      int sk[4];
+      int sk[5];
       CK(cudaMemcpy(sk, c->lj.skin, sizeof(sk), cudaMemcpyDeviceToHost), "skin");
-      c->stats.list_trips += sk[3];
-      if (sk[2]) c->lj.headroom *= 1.5f;  // a refreshed row did not fit: more room
-      CK(cudaMemsetAsync(c->lj.skin + 3, 0, sizeof(int), c->st), "skin");
+      c->stats.list_trips += sk[4];
+      if (sk[3]) c->lj.headroom *= 1.5f;  // a refreshed row did not fit: more room
+      CK(cudaMemsetAsync(c->lj.skin + 4, 0, sizeof(int), c->st), "skin");
     }
     CK(cudaMemsetAsync(c->status, 0, sizeof(int), c->st), "status");
     Grid g = c->cfg.periodic ? make_grid_periodic(c->cfg.box, c->cfg.lj_rs)
@@ -888,10 +901,11 @@ md_status run_window(md_ctx* c) {
   return MD_OK;
 }
 
-// One iteration of cpu/cpumd/Host.cpp:141-195.  In the precision form with a
-// periodic box, correct(t) and predict(t+1) run as one kernel unless step
-// t+1 rebuilds a list, step t records output, or this is the last step of
-// the call (the state between calls is always the corrected one).
+// One iteration of cpu/cpumd/Host.cpp:141-195.  correct(t) and predict(t+1)
+// run as one kernel, with the LJ forces where those are all (the cluster path
+// and the plain form), unless step t+1 rebuilds a list, step t records output,
+// or this is the last step of the call (the state between calls is always the
+// corrected one); with walls the predict follows the second look at the forces.
 md_status step_once(md_ctx* c, bool last) {
   const int t = c->t;
   if (due(c, t)) {
@@ -908,8 +922,9 @@ md_status step_once(md_ctx* c, bool last) {
   const bool output = c->cfg.output_timesteps > 0 && c->printout == t;
   const bool anim = anim_due(c, t);
   const bool equi = equi_due(c, t);
-  const bool fuse =
-      c->mixed() && !c->walls() && !last && !output && !anim && !equi && !due(c, t + 1);
+  // nothing needs the corrected state of this step: the next predict may follow
+  const bool next = !last && !output && !anim && !equi && !due(c, t + 1);
+  const bool fuse = next && !c->walls();
   if (c->cluster && fuse) {
     {
       Timed tm(c, 6);
@@ -918,6 +933,9 @@ md_status step_once(md_ctx* c, bool last) {
     advance_fused(c);
     return MD_OK;
   }
+  int* const hits = c->status + 6;
+  const int* const flag = c->wall_flag + (t & 1);
+  int* const flag_next = c->wall_flag + ((t + 1) & 1);
   if (c->cluster) {
     // forces and correct of step t in one kernel, without the predict (a list
     // build, a record, a frame, new velocities or the call's end follows)
@@ -928,12 +946,35 @@ md_status step_once(md_ctx* c, bool last) {
     std::swap(c->pos, c->pos_alt);
     std::swap(c->posf, c->posf_alt);
     c->stats.launches++;
+  } else if (c->fused64()) {
+    // plain form: forces and correct (then the next predict) in one kernel;
+    // with walls a second one evaluates the forces again if an atom hit one
+    // and does the predict
+    Timed tm(c, 0);
+    Gear64 g;
+    gear64_args(gear_args(c, t + 1), c->pos_alt, fuse, g);
+    ForceArgs a = lj_args(c, fuse ? nullptr : c->f3, nullptr);
+    a.gear64 = &g;
+    launch_lj_step64(a, c->st);
+    std::swap(c->pos, c->pos_alt);
+    c->stats.launches++;
+    if (c->walls()) {
+      gear64_args(gear_args(c, t + 1), next ? c->pos_alt : c->pos, next, g);
+      a = lj_args(c, c->f3, nullptr);
+      a.gear64 = &g;
+      a.run_if = flag;
+      a.hits = hits;
+      a.flag_next = flag_next;
+      launch_lj_redo64(a, c->st);
+      if (next) std::swap(c->pos, c->pos_alt);
+      c->stats.launches++;
+    }
+    c->predicted = next;
   } else {
     {
       md_status fs = forces(c, c->f3, true);
       if (fs != MD_OK) return fs;
     }
-    if (c->walls()) CK(cudaMemsetAsync(c->wall_flag, 0, sizeof(int), c->st), "wall flag");
     {
       Timed tm(c, 3);
       if (fuse) {
@@ -944,15 +985,12 @@ md_status step_once(md_ctx* c, bool last) {
       }
       c->stats.launches++;
     }
-  }
-  if (c->walls()) {
-    int flag = 0;
-    CK(cudaMemcpyAsync(&flag, c->wall_flag, sizeof(int), cudaMemcpyDeviceToHost, c->st), "wall");
-    CK(cudaStreamSynchronize(c->st), "wall");
-    if (flag) {
-      c->stats.wall_hits++;
-      forces(c, c->f3);
-      launch_accel(c->pos, c->acc, c->f3, c->n, c->sp, c->st);
+    if (c->walls()) {
+      // the forces again after a wall hit, decided on the device
+      forces(c, c->f3, false, flag);
+      const bool predict = next && !c->mixed();
+      launch_wall_redo(gear_args(c, predict ? t + 1 : t), flag, hits, flag_next, predict, c->st);
+      c->predicted = predict;
       c->stats.launches++;
     }
   }
@@ -1063,6 +1101,9 @@ md_status md_create(const md_config* cfg, md_ctx** out) {
   for (double** p : vecs)
     if ((e = cudaMalloc(p, sizeof(double) * 3 * N)) != cudaSuccess) return bail(e, "state");
   if ((e = cudaMalloc(&c->posf, sizeof(float4) * N)) != cudaSuccess) return bail(e, "posf");
+  if (c->fused64() &&
+      (e = cudaMalloc(&c->pos_alt, sizeof(md_double4) * N)) != cudaSuccess)
+    return bail(e, "pos");
   if (c->cluster) {
     if ((e = cudaMalloc(&c->io, sizeof(double) * 4 * N)) != cudaSuccess) return bail(e, "io");
     if ((e = cudaMalloc(&c->pos_alt, sizeof(md_double4) * N)) != cudaSuccess)
@@ -1070,10 +1111,10 @@ md_status md_create(const md_config* cfg, md_ctx** out) {
     if ((e = cudaMalloc(&c->posf_alt, sizeof(float4) * N)) != cudaSuccess)
       return bail(e, "posf");
   }
-  if ((e = cudaMalloc(&c->status, sizeof(int) * 4)) != cudaSuccess) return bail(e, "flags");
-  c->wall_flag = c->status + 1;
+  if ((e = cudaMalloc(&c->status, sizeof(int) * kStatusInts)) != cudaSuccess) return bail(e, "flags");
+  c->wall_flag = c->status + 4;
   c->missing = c->status + 2;
-  if ((e = cudaMemset(c->status, 0, sizeof(int) * 4)) != cudaSuccess) return bail(e, "flags");
+  if ((e = cudaMemset(c->status, 0, sizeof(int) * kStatusInts)) != cudaSuccess) return bail(e, "flags");
   if ((e = cudaMalloc(&c->sc.dpart, sizeof(double) * (8 * 1024 + 64))) != cudaSuccess)
     return bail(e, "scratch");
   if ((e = cudaMalloc(&c->sc.umax, sizeof(unsigned long long) * 4)) != cudaSuccess)
@@ -1230,7 +1271,7 @@ md_status md_begin(md_ctx* c, float vxcm) {
   CK(cudaMemsetAsync(c->acc, 0, B, c->st), "begin");
   CK(cudaMemsetAsync(c->b, 0, B, c->st), "begin");
   CK(cudaMemsetAsync(c->c, 0, B, c->st), "begin");
-  CK(cudaMemsetAsync(c->status, 0, sizeof(int) * 4, c->st), "begin");
+  CK(cudaMemsetAsync(c->status, 0, sizeof(int) * kStatusInts, c->st), "begin");
   k_begin<<<(c->n + 255) / 256, 256, 0, c->st>>>(c->pos, c->vel, c->n, c->box_size / 2,
                                                   c->walls(), (double)vxcm);
   c->stats = md_stats{};
@@ -1414,11 +1455,10 @@ md_status md_get_stats(const md_ctx* c, md_stats* out) {
   if (skin) {
     // skin refreshes since the last list build are still on the device
     int sk[5] = {0, 0, 0, 0, 0};
-    const size_t words = c->cluster ? 5 : 4;  // the row-list flags hold 4 ints
     if (cudaStreamSynchronize(c->st) != cudaSuccess ||
-        cudaMemcpy(sk, skin, sizeof(int) * words, cudaMemcpyDeviceToHost) != cudaSuccess)
+        cudaMemcpy(sk, skin, sizeof(sk), cudaMemcpyDeviceToHost) != cudaSuccess)
       return MD_CUDA_ERROR;
-    out->list_trips += c->cluster ? sk[4] : sk[3];
+    out->list_trips += sk[4];
   }
   return MD_OK;
 }

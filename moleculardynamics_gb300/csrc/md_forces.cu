@@ -23,6 +23,7 @@
 
 #include "md_exact64.cuh"
 #include "md_forces.h"
+#include "md_gear64.cuh"
 #include "md_neighbor.cuh"
 #include "md_potential.cuh"
 #include "md_tma.cuh"
@@ -161,7 +162,7 @@ __device__ __forceinline__ void lj64_energy(double r2, double ijx, double ijy, d
 // positions).
 template <bool ENERGY>
 __device__ __noinline__ void lj64_refresh(int i, const md_double4* __restrict__ pos,
-                                          double* __restrict__ f3, int ld,
+                                          double* sums, int ld,
                                           uint32_t* __restrict__ list, int* __restrict__ len,
                                           const RowWalker& w, int* skin, int cap, float rv2,
                                           float4* __restrict__ pos_build, double rcutsq,
@@ -201,12 +202,12 @@ __device__ __noinline__ void lj64_refresh(int i, const md_double4* __restrict__ 
       kept++;
     }
   });
-  if (kept > cap) atomicOr(&skin[2], 1);
+  if (kept > cap) atomicOr(&skin[3], 1);
   len[i] = kept < cap ? kept : cap;
   pos_build[i] = pc;
-  f3[3 * i] = fx;
-  f3[3 * i + 1] = fy;
-  f3[3 * i + 2] = fz;
+  sums[0] = fx;
+  sums[1] = fy;
+  sums[2] = fz;
 }
 
 constexpr int kLj64Cap = 96;  // screened entries of a group in shared memory
@@ -223,41 +224,96 @@ constexpr int kLj64Cap = 96;  // screened entries of a group in shared memory
 // chains: 64 registers (8 blocks per SM) took 255 us for 108,000 atoms, 72
 // registers 259, 80 registers 267, 96 unbounded 280; one thread per atom with
 // the FP64 instructions took 1010.
-template <int G, bool ENERGY>
-__global__ void __launch_bounds__(128, 8)
-    k_lj_fp64(const md_double4* __restrict__ pos, double* __restrict__ f3, int n, int ld,
-              uint32_t* __restrict__ list, int* __restrict__ len, RowWalker w, int* skin,
-              int parity, int cap, float rv2, float4* __restrict__ pos_build, double rcutsq,
-              const __grid_constant__ LjPairConst c, double* __restrict__ epart) {
+//
+// FORCE: forces (and energies) alone.  STEP: the correct of the step follows
+// for each atom in the lanes that hold its force (md_gear64.cuh), and where
+// nothing else is due the predict of the next step; the new positions go to
+// another buffer, as other blocks still read the present ones.  REDO: after a
+// correct with a wall hit (*run_if) the forces and a = F/m again, and in any
+// case the predict if asked for; the count of such steps and the flag of the
+// next one are kept on the device, so a step with walls needs no host wait.
+enum { LJ64_FORCE = 0, LJ64_STEP = 1, LJ64_REDO = 2 };
+struct Lj64Args {
+  const md_double4* pos;
+  double* f3;
+  int n, ld;
+  uint32_t* list;
+  int* len;
+  RowWalker w;
+  int* skin;
+  SkinFlags sf;
+  int cap;
+  float rv2;
+  float4* pos_build;
+  double rcutsq;
+  LjPairConst c;
+  double* epart;
+  const int* run_if;
+  int* hits;       // REDO: steps with a wall hit
+  int* flag_next;  // REDO: the wall flag of the next step
+  int store;       // STEP: forces also to f3
+  Gear64 g;
+};
+
+template <int G, int MODE, bool ENERGY>
+__global__ void __launch_bounds__(128, 8) k_lj_fp64(const __grid_constant__ Lj64Args a) {
   constexpr int kAtoms = 32 / G;  // atoms per warp
   __shared__ uint32_t queue[128 / G][kLj64Cap];
   __shared__ double term[4][3][32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gl = lane & (G - 1), group = lane / G;
-  double ev[3] = {0.0, 0.0, 0.0};
-  const bool tripped = (skin[parity] | skin[2]) != 0;
   const int t = blockIdx.x * 128 + tid;
-  if (t == 0) skin[parity ^ 1] = 0;  // the next step's flag starts clear
-  if (tripped) {
-    // one thread per atom; the grid holds at least n threads
-    if (t < n)
-      lj64_refresh<ENERGY>(t, pos, f3, ld, list, len, w, skin, cap, rv2, pos_build, rcutsq, c, ev);
-    if (t == 0) atomicAdd(&skin[3], 1);
+  const bool gate = !a.run_if || *a.run_if != 0;
+  if (MODE == LJ64_REDO && t == 0) {
+    if (gate) atomicAdd(a.hits, 1);
+    *a.flag_next = 0;
+  }
+  if (!gate && !(MODE == LJ64_REDO && a.g.predict)) return;
+  if (t == 0 && gate) a.skin[a.sf.clear] = 0;  // the flag of step t + 2 starts clear
+  double ev[3] = {0.0, 0.0, 0.0};
+  // The trip flag of the positions.  A correct without the predict (STEP)
+  // leaves the trip of the corrected positions in the next step's flag: read
+  // too by the launches that evaluate them.  One thread reads for the block:
+  // REDO's own predict may set that flag meanwhile, and a block that sees it
+  // walks full rows, which any block may.
+  __shared__ int s_trip;
+  if (tid == 0)
+    s_trip = a.skin[a.sf.read] | a.skin[3] |
+             (ENERGY || MODE == LJ64_REDO ? a.skin[(a.sf.read + 1) % 3] : 0);
+  __syncthreads();
+  const bool tripped = s_trip != 0;
+  const int i = (blockIdx.x * 4 + warp) * kAtoms + group;
+  const bool live = i < a.n;
+  double acc = 0.0;  // lane gl < 3: component gl of the force
+  int ti = SP_NG;
+  if (!gate) {
+    // the predict alone
+  } else if (tripped) {
+    // one thread per atom of the block
+    double* sums = &term[0][0][0];
+    const int first = blockIdx.x * 4 * kAtoms;
+    if (tid < 4 * kAtoms && first + tid < a.n)
+      lj64_refresh<ENERGY>(first + tid, a.pos, sums + 3 * tid, a.ld, a.list, a.len, a.w, a.skin,
+                           a.cap, a.rv2, a.pos_build, a.rcutsq, a.c, ev);
+    if (t == 0) atomicAdd(&a.skin[4], 1);
+    __syncthreads();  // gate and trip are the same for the whole launch
+    if (live && gl < 3) acc = sums[3 * (warp * kAtoms + group) + gl];
+    if (live) ti = species64(a.pos[i].w);
   } else {
-    const int i = (blockIdx.x * 4 + warp) * kAtoms + group;
-    const bool live = i < n;
+    const LjPairConst& c = a.c;
+    const md_double4* __restrict__ pos = a.pos;
+    const uint32_t* __restrict__ list = a.list;
     const md_double4 pi = live ? pos[i] : md_double4{0, 0, 0, 0};
-    const int ti = species64(pi.w);
-    const double box = w.g.box;
+    ti = species64(pi.w);
+    const double box = a.w.g.box;
     const float xf = trunc32(pi.x), yf = trunc32(pi.y), zf = trunc32(pi.z);
     // screen: each coordinate is off by less than 2^-23 of itself, and a pair
     // inside the cutoff has |x_j| <= |x_i| + rcut (+ the box, for an image)
-    const float rc2 = (float)rcutsq * 1.000001f, rc = sqrtf(rc2), bf = w.g.box_f;
+    const float rc2 = (float)a.rcutsq * 1.000001f, rc = sqrtf(rc2), bf = a.w.g.box_f;
     const float off = (fmaxf(fabsf(xf), fmaxf(fabsf(yf), fabsf(zf))) + fabsf(bf) + rc) * 0x1p-20f;
     const float thr = rc2 + off * (8.0f * rc + 16.0f * off);
     uint32_t* q = queue[warp * kAtoms + group];
-    double acc = 0.0;  // lane gl < 3: component gl
-    const int L = live ? len[i] : 0;
+    const int L = live ? a.len[i] : 0;
     int k0 = 0;
     for (;;) {
       // screen until the queue could overflow or every row of the warp ends
@@ -268,7 +324,7 @@ __global__ void __launch_bounds__(128, 8)
         bool keep = false;
         uint32_t e = 0;
         if (go && k < L) {
-          e = list[(size_t)k * ld + i];
+          e = list[(size_t)k * a.ld + i];
           const md_double4 pj = pos[entry_index(e)];
           float dx = xf - trunc32(pj.x), dy = yf - trunc32(pj.y), dz = zf - trunc32(pj.z);
           if (e >> 26) {
@@ -303,7 +359,7 @@ __global__ void __launch_bounds__(128, 8)
           const double ijx = xsub(pi.x, xj), ijy = xsub(pi.y, yj), ijz = xsub(pi.z, zj);
           const double r2 = xadd(xadd(sq64(ijx), sq64(ijy)), sq64(ijz));
           const int tj = species64(pj.w);
-          in = below64(r2, rcutsq) && (tj == SP_NG || ti == SP_NG);
+          in = below64(r2, a.rcutsq) && (tj == SP_NG || ti == SP_NG);
           if (in) {
             const int sel = lj_select(ti, tj);
             const double sq = sel == 0 ? c.sq[0] : (sel == 1 ? c.sq[1] : c.sq[2]);
@@ -328,9 +384,13 @@ __global__ void __launch_bounds__(128, 8)
       }
       if (!__any_sync(0xffffffffu, k0 < L)) break;
     }
-    if (live && gl < 3) f3[3 * i + gl] = acc;
   }
-  if (ENERGY) block_partial<3>(ev, epart);
+  if (gate && (MODE != LJ64_STEP || a.store) && live && gl < 3) a.f3[3 * (size_t)i + gl] = acc;
+  if (MODE == LJ64_STEP)
+    gear64_component<GEAR64_CORRECT>(a.g, live, i, gl, group * G, ti, acc, false);
+  if (MODE == LJ64_REDO)
+    gear64_component<GEAR64_REDO>(a.g, live, i, gl, group * G, ti, acc, gate);
+  if (ENERGY) block_partial<3>(ev, a.epart);
 }
 
 // ------------------------------------------------------------------ LJ FP32
@@ -436,7 +496,7 @@ __device__ __forceinline__ void lj32_atom(int i, const float4* __restrict__ posf
         kept++;
       }
     });
-    if (kept > cap) atomicOr(&skin[2], 1);
+    if (kept > cap) atomicOr(&skin[3], 1);
     len[i] = kept < cap ? kept : cap;
     pos_build[i] = pc;
   }
@@ -464,17 +524,18 @@ template <bool ENERGY>
 __global__ void __launch_bounds__(128)
     k_lj_fp32(const float4* __restrict__ posf, const md_double4* __restrict__ pos,
               double* __restrict__ f3, int n, int ld, uint32_t* __restrict__ list,
-              int* __restrict__ len, RowWalker w, int* skin, int parity, int cap, float rv2,
+              int* __restrict__ len, RowWalker w, int* skin, SkinFlags sf, int cap, float rv2,
               float4* __restrict__ pos_build, double rcutsq, Species sp,
-              double* __restrict__ epart) {
+              double* __restrict__ epart, const int* __restrict__ run_if) {
+  if (run_if && *run_if == 0) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   double ev[3] = {0.0, 0.0, 0.0};
-  const bool tripped = (skin[parity] | skin[2]) != 0;
+  const bool tripped = (skin[sf.read] | skin[3]) != 0;
   if (i < n)
     lj32_atom<ENERGY>(i, posf, pos, f3, ld, list, len, w, tripped, skin, cap, rv2, pos_build,
                       rcutsq, sp, ev);
-  if (tripped && i == 0) atomicAdd(&skin[3], 1);
-  if (i == 0) skin[parity ^ 1] = 0;  // the next step's flag starts clear
+  if (tripped && i == 0) atomicAdd(&skin[4], 1);
+  if (i == 0) skin[sf.clear] = 0;  // the flag of step t + 2 starts clear
   if (ENERGY) block_partial<3>(ev, epart);
 }
 
@@ -490,21 +551,22 @@ __global__ void __launch_bounds__(kListTileAtoms, 8)
     k_lj_tma(const __grid_constant__ CUtensorMap tmap, const float4* __restrict__ posf,
              const md_double4* __restrict__ pos, double* __restrict__ f3, int n, int ld,
              uint32_t* __restrict__ list, int* __restrict__ len, RowWalker w, int* skin,
-             int parity, int cap, float rv2, float4* __restrict__ pos_build, double rcutsq,
-             Species sp, int* status, int wait_limit) {
+             SkinFlags sf, int cap, float rv2, float4* __restrict__ pos_build, double rcutsq,
+             Species sp, int* status, int wait_limit, const int* __restrict__ run_if) {
+  if (run_if && *run_if == 0) return;  // the whole block
   __shared__ __align__(128) uint32_t tile[2][kListTileSlots][kListTileAtoms];
   __shared__ __align__(8) uint64_t bar[2];
   __shared__ int s_max[kListTileAtoms / 32];
   const int tid = threadIdx.x;
   const int i = blockIdx.x * kListTileAtoms + tid;
-  const bool tripped = (skin[parity] | skin[2]) != 0;
+  const bool tripped = (skin[sf.read] | skin[3]) != 0;
   if (tripped) {
     if (i < n)
       lj32_atom_tripped(i, posf, pos, f3, ld, list, len, w, skin, cap, rv2, pos_build, rcutsq,
                         sp);
     if (i == 0) {
-      atomicAdd(&skin[3], 1);
-      skin[parity ^ 1] = 0;
+      atomicAdd(&skin[4], 1);
+      skin[sf.clear] = 0;
     }
     return;
   }
@@ -615,7 +677,7 @@ __global__ void __launch_bounds__(kListTileAtoms, 8)
     f3[3 * i + 1] = (double)hy - (double)ly;
     f3[3 * i + 2] = (double)hz - (double)lz;
   }
-  if (i == 0) skin[parity ^ 1] = 0;  // the next step's flag starts clear
+  if (i == 0) skin[sf.clear] = 0;  // the flag of step t + 2 starts clear
 }
 
 // --------------------------------------------------------------- bond order
@@ -1287,17 +1349,74 @@ static int lj64_lanes(int n) {
   return n * 32LL <= room ? 32 : (n * 16LL <= room ? 16 : (n * 8LL <= room ? 8 : 4));
 }
 
+static LjPairConst lj_pair_const(const Species& sp, double rcutsq) {
+  LjPairConst c;
+  for (int t = 0; t < 3; t++) {
+    const double sig = sp.sig[t], eps = sp.eps[t];
+    c.sq[t] = sig * sig;
+    c.con[t] = 24.0 * eps / c.sq[t];
+    c.eps2[t] = 2.0 * eps;
+    const double src2 = c.sq[t] / rcutsq, src6 = src2 * src2 * src2;
+    const double src12 = src6 * src6;
+    c.eshift[t] = c.eps2[t] * (src12 - src6);
+    uint64_t b;
+    memcpy(&b, &c.sq[t], sizeof(b));
+    c.yq[t] = divisor_fraction(b);
+  }
+  return c;
+}
+
 template <int G>
-static void launch_lj64(const ForceArgs& a, const LjPairConst& c, bool energy, cudaStream_t st) {
-  const int B = nblk((long long)a.n * G, 128);
-  if (energy)
-    k_lj_fp64<G, true><<<B, 128, 0, st>>>(a.pos, a.f3, a.n, a.ld, a.list, a.len, a.walker, a.skin,
-                                          a.parity, a.cap, a.rv2, a.pos_build, a.rcutsq, c,
-                                          a.epart);
+static void launch_lj64_g(const Lj64Args& k, int mode, bool energy, cudaStream_t st) {
+  const int B = nblk((long long)k.n * G, 128);
+  if (mode == LJ64_STEP)
+    k_lj_fp64<G, LJ64_STEP, false><<<B, 128, 0, st>>>(k);
+  else if (mode == LJ64_REDO)
+    k_lj_fp64<G, LJ64_REDO, false><<<B, 128, 0, st>>>(k);
+  else if (energy)
+    k_lj_fp64<G, LJ64_FORCE, true><<<B, 128, 0, st>>>(k);
   else
-    k_lj_fp64<G, false><<<B, 128, 0, st>>>(a.pos, a.f3, a.n, a.ld, a.list, a.len, a.walker,
-                                           a.skin, a.parity, a.cap, a.rv2, a.pos_build, a.rcutsq,
-                                           c, nullptr);
+    k_lj_fp64<G, LJ64_FORCE, false><<<B, 128, 0, st>>>(k);
+}
+
+static void launch_lj64(const ForceArgs& a, int mode, bool energy, cudaStream_t st) {
+  Lj64Args k{};
+  k.pos = a.pos;
+  k.f3 = a.f3;
+  k.n = a.n;
+  k.ld = a.ld;
+  k.list = a.list;
+  k.len = a.len;
+  k.w = a.walker;
+  k.skin = a.skin;
+  k.sf = a.sf;
+  k.cap = a.cap;
+  k.rv2 = a.rv2;
+  k.pos_build = a.pos_build;
+  k.rcutsq = a.rcutsq;
+  k.c = lj_pair_const(a.sp, a.rcutsq);
+  k.epart = energy ? a.epart : nullptr;
+  k.run_if = energy ? nullptr : a.run_if;
+  if (mode != LJ64_FORCE) {
+    k.g = *a.gear64;
+    k.hits = a.hits;
+    k.flag_next = a.flag_next;
+    k.store = a.f3 != nullptr;
+  }
+  switch (lj64_lanes(a.n)) {
+    case 32: launch_lj64_g<32>(k, mode, energy, st); break;
+    case 16: launch_lj64_g<16>(k, mode, energy, st); break;
+    case 8: launch_lj64_g<8>(k, mode, energy, st); break;
+    default: launch_lj64_g<4>(k, mode, energy, st);
+  }
+}
+
+void launch_lj_step64(const ForceArgs& a, cudaStream_t st) {
+  if (a.n > 0) launch_lj64(a, LJ64_STEP, false, st);
+}
+
+void launch_lj_redo64(const ForceArgs& a, cudaStream_t st) {
+  if (a.n > 0) launch_lj64(a, LJ64_REDO, false, st);
 }
 
 void launch_lj(const ForceArgs& a, bool fp32, bool energy, cudaStream_t st) {
@@ -1305,46 +1424,28 @@ void launch_lj(const ForceArgs& a, bool fp32, bool energy, cudaStream_t st) {
   const int B = nblk(a.n, T);
   if (B == 0) return;
   if (!fp32) {
-    LjPairConst c;
-    for (int t = 0; t < 3; t++) {
-      const double sig = a.sp.sig[t], eps = a.sp.eps[t];
-      c.sq[t] = sig * sig;
-      c.con[t] = 24.0 * eps / c.sq[t];
-      c.eps2[t] = 2.0 * eps;
-      const double src2 = c.sq[t] / a.rcutsq, src6 = src2 * src2 * src2;
-      const double src12 = src6 * src6;
-      c.eshift[t] = c.eps2[t] * (src12 - src6);
-      uint64_t b;
-      memcpy(&b, &c.sq[t], sizeof(b));
-      c.yq[t] = divisor_fraction(b);
-    }
-    switch (lj64_lanes(a.n)) {
-      case 32: launch_lj64<32>(a, c, energy, st); break;
-      case 16: launch_lj64<16>(a, c, energy, st); break;
-      case 8: launch_lj64<8>(a, c, energy, st); break;
-      default: launch_lj64<4>(a, c, energy, st);
-    }
+    launch_lj64(a, LJ64_FORCE, energy, st);
   } else if (!energy && a.tmap) {
     const int TB = nblk(a.n, kListTileAtoms);
     if (a.all_ng)
       k_lj_tma<true><<<TB, kListTileAtoms, 0, st>>>(*a.tmap, a.posf, a.pos, a.f3, a.n, a.ld,
-                                                    a.list, a.len, a.walker, a.skin, a.parity,
+                                                    a.list, a.len, a.walker, a.skin, a.sf,
                                                     a.cap, a.rv2, a.pos_build, a.rcutsq, a.sp,
-                                                    a.status, a.wait_limit);
+                                                    a.status, a.wait_limit, a.run_if);
     else
       k_lj_tma<false><<<TB, kListTileAtoms, 0, st>>>(*a.tmap, a.posf, a.pos, a.f3, a.n, a.ld,
-                                                     a.list, a.len, a.walker, a.skin, a.parity,
+                                                     a.list, a.len, a.walker, a.skin, a.sf,
                                                      a.cap, a.rv2, a.pos_build, a.rcutsq, a.sp,
-                                                     a.status, a.wait_limit);
+                                                     a.status, a.wait_limit, a.run_if);
   } else {
     if (energy)
       k_lj_fp32<true><<<B, T, 0, st>>>(a.posf, a.pos, a.f3, a.n, a.ld, a.list, a.len, a.walker,
-                                       a.skin, a.parity, a.cap, a.rv2, a.pos_build, a.rcutsq,
-                                       a.sp, a.epart);
+                                       a.skin, a.sf, a.cap, a.rv2, a.pos_build, a.rcutsq,
+                                       a.sp, a.epart, nullptr);
     else
       k_lj_fp32<false><<<B, T, 0, st>>>(a.posf, a.pos, a.f3, a.n, a.ld, a.list, a.len, a.walker,
-                                        a.skin, a.parity, a.cap, a.rv2, a.pos_build, a.rcutsq,
-                                        a.sp, a.epart);
+                                        a.skin, a.sf, a.cap, a.rv2, a.pos_build, a.rcutsq,
+                                        a.sp, a.epart, a.run_if);
   }
 }
 

@@ -4,6 +4,16 @@
 
 namespace mdgb {
 
+struct Gear64;
+
+// Trip flags of a row list by step: the force launches of step t read [t % 3],
+// the update to the positions of step t + 1 sets [(t + 1) % 3] and the force
+// launch of step t clears [(t + 2) % 3], so that one kernel can do all three.
+struct SkinFlags {
+  int read, clear;
+};
+inline SkinFlags skin_flags(int step) { return {step % 3, (step + 2) % 3}; }
+
 struct ForceArgs {
   const md_double4* pos;
   const float4* posf;   // FP32 copy (precision form)
@@ -17,7 +27,7 @@ struct ForceArgs {
   int* status;
   RowWalker walker;     // full rows, walked when the skin is tripped
   int* skin;            // NeighborList::skin
-  int parity;           // step parity: skin[parity] is this step's trip flag
+  SkinFlags sf;
   int cap;              // compact row capacity
   float rv2;            // compact filter radius squared
   float4* pos_build;    // skin reference positions
@@ -25,6 +35,10 @@ struct ForceArgs {
   Species sp;
   double* epart;        // 3 doubles per block when energy is requested
   int wait_limit = 1 << 20;  // polls of a bounded mbarrier wait (0: give up at once)
+  const int* run_if = nullptr;  // force launches only: return at once unless *run_if != 0
+  // the FP64 kernel with the Gear update (launch_lj_step64, launch_lj_redo64)
+  const Gear64* gear64 = nullptr;
+  int *hits = nullptr, *flag_next = nullptr;  // redo: steps with a wall hit; next step's flag
 };
 
 struct MbArgs {
@@ -57,6 +71,11 @@ struct MbArgs {
 };
 
 void launch_lj(const ForceArgs& a, bool fp32, bool energy, cudaStream_t st);
+// FP64: forces and correct (then predict, gear64->predict) in one kernel;
+// f3 NULL: the forces are not stored.  redo: after a correct with walls, the
+// forces and a = F/m again if *run_if, then the predict.
+void launch_lj_step64(const ForceArgs& a, cudaStream_t st);
+void launch_lj_redo64(const ForceArgs& a, cudaStream_t st);
 void launch_mb(const MbArgs& a, bool fp32, bool energy, cudaStream_t st);
 int lj_blocks(int n, bool fp32);  // blocks of an energy launch of launch_lj
 int mb_blocks(int n);            // atoms with entries in epart1, epart2

@@ -8,9 +8,11 @@
 // them in a fixed order.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 
 #include "mdgb.h"
 #include "md_gear.cuh"
+#include "md_gear64.cuh"
 #include "md_integrate.h"
 #include "md_potential.cuh"
 
@@ -47,62 +49,35 @@ __device__ __forceinline__ void skin_check(const GearArgs& a, int i, double x, d
 
 enum { G_PREDICT = 0, G_CORRECT = 1, G_CORRECT_PREDICT = 2 };
 
-// cpu/common/Device.cpp:17-39 (predict) and :44-120 (correct).  EXACT keeps
-// every rounding of the reference; otherwise products fuse into FMAs and
-// F/m becomes F * (1/m) (the precision form, still FP64 state).
-template <int MODE, bool EXACT>
+// cpu/common/Device.cpp:17-39 (predict) and :44-120 (correct) of the precision
+// form: FP64 state, products fused into FMAs, F/m as F * (1/m).
+template <int MODE>
 __global__ void __launch_bounds__(256) k_gear(GearArgs a) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n) return;
   const GearCoef k = a.k;
   md_double4 r = a.pos[i];
   const int type = (int)r.w;
-  double rr[3] = {r.x, r.y, r.z}, v[3], ac[3], b[3], c[3];
+  GearAtom s;
+  s.r[0] = r.x;
+  s.r[1] = r.y;
+  s.r[2] = r.z;
 #pragma unroll
   for (int d = 0; d < 3; d++) {
-    v[d] = a.vel[3 * i + d];
-    ac[d] = a.acc[3 * i + d];
-    b[d] = a.b[3 * i + d];
-    c[d] = a.c[3 * i + d];
+    s.v[d] = a.vel[3 * i + d];
+    s.a[d] = a.acc[3 * i + d];
+    s.b[d] = a.b[3 * i + d];
+    s.c[d] = a.c[3 * i + d];
   }
   if (MODE != G_PREDICT) {
-    const double mass = mass_of(type, a.sp);
     const double im = type == SP_N ? a.inv_mass[0] : (type == SP_O ? a.inv_mass[1] : a.inv_mass[2]);
-    if (EXACT) {
+    double f[3];
 #pragma unroll
-      for (int d = 0; d < 3; d++) {
-        const double ai = xdiv(a.f3[3 * i + d], mass);
-        const double corr = xsub(ai, ac[d]);
-        rr[d] = xadd(rr[d], xmul(k.cr, corr));
-        v[d] = xadd(v[d], xmul(k.cv, corr));
-        ac[d] = ai;
-        b[d] = xadd(b[d], xmul(k.cb, corr));
-        c[d] = xadd(c[d], xmul(k.cc, corr));
-      }
-    } else {
-      GearAtom s;
-      double f[3];
-#pragma unroll
-      for (int d = 0; d < 3; d++) {
-        s.r[d] = rr[d];
-        s.v[d] = v[d];
-        s.a[d] = ac[d];
-        s.b[d] = b[d];
-        s.c[d] = c[d];
-        f[d] = a.f3[3 * i + d];
-      }
-      gear_correct_fma(s, f, im, k);
-#pragma unroll
-      for (int d = 0; d < 3; d++) {
-        rr[d] = s.r[d];
-        v[d] = s.v[d];
-        ac[d] = s.a[d];
-        b[d] = s.b[d];
-        c[d] = s.c[d];
-      }
-    }
+    for (int d = 0; d < 3; d++) f[d] = a.f3[3 * i + d];
+    gear_correct_fma(s, f, im, k);
     if (MODE == G_CORRECT && a.walls) {
       const double np = a.npos;
+      double *rr = s.r, *v = s.v;
       bool hit = false;
       if (rr[0] > np && rr[1] > 0) { hit = true; v[0] = xmul(-v[0], (double)a.energy_loss); rr[0] = np; }
       if (rr[0] > np && rr[1] < 0) { hit = true; rr[0] = -np; }
@@ -111,53 +86,56 @@ __global__ void __launch_bounds__(256) k_gear(GearArgs a) {
       if (fabs(rr[2]) > np) { hit = true; v[2] = -v[2]; rr[2] = xmul(np, xdiv(rr[2], fabs(rr[2]))); }
       if (hit) atomicOr(a.wall_flag, 1);
     }
-    if (!(isfinite(rr[0]) && isfinite(rr[1]) && isfinite(rr[2]) && isfinite(v[0]) &&
-          isfinite(v[1]) && isfinite(v[2])))
-      atomicOr(a.status, ST_NONFINITE);
+    if (!gear_finite(s)) atomicOr(a.status, ST_NONFINITE);
   }
-  if (MODE != G_CORRECT) {
-    if (EXACT) {
-#pragma unroll
-      for (int d = 0; d < 3; d++) {
-        rr[d] = xadd(xadd(xadd(xadd(rr[d], xmul(k.c1, v[d])), xmul(k.c2, ac[d])),
-                          xmul(k.c3, b[d])),
-                     xmul(k.c4, c[d]));
-        v[d] = xadd(xadd(xadd(v[d], xmul(k.c1, ac[d])), xmul(k.c2, b[d])), xmul(k.c3, c[d]));
-        ac[d] = xadd(xadd(ac[d], xmul(k.c1, b[d])), xmul(k.c2, c[d]));
-        b[d] = xadd(b[d], xmul(k.c1, c[d]));
-      }
-    } else {
-      GearAtom s;
-#pragma unroll
-      for (int d = 0; d < 3; d++) {
-        s.r[d] = rr[d];
-        s.v[d] = v[d];
-        s.a[d] = ac[d];
-        s.b[d] = b[d];
-        s.c[d] = c[d];
-      }
-      gear_predict_fma(s, k);
-#pragma unroll
-      for (int d = 0; d < 3; d++) {
-        rr[d] = s.r[d];
-        v[d] = s.v[d];
-        ac[d] = s.a[d];
-        b[d] = s.b[d];
-      }
-    }
-  }
+  if (MODE != G_CORRECT) gear_predict_fma(s, k);
 #pragma unroll
   for (int d = 0; d < 3; d++) {
-    a.vel[3 * i + d] = v[d];
-    a.acc[3 * i + d] = ac[d];
-    a.b[3 * i + d] = b[d];
-    if (MODE != G_PREDICT) a.c[3 * i + d] = c[d];
+    a.vel[3 * i + d] = s.v[d];
+    a.acc[3 * i + d] = s.a[d];
+    a.b[3 * i + d] = s.b[d];
+    if (MODE != G_PREDICT) a.c[3 * i + d] = s.c[d];
   }
-  r.x = rr[0];
-  r.y = rr[1];
-  r.z = rr[2];
+  r.x = s.r[0];
+  r.y = s.r[1];
+  r.z = s.r[2];
   a.pos[i] = r;
-  skin_check(a, i, rr[0], rr[1], rr[2], type);
+  skin_check(a, i, s.r[0], s.r[1], s.r[2], type);
+}
+
+// The plain form's update on its own: four lanes per atom.  hit: REDO's flag.
+template <int MODE>
+__global__ void __launch_bounds__(128)
+    k_gear64(const __grid_constant__ Gear64 a, const double* __restrict__ f3, int n,
+             const int* __restrict__ hit, int* hits, int* flag_next) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = t >> 2, d = t & 3;
+  const bool gate = MODE != GEAR64_REDO || *hit != 0;
+  if (MODE == GEAR64_REDO && t == 0) {
+    if (gate) atomicAdd(hits, 1);
+    *flag_next = 0;
+  }
+  if (!gate && !a.predict) return;
+  const bool on = i < n;
+  const double w = on ? a.pos[i].w : 2.0;
+  const double f = MODE != GEAR64_PREDICT && on && d < 3 ? f3[3 * (size_t)i + d] : 0.0;
+  gear64_component<MODE>(a, on, i, d, threadIdx.x & 28, (int)w, f, gate);
+}
+
+// the precision form: a = F/m (FP64 quotient, as k_accel) after a wall hit
+__global__ void k_wall_accel(const md_double4* __restrict__ pos, double* __restrict__ acc,
+                             const double* __restrict__ f3, int n, Species sp,
+                             const int* __restrict__ hit, int* hits, int* flag_next) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool gate = *hit != 0;
+  if (i == 0) {
+    if (gate) atomicAdd(hits, 1);
+    *flag_next = 0;
+  }
+  if (!gate || i >= n) return;
+  const double mass = mass_of((int)pos[i].w, sp);
+#pragma unroll
+  for (int d = 0; d < 3; d++) acc[3 * i + d] = xdiv(f3[3 * i + d], mass);
 }
 
 // cpu/common/Device.cpp:125-133
@@ -801,26 +779,72 @@ __global__ void k_equi_scale(double* __restrict__ vel, int n3, double s) {
 
 }  // namespace
 
+void gear64_args(const GearArgs& a, md_double4* pos_next, bool predict, Gear64& g) {
+  g.pos = a.pos;
+  g.pos_next = pos_next;
+  g.vel = a.vel;
+  g.acc = a.acc;
+  g.b = a.b;
+  g.c = a.c;
+  g.k = a.k;
+  for (int t = 0; t < 3; t++) {
+    g.mass[t] = (double)a.sp.mass[t];
+    uint64_t b;
+    memcpy(&b, &g.mass[t], sizeof(b));
+    g.ymass[t] = divisor_fraction(b);
+  }
+  g.npos = a.npos;
+  g.energy_loss = (double)a.energy_loss;
+  g.walls = a.walls;
+  g.wall_flag = a.wall_flag;
+  g.trip = a.trip;
+  g.pos_build = a.pos_build;
+  g.trip2 = a.trip2;
+  g.status = a.status;
+  g.predict = predict;
+}
+
+// blocks of 128 atoms' components; one warp (8 atoms) a block for the smallest
+// systems, so that their few warps do not share schedulers
+template <int MODE>
+static void launch_gear64(const GearArgs& a, bool predict, const int* hit, int* hits,
+                          int* flag_next, cudaStream_t st) {
+  if (a.n <= 0) return;
+  Gear64 g;
+  gear64_args(a, a.pos, predict, g);
+  const int T = a.n <= 8 * 152 ? 32 : 128;
+  k_gear64<MODE><<<nblk(4LL * a.n, T), T, 0, st>>>(g, a.f3, a.n, hit, hits, flag_next);
+}
+
 void launch_predict(const GearArgs& a, cudaStream_t st) {
   if (a.n <= 0) return;
   if (a.exact)
-    k_gear<G_PREDICT, true><<<nblk(a.n, 256), 256, 0, st>>>(a);
+    launch_gear64<GEAR64_PREDICT>(a, true, nullptr, nullptr, nullptr, st);
   else
-    k_gear<G_PREDICT, false><<<nblk(a.n, 256), 256, 0, st>>>(a);
+    k_gear<G_PREDICT><<<nblk(a.n, 256), 256, 0, st>>>(a);
 }
 void launch_correct(const GearArgs& a, cudaStream_t st) {
   if (a.n <= 0) return;
   if (a.exact)
-    k_gear<G_CORRECT, true><<<nblk(a.n, 256), 256, 0, st>>>(a);
+    launch_gear64<GEAR64_CORRECT>(a, false, nullptr, nullptr, nullptr, st);
   else
-    k_gear<G_CORRECT, false><<<nblk(a.n, 256), 256, 0, st>>>(a);
+    k_gear<G_CORRECT><<<nblk(a.n, 256), 256, 0, st>>>(a);
 }
 void launch_correct_predict(const GearArgs& a, cudaStream_t st) {
   if (a.n <= 0) return;
   if (a.exact)
-    k_gear<G_CORRECT_PREDICT, true><<<nblk(a.n, 256), 256, 0, st>>>(a);
+    launch_gear64<GEAR64_CORRECT>(a, true, nullptr, nullptr, nullptr, st);
   else
-    k_gear<G_CORRECT_PREDICT, false><<<nblk(a.n, 256), 256, 0, st>>>(a);
+    k_gear<G_CORRECT_PREDICT><<<nblk(a.n, 256), 256, 0, st>>>(a);
+}
+void launch_wall_redo(const GearArgs& a, const int* hit, int* hits, int* flag_next, bool predict,
+                      cudaStream_t st) {
+  if (a.n <= 0) return;
+  if (a.exact)
+    launch_gear64<GEAR64_REDO>(a, predict, hit, hits, flag_next, st);
+  else
+    k_wall_accel<<<nblk(a.n, 256), 256, 0, st>>>(a.pos, a.acc, a.f3, a.n, a.sp, hit, hits,
+                                                 flag_next);
 }
 void launch_accel(const md_double4* pos, double* acc, const double* f3, int n, Species sp,
                   cudaStream_t st) {

@@ -38,6 +38,13 @@ void launch_predict(const GearArgs& a, cudaStream_t st);
 void launch_correct(const GearArgs& a, cudaStream_t st);
 // correct for this step and predict for the next in one pass (no walls)
 void launch_correct_predict(const GearArgs& a, cudaStream_t st);
+// after a correct with walls: a = F/m where *hit, the count of such steps, the
+// next step's flag cleared; FP64 form with `predict`: then the next predict
+void launch_wall_redo(const GearArgs& a, const int* hit, int* hits, int* flag_next, bool predict,
+                      cudaStream_t st);
+// the FP64 form's arguments for the kernels that fuse the update
+struct Gear64;
+void gear64_args(const GearArgs& a, md_double4* pos_next, bool predict, Gear64& g);
 void launch_accel(const md_double4* pos, double* acc, const double* f3, int n, Species sp,
                   cudaStream_t st);
 void launch_posf(const md_double4* pos, float4* posf, int n, cudaStream_t st);

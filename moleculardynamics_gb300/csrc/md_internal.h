@@ -51,8 +51,8 @@ struct NeighborList {
   double trip_dist = 0;        // an atom displaced by more than this trips the list
   float rv2_keep = 0.f;        // squared filter radius (rv plus FP32 margin)
   float headroom = 1.25f;      // compact row capacity / longest row at build
-  // skin flags: [0], [1] trip flag of even / odd steps, [2] refresh overflow
-  // (sticky until the next build), [3] refreshes done
+  // skin flags: [0..2] trip flag of step t at t % 3, [3] refresh overflow
+  // (sticky until the next build), [4] refreshes done
   int* skin = nullptr;
   // host copies of the last build's sizes
   int maxcell = 0, nlargest = 0, nlistsize = 0, max_len = 0;

@@ -460,11 +460,11 @@ int list_build(NeighborList& nl, md_double4* pos, int n, const Grid& g, int comp
   nl.trip_dist = compact ? 0.5 * ((double)rv - rc) - (double)margin : 1e300;
   nl.rv2_keep = rv2;
   if (!nl.skin) {
-    if ((e = cudaMalloc(&nl.skin, sizeof(int) * 4)) != cudaSuccess) return e;
-    // [3], the trip count, is cleared by its reader after each build: zero it once here
-    cudaMemsetAsync(nl.skin, 0, sizeof(int) * 4, st);
+    if ((e = cudaMalloc(&nl.skin, sizeof(int) * 5)) != cudaSuccess) return e;
+    // [4], the trip count, is cleared by its reader after each build: zero it once here
+    cudaMemsetAsync(nl.skin, 0, sizeof(int) * 5, st);
   }
-  cudaMemsetAsync(nl.skin, 0, sizeof(int) * 3, st);
+  cudaMemsetAsync(nl.skin, 0, sizeof(int) * 4, st);
   return (int)cudaGetLastError();
 }
 
