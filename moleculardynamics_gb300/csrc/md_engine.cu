@@ -276,12 +276,12 @@ md_status ensure_epart(md_ctx* c, long long need) {
 }
 
 // slots per atom of the bond-order short lists (read in 16-byte words)
-int mb_pitch(const md_ctx* c) { return (std::max(c->mb.cap, 1) + 3) & ~3; }
+int mb_pitch(const md_ctx* c) { return std::max(c->mb.cap, 4); }
 
 md_status ensure_mb_scratch(md_ctx* c) {
   const size_t nmb = (size_t)std::max(c->cfg.n_mb, 1);
   const size_t es = c->mixed() ? sizeof(float) : sizeof(double);
-  if (!c->mb_fslot)
+  if (!c->mixed() && !c->mb_fslot)
     CK(cudaMalloc(&c->mb_fslot, 4 * es * kMbSlotCount * nmb), "mb third-body forces");
   const long long need = (long long)mb_pitch(c) * (long long)nmb;
   if (need <= c->mb_elems && c->mb_sl) return MD_OK;
@@ -330,7 +330,8 @@ MbArgs mb_args(md_ctx* c, double* f3, int ljexist) {
   a.n = c->cfg.n_mb;
   a.list = c->mb.list;
   a.len = c->mb.len;
-  a.ld = c->mb.ld;
+  a.ri = (size_t)c->mb.cap;
+  a.rk = 1;
   a.grid = c->mb.grid;
   a.cell3 = c->mb.cell3;
   a.ref_rows = nullptr;
@@ -669,7 +670,7 @@ md_status make_record(md_ctx* c, int t, double* rec16) {
     c->stats.launches += 2;
   }
   if (c->cfg.use_mb && c->cfg.n_mb > 0) {
-    int B = mb_blocks(c->cfg.n_mb);
+    int B = mb_blocks(c->cfg.n_mb, c->mixed());
     md_status s = ensure_epart(c, 3LL * B);
     if (s != MD_OK) return s;
     MbArgs a = mb_args(c, c->f3_tmp, 0);
@@ -1814,7 +1815,7 @@ md_status md_surrogate_collect(md_surrogate* s, md_ctx* c, int stride, int offse
   const int n = c->cfg.n_mb;
   int r = sur_descriptors(*s, c->pos, n, make_walker(c->mb), false, c->status, c->st);
   if (r) return cuda_fail(c, (cudaError_t)r, "surrogate descriptors");
-  const int B = mb_blocks(n);
+  const int B = mb_blocks(n, c->mixed());
   md_status ms = ensure_epart(c, 3LL * B);
   if (ms != MD_OK) return ms;
   MbArgs a = mb_args(c, c->f3_tmp, 0);

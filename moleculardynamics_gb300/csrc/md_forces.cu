@@ -10,13 +10,12 @@
 // pair set equals the FP64 one; per-atom sums are FP32 chunks of 16 pairs
 // folded into a compensated (Kahan) FP32 pair (hi, lo), stored as FP64.
 // Bond order: a short list per atom (candidates within rcut now), then
-//   pass 1: one warp per atom i, one lane per pair (i, j); the lane loops over
-//           the third bodies m of i's short list (BondOrderFuncs.h:12-143,
-//           242-278) and stores xi_ij, xi_ji and Va_ij per (i, slot);
-//   pass 2: one warp per atom k, one lane per i of k's short list; the lane
-//           loops over j of i's short list that lie in k's candidate row and
-//           adds k's third-body force (BondOrderFuncs.h:148-237, 339-393).
-// Lane sums are combined with warp shuffles.
+//   FP64: one block per atom i evaluates its bonds i-j with every third body m
+//           once (BondOrderFuncs.h:12-143, 242-278) and leaves the force on
+//           each m in a slot (:148-237), which m's warp collects (:339-393);
+//   FP32: pass 1, one warp per atom i, one lane per pair (i, j), and pass 2,
+//           one warp per atom k, one lane per i of k's short list, over the
+//           bonds i-j whose j lies in k's candidate row.
 #include <cmath>
 #include <cstring>
 #include <type_traits>
@@ -727,24 +726,37 @@ struct PosT<float> {
   }
 };
 
-// short list: candidates within rcut at the current positions, row order
+// Short list: candidates within rcut at the current positions, row order.  A
+// warp per atom, 32 candidates at a time (a ballot keeps the order).  FP64: a
+// pair clear of the cutoff by more than the truncation of its FP32 copies
+// needs no FP64 operation; the others, and in FP32 the pairs within 1e-5 of
+// the cutoff, are decided in FP64.
 template <typename T>
 __global__ void __launch_bounds__(128)
     k_mb_short(const md_double4* __restrict__ pos, const float4* __restrict__ posf, int n,
-               int ld, const uint32_t* __restrict__ list, const int* __restrict__ len, Grid g,
-               double rcutsq, uint32_t* __restrict__ sl, int pitch, int* __restrict__ slen,
-               const int* __restrict__ run_if) {
+               const uint32_t* __restrict__ list, size_t ri, size_t rk,
+               const int* __restrict__ len, Grid g, double rcutsq, uint32_t* __restrict__ sl,
+               size_t si, size_t ss, int* __restrict__ slen, const int* __restrict__ run_if) {
   if (run_if && *run_if == 0) return;  // the whole launch: a gated call with nothing to do
-  // one warp per atom, lanes over its row: the kept entries in row order
-  // (ballot prefix), 32 candidates tested at a time
+  constexpr bool k64 = sizeof(T) == 8;
   const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (i >= n) return;  // whole warp
-  T xi, yi, zi;
-  int ti;
-  PosT<T>::load(pos, posf, i, xi, yi, zi, ti);
-  const T rc2 = (T)rcutsq;
-  const T band = (T)1e-5 * rc2;
+  auto load = [&](int j) {
+    if (!k64) return posf[j];
+    const md_double4 p = pos[j];
+    return make_float4(trunc32(p.x), trunc32(p.y), trunc32(p.z), 0.f);
+  };
+  const float4 pi = load(i);
+  const float rc2 = (float)rcutsq;
+  float band = 1e-5f * rc2;
+  if (k64) {
+    // each coordinate is off by less than 2^-23 of itself (k_lj_fp64's bound)
+    const float rc = sqrtf(rc2) * 1.000001f;
+    const float off =
+        (fmaxf(fabsf(pi.x), fmaxf(fabsf(pi.y), fabsf(pi.z))) + fabsf(g.box_f) + rc) * 0x1p-20f;
+    band += off * (8.0f * rc + 16.0f * off);
+  }
   int cnt = 0;
   const int L = len[i];
   for (int k0 = 0; k0 < L; k0 += 32) {
@@ -752,70 +764,52 @@ __global__ void __launch_bounds__(128)
     bool keep = false;
     uint32_t e = 0;
     if (k < L) {
-      e = list[(size_t)k * ld + i];
-      const int j = entry_index(e);
-      T xj, yj, zj;
-      int tj;
-      PosT<T>::load(pos, posf, j, xj, yj, zj, tj);
-      PosT<T>::image(xj, yj, zj, e, g);
-      T r2;
-      if (sizeof(T) == 8)
-        r2 = (T)norm2_exact((double)(xi - xj), (double)(yi - yj), (double)(zi - zj));
-      else
-        r2 = (xi - xj) * (xi - xj) + (yi - yj) * (yi - yj) + (zi - zj) * (zi - zj);
+      e = list[(size_t)i * ri + (size_t)k * rk];
+      const float4 pj = load(entry_index(e));
+      float x = pj.x, y = pj.y, z = pj.z;
+      PosT<float>::image(x, y, z, e, g);
+      const float r2 = (pi.x - x) * (pi.x - x) + (pi.y - y) * (pi.y - y) + (pi.z - z) * (pi.z - z);
       keep = r2 < rc2;
-      if (sizeof(T) == 4 && r2 > rc2 - band && r2 < rc2 + band) {
+      if (!(fabsf(r2 - rc2) >= band)) {  // near the cutoff, or not a number
         double a[3], b[3];
         int t0;
         PosT<double>::load(pos, posf, i, a[0], a[1], a[2], t0);
-        PosT<double>::load(pos, posf, j, b[0], b[1], b[2], t0);
+        PosT<double>::load(pos, posf, entry_index(e), b[0], b[1], b[2], t0);
         PosT<double>::image(b[0], b[1], b[2], e, g);
         keep = norm2_exact(xsub(a[0], b[0]), xsub(a[1], b[1]), xsub(a[2], b[2])) < rcutsq;
       }
     }
     const unsigned mask = __ballot_sync(0xffffffffu, keep);
-    if (keep) sl[(size_t)i * pitch + cnt + __popc(mask & ((1u << lane) - 1u))] = e;
+    if (keep) sl[(size_t)i * si + (size_t)(cnt + __popc(mask & ((1u << lane) - 1u))) * ss] = e;
     cnt += __popc(mask);
   }
   if (lane == 0) slen[i] = cnt;
 }
 
-// FP64: the nearly rounded forms of md_exact64.cuh; FP32: the approximation
-// instructions
-__device__ __forceinline__ double mb_rcp(double b) { return rcp64(b); }
-__device__ __forceinline__ float mb_rcp(float b) { return __fdividef(1.0f, b); }
-__device__ __forceinline__ double mb_rsqrt(double x) { return rsqrt64(x); }
-__device__ __forceinline__ float mb_rsqrt(float x) { return rsqrtf(x); }
-__device__ __forceinline__ double mb_exp(double x) { return exp64(x); }
-__device__ __forceinline__ float mb_exp(float x) { return __expf(x); }
-
 // common/arvdwfc.cpp:54-59, (1 - tanh x) / 2 as 1 / (1 + e^2x) and its
 // derivative -ALFA (1 - tanh^2 x) / 2 = -2 ALFA fc (1 - fc)
-template <typename T>
-__device__ __forceinline__ void mb_cutoff(T r, T& fc, T& dfc) {
-  fc = mb_rcp((T)1.0 + mb_exp((T)(2.0f * MD_ALFA) * (r - (T)MD_R0)));
-  const T t = (T)(2.0f * MD_ALFA) * fc;
+__device__ __forceinline__ void mb_cutoff(double r, double& fc, double& dfc) {
+  fc = rcp64(1.0 + exp64((double)(2.0f * MD_ALFA) * (r - (double)MD_R0)));
+  const double t = (double)(2.0f * MD_ALFA) * fc;
   dfc = fma(t, fc, -t);
 }
 
 // the angular function and its derivative prefactor (angular in
 // md_potential.cuh) from one reciprocal; MD_H is 0
-template <typename T>
-__device__ __forceinline__ void mb_angular(T c, T& g, T& gpre) {
+__device__ __forceinline__ void mb_angular(double c, double& g, double& gpre) {
   static_assert(MD_H == 0.0f, "cos enters as H - cos");
-  const T iq = mb_rcp(fma(c, c, (T)MD_D));
-  const T h = (T)MD_C * iq;
-  g = (T)(1.0f + MD_C / MD_D) - h;
-  gpre = (h * iq) * ((T)2.0 * c);
+  const double iq = rcp64(fma(c, c, (double)MD_D));
+  const double h = (double)MD_C * iq;
+  g = (double)(1.0f + MD_C / MD_D) - h;
+  gpre = (h * iq) * (2.0 * c);
 }
 
 // Neighbours of the block's atom i (up to 32 of its short list), in shared
 // memory: the vector r_i - r_s, the distance, its reciprocal, the unit vector
 // and the cutoff, and as the partner j of a bond the pair terms.
-template <typename T>
 struct Nb {
-  T d[3][32], u[3][32], r[32], ir[32], fc[32], dfc[32];
-  T E[32], va[32], dva[32], dv[32], v0[32];  // pair terms: E, Va, Va', Vr' + Vdw', Vr + Vdw
+  double d[3][32], u[3][32], r[32], ir[32], fc[32], dfc[32];
+  double E[32], va[32], dva[32], dv[32], v0[32];  // pair terms: E, Va, Va', Vr' + Vdw', Vr + Vdw
   int id[32];
   // bit 6: not a third body of i's bonds (NG), 7: not a bond (NG, or beyond
   // the pair cutoff); bits 0-2: in the cell below i's along x, y, z, 3-5: above
@@ -824,20 +818,20 @@ struct Nb {
 constexpr int kNbNoThird = 64, kNbNoBond = 128;
 
 // one neighbour per thread (tid < 32)
-template <typename T, bool PAIR>
-__device__ __forceinline__ void mb_stage(Nb<T>& N, int q, uint32_t e, T xi, T yi, T zi, int ti,
+template <bool PAIR>
+__device__ __forceinline__ void mb_stage(Nb& N, int q, uint32_t e, double xi, double yi, double zi, int ti,
                                          const md_double4* pos, const float4* posf, const Grid& g,
                                          const int* cell3, int i) {
   const int j = entry_index(e);
-  T x, y, z;
+  double x, y, z;
   int tj;
-  PosT<T>::load(pos, posf, j, x, y, z, tj);
-  PosT<T>::image(x, y, z, e, g);
-  const T dx = xi - x, dy = yi - y, dz = zi - z;
-  const T r2 = dx * dx + dy * dy + dz * dz;
-  const T ir = mb_rsqrt(r2), r = r2 * ir;
-  T fc, dfc;
-  mb_cutoff<T>(r, fc, dfc);
+  PosT<double>::load(pos, posf, j, x, y, z, tj);
+  PosT<double>::image(x, y, z, e, g);
+  const double dx = xi - x, dy = yi - y, dz = zi - z;
+  const double r2 = dx * dx + dy * dy + dz * dz;
+  const double ir = rsqrt64(r2), r = r2 * ir;
+  double fc, dfc;
+  mb_cutoff(r, fc, dfc);
   N.d[0][q] = dx, N.d[1][q] = dy, N.d[2][q] = dz;
   N.u[0][q] = dx * ir, N.u[1][q] = dy * ir, N.u[2][q] = dz * ir;
   N.r[q] = r;
@@ -846,7 +840,7 @@ __device__ __forceinline__ void mb_stage(Nb<T>& N, int q, uint32_t e, T xi, T yi
   N.dfc[q] = dfc;
   N.id[q] = j;
   int flag = tj == SP_NG ? kNbNoThird | kNbNoBond : 0;
-  if (r2 > (T)MD_CUTOFF_RIJSQ) flag |= kNbNoBond;
+  if (r2 > (double)MD_CUTOFF_RIJSQ) flag |= kNbNoBond;
   if (cell3) {
     const int4 a = reinterpret_cast<const int4*>(cell3)[i],
                b = reinterpret_cast<const int4*>(cell3)[j];
@@ -861,17 +855,17 @@ __device__ __forceinline__ void mb_stage(Nb<T>& N, int q, uint32_t e, T xi, T yi
   N.flag[q] = flag;
   if (PAIR) {
     // common/arvdwfc.cpp:17-48 with the powers of one exponential
-    const T de = get_de<T>(ti, tj), re = get_re<T>(ti, tj), beta = get_beta<T>(ti, tj);
-    const T x1 = mb_exp(-beta * (r - re)), x2 = x1 * x1, x4 = x2 * x2;
-    const T va = MD_S * de / (MD_S - 1.0f) * x1;
-    const T vr = de / (MD_S - 1.0f) * x2 + 7.0e-8f * (x4 * x4 * x2);
-    const T eplus = mb_exp(MD_ALFAV * (r - get_r0v<T>(ti, tj)));
-    const T gmexp = MD_GM * mb_rcp(eplus);
-    const T a = eplus + gmexp, b = MD_ALFAV * (eplus - gmexp), db = MD_ALFAVSQ * a;
-    const T v = 1.0f + 50.0f * MD_GM + MD_GMSQ + 10.0f * (MD_GM - 1.0f) * b;
-    const T ia = mb_rcp(a), ia2 = ia * ia;
-    const T dvdw = -1.0e-4f * ((10.0f * (MD_GM - 1.0f) * db * a - 2.0f * b * v) * (ia2 * ia));
-    N.E[q] = mb_exp((T)MD_LAMDA3 * (r - re));
+    const double de = get_de<double>(ti, tj), re = get_re<double>(ti, tj), beta = get_beta<double>(ti, tj);
+    const double x1 = exp64(-beta * (r - re)), x2 = x1 * x1, x4 = x2 * x2;
+    const double va = MD_S * de / (MD_S - 1.0f) * x1;
+    const double vr = de / (MD_S - 1.0f) * x2 + 7.0e-8f * (x4 * x4 * x2);
+    const double eplus = exp64(MD_ALFAV * (r - get_r0v<double>(ti, tj)));
+    const double gmexp = MD_GM * rcp64(eplus);
+    const double a = eplus + gmexp, b = MD_ALFAV * (eplus - gmexp), db = MD_ALFAVSQ * a;
+    const double v = 1.0f + 50.0f * MD_GM + MD_GMSQ + 10.0f * (MD_GM - 1.0f) * b;
+    const double ia = rcp64(a), ia2 = ia * ia;
+    const double dvdw = -1.0e-4f * ((10.0f * (MD_GM - 1.0f) * db * a - 2.0f * b * v) * (ia2 * ia));
+    N.E[q] = exp64((double)MD_LAMDA3 * (r - re));
     N.va[q] = va;
     N.dva[q] = beta * va;
     N.dv[q] = beta * 2.0f * vr + dvdw;
@@ -884,25 +878,23 @@ __device__ __forceinline__ void mb_stage(Nb<T>& N, int q, uint32_t e, T xi, T yi
 // the factor E; xj, yj the same for the angle at j) and the coefficients of
 // the forces on m along u_im (a for the angle at i, b at j) and along
 // r_j - r_m (p, q), each still without its bond's factor.
-template <typename T>
 struct Angle {
-  T x, y, xj, yj, a, b, p, q;
+  double x, y, xj, yj, a, b, p, q;
 };
-template <typename T>
-__device__ __forceinline__ Angle<T> mb_angle(const Nb<T>& J, int j, const Nb<T>& M, int m) {
-  const T vx = M.d[0][m] - J.d[0][j], vy = M.d[1][m] - J.d[1][j], vz = M.d[2][m] - J.d[2][j];
-  const T rij = J.r[j], irij = J.ir[j], rim = M.r[m], irim = M.ir[m], fi = M.fc[m];
-  const T r2 = vx * vx + vy * vy + vz * vz;
-  const T irjm = mb_rsqrt(r2), rjm = r2 * irjm;
-  T fj, dfj, gi, pi, gj, pj;
-  mb_cutoff<T>(rjm, fj, dfj);
+__device__ __forceinline__ Angle mb_angle(const Nb& J, int j, const Nb& M, int m) {
+  const double vx = M.d[0][m] - J.d[0][j], vy = M.d[1][m] - J.d[1][j], vz = M.d[2][m] - J.d[2][j];
+  const double rij = J.r[j], irij = J.ir[j], rim = M.r[m], irim = M.ir[m], fi = M.fc[m];
+  const double r2 = vx * vx + vy * vy + vz * vz;
+  const double irjm = rsqrt64(r2), rjm = r2 * irjm;
+  double fj, dfj, gi, pi, gj, pj;
+  mb_cutoff(rjm, fj, dfj);
   // cosines of the angles at i (unit vectors) and at j (projection)
-  const T ci = J.u[0][j] * M.u[0][m] + J.u[1][j] * M.u[1][m] + J.u[2][j] * M.u[2][m];
-  const T cj = fma(-rim, ci, rij) * irjm;
-  mb_angular<T>(ci, gi, pi);
-  mb_angular<T>(cj, gj, pj);
-  const T xi = fi * pi, xj = fj * pj;
-  Angle<T> A;
+  const double ci = J.u[0][j] * M.u[0][m] + J.u[1][j] * M.u[1][m] + J.u[2][j] * M.u[2][m];
+  const double cj = fma(-rim, ci, rij) * irjm;
+  mb_angular(ci, gi, pi);
+  mb_angular(cj, gj, pj);
+  const double xi = fi * pi, xj = fj * pj;
+  Angle A;
   A.x = fi * gi;
   A.y = xi * fma(-ci, irij, irim);
   A.xj = fj * gj;
@@ -943,48 +935,47 @@ __device__ __forceinline__ double quarter_sum(double v0, double v1, double v2, d
 // the bond's factors are known; then lane m adds over the eight bonds.  More
 // than 32 neighbours take the triplets twice, in tiles of 32.
 //
-// The FP64 instance is bound by the FP64 pipe (77 operations per triplet), the
-// FP32 one by instruction issue.
+// Bound by the FP64 pipe (77 operations per triplet; 86% busy).
 // SLOTS: with the engine's own rows; caller-supplied rows may lack symmetry,
 // and k_mb_pass2 evaluates their third bodies.
-template <typename T, bool ENERGY, bool SLOTS>
+template <bool ENERGY, bool SLOTS>
 __global__ void __launch_bounds__(128)
     k_mb_bonds(const md_double4* __restrict__ pos, const float4* __restrict__ posf,
                double* __restrict__ f3, int n, const uint32_t* __restrict__ sl, int pitch,
                const int* __restrict__ slen, Grid g, const int* __restrict__ cell3, int ljexist,
-               T* __restrict__ wi_s, T* __restrict__ wj_s, T* __restrict__ fslot,
+               double* __restrict__ wi_s, double* __restrict__ wj_s, double* __restrict__ fslot,
                int* __restrict__ missing, double* __restrict__ epart,
                double* __restrict__ eatom, const int* __restrict__ run_if) {
   if (!ENERGY && run_if && *run_if == 0) return;
-  __shared__ Nb<T> NA, NB;
-  __shared__ T table[4][4][8][kMbPitch];  // warp, coefficient, bond, m
-  __shared__ T wsm[4][2][8];              // factors of the warp's bonds
-  __shared__ double fsum[4][4];
+  __shared__ Nb NA, NB;
+  __shared__ double table[4][4][8][kMbPitch];  // warp, coefficient, bond, m
+  __shared__ double wsm[4][2][8];              // factors of the warp's bonds
+  __shared__ double bsum[4][32];               // force of a bond, its energy
   const int i = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int jj = lane >> 2, quad = lane & 3;
-  T xi, yi, zi;
+  double xi, yi, zi;
   int ti;
-  PosT<T>::load(pos, posf, i, xi, yi, zi, ti);
+  PosT<double>::load(pos, posf, i, xi, yi, zi, ti);
   const int S = slen[i];
   const uint32_t* row = sl + (size_t)i * pitch;
-  T fx = 0, fy = 0, fz = 0;
+  double fx = 0, fy = 0, fz = 0;
   double energy = 0.0;
   int miss = 0;
   const bool once = S <= 32;
   for (int j0 = 0; j0 < S; j0 += 32) {
     __syncthreads();
     if (tid < 32 && j0 + tid < S)
-      mb_stage<T, true>(NA, tid, row[j0 + tid], xi, yi, zi, ti, pos, posf, g, cell3, i);
+      mb_stage<true>(NA, tid, row[j0 + tid], xi, yi, zi, ti, pos, posf, g, cell3, i);
     __syncthreads();
     const int j = 8 * warp + jj;  // bond of this lane in the tile
     const bool bond = j0 + j < S && !(NA.flag[j & 31] & kNbNoBond);
-    T x = 0, y = 0, xj = 0, yj = 0;
-    auto triplets = [&](const Nb<T>& M, int m0, bool sums, bool store) {
+    double x = 0, y = 0, xj = 0, yj = 0;
+    auto triplets = [&](const Nb& M, int m0, bool sums, bool store) {
       const int mn = min(32, S - m0);
       if (bond)
         for (int m = quad; m < mn; m += 4) {
           if (m0 + m == j0 + j) continue;
-          const Angle<T> A = mb_angle<T>(NA, j, M, m);
+          const Angle A = mb_angle(NA, j, M, m);
           if (sums && !(M.flag[m] & kNbNoThird)) {
             x += A.x;
             y += A.y;
@@ -1000,11 +991,11 @@ __global__ void __launch_bounds__(128)
         }
     };
     // the tile of third bodies at m0: the bonds' own tile or a second one
-    auto tile = [&](int m0) -> const Nb<T>& {
+    auto tile = [&](int m0) -> const Nb& {
       if (m0 == j0) return NA;
       __syncthreads();
       if (tid < 32 && m0 + tid < S)
-        mb_stage<T, false>(NB, tid, row[m0 + tid], xi, yi, zi, ti, pos, posf, g, cell3, i);
+        mb_stage<false>(NB, tid, row[m0 + tid], xi, yi, zi, ti, pos, posf, g, cell3, i);
       __syncthreads();
       return NB;
     };
@@ -1017,21 +1008,23 @@ __global__ void __launch_bounds__(128)
       yj += __shfl_xor_sync(0xffffffffu, yj, o);
     }
     if (quad == 0 && j0 + j < S) {
-      T wi = (T)NAN, wj = (T)NAN;
+      double wi = (double)NAN, wj = (double)NAN;
       if (bond) {
-        const T E = NA.E[j], va = NA.va[j], lam = (T)MD_LAMDA3;
-        const T bi = mb_rcp(fma(E, x, (T)1.0)), bj = mb_rcp(fma(E, xj, (T)1.0));
-        const T pi = bi * bi * E, pj = bj * bj * E;  // E / (1 + xi)^2
-        const T bo = (T)0.5 * (bi + bj);
-        const T db = (T)0.5 * (pi * fma(lam, x, y) + pj * fma(lam, xj, yj));
+        const double E = NA.E[j], va = NA.va[j], lam = (double)MD_LAMDA3;
+        const double bi = rcp64(fma(E, x, 1.0)), bj = rcp64(fma(E, xj, 1.0));
+        const double pi = bi * bi * E, pj = bj * bj * E;  // E / (1 + xi)^2
+        const double bo = 0.5 * (bi + bj);
+        const double db = 0.5 * (pi * fma(lam, x, y) + pj * fma(lam, xj, yj));
         // what the third bodies need of this bond: va E / (4 (1 + xi)^2)
-        wi = (T)0.25 * va * pi;
-        wj = (T)0.25 * va * pj;
-        const T f = NA.dv[j] - bo * NA.dva[j] - va * db;
-        fx = fma(f, NA.u[0][j], fx);
-        fy = fma(f, NA.u[1][j], fy);
-        fz = fma(f, NA.u[2][j], fz);
-        if (ENERGY) energy += (double)((T)0.5 * (NA.v0[j] - bo * va));
+        wi = 0.25 * va * pi;
+        wj = 0.25 * va * pj;
+        const double f = NA.dv[j] - bo * NA.dva[j] - va * db;
+        bsum[0][j] = f * NA.u[0][j];
+        bsum[1][j] = f * NA.u[1][j];
+        bsum[2][j] = f * NA.u[2][j];
+        if (ENERGY) bsum[3][j] = 0.5 * (NA.v0[j] - bo * va);
+      } else {
+        bsum[0][j] = bsum[1][j] = bsum[2][j] = bsum[3][j] = 0.0;
       }
       wsm[warp][0][jj] = wi;
       wsm[warp][1][jj] = wj;
@@ -1040,11 +1033,11 @@ __global__ void __launch_bounds__(128)
     }
     __syncwarp();
     for (int m0 = 0; m0 < S; m0 += 32) {
-      const Nb<T>& M = tile(m0);
+      const Nb& M = tile(m0);
       if (!once) triplets(M, m0, false, true);
       __syncwarp();
       // lane m: coefficients of this warp's bonds along u_im (c) and r_j - r_m
-      T c = 0, cu = 0, s = 0, gx = 0, gy = 0, gz = 0;
+      double c = 0, cu = 0, s = 0, gx = 0, gy = 0, gz = 0;
       const int m = lane;
       if (m0 + m < S) {
         const int fm = M.flag[m];
@@ -1060,10 +1053,10 @@ __global__ void __launch_bounds__(128)
             miss += seen && NA.flag[jb] & kNbNoThird;
             continue;
           }
-          const T wi = wsm[warp][0][b], wj = wsm[warp][1][b];
-          const T ck = fma(wi, table[warp][0][b][m], wj * table[warp][1][b][m]);
+          const double wi = wsm[warp][0][b], wj = wsm[warp][1][b];
+          const double ck = fma(wi, table[warp][0][b][m], wj * table[warp][1][b][m]);
           if (seen) {
-            const T cv = fma(wi, table[warp][2][b][m], wj * table[warp][3][b][m]);
+            const double cv = fma(wi, table[warp][2][b][m], wj * table[warp][3][b][m]);
             c += ck;
             s += cv;
             gx = fma(-cv, NA.d[0][jb], gx);
@@ -1082,21 +1075,27 @@ __global__ void __launch_bounds__(128)
         table[warp][0][4][m] = cu;
       }
       __syncthreads();
+      if (warp == 0 && m0 == j0 && j0 + lane < S) {
+        fx += bsum[0][lane];
+        fy += bsum[1][lane];
+        fz += bsum[2][lane];
+        if (ENERGY) energy += (double)bsum[3][lane];
+      }
       if (warp == 0 && m0 + m < S) {
-        T v[5];
+        double v[5];
 #pragma unroll
         for (int d = 0; d < 5; d++)
           v[d] = (table[0][0][d][m] + table[1][0][d][m]) + (table[2][0][d][m] + table[3][0][d][m]);
         // the bond's own force: both ends of the angle's derivative along u_im
         if (!(M.flag[m] & kNbNoThird)) {
-          const T w = (T)-2.0 * (v[3] + v[4]);
+          const double w = -2.0 * (v[3] + v[4]);
           fx = fma(w, M.u[0][m], fx);
           fy = fma(w, M.u[1][m], fy);
           fz = fma(w, M.u[2][m], fz);
         }
         if (SLOTS && m0 + m < kMbSlots) {
-          T* o = fslot + 4 * ((size_t)i * kMbSlots + m0 + m);
-          const T ox = fma(v[3], M.u[0][m], v[0]), oy = fma(v[3], M.u[1][m], v[1]),
+          double* o = fslot + 4 * ((size_t)i * kMbSlots + m0 + m);
+          const double ox = fma(v[3], M.u[0][m], v[0]), oy = fma(v[3], M.u[1][m], v[1]),
                   oz = fma(v[3], M.u[2][m], v[2]);
           o[0] = j0 ? o[0] + ox : ox;
           o[1] = j0 ? o[1] + oy : oy;
@@ -1106,16 +1105,15 @@ __global__ void __launch_bounds__(128)
       __syncthreads();
     }
   }
-  // the force on i: quarters of each warp's lanes, then the four warps
-  const double q = quarter_sum((double)fx, (double)fy, (double)fz, energy, lane);
-  if ((lane & 7) == 0) fsum[warp][lane >> 3] = q;
   if (SLOTS) {
     const int mw = __reduce_add_sync(0xffffffffu, miss);
     if (lane == 0 && mw) atomicAdd(missing, mw);
   }
-  __syncthreads();
+  if (warp != 0) return;
+  // the force on i, from warp 0's lanes
+  const double q = quarter_sum(fx, fy, fz, energy, lane);
+  const double v = __shfl_sync(0xffffffffu, q, (lane & 3) * 8);
   if (tid < 4) {
-    const double v = (fsum[0][tid] + fsum[1][tid]) + (fsum[2][tid] + fsum[3][tid]);
     if (tid < 3) {
       const size_t o = 3 * (size_t)i + tid;
       f3[o] = ljexist ? f3[o] + v : v;
@@ -1278,20 +1276,20 @@ __global__ void __launch_bounds__(128)
 // symmetric up to the last bit of a distance at the cutoff and the reference's
 // cells at the edge of its box; where k is missing in i's list (or beyond the
 // slots), the lane evaluates i's bonds itself.
-template <typename T, bool ENERGY>
+template <bool ENERGY>
 __global__ void __launch_bounds__(128)
     k_mb_gather(const md_double4* __restrict__ pos, const float4* __restrict__ posf,
                 double* __restrict__ f3, int n, const uint32_t* __restrict__ sl, int pitch,
                 const int* __restrict__ slen, Grid g, const int* __restrict__ cell3,
-                double rcutsq, const T* __restrict__ wi_s, const T* __restrict__ wj_s,
-                const T* __restrict__ fslot, int* __restrict__ missing,
+                double rcutsq, const double* __restrict__ wi_s, const double* __restrict__ wj_s,
+                const double* __restrict__ fslot, int* __restrict__ missing,
                 double* __restrict__ epart, const int* __restrict__ run_if) {
   if (!ENERGY && run_if && *run_if == 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int k = blockIdx.x * 4 + warp;
   if (k >= n) return;
   const int Sk = slen[k];
-  T fx = 0, fy = 0, fz = 0;
+  double fx = 0, fy = 0, fz = 0;
   int miss = 0;
   for (int s = lane; s < Sk; s += 32) {
     const uint32_t e = sl[(size_t)k * pitch + s];
@@ -1307,21 +1305,21 @@ __global__ void __launch_bounds__(128)
       if (entry_index(w.x) == k) q = q0;
     }
     if (q >= 0 && q < lim) {
-      const T* o = fslot + 4 * ((size_t)i * kMbSlots + q);
+      const double* o = fslot + 4 * ((size_t)i * kMbSlots + q);
       fx += o[0];
       fy += o[1];
       fz += o[2];
     } else {
-      T xk, yk, zk;
+      double xk, yk, zk;
       int tk;
-      PosT<T>::load(pos, posf, k, xk, yk, zk, tk);
-      const Pass2I<T> I = pass2_entry<T>(e, xk, yk, zk, pos, posf, g);
+      PosT<double>::load(pos, posf, k, xk, yk, zk, tk);
+      const Pass2I<double> I = pass2_entry<double>(e, xk, yk, zk, pos, posf, g);
       for (int sj = 0; sj < Si; sj++)
-        pass2_pair<T>(I, (size_t)i * pitch + sj, k, xk, yk, zk, pos, posf, sl, g, cell3, nullptr,
-                      0, 0, (T)rcutsq, (T)MD_CUTOFF_RIJSQ, wi_s, wj_s, fx, fy, fz, miss);
+        pass2_pair<double>(I, (size_t)i * pitch + sj, k, xk, yk, zk, pos, posf, sl, g, cell3, nullptr,
+                      0, 0, rcutsq, (double)MD_CUTOFF_RIJSQ, wi_s, wj_s, fx, fy, fz, miss);
     }
   }
-  const double v = quarter_sum((double)fx, (double)fy, (double)fz, 0.0, lane);
+  const double v = quarter_sum(fx, fy, fz, 0.0, lane);
   const int c = lane >> 3;
   if ((lane & 7) == 0 && c < 3) f3[3 * (size_t)k + c] += v;
   const int m = __reduce_add_sync(0xffffffffu, miss);
@@ -1332,6 +1330,279 @@ __global__ void __launch_bounds__(128)
     w += __shfl_xor_sync(0xffffffffu, w, 16);
     if (lane == 0) epart[k] = w;
   }
+}
+
+// ---- the precision form: pass 1 and pass 2 ----
+// The order and the roundings of these FP32 sums are part of the form's
+// results: the bond order jumps where a pair passes the cutoff, so two runs
+// that differ in the last FP32 bit part by 1e-2 of a velocity once a pair
+// crosses it a step earlier.  Measured: k_mb_bonds<float> took 228 us per
+// evaluation of 32,768 atoms against 420 here, but its runs of 50 steps left
+// the present ones' tolerance for 45% of the seeds.
+
+// Third bodies m of the warp's atom i (pass 1): what depends on i and m
+// only, computed once per warp instead of once per pair i-j.
+constexpr int kThirdMax = 64;
+struct ThirdSm {
+  float x[kThirdMax], y[kThirdMax], z[kThirdMax];  // position at its image
+  float r[kThirdMax], ir[kThirdMax], fc[kThirdMax], dfc[kThirdMax];  // r_im, 1 / r_im
+  float ux[kThirdMax], uy[kThirdMax], uz[kThirdMax];                // (r_i - r_m) / r_im
+  int id[kThirdMax];                                            // atom, -1 for an NG atom
+};
+
+// 64 registers without spills, 8 blocks per SM instead of 7
+template <bool ENERGY>
+__global__ void __launch_bounds__(128, 8)
+    k_mb_pass1_32(const md_double4* __restrict__ pos, const float4* __restrict__ posf,
+               double* __restrict__ f3, int n, const uint32_t* __restrict__ sl,
+               const int* __restrict__ slen, Grid g, int ljexist, float* __restrict__ xsi_s,
+               float* __restrict__ xsj_s, double* __restrict__ epart,
+               double* __restrict__ eatom, const int* __restrict__ run_if) {
+  if (!ENERGY && run_if && *run_if == 0) return;
+  const int warps = blockDim.x >> 5;
+  const int i = blockIdx.x * warps + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  using T = float;
+  double ev[2] = {0.0, 0.0};
+  __shared__ ThirdSm third_sm[4];
+  ThirdSm& TS = third_sm[(threadIdx.x >> 5) & 3];
+  if (i < n) {
+    T xi, yi, zi;
+    int ti;
+    PosT<T>::load(pos, posf, i, xi, yi, zi, ti);
+    const int S = slen[i];
+    T fx = 0, fy = 0, fz = 0;
+    const T cut_rijsq = (T)MD_CUTOFF_RIJSQ;
+    const T nanv = (T)NAN;
+    const bool staged = S <= kThirdMax && blockDim.x <= 128;  // warp-uniform
+    if (staged) {
+      for (int m = lane; m < S; m += 32) {
+        const uint32_t em = sl[(size_t)m * n + i];
+        const int mp = entry_index(em);
+        T xm, ym, zm;
+        int tm;
+        PosT<T>::load(pos, posf, mp, xm, ym, zm, tm);
+        PosT<T>::image(xm, ym, zm, em, g);
+        TS.id[m] = tm == SP_NG ? -1 : mp;
+        TS.x[m] = xm;
+        TS.y[m] = ym;
+        TS.z[m] = zm;
+        const float imx = xi - xm, imy = yi - ym, imz = zi - zm;
+        const float r2 = imx * imx + imy * imy + imz * imz;
+        const float irim = rsqrtf(r2), rim = r2 * irim;
+        float fci, dfci;
+        cutoff<float>(rim, fci, dfci);
+        TS.r[m] = rim;
+        TS.ir[m] = irim;
+        TS.fc[m] = fci;
+        TS.dfc[m] = dfci;
+        TS.ux[m] = imx * irim;
+        TS.uy[m] = imy * irim;
+        TS.uz[m] = imz * irim;
+      }
+      __syncwarp();
+    }
+    for (int s = lane; s < S; s += 32) {
+      const uint32_t e = sl[(size_t)s * n + i];
+      const int j = entry_index(e);
+      T xj, yj, zj;
+      int tj;
+      PosT<T>::load(pos, posf, j, xj, yj, zj, tj);
+      PosT<T>::image(xj, yj, zj, e, g);
+      const size_t slot = (size_t)s * n + i;
+      const T ijx = xi - xj, ijy = yi - yj, ijz = zi - zj;
+      T rij = ijx * ijx + ijy * ijy + ijz * ijz;
+      if (tj == SP_NG || rij > cut_rijsq) {
+        xsi_s[slot] = nanv;
+        xsj_s[slot] = nanv;
+        continue;
+      }
+      rij = md_sqrt(rij);
+      // BondOrderFuncs.h:242-278 bondForces
+      T va = 0, dva = 0, vr = 0, dvr = 0, vdw, dvdw, bo = 0;
+      T dbx = 0, dby = 0, dbz = 0;
+      T fcut, dfcut;
+      cutoff<T>(fdiv<T>(rij, 10), fcut, dfcut);
+      T xs_i = nanv, xs_j = nanv;
+      if (fcut > 0) {
+        const T de = get_de<T>(ti, tj), re = get_re<T>(ti, tj), beta = get_beta<T>(ti, tj);
+        attractive<T>(va, dva, rij, de, beta, re);
+        repulsive<T>(vr, dvr, rij, de, beta, re);
+        // BondOrderFuncs.h:12-143 bondOrder1
+        const T drijx = fdiv<T>(ijx, rij), drijy = fdiv<T>(ijy, rij), drijz = fdiv<T>(ijz, rij);
+        const T E = md_exp((T)MD_LAMDA3 * (rij - re));
+        const T inv_rij = fdiv<T>(1.0f, rij), half_inv_rij = 0.5f * inv_rij;
+        T xsi = 0, xsj = 0;
+        T dxsix = 0, dxsiy = 0, dxsiz = 0, dxsjx = 0, dxsjy = 0, dxsjz = 0;
+        for (int m = 0; m < S; m++) {
+          T xm, ym, zm, rim, inv_rim, fci, dfci, drimx, drimy, drimz;
+          if (staged) {
+            const int mp = TS.id[m];
+            if (mp < 0 || mp == j) continue;
+            xm = TS.x[m];
+            ym = TS.y[m];
+            zm = TS.z[m];
+            rim = TS.r[m];
+            inv_rim = TS.ir[m];
+            fci = TS.fc[m];
+            dfci = TS.dfc[m];
+            drimx = TS.ux[m];
+            drimy = TS.uy[m];
+            drimz = TS.uz[m];
+          } else {
+            const uint32_t em = sl[(size_t)m * n + i];
+            const int mp = entry_index(em);
+            int tm;
+            PosT<T>::load(pos, posf, mp, xm, ym, zm, tm);
+            if (tm == SP_NG || mp == j) continue;
+            PosT<T>::image(xm, ym, zm, em, g);
+            const T imx = xi - xm, imy = yi - ym, imz = zi - zm;
+            rim = md_sqrt(imx * imx + imy * imy + imz * imz);
+            cutoff<T>(rim, fci, dfci);
+            drimx = fdiv<T>(imx, rim);
+            drimy = fdiv<T>(imy, rim);
+            drimz = fdiv<T>(imz, rim);
+            inv_rim = fdiv<T>(1.0f, rim);
+          }
+          const T jmx = xj - xm, jmy = yj - ym, jmz = zj - zm;
+          T rjm, inv_rjm = 0;
+          {  // the distance and its reciprocal from one rsqrt
+            const float r2 = (float)(jmx * jmx + jmy * jmy + jmz * jmz);
+            const float ir = rsqrtf(r2);
+            inv_rjm = ir;
+            rjm = r2 * ir;
+          }
+          T fcj, dfcj;
+          cutoff<T>(rjm, fcj, dfcj);
+          if (fci > 0) {
+            // d cos / d r_i = drij (1/rim - cos/rij) + drim (1/rij - cos/rim): the
+            // reference's quotient per component (BondOrderFuncs.h) in two scalars
+            const T num2 = rij * rij + rim * rim - rjm * rjm;
+            const T icos = num2 * half_inv_rij * inv_rim;
+            T gth, gpre;
+            angular1<T>(icos, gth, gpre);
+            xsi += fci * gth * E;
+            const T fE = fci * E;
+            const T cm = dfci * gth * E + fE * gpre * (inv_rij - icos * inv_rim);
+            const T cj = fE * (gpre * (inv_rim - icos * inv_rij) + gth * (T)MD_LAMDA3);
+            dxsix = fma(drimx, cm, fma(drijx, cj, dxsix));
+            dxsiy = fma(drimy, cm, fma(drijy, cj, dxsiy));
+            dxsiz = fma(drimz, cm, fma(drijz, cj, dxsiz));
+          }
+          if (fcj > 0) {
+            // d cos / d r_i = drij (1/rjm - cos/rij) - drim rim / (rij rjm)
+            const T num2 = rij * rij + rjm * rjm - rim * rim;
+            const T jcos = num2 * half_inv_rij * inv_rjm;
+            T gth, gpre;
+            angular1<T>(jcos, gth, gpre);
+            xsj += fcj * gth * E;
+            const T fE = fcj * E;
+            const T cj = fE * (gpre * (inv_rjm - jcos * inv_rij) + (T)MD_LAMDA3 * gth);
+            const T cm = -fE * gpre * rim * inv_rij * inv_rjm;
+            dxsjx = fma(drijx, cj, fma(drimx, cm, dxsjx));
+            dxsjy = fma(drijy, cj, fma(drimy, cm, dxsjy));
+            dxsjz = fma(drijz, cj, fma(drimz, cm, dxsjz));
+          }
+        }
+        xs_i = xsi;
+        xs_j = xsj;
+        const T bij = fdiv<T>(1.0f, 1.0f + xsi), pbi = fdiv<T>(1.0f, (1.0f + xsi) * (1.0f + xsi));
+        const T bji = fdiv<T>(1.0f, 1.0f + xsj), pbj = fdiv<T>(1.0f, (1.0f + xsj) * (1.0f + xsj));
+        bo = 0.5f * (bij + bji);
+        dbx = 0.5f * (pbi * dxsix + pbj * dxsjx);
+        dby = 0.5f * (pbi * dxsiy + pbj * dxsjy);
+        dbz = 0.5f * (pbi * dxsiz + pbj * dxsjz);
+        // what pass 2 needs of this pair: va E / (4 (1 + xi)^2) for either
+        // end (its force is -factor x the derivative of the angle terms)
+        xs_i = (T)0.25 * va * E * pbi;
+        xs_j = (T)0.25 * va * E * pbj;
+      }
+      xsi_s[slot] = xs_i;
+      xsj_s[slot] = xs_j;
+      vander_waals<T>(vdw, dvdw, rij, get_r0v<T>(ti, tj));
+      const T fij = dvr - bo * dva + dvdw;
+      fx += fdiv<T>(fij * ijx, rij) - dbx * va;
+      fy += fdiv<T>(fij * ijy, rij) - dby * va;
+      fz += fdiv<T>(fij * ijz, rij) - dbz * va;
+      if (ENERGY) ev[0] += (double)(0.5f * ((vr - bo * va) + vdw));
+    }
+    double sx = warp_sum((double)fx), sy = warp_sum((double)fy), sz = warp_sum((double)fz);
+    if (ENERGY && eatom) {
+      // per-atom share: sum over j of 1/2 (Vr - b Va + Vdw) (the i-sum of
+      // common/DebugCalculations.cpp:129-270 restricted to the force's pairs)
+      const double ei = warp_sum(ev[0]);
+      if (lane == 0) eatom[i] = ei;
+    }
+    if (lane == 0) {
+      if (ljexist) {
+        f3[3 * i] += sx;
+        f3[3 * i + 1] += sy;
+        f3[3 * i + 2] += sz;
+      } else {
+        f3[3 * i] = sx;
+        f3[3 * i + 1] = sy;
+        f3[3 * i + 2] = sz;
+      }
+      if (ENERGY) {
+        const md_double4 p = pos[i];
+        ev[1] = p.x * sx + p.y * sy + p.z * sz;
+      }
+    }
+  }
+  if (ENERGY) block_partial<2>(ev, epart);
+}
+
+// Pass 2 of the precision form: one warp per atom k, one entry i of k's short
+// list per lane, over i's bonds i-j; 40 registers, 12 blocks per SM instead of
+// 10.  (Spreading the bonds of k over all 32 lanes was measured slower, 348
+// against 249 us on 32,768 atoms: lanes of one i read 32 different lines of the
+// slot arrays, where lanes of neighbouring i, stored side by side, share
+// sectors.)  ref_rows is NULL here; it stays an argument because without the
+// branch the compiler fuses other products into FMAs, which moves the last bit.
+template <bool ENERGY>
+__global__ void __launch_bounds__(128, 12)
+    k_mb_pass2_32(const md_double4* __restrict__ pos, const float4* __restrict__ posf,
+               double* __restrict__ f3, int n, const uint32_t* __restrict__ sl,
+               const int* __restrict__ slen, Grid g, const int* __restrict__ cell3,
+               const int* __restrict__ ref_rows, int ref_nls, int ref_nlargest, double rcutsq,
+               const float* __restrict__ wi_s, const float* __restrict__ wj_s,
+               int* __restrict__ missing, double* __restrict__ epart,
+               const int* __restrict__ run_if) {
+  if (!ENERGY && run_if && *run_if == 0) return;
+  using T = float;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int k = blockIdx.x * 4 + warp;
+  double ev[1] = {0.0};
+  if (k < n) {
+    T xk, yk, zk;
+    int tk;
+    PosT<T>::load(pos, posf, k, xk, yk, zk, tk);
+    const int Sk = slen[k];
+    const T rc2 = (T)rcutsq, cut_rijsq = (T)MD_CUTOFF_RIJSQ;
+    T fx = 0, fy = 0, fz = 0;
+    int miss = 0;
+    for (int s = lane; s < Sk; s += 32) {
+      const Pass2I<T> I = pass2_entry<T>(sl[(size_t)s * n + k], xk, yk, zk, pos, posf, g);
+      const int Si = slen[I.id];
+      for (int sj = 0; sj < Si; sj++)
+        pass2_pair<T>(I, (size_t)sj * n + I.id, k, xk, yk, zk, pos, posf, sl, g, cell3,
+                      ref_rows, ref_nls, ref_nlargest, rc2, cut_rijsq, wi_s, wj_s, fx, fy, fz,
+                      miss);
+    }
+    const double sx = warp_sum((double)fx), sy = warp_sum((double)fy), sz = warp_sum((double)fz);
+    const int m = __reduce_add_sync(0xffffffffu, miss);
+    if (lane == 0) {
+      f3[3 * k] += sx;
+      f3[3 * k + 1] += sy;
+      f3[3 * k + 2] += sz;
+      if (m) atomicAdd(missing, m);
+      if (ENERGY) {
+        const md_double4 p = pos[k];
+        ev[0] = p.x * sx + p.y * sy + p.z * sz;
+      }
+    }
+  }
+  if (ENERGY) block_partial<1>(ev, epart);
 }
 
 inline int nblk(long long n, int t) { return (int)((n + t - 1) / t); }
@@ -1452,39 +1723,54 @@ void launch_lj(const ForceArgs& a, bool fp32, bool energy, cudaStream_t st) {
 int lj_blocks(int n, bool fp32) {
   return fp32 ? nblk(n, 128) : nblk((long long)n * lj64_lanes(n), 128);
 }
-int mb_blocks(int n) { return n; }
+int mb_blocks(int n, bool fp32) { return fp32 ? nblk(n, 4) : n; }
 
-template <typename T, bool ENERGY>
-static void launch_mb_t(const MbArgs& a, cudaStream_t st) {
-  if (a.n <= 0) return;
+template <bool ENERGY>
+static void launch_mb64(const MbArgs& a, cudaStream_t st) {
   const int* gate = ENERGY ? nullptr : a.run_if;
-  T *wi = (T*)a.xsi, *wj = (T*)a.xsj, *fs = (T*)a.fslot;
+  double *wi = (double*)a.xsi, *wj = (double*)a.xsj, *fs = (double*)a.fslot;
   double *e1 = ENERGY ? a.epart1 : nullptr, *e2 = ENERGY ? a.epart2 : nullptr;
   double* ea = ENERGY ? a.eatom : nullptr;
   const int B = nblk(a.n, 4);
-  k_mb_short<T><<<B, 128, 0, st>>>(a.pos, a.posf, a.n, a.ld, a.list, a.len, a.grid, a.rcutsq,
-                                   a.sl, a.pitch, a.slen, gate);
+  k_mb_short<double><<<B, 128, 0, st>>>(a.pos, a.posf, a.n, a.list, a.ri, a.rk, a.len, a.grid,
+                                        a.rcutsq, a.sl, (size_t)a.pitch, 1, a.slen, gate);
   if (!a.ref_rows) {
-    k_mb_bonds<T, ENERGY, true><<<a.n, 128, 0, st>>>(a.pos, a.posf, a.f3, a.n, a.sl, a.pitch,
-                                                     a.slen, a.grid, a.cell3, a.ljexist, wi, wj,
-                                                     fs, a.missing, e1, ea, gate);
-    k_mb_gather<T, ENERGY><<<B, 128, 0, st>>>(a.pos, a.posf, a.f3, a.n, a.sl, a.pitch, a.slen,
-                                              a.grid, a.cell3, a.rcutsq, wi, wj, fs, a.missing,
-                                              e2, gate);
-  } else if constexpr (sizeof(T) == 8 && !ENERGY) {
-    k_mb_bonds<T, false, false><<<a.n, 128, 0, st>>>(a.pos, a.posf, a.f3, a.n, a.sl, a.pitch,
-                                                     a.slen, a.grid, nullptr, a.ljexist, wi, wj,
-                                                     nullptr, a.missing, nullptr, nullptr, gate);
+    k_mb_bonds<ENERGY, true><<<a.n, 128, 0, st>>>(
+        a.pos, a.posf, a.f3, a.n, a.sl, a.pitch, a.slen, a.grid, a.cell3, a.ljexist, wi, wj, fs,
+        a.missing, e1, ea, gate);
+    k_mb_gather<ENERGY><<<B, 128, 0, st>>>(a.pos, a.posf, a.f3, a.n, a.sl, a.pitch,
+                                                   a.slen, a.grid, a.cell3, a.rcutsq, wi, wj, fs,
+                                                   a.missing, e2, gate);
+  } else if constexpr (!ENERGY) {
+    k_mb_bonds<false, false><<<a.n, 128, 0, st>>>(
+        a.pos, a.posf, a.f3, a.n, a.sl, a.pitch, a.slen, a.grid, nullptr, a.ljexist, wi, wj,
+        nullptr, a.missing, nullptr, nullptr, gate);
     k_mb_pass2<<<B, 128, 0, st>>>(a.pos, a.f3, a.n, a.sl, a.pitch, a.slen, a.grid, a.ref_rows,
                                   a.ref_nls, a.ref_nlargest, a.rcutsq, wi, wj, a.missing);
   }
 }
 
+template <bool ENERGY>
+static void launch_mb32(const MbArgs& a, cudaStream_t st) {
+  const int* gate = ENERGY ? nullptr : a.run_if;
+  float *wi = (float*)a.xsi, *wj = (float*)a.xsj;
+  const int B = nblk(a.n, 4);
+  k_mb_short<float><<<B, 128, 0, st>>>(a.pos, a.posf, a.n, a.list, a.ri, a.rk, a.len, a.grid,
+                                       a.rcutsq, a.sl, 1, (size_t)a.n, a.slen, gate);
+  k_mb_pass1_32<ENERGY><<<B, 128, 0, st>>>(a.pos, a.posf, a.f3, a.n, a.sl, a.slen, a.grid,
+                                           a.ljexist, wi, wj, ENERGY ? a.epart1 : nullptr,
+                                           ENERGY ? a.eatom : nullptr, gate);
+  k_mb_pass2_32<ENERGY><<<B, 128, 0, st>>>(a.pos, a.posf, a.f3, a.n, a.sl, a.slen, a.grid,
+                                           a.cell3, a.ref_rows, a.ref_nls, a.ref_nlargest, a.rcutsq,
+                                           wi, wj, a.missing, ENERGY ? a.epart2 : nullptr, gate);
+}
+
 void launch_mb(const MbArgs& a, bool fp32, bool energy, cudaStream_t st) {
+  if (a.n <= 0) return;
   if (fp32)
-    energy ? launch_mb_t<float, true>(a, st) : launch_mb_t<float, false>(a, st);
+    energy ? launch_mb32<true>(a, st) : launch_mb32<false>(a, st);
   else
-    energy ? launch_mb_t<double, true>(a, st) : launch_mb_t<double, false>(a, st);
+    energy ? launch_mb64<true>(a, st) : launch_mb64<false>(a, st);
 }
 
 }  // namespace mdgb

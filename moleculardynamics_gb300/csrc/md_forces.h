@@ -46,9 +46,9 @@ struct MbArgs {
   const float4* posf;
   double* f3;
   int n;                // many-body atoms [0, n)
-  const uint32_t* list; // full candidate rows, list[k * ld + i]
+  const uint32_t* list; // full candidate rows, list[i * ri + k * rk]
   const int* len;
-  int ld;
+  size_t ri, rk;
   Grid grid;
   const int* cell3;     // build-time cells of the many-body list
   const int* ref_rows;  // or: rows in the reference layout (membership by scan)
@@ -56,16 +56,17 @@ struct MbArgs {
   int ref_nlargest;
   double rcutsq;
   int ljexist;          // accumulate onto F (BondOrderFuncs.h:325-336)
-  uint32_t* sl;         // short lists, sl[i * pitch + s] (scratch, n * pitch)
+  uint32_t* sl;         // short lists (scratch, n * pitch): FP64 sl[i * pitch + s], FP32
+                        // sl[s * n + i]; xsi, xsj alike
   int pitch;            // slots per atom; a multiple of 4 unless ref_rows is set
   int* slen;
   void* xsi;            // per (i, slot), T: the bond's factor va E / (4 (1 + xi_ij)^2)
   void* xsj;            // and va E / (4 (1 + xi_ji)^2), NaN where there is no bond
-  void* fslot = nullptr;  // forces on third bodies, 4 T for each of an atom's kMbSlotCount
+  void* fslot = nullptr;  // FP64: forces on third bodies, 4 for each of an atom's kMbSlotCount
                           // first slots (not needed with ref_rows)
   int* missing;
   const int* run_if = nullptr;  // force launches only: return at once unless *run_if != 0
-  double* epart1;       // energy launches: 2 doubles per atom (bonds)
+  double* epart1;       // energy launches: 2 doubles per entry of mb_blocks (bonds)
   double* epart2;       // and 1 (third bodies)
   double* eatom = nullptr;  // energy launches: per-atom energy (sum over j of half the pair)
 };
@@ -78,7 +79,7 @@ void launch_lj_step64(const ForceArgs& a, cudaStream_t st);
 void launch_lj_redo64(const ForceArgs& a, cudaStream_t st);
 void launch_mb(const MbArgs& a, bool fp32, bool energy, cudaStream_t st);
 int lj_blocks(int n, bool fp32);  // blocks of an energy launch of launch_lj
-int mb_blocks(int n);            // atoms with entries in epart1, epart2
+int mb_blocks(int n, bool fp32);  // entries of an energy launch in epart1, epart2
 constexpr int kMbSlotCount = 64;
 
 }  // namespace mdgb

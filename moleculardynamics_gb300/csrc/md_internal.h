@@ -28,8 +28,9 @@ struct CellTable {
   int cap = 0;  // power of two
 };
 
-// One neighbour list: atoms [0, n) of the engine, rows in ELL slot-major
-// layout list[k * n + i] of packed entries (md_common.cuh).
+// One neighbour list: atoms [0, n) of the engine, rows of packed entries
+// (md_common.cuh): compact rows slot-major, list[k * ld + i], full candidate
+// rows by atom, list[i * cap + k].
 struct NeighborList {
   int n = 0;
   Grid grid{};
@@ -41,7 +42,8 @@ struct NeighborList {
   uint32_t* list = nullptr;
   int* len = nullptr;
   int ld = 0;                  // leading dimension: list[k * ld + i], ld = n rounded up to 32
-  int cap = 0;                 // slots per row allocated
+  int cap = 0;                 // slots per row allocated (a multiple of 4)
+  int list_n = 0;              // atoms the rows were allocated for
   CUtensorMap tmap;            // TMA descriptor of the list (compact lists)
   int tmap_ok = 0;
   long long list_elems = 0;    // allocated list entries

@@ -15,6 +15,7 @@
 // far enough for a dropped candidate to come within rcut, and otherwise walks
 // the full row (same candidates, same order as the reference).
 #include <cmath>
+#include <type_traits>
 #include <cstdio>
 #include <cstring>
 
@@ -174,42 +175,101 @@ __global__ void k_pos_build(const md_double4* __restrict__ pos, int n, float4* _
   pb[i] = make_float4((float)p.x, (float)p.y, (float)p.z, __int_as_float((int)p.w));
 }
 
-// MODE 0: count (len[i] and maxima); MODE 1: write ELL rows.
+// Rows, a warp per atom: 27 lanes look up the cells around the atom's own, a
+// warp scan joins them into one candidate sequence in the reference's order,
+// and the lanes test 32 candidates at a time (a ballot keeps the order).
+// MODE 0 counts (len[i] and maxima), 1 writes, 2 does both, with rows longer
+// than cap truncated and reported through the counters.  An entry k of atom i
+// goes to list[i * ri + k * rk].
+// A thread per atom walked its 600 candidates one dependent load after another:
+// 57 us (count) and 129 us (write) for 864 atoms, 177 and 380 for 108,000.
 template <int MODE>
-__global__ void k_rows(RowWalker w, const md_double4* __restrict__ pos,
-                       const float4* __restrict__ pb, int compact, float rv2, float box_f,
-                       uint32_t* __restrict__ list, int* __restrict__ len, int ld,
-                       int* __restrict__ counters) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= w.n) return;
+__global__ void __launch_bounds__(128)
+    k_rows(RowWalker w, const md_double4* __restrict__ pos, const float4* __restrict__ pb,
+           int compact, float rv2, float box_f, uint32_t* __restrict__ list,
+           int* __restrict__ len, size_t ri, size_t rk, int cap, int* __restrict__ counters) {
+  const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (i >= w.n) return;  // whole warp
   const float4 pi = pb[i];
-  int full = 0, kept = 0;
-  walk_row(w, pos, i, [&](int m, int ix, int iy, int iz) {
-    full++;
-    bool keep = true;
-    if (compact) {
-      float4 pm = pb[m];
-      float dx = pi.x - (pm.x + (float)ix * box_f);
-      float dy = pi.y - (pm.y + (float)iy * box_f);
-      float dz = pi.z - (pm.z + (float)iz * box_f);
+  const bool whole = w.g.periodic && w.g.cells == 1;  // minimum images of all atoms
+  int first = 0, count = 0, img = 0;  // this lane's cell
+  if (!whole && lane < 27) {
+    const int4 c4 = reinterpret_cast<const int4*>(w.cell3)[i];
+    int nc[3] = {c4.x + lane / 9 - 1, c4.y + lane / 3 % 3 - 1, c4.z + lane % 3 - 1};
+    bool out = false;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      if (!w.g.periodic) {
+        out |= nc[d] >= w.g.cells || nc[d] < 0;
+      } else if (nc[d] < 0) {
+        nc[d] += w.g.cells;
+        img |= 3 << (2 * d);
+      } else if (nc[d] >= w.g.cells) {
+        nc[d] -= w.g.cells;
+        img |= 1 << (2 * d);
+      }
+    }
+    const int s = out ? -1 : table_find(w.keys, w.cap, cell_key(nc[0], nc[1], nc[2]));
+    if (s >= 0) {
+      first = w.start[s];
+      count = w.count[s];
+    }
+  }
+  int pre = count;  // inclusive, then exclusive
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, pre, o);
+    if (lane >= o) pre += y;
+  }
+  const int total = whole ? w.n : __shfl_sync(0xffffffffu, pre, 31);
+  pre -= count;
+  const md_double4 ei = whole ? pos[i] : md_double4{0, 0, 0, 0};
+  int kept = 0, self = 0;
+  for (int q0 = 0; q0 < total; q0 += 32) {
+    const int q = q0 + lane;
+    int m = q, im = 0;
+    if (!whole) {
+      // the last cell that starts at or before q
+      int c = 0;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const int p = __shfl_sync(0xffffffffu, pre, (c + o) & 31);
+        if (c + o < 27 && p <= q) c += o;
+      }
+      const int p = __shfl_sync(0xffffffffu, pre, c), f = __shfl_sync(0xffffffffu, first, c);
+      im = __shfl_sync(0xffffffffu, img, c);
+      if (q < total) m = w.sorted[f + q - p];
+    }
+    bool keep = q < total && m != i;
+    if (q < total && m == i) self = 1;
+    if (keep && whole) {
+      const md_double4 em = pos[m];
+      im = (min_image(ei.x, em.x, w.g.box) & 3) | ((min_image(ei.y, em.y, w.g.box) & 3) << 2) |
+           ((min_image(ei.z, em.z, w.g.box) & 3) << 4);
+    }
+    const uint32_t e = (uint32_t)m | ((uint32_t)im << kIndexBits);
+    if (keep && compact) {
+      const float4 pm = pb[m];
+      const float dx = pi.x - (pm.x + (float)entry_img(e, 0) * box_f);
+      const float dy = pi.y - (pm.y + (float)entry_img(e, 1) * box_f);
+      const float dz = pi.z - (pm.z + (float)entry_img(e, 2) * box_f);
       keep = dx * dx + dy * dy + dz * dz < rv2;
     }
-    if (keep) {
-      if (MODE == 1) list[(size_t)kept * ld + i] = pack_entry(m, ix, iy, iz);
-      kept++;
+    const unsigned mask = __ballot_sync(0xffffffffu, keep);
+    if (MODE != 0 && keep) {
+      const int k = kept + __popc(mask & ((1u << lane) - 1u));
+      if (k < cap) list[(size_t)i * ri + (size_t)k * rk] = e;
     }
-  });
-  if (MODE == 0) {
-    len[i] = kept;
-    // one atomic per warp for each counter
-    const unsigned m = __activemask();
-    const unsigned fmax_w = __reduce_max_sync(m, (unsigned)full);
-    const unsigned kmax_w = __reduce_max_sync(m, (unsigned)kept);
-    const unsigned ksum_w = __reduce_add_sync(m, (unsigned)kept);
-    if ((int)(threadIdx.x & 31) == __ffs(m) - 1) {
-      atomicMax(&counters[1], (int)fmax_w);
-      atomicMax(&counters[2], (int)kmax_w);
-      atomicAdd((unsigned long long*)(counters + 4), (unsigned long long)ksum_w);
+    kept += __popc(mask);
+  }
+  if (MODE != 1) {
+    const int full = total - (__any_sync(0xffffffffu, self) ? 1 : 0);
+    if (lane == 0) {
+      len[i] = kept;
+      atomicMax(&counters[1], full);
+      atomicMax(&counters[2], kept);
+      atomicAdd((unsigned long long*)(counters + 4), (unsigned long long)kept);
     }
   }
 }
@@ -421,9 +481,25 @@ int list_build(NeighborList& nl, md_double4* pos, int n, const Grid& g, int comp
   float margin = (float)(1e-6 * (fabs(g.box) + rv) + 1e-6);
   float rv_keep = rv + margin;
   float rv2 = compact ? rv_keep * rv_keep : 0.f;
-  if (n > 0)
-    k_rows<0><<<blocks(n, 128), 128, 0, st>>>(w, pos, nl.pos_build, compact, rv2, g.box_f,
-                                              nullptr, nl.len, n, sc.counts);
+  nl.ld = ((n > 0 ? n : 1) + 31) / 32 * 32;
+  // compact rows slot-major (the LJ kernels read one slot of many atoms), full
+  // rows atom by atom (a warp reads its atom's candidates)
+  const auto rows = [&](auto mode) {
+    constexpr int M = decltype(mode)::value;
+    const size_t ri = compact ? 1 : (size_t)nl.cap, rk = compact ? (size_t)nl.ld : 1;
+    k_rows<M><<<blocks(n, 4), 128, 0, st>>>(w, pos, nl.pos_build, compact, rv2, g.box_f, nl.list,
+                                            nl.len, ri, rk, nl.cap, sc.counts);
+  };
+  // one pass into the capacity of the previous build; the writing pass again
+  // only when a row outgrew it
+  const bool have =
+      nl.list && nl.cap > 0 && nl.list_n == n && (long long)nl.cap * nl.ld <= nl.list_elems;
+  if (n > 0) {
+    if (have)
+      rows(std::integral_constant<int, 2>());
+    else
+      rows(std::integral_constant<int, 0>());
+  }
   int hc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   int status = 0;
   cudaMemcpyAsync(hc, sc.counts, sizeof(hc), cudaMemcpyDeviceToHost, st);
@@ -448,14 +524,14 @@ int list_build(NeighborList& nl, md_double4* pos, int n, const Grid& g, int comp
   nl.max_len = hc[2];
   int need_cap = hc[2] > 0 ? hc[2] : 1;
   if (compact) need_cap = (int)(need_cap * nl.headroom) + 8;  // room for skin refreshes
-  nl.ld = ((n > 0 ? n : 1) + 31) / 32 * 32;
-  long long elems = (long long)need_cap * nl.ld;
-  if ((e = grow(nl.list, nl.list_elems, elems)) != cudaSuccess) return e;
-  nl.cap = need_cap;
+  need_cap = (need_cap + 3) & ~3;
+  if (!have || need_cap > nl.cap) {
+    if ((e = grow(nl.list, nl.list_elems, (long long)need_cap * nl.ld)) != cudaSuccess) return e;
+    nl.cap = need_cap;
+    nl.list_n = n;
+    if (n > 0) rows(std::integral_constant<int, 1>());
+  }
   nl.tmap_ok = compact && n > 0 ? encode_list_map(nl) : 0;
-  if (n > 0)
-    k_rows<1><<<blocks(n, 128), 128, 0, st>>>(w, pos, nl.pos_build, compact, rv2, g.box_f,
-                                              nl.list, nl.len, nl.ld, sc.counts);
   double rc = rcut;
   nl.trip_dist = compact ? 0.5 * ((double)rv - rc) - (double)margin : 1e300;
   nl.rv2_keep = rv2;

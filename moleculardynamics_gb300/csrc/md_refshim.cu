@@ -289,7 +289,8 @@ void mdgb_many_body_forces(const double* pos4, double* f3, int n, int nlargestsi
   a.n = n;
   a.list = s.ell;
   a.len = s.len;
-  a.ld = n;
+  a.ri = 1;
+  a.rk = (size_t)n;
   a.grid = Grid{};
   a.cell3 = nullptr;
   a.ref_rows = s.rows;

@@ -117,7 +117,8 @@ extern "C" int mdgb_many_body_forces_static(const double* d_pos4, double* d_f3, 
   a.n = n;
   a.list = ell;
   a.len = len;
-  a.ld = n;
+  a.ri = 1;
+  a.rk = (size_t)n;
   a.grid = Grid{};
   a.cell3 = nullptr;
   a.ref_rows = d_list;
