@@ -242,6 +242,7 @@ __global__ void k_cl_segments(ClusterSegment* __restrict__ seg, const int* __res
   if (s >= *nseg_dev) return;
   ClusterSegment& S = seg[s];
   const ClusterReplica r = reps[S.rep];
+  S.r = r;
   if (r.G == 1) {
     ClusterPiece pc;
     pc.src = start[r.cell0];
@@ -304,29 +305,21 @@ __global__ void k_cl_segments(ClusterSegment* __restrict__ seg, const int* __res
 // ---- per-block segment context in shared memory ----
 struct SegShared {
   ClusterSegment S;
-  ClusterReplica r;
-  int self0;          // staged offset of the segment's first own atom
   int off[9][kOffW];  // staged offset of z slot w (cell cz0-1+w) of each group; w = zspan: end
 };
 
-__device__ __forceinline__ void load_segment(SegShared& sh, const ClusterSegment* seg,
-                                             const ClusterReplica* reps, int sidx) {
+__device__ __forceinline__ void load_segment(SegShared& sh, const ClusterSegment* seg, int sidx) {
   const int* src = (const int*)&seg[sidx];
   int* dst = (int*)&sh.S;
   for (int k = threadIdx.x; k < (int)(sizeof(ClusterSegment) / 4); k += blockDim.x)
     dst[k] = src[k];
-  __syncthreads();
-  const int* rs = (const int*)&reps[sh.S.rep];
-  int* rd = (int*)&sh.r;
-  for (int k = threadIdx.x; k < (int)(sizeof(ClusterReplica) / 4); k += blockDim.x) rd[k] = rs[k];
-  if (threadIdx.x == 0) sh.self0 = sh.S.self0;  // computed at the build (k_cl_segments)
 }
 
 // staged copy of positions with the pieces' periodic images applied
 __device__ __forceinline__ void stage(const SegShared& sh, const float4* __restrict__ src,
                                       float4* st) {
   const ClusterSegment& S = sh.S;
-  const float Lf = sh.r.Lf, Llo = sh.r.Llo;
+  const float Lf = sh.S.r.Lf, Llo = sh.S.r.Llo;
   for (int k = 0; k < S.npieces; k++) {
     const ClusterPiece pc = S.piece[k];
     const float sx = (float)pc.ix, sy = (float)pc.iy, sz = (float)pc.iz;
@@ -372,7 +365,7 @@ __device__ __forceinline__ bool stage_bulk(const SegShared& sh, const float4* __
     return false;
   }
   if (!S.img) return true;
-  const float Lf = sh.r.Lf, Llo = sh.r.Llo;
+  const float Lf = sh.S.r.Lf, Llo = sh.S.r.Llo;
   for (int k = 0; k < S.npieces; k++) {
     const ClusterPiece& pc = S.piece[k];
     if ((pc.ix | pc.iy | pc.iz) == 0) continue;
@@ -390,7 +383,7 @@ __device__ __forceinline__ bool stage_bulk(const SegShared& sh, const float4* __
 
 __device__ __forceinline__ void fill_offsets(SegShared& sh, const int* __restrict__ start) {
   const ClusterSegment& S = sh.S;
-  const ClusterReplica& r = sh.r;
+  const ClusterReplica& r = sh.S.r;
   if (r.G == 1) return;
   const int zspan = S.cz1 - S.cz0 + 3;
   for (int k = threadIdx.x; k < 9 * (zspan + 1); k += blockDim.x) {
@@ -416,13 +409,13 @@ __device__ __forceinline__ void fill_offsets(SegShared& sh, const int* __restric
 
 // staged offset of the segment's own atom p
 __device__ __forceinline__ int self_offset(const SegShared& sh, int p) {
-  return sh.self0 + (p - sh.S.p0);
+  return sh.S.self0 + (p - sh.S.p0);
 }
 
 // visit(q) for every staged candidate of atom p's 27-cell row, in row order
 template <typename F>
 __device__ __forceinline__ void walk_staged(const SegShared& sh, int self, F&& visit) {
-  if (sh.r.G == 1) {
+  if (sh.S.r.G == 1) {
     for (int q = 0; q < sh.S.staged; q++)
       if (q != self) visit(q);
     return;
@@ -557,13 +550,13 @@ __global__ void __launch_bounds__(256)
               int* __restrict__ counters, int grouped) {
   extern __shared__ float4 st[];
   __shared__ SegShared sh;
-  load_segment(sh, seg, reps, blockIdx.x);
+  load_segment(sh, seg, blockIdx.x);
   __syncthreads();
   stage(sh, pb, st);
   fill_offsets(sh, start);
   __syncthreads();
-  const bool minimg = sh.r.G == 1;
-  const float Lf = sh.r.Lf, invL = 1.0f / sh.r.Lf;
+  const bool minimg = sh.S.r.G == 1;
+  const float Lf = sh.S.r.Lf, invL = 1.0f / sh.S.r.Lf;
   int mx = 0;
   unsigned long long tot = 0;
   for (int base = sh.S.p0; base < sh.S.p1; base += blockDim.x) {
@@ -717,8 +710,8 @@ __device__ __noinline__ bool band_inside(const SegShared& sh, const md_double4* 
   int ix, iy, iz;
   const int j = staged_source(sh.S, q, ix, iy, iz);
   const md_double4 a = pos[p], b = pos[j];
-  const double L = sh.r.L;
-  if (sh.r.G == 1) {
+  const double L = sh.S.r.L;
+  if (sh.S.r.G == 1) {
     ix = min_image(a.x, b.x, L);
     iy = min_image(a.y, b.y, L);
     iz = min_image(a.z, b.z, L);
@@ -740,51 +733,89 @@ struct LjParams {
 };
 
 // The padded-row loops decide pairs within 1e-5 of the cutoff afterwards:
-// the atom's row is walked again (entries from global memory, in row order),
-// and every pair in the band that the FP64 decision keeps is added, in row
-// order, to one FP32 sum, folded once into the compensated force.  Rare
-// (about one atom in 600 has such a pair).
+// the row's 16-slot chunks that have such a pair (bit t of `chunks`: chunk t,
+// bit 31: any from 31 on) are walked again, entries from global memory in row
+// order, and every pair in the band that the FP64 decision keeps is added, in
+// row order, to one FP32 sum, folded once into the compensated force.  Rare
+// (about one atom in 600 has such a pair), but the chunk's entries are loaded
+// together: walking the whole row one dependent load after another took 9 us,
+// as long as the rest of a block's segment, and every launch waits for one.
 template <bool ALL_NG>
 __device__ __noinline__ float3 band_pass(const SegShared& sh, const float4* st,
                                          const md_double4* pos, double rcutsq,
-                                         const uint16_t* rows, int ld, int grouped, int p, int L,
-                                         float4 pi, float rc_lo, float rc_hi, LjParams lp) {
+                                         const uint16_t* rows, int ld, int grouped, int p,
+                                         uint32_t chunks, int L, float4 pi, float rc_lo,
+                                         float rc_hi, LjParams lp) {
   float ex = 0.f, ey = 0.f, ez = 0.f;
   const int ti = __float_as_int(pi.w);
-  for (int k = 0; k < L; k++) {
-    const int e = rows[row_slot(k, p, ld, grouped)];
-    const int q = grouped ? e >> 4 : e;
-    const float4 pj = st[q];
-    const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-    const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-    if (!(r2 > rc_lo && r2 < rc_hi)) continue;
-    float fij;
-    const float inv = rcp_approx(r2);
-    if (ALL_NG) {
-      const float inv2 = inv * inv;
-      fij = (inv2 * inv2) * fmaf(lp.p, inv2 * inv, -lp.q);
+  auto chunk = [&](int k0) {
+    uint32_t w[8];
+    if (grouped) {
+      const uint4* r = reinterpret_cast<const uint4*>(rows) + (size_t)(k0 >> 3) * ld + p;
+      const uint4 a = r[0], b = r[ld];
+      w[0] = a.x, w[1] = a.y, w[2] = a.z, w[3] = a.w;
+      w[4] = b.x, w[5] = b.y, w[6] = b.z, w[7] = b.w;
     } else {
-      const int tj = __float_as_int(pj.w);
-      if (!(tj == SP_NG || ti == SP_NG)) continue;
-      const int sel = lj_select(ti, tj);
-      const float s2 = sel == SP_N ? lp.s2[0] : (sel == SP_O ? lp.s2[1] : lp.s2[2]);
-      const float c24 = sel == SP_N ? lp.c24[0] : (sel == SP_O ? lp.c24[1] : lp.c24[2]);
-      const float sr2 = s2 * inv;
-      const float sr6 = sr2 * sr2 * sr2;
-      fij = c24 * inv * sr6 * fmaf(2.0f, sr6, -1.0f);
+#pragma unroll
+      for (int k = 0; k < 8; k++)
+        w[k] = (uint32_t)rows[(size_t)(k0 + 2 * k) * ld + p] |
+               ((uint32_t)rows[(size_t)(k0 + 2 * k + 1) * ld + p] << 16);
     }
-    if (!band_inside(sh, pos, p, q, rcutsq)) continue;
-    ex = fmaf(dx, fij, ex);
-    ey = fmaf(dy, fij, ey);
-    ez = fmaf(dz, fij, ez);
+    // slots of the chunk in the band (past L: the sentinel, never in it)
+    uint32_t in = 0;
+#pragma unroll
+    for (int k = 0; k < 16; k++) {
+      const uint32_t e = (w[k >> 1] >> ((k & 1) * 16)) & 0xFFFFu;
+      const float4 pj = st[grouped ? e >> 4 : e];
+      const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+      const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+      in |= (uint32_t)(r2 > rc_lo && r2 < rc_hi) << k;
+    }
+    for (; in; in &= in - 1) {
+      const int k = __ffs(in) - 1;
+      const uint32_t e = (pick8(w, k >> 1) >> ((k & 1) * 16)) & 0xFFFFu;
+      const int q = (int)(grouped ? e >> 4 : e);
+      const float4 pj = st[q];
+      const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+      const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+      float fij;
+      const float inv = rcp_approx(r2);
+      if (ALL_NG) {
+        const float inv2 = inv * inv;
+        fij = (inv2 * inv2) * fmaf(lp.p, inv2 * inv, -lp.q);
+      } else {
+        const int tj = __float_as_int(pj.w);
+        if (!(tj == SP_NG || ti == SP_NG)) continue;
+        const int sel = lj_select(ti, tj);
+        const float s2 = sel == SP_N ? lp.s2[0] : (sel == SP_O ? lp.s2[1] : lp.s2[2]);
+        const float c24 = sel == SP_N ? lp.c24[0] : (sel == SP_O ? lp.c24[1] : lp.c24[2]);
+        const float sr2 = s2 * inv;
+        const float sr6 = sr2 * sr2 * sr2;
+        fij = c24 * inv * sr6 * fmaf(2.0f, sr6, -1.0f);
+      }
+      if (!band_inside(sh, pos, p, q, rcutsq)) continue;
+      ex = fmaf(dx, fij, ex);
+      ey = fmaf(dy, fij, ey);
+      ez = fmaf(dz, fij, ez);
+    }
+  };
+  for (; chunks; chunks &= chunks - 1) {
+    const int t = __ffs(chunks) - 1;
+    for (int k0 = t * kClusterTileSlots; k0 < L && (t == 31 || k0 < (t + 1) * kClusterTileSlots);
+         k0 += kClusterTileSlots)
+      chunk(k0);
   }
   return make_float3(ex, ey, ez);
+}
+__device__ __forceinline__ uint32_t band_bit(bool band, int chunk) {
+  return (uint32_t)band << min(chunk, 31);
 }
 
 // Arguments of the segment force kernel (device copy of ClusterForceArgs).
 struct ClStep {
   int nseg;
-  int* sched;  // [0] next segment to hand out, [1] blocks finished
+  int* sched;  // [0] segments handed out; launches outside the step loop: [1] blocks finished
+  int* sched_clear;  // step loop: the next launch's counter (else NULL)
   const ClusterSegment* seg;
   const ClusterReplica* reps;
   const int* start;
@@ -872,7 +903,7 @@ __global__ void __launch_bounds__(224, 3)
   __syncthreads();
   const int sidx = s_seg;
   if (sidx >= a.nseg) break;
-  load_segment(sh, a.seg, a.reps, sidx);
+  load_segment(sh, a.seg, sidx);
   __syncthreads();
   // block tiles: the segment's first two row tiles go to L2 while the
   // neighbourhood streams in (no completion to wait for)
@@ -888,11 +919,11 @@ __global__ void __launch_bounds__(224, 3)
   put_sentinel(st, sh.S.staged);
   if (tripped) fill_offsets(sh, a.start);
   __syncthreads();
-  const bool minimg = sh.r.G == 1;
+  const bool minimg = sh.S.r.G == 1;
   // without minimum images or energies the sentinel-padded rows need no
   // per-slot validity test (the sentinel lies beyond every cutoff)
   const bool fast = !ENERGY && !minimg;
-  const float Lf = sh.r.Lf, invL = 1.0f / sh.r.Lf;
+  const float Lf = sh.S.r.Lf, invL = 1.0f / sh.S.r.Lf;
   const float rc2 = (float)a.rcutsq;
   const float rc_lo = rc2 * (1.0f - 1e-5f), rc_hi = rc2 * (1.0f + 1e-5f);
   // |r2 - rc_mid| < rc_half covers (rc_lo, rc_hi) with a little to spare
@@ -935,7 +966,7 @@ __global__ void __launch_bounds__(224, 3)
     const float4 pi = st[self];
     const int ti = __float_as_int(pi.w);
     float hx = 0.f, hy = 0.f, hz = 0.f, lx = 0.f, ly = 0.f, lz = 0.f;
-    bool band_any = false;  // a padded-row chunk had a pair in the cutoff band
+    uint32_t bands = 0u;  // padded-row chunks with a pair in the cutoff band
     // energies (ENERGY): E, shifted E and the virial of the atom's pairs,
     // summed like the forces (FP32 within a 16-slot chunk, compensated
     // across chunks, widened to FP64 once per atom)
@@ -1046,7 +1077,7 @@ __global__ void __launch_bounds__(224, 3)
     };
     // 16 padded row slots; pairs in the band are added afterwards, each
     // decided in FP64 (rare: about one atom in 600 has one)
-    auto chunk16_fast = [&](auto&& get) {
+    auto chunk16_fast = [&](auto&& get, int chunk) {
       float ax = 0.f, ay = 0.f, az = 0.f, bx = 0.f, by = 0.f, bz = 0.f;
       bool band = false;
 #pragma unroll
@@ -1054,7 +1085,7 @@ __global__ void __launch_bounds__(224, 3)
         pair_fast(get(kk), ax, ay, az, band);
         pair_fast(get(kk + 1), bx, by, bz, band);
       }
-      band_any |= band;  // decided after the row (band_pass)
+      bands |= band_bit(band, chunk);  // decided after the row (band_pass)
       kahan_add(hx, lx, ax + bx);
       kahan_add(hy, ly, ay + by);
       kahan_add(hz, lz, az + bz);
@@ -1097,7 +1128,7 @@ __global__ void __launch_bounds__(224, 3)
         if (!fast)
           chunk16(get, L - t * kClusterTileSlots, wmax - t * kClusterTileSlots);
         else if (live)
-          chunk16_fast(get);
+          chunk16_fast(get, t);
         __syncwarp();  // the warp is done with buffer b
         if (lane == 0 && t + 2 < Tw) {
           fence_proxy_async();
@@ -1147,7 +1178,7 @@ __global__ void __launch_bounds__(224, 3)
         if (!fast)
           chunk16(get, L - t0, wmax - t0);
         else if (live)
-          chunk16_fast(get);
+          chunk16_fast(get, t0 / kClusterTileSlots);
       }
     } else if (!tripped) {
       const int L = live ? (int)a.len[p] : 0;
@@ -1184,7 +1215,7 @@ __global__ void __launch_bounds__(224, 3)
             if (!fast)
               chunk16(get, L - t * kClusterTileSlots, wrem);
             else if (live)
-              chunk16_fast(get);
+              chunk16_fast(get, t);
           }
         }
         // everyone is done with buffer b (and every wait succeeded)
@@ -1244,13 +1275,13 @@ __global__ void __launch_bounds__(224, 3)
       kept_new = kept;
       a.pos_build[p] = a.posf[p];
     }
-    if (fast && !tripped && live && band_any) {
+    if (fast && !tripped && live && bands) {
       LjParams lp;
       lp.s2[0] = s2_n, lp.s2[1] = s2_o, lp.s2[2] = s2_ng;
       lp.c24[0] = c_n, lp.c24[1] = c_o, lp.c24[2] = c_ng;
       lp.p = lj_p, lp.q = lj_q;
       const float3 e = band_pass<ALL_NG>(sh, st, a.pos, a.rcutsq, a.rows, a.ld, a.grouped, p,
-                                         (int)a.len[p], pi, rc_lo, rc_hi, lp);
+                                         bands, (int)a.len[p], pi, rc_lo, rc_hi, lp);
       kahan_add(hx, lx, e.x);
       kahan_add(hy, ly, e.y);
       kahan_add(hz, lz, e.z);
@@ -1394,7 +1425,7 @@ __device__ __forceinline__ void lean_checked(const SegShared& sh, const float4* 
 __device__ __noinline__ LeanSum lean_refresh(const SegShared& sh, const float4* st, const ClStep& a,
                                              int p, int self, float4 pi, LeanConst k) {
   LeanSum s = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0};
-  const bool minimg = sh.r.G == 1;
+  const bool minimg = sh.S.r.G == 1;
   int inchunk = 0;
   float cx = 0.f, cy = 0.f, cz = 0.f;
   walk_staged(sh, self, [&](int q) {
@@ -1467,13 +1498,22 @@ __global__ void __launch_bounds__(224, 4) k_lj_lean(const ClStep a) {
   const int tid = threadIdx.x;
   __shared__ SegShared sh;
   __shared__ __align__(8) uint64_t bar;
-  __shared__ int s_trip, s_seg;
+  __shared__ int s_trip, s_next;
+  // Before the launch this one depends on has finished (the step launches may
+  // start early, see launch_lj_cluster): only what a list build alone writes.
+  int sidx = blockIdx.x;  // the first segment; later ones from the counter
   if (tid == 0) {
-    s_trip = (a.skin[a.flag_read] | a.skin[3]) != 0;
     mbar_init(&bar, 1);
     fence_mbar_init();
   }
+  load_segment(sh, a.seg, sidx);
+  grid_wait();
+  if (tid == 0) {
+    s_trip = (a.skin[a.flag_read] | a.skin[3]) != 0;
+    if (blockIdx.x == 0 && a.sched_clear) *a.sched_clear = 0;
+  }
   __syncthreads();
+  grid_launch_dependents();
   const bool tripped = s_trip != 0;
   LeanConst k;
   k.rc_lo = a.lean_c[0];
@@ -1485,20 +1525,18 @@ __global__ void __launch_bounds__(224, 4) k_lj_lean(const ClStep a) {
   uint32_t phase = 0u;
   bool trip_next = false;
   for (;;) {
-    if (tid == 0) s_seg = atomicAdd(&a.sched[0], 1);
-    __syncthreads();
-    const int sidx = s_seg;
-    if (sidx >= a.nseg) break;
-    load_segment(sh, a.seg, a.reps, sidx);
-    __syncthreads();
+    // the next segment's number is on its way while this one computes; a grid
+    // with a block for every segment needs none
+    int next = a.nseg;
+    if (tid == 0 && (int)gridDim.x < a.nseg) next = gridDim.x + atomicAdd(a.sched, 1);
     if (!stage_bulk(sh, a.posf, st, &bar, phase, a.status, a.wait_limit)) break;
     phase ^= 1u;
     put_sentinel(st, sh.S.staged);
     if (tripped) fill_offsets(sh, a.start);
     __syncthreads();
-    const bool minimg = sh.r.G == 1;
-    k.Lf = sh.r.Lf;
-    k.invL = 1.0f / sh.r.Lf;
+    const bool minimg = sh.S.r.G == 1;
+    k.Lf = sh.S.r.Lf;
+    k.invL = 1.0f / sh.S.r.Lf;
     const int p1 = sh.S.p1;
     for (int base = sh.S.p0; base < p1; base += blockDim.x) {
       const int p = base + tid;
@@ -1534,7 +1572,7 @@ __global__ void __launch_bounds__(224, 4) k_lj_lean(const ClStep a) {
           n1 = __ldg(rp + gs);
         }
         const char* sb = reinterpret_cast<const char*>(st);
-        bool band_any = false;
+        uint32_t bands = 0u;
         for (int t0 = 0; t0 < wmax; t0 += kClusterTileSlots) {
           const uint4 w0 = n0, w1 = n1;
           if (t0 + kClusterTileSlots < wmax) {
@@ -1561,16 +1599,16 @@ __global__ void __launch_bounds__(224, 4) k_lj_lean(const ClStep a) {
             one(cw[w] & 0xFFFFu, ax, ay, az);
             one(cw[w] >> 16, bx, by, bz);
           }
-          band_any |= band;
+          bands |= band_bit(band, t0 / kClusterTileSlots);
           kahan_add(hx, lx, ax + bx);
           kahan_add(hy, ly, ay + by);
           kahan_add(hz, lz, az + bz);
         }
-        if (live && band_any) {
+        if (live && bands) {
           LjParams lp;
           lp.p = k.lj_p, lp.q = k.lj_q;
-          const float3 e = band_pass<true>(sh, st, a.pos, a.rcutsq, a.rows, a.ld, 1, p, L, pi,
-                                           k.rc_lo, k.rc_hi, lp);
+          const float3 e = band_pass<true>(sh, st, a.pos, a.rcutsq, a.rows, a.ld, 1, p, bands, L,
+                                           pi, k.rc_lo, k.rc_hi, lp);
           kahan_add(hx, lx, e.x);
           kahan_add(hy, ly, e.y);
           kahan_add(hz, lz, e.z);
@@ -1625,9 +1663,14 @@ __global__ void __launch_bounds__(224, 4) k_lj_lean(const ClStep a) {
         trip_next |= ddx * ddx + ddy * ddy + ddz * ddz > a.g.trip2;
       }
     }
+    if (tid == 0) s_next = next;
     __syncthreads();  // the next segment overwrites sh and the stage
+    sidx = s_next;
+    if (sidx >= a.nseg) break;
+    load_segment(sh, a.seg, sidx);
+    __syncthreads();
   }
-  if (tid == 0) {
+  if (!a.sched_clear && tid == 0) {
     __threadfence();
     if (atomicAdd(&a.sched[1], 1) == (int)gridDim.x - 1) {
       a.sched[0] = 0;
@@ -1648,11 +1691,11 @@ __global__ void __launch_bounds__(256)
                   const md_double4* __restrict__ pos, int nls, int* __restrict__ out,
                   signed char* __restrict__ img, int* __restrict__ nlargest) {
   __shared__ SegShared sh;
-  load_segment(sh, seg, reps, blockIdx.x);
+  load_segment(sh, seg, blockIdx.x);
   __syncthreads();
   fill_offsets(sh, start);
   __syncthreads();
-  const double L = sh.r.L;
+  const double L = sh.S.r.L;
   for (int p = sh.S.p0 + threadIdx.x; p < sh.S.p1; p += blockDim.x) {
     const int self = self_offset(sh, p);
     const size_t o = (size_t)orig[p] * nls;
@@ -1661,7 +1704,7 @@ __global__ void __launch_bounds__(256)
     walk_staged(sh, self, [&](int q) {
       int ix, iy, iz;
       const int j = staged_source(sh.S, q, ix, iy, iz);
-      if (sh.r.G == 1) {
+      if (sh.S.r.G == 1) {
         const md_double4 b = pos[j];
         ix = min_image(a.x, b.x, L);
         iy = min_image(a.y, b.y, L);
@@ -1836,9 +1879,9 @@ int cluster_build(ClusterList& cl, const std::vector<ClusterReplica>& reps_in, f
   }
   if (!cl.counters && (e = cudaMalloc(&cl.counters, sizeof(int) * 8)) != cudaSuccess) return e;
   if (!cl.sched) {
-    if ((e = cudaMalloc(&cl.sched, sizeof(int) * 2)) != cudaSuccess) return e;
-    cudaMemsetAsync(cl.sched, 0, sizeof(int) * 2, st);
+    if ((e = cudaMalloc(&cl.sched, sizeof(int) * 8)) != cudaSuccess) return e;
   }
+  cudaMemsetAsync(cl.sched, 0, sizeof(int) * 8, st);
   cudaMemsetAsync(cl.counters, 0, sizeof(int) * 8, st);
   cudaMemsetAsync(cl.count, 0, sizeof(int) * ((size_t)cl.ncells + 1), st);
   cudaMemsetAsync(cl.fill, 0, sizeof(int) * ((size_t)cl.ncells + 1), st);
@@ -2035,9 +2078,12 @@ void launch_lj_cluster(const ClusterForceArgs& f, bool energy, cudaStream_t st) 
       block_tiles ? nbuf * kClusterTileSlots * (size_t)(cl.block + 8) * sizeof(uint16_t)
                   : (cl.row_loads == 3 ? (size_t)(cl.block / 32) * 2 * kWarpTileBytes : 0);
   const size_t smem = tiles + stage_bytes(cl.max_staged);
+  // every-step launches of one species on grouped rows: the lean kernel
+  const bool lean = cl.grouped && f.all_ng && !energy;
   ClStep a;
   a.nseg = cl.nseg;
-  a.sched = cl.sched;
+  a.sched = f.in_steps && lean ? cl.sched + f.step % 3 : cl.sched + 4;
+  a.sched_clear = f.in_steps && lean ? cl.sched + (f.step + 1) % 3 : nullptr;
   a.seg = cl.seg;
   a.reps = cl.rep;
   a.start = cl.start;
@@ -2102,16 +2148,31 @@ void launch_lj_cluster(const ClusterForceArgs& f, bool energy, cudaStream_t st) 
     MDGB_CL_LAUNCH2(E, A, G, 2, cl.rmap_w);      \
   else                                           \
     MDGB_CL_LAUNCH2(E, A, G, 1, cl.rmap)
-  if (cl.grouped && f.all_ng && !energy) {
-    // every-step launches of one species on grouped rows: the lean kernel
+  if (lean) {
     const int gear = !f.gear ? 0 : (f.gear->correct_only ? 2 : 1);
     const size_t sm = stage_bytes(cl.max_staged);
+    // Launches of the step loop may start while the previous one drains
+    // (programmatic dependent launch): their blocks set up the segment and
+    // wait in the kernel for the previous launch to finish.
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.blockDim = cl.block;
+    cfg.dynamicSmemBytes = sm;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = f.in_steps ? 1 : 0;
+    auto launch = [&](auto kern) {
+      cfg.gridDim = grid_for((const void*)kern);
+      cudaLaunchKernelEx(&cfg, kern, a);
+    };
     if (gear == 1)
-      k_lj_lean<1><<<grid_for((const void*)k_lj_lean<1>), cl.block, sm, st>>>(a);
+      launch(k_lj_lean<1>);
     else if (gear == 2)
-      k_lj_lean<2><<<grid_for((const void*)k_lj_lean<2>), cl.block, sm, st>>>(a);
+      launch(k_lj_lean<2>);
     else
-      k_lj_lean<0><<<grid_for((const void*)k_lj_lean<0>), cl.block, sm, st>>>(a);
+      launch(k_lj_lean<0>);
   } else if (energy) {
     if (f.all_ng) { MDGB_CL_LAUNCH(true, true, 0); } else { MDGB_CL_LAUNCH(true, false, 0); }
   } else if (f.gear && f.gear->correct_only) {

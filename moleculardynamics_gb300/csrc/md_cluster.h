@@ -53,6 +53,7 @@ struct ClusterSegment {
   int img;           // some piece carries a periodic image
   int group[10];     // first piece of each (dx, dy) group (9 groups + end)
   ClusterPiece piece[kClusterMaxPieces];
+  ClusterReplica r;  // the replica, so that a block loads all it needs at once
 };
 
 struct ClusterList {
@@ -87,7 +88,7 @@ struct ClusterList {
   int Z = kClusterMaxZ;                           // cells per segment (upper bound)
   int block = 128;                                // threads per segment block (<= 224)
   int stage_cap = kClusterMaxStaged;              // staged atoms per segment (soft cap)
-  int row_loads = 1;                              // 1 block TMA tiles, 2 register prefetch,
+  int row_loads = 2;                              // 1 block TMA tiles, 2 register prefetch,
                                                   // 3 per-warp TMA tiles
   int grouped = 0;                                // rows grouped by eight slots with byte
                                                   // offsets (the register-prefetch scheme):
@@ -96,7 +97,10 @@ struct ClusterList {
   CUtensorMap rmap_w;                             // the same with per-warp boxes
   int rmap_ok = 0;
   int* counters = nullptr;                        // device: max staged, max len, entries, max cell
-  int* sched = nullptr;                           // device: persistent kernel's work counters
+  // device: work counters of the persistent kernels.  [0..2] step launches, by
+  // step mod 3 (the launch of step t clears the counter of t + 1); [4], [5]
+  // other launches: next segment, blocks finished (the last one clears both)
+  int* sched = nullptr;
   bool built = false;
   int version = 0;  // counts builds (each may change the order)
 };
@@ -139,6 +143,7 @@ struct ClusterForceArgs {
   const ClusterGearArgs* gear;  // NULL: forces only
   int* skin = nullptr;          // skin flags (NULL: the list's own)
   int wait_limit = 1 << 20;     // polls of a bounded mbarrier wait (0: give up at once)
+  bool in_steps = false;        // the step loop's launch of step `step` (one per step)
 };
 void launch_lj_cluster(const ClusterForceArgs& a, bool energy, cudaStream_t st);
 // inv[orig[p]] = p

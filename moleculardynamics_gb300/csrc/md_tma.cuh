@@ -120,6 +120,13 @@ __device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, i
                : "memory");
 }
 
+// Programmatic dependent launch: wait for the launches this one depends on
+// (no-op for a launch without the attribute); let the next one's blocks start
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_dependents() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // L2 prefetch of the line holding p (no register result, no wait)
 __device__ __forceinline__ void prefetch_l2(const void* p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
