@@ -61,9 +61,23 @@ __device__ __forceinline__ int wrapc(int c, int G, int& img) {
 
 __device__ __forceinline__ int zimg(int z, int G) { return z < 0 ? -1 : (z >= G ? 1 : 0); }
 
-// 1. wrap into [-L/2, L/2) and find the dense cell (the arithmetic of
-// md_neighbor.cu's periodic grid: x - L floor((x + L/2) / L), then
-// (int)((x + L/2) / cs) clamped to the grid); count atoms per cell
+// The exact cell arithmetic for one coordinate (md_neighbor.cu's periodic
+// grid): x - L floor((x + L/2) / L), then (int)((x + L/2) / cs) clamped to the
+// grid; -1 for a position that is no number.
+__device__ __noinline__ int wrap_cell_exact(double& x, double L, double cs, int G) {
+  const double h = L * 0.5;
+  x = xsub(x, xmul(floor(xdiv(xadd(x, h), L)), L));
+  const double s = xdiv(xadd(x, h), cs);
+  if (!(s >= 0.0 && s < 2.0e9)) return -1;
+  return min(__double2int_rz(s), G - 1);
+}
+
+// 1. wrap into [-L/2, L/2) and find the dense cell; count atoms per cell.  An
+// atom inside its box (nearly all between builds) needs no wrap, and a product
+// with 1/cs, within 2 ulp of the quotient, decides its cell unless it lies
+// within 2^-20 of an integer: one addition and one product on the FP64 pipe,
+// the rest by the bits (123 us per 1M atoms with comparisons, roundings and
+// conversions there).
 __global__ void k_cl_assign(md_double4* __restrict__ pos, int n, const ClusterReplica* reps,
                             int nrep, int* __restrict__ cell, int* __restrict__ count,
                             int* __restrict__ counters, int* __restrict__ status) {
@@ -73,36 +87,39 @@ __global__ void k_cl_assign(md_double4* __restrict__ pos, int n, const ClusterRe
   md_double4 p = pos[i];
   double x[3] = {p.x, p.y, p.z};
   const double h = r.L * 0.5;
+  const uint64_t lbits = (uint64_t)__double_as_longlong(r.L);
   int c[3];
-  bool bad = false;
+  bool bad = false, moved = false;
 #pragma unroll
   for (int d = 0; d < 3; d++) {
-    // floor((x + h) / L) and trunc((x + h) / cs) with the exact divisions,
-    // which GB300's narrow FP64 pipe makes costly: a product with the
-    // reciprocal (within 2 ulp of the quotient) decides unless the quotient
-    // lies within 1e-12 of an integer
     const double xa = xadd(x[d], h);
-    double q = 0.0;  // 0 <= x + L/2 < L: the rounded quotient lies in [0, 1)
-    if (!(xa >= 0.0 && xa < r.L)) {
-      const double qa = xa * r.invL;
-      q = fabs(qa - rint(qa)) > 1e-12 * fmax(1.0, fabs(qa)) ? floor(qa) : floor(xdiv(xa, r.L));
-      x[d] = xsub(x[d], xmul(q, r.L));
+    int cc = -1;
+    // 0 <= xa < L by the bit patterns (a negative number's is the larger)
+    if ((uint64_t)__double_as_longlong(xa) < lbits) {
+      const uint64_t b = (uint64_t)__double_as_longlong(xa * r.invcs);
+      const int sh = 1043 - (int)(b >> 52);  // s 2^32 = mantissa >> sh
+      const uint64_t m = (b & 0xFFFFFFFFFFFFFull) | (1ull << 52);
+      const uint64_t f = sh < 0 ? 0 : (sh > 63 ? 0 : m >> sh);
+      const uint32_t frac = (uint32_t)f;
+      if (sh >= 0 && frac - 4096u < 0xFFFFE000u) cc = min((int)(f >> 32), r.G - 1);
     }
-    const double xb = q == 0.0 ? xa : xadd(x[d], h);
-    const double sa = xb * r.invcs;
-    double s = fabs(sa - rint(sa)) > 1e-12 * fmax(1.0, fabs(sa)) ? sa : xdiv(xb, r.cs);
-    if (!(s >= 0.0 && s < 2.0e9)) {
-      bad = true;
-      s = 0.0;
+    if (cc < 0) {
+      cc = wrap_cell_exact(x[d], r.L, r.cs, r.G);
+      moved = true;
+      if (cc < 0) {
+        bad = true;
+        cc = 0;
+      }
     }
-    const int cc = __double2int_rz(s);
-    c[d] = cc >= r.G ? r.G - 1 : cc;
+    c[d] = cc;
   }
   if (bad) atomicOr(status, ST_NONFINITE);
-  p.x = x[0];
-  p.y = x[1];
-  p.z = x[2];
-  pos[i] = p;
+  if (moved) {
+    p.x = x[0];
+    p.y = x[1];
+    p.z = x[2];
+    pos[i] = p;
+  }
   const int id = r.G == 1 ? r.cell0 : cid(r, c[0], c[1], c[2]);
   cell[i] = id;
   const int old = atomicAdd(&count[id], 1);
@@ -135,30 +152,33 @@ __global__ void k_cl_rank(const int* __restrict__ unsorted, const int* __restric
   perm[lo + rank] = a;
 }
 
-template <typename T>
-__global__ void k_gather(const T* __restrict__ src, T* __restrict__ dst,
-                         const int* __restrict__ perm, int n) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p < n) dst[p] = src[perm[p]];
-}
-
-__global__ void k_gather3(const double* __restrict__ src, double* __restrict__ dst,
-                          const int* __restrict__ perm, int n) {
+// 2. the state into cell order, with the FP32 copies of the positions
+struct Permute {
+  const md_double4* pos;
+  md_double4* pos_out;
+  const double* v3[5];  // NULL: not there
+  double* v3_out[5];
+  const int* orig;
+  int* orig_out;
+  float4 *pb, *posf;
+};
+__global__ void k_cl_permute(const __grid_constant__ Permute a, const int* __restrict__ perm,
+                             int n) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n) return;
-  const int a = perm[p];
+  const int s = perm[p];
+  const md_double4 r = a.pos[s];
+  a.pos_out[p] = r;
+  a.orig_out[p] = a.orig[s];
+  const float4 f = make_float4((float)r.x, (float)r.y, (float)r.z, __int_as_float((int)r.w));
+  a.pb[p] = f;
+  a.posf[p] = f;
 #pragma unroll
-  for (int d = 0; d < 3; d++) dst[3 * p + d] = src[3 * a + d];
-}
-
-__global__ void k_cl_posf(const md_double4* __restrict__ pos, float4* __restrict__ pb,
-                          float4* __restrict__ posf, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const md_double4 p = pos[i];
-  const float4 v = make_float4((float)p.x, (float)p.y, (float)p.z, __int_as_float((int)p.w));
-  pb[i] = v;
-  posf[i] = v;
+  for (int k = 0; k < 5; k++)
+    if (a.v3[k]) {
+#pragma unroll
+      for (int d = 0; d < 3; d++) a.v3_out[k][3 * (size_t)p + d] = a.v3[k][3 * (size_t)s + d];
+    }
 }
 
 // 3a. greedy cut of each z-column: a segment starts at z = 0 and wherever
@@ -234,16 +254,25 @@ __global__ void k_seg_emit(const ClusterReplica* __restrict__ reps, int nrep, in
 }
 
 // 3c. pieces of each segment: for each (dx, dy) group the z range
-// cz0-1 .. cz1+1, split where the periodic image changes
+// cz0-1 .. cz1+1, split where the periodic image changes.  A warp per segment,
+// a group (up to three pieces) per lane.  The first thread also leaves the
+// segment count and the status beside the counters for the host's one copy.
 __global__ void k_cl_segments(ClusterSegment* __restrict__ seg, const int* __restrict__ nseg_dev,
                               const ClusterReplica* __restrict__ reps,
-                              const int* __restrict__ start, int* __restrict__ counters) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+                              const int* __restrict__ start, int* __restrict__ counters,
+                              const int* __restrict__ status) {
+  const int s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int g = threadIdx.x & 31;
+  if (s == 0 && g == 0) {
+    counters[5] = *nseg_dev;
+    counters[6] = *status;
+  }
   if (s >= *nseg_dev) return;
   ClusterSegment& S = seg[s];
   const ClusterReplica r = reps[S.rep];
-  S.r = r;
   if (r.G == 1) {
+    if (g) return;
+    S.r = r;
     ClusterPiece pc;
     pc.src = start[r.cell0];
     pc.count = start[r.cell0 + 1] - pc.src;
@@ -252,7 +281,7 @@ __global__ void k_cl_segments(ClusterSegment* __restrict__ seg, const int* __res
     S.p0 = pc.src;
     S.p1 = pc.src + pc.count;
     S.piece[0] = pc;
-    for (int g = 0; g < 10; g++) S.group[g] = g == 9 ? 1 : 0;
+    for (int k = 0; k < 10; k++) S.group[k] = k == 9 ? 1 : 0;
     S.npieces = 1;
     S.staged = pc.count;
     S.self0 = 0;
@@ -260,46 +289,68 @@ __global__ void k_cl_segments(ClusterSegment* __restrict__ seg, const int* __res
     atomicMax(&counters[0], S.staged);
     return;
   }
-  const int G = r.G;
-  S.p0 = start[cid(r, S.cx, S.cy, S.cz0)];
-  S.p1 = start[cid(r, S.cx, S.cy, S.cz1) + 1];
-  int np = 0, dst = 0;
-  for (int dx = -1; dx < 2; dx++)
-    for (int dy = -1; dy < 2; dy++) {
-      S.group[(dx + 1) * 3 + (dy + 1)] = np;
-      int ix, iy;
-      const int cx = wrapc(S.cx + dx, G, ix), cy = wrapc(S.cy + dy, G, iy);
-      const int zend = S.cz1 + 1;
-      for (int z = S.cz0 - 1; z <= zend;) {
-        const int iz = zimg(z, G);
-        int zb = z;
-        while (zb + 1 <= zend && zimg(zb + 1, G) == iz) zb++;
-        ClusterPiece pc;
-        pc.src = start[cid(r, cx, cy, z - iz * G)];
-        pc.count = start[cid(r, cx, cy, zb - iz * G) + 1] - pc.src;
-        pc.dst = dst;
-        pc.ix = (signed char)ix;
-        pc.iy = (signed char)iy;
-        pc.iz = (signed char)iz;
-        pc.pad = 0;
-        S.piece[np++] = pc;
-        dst += pc.count;
-        z = zb + 1;
-      }
+  const int G = r.G, cx0 = S.cx, cy0 = S.cy, cz0 = S.cz0, cz1 = S.cz1;
+  ClusterPiece pc[3];
+  int np = 0, atoms = 0, img = 0;
+  if (g < 9) {
+    int ix, iy;
+    const int cx = wrapc(cx0 + g / 3 - 1, G, ix), cy = wrapc(cy0 + g % 3 - 1, G, iy);
+    // the z range below, inside and above the box
+#pragma unroll
+    for (int iz = -1; iz < 2; iz++) {
+      const int lo = max(cz0 - 1, iz * G), hi = min(cz1 + 1, iz * G + G - 1);
+      if (lo > hi) continue;
+      ClusterPiece q;
+      q.src = start[cid(r, cx, cy, lo - iz * G)];
+      q.count = start[cid(r, cx, cy, hi - iz * G) + 1] - q.src;
+      q.dst = atoms;
+      q.ix = (signed char)ix;
+      q.iy = (signed char)iy;
+      q.iz = (signed char)iz;
+      q.pad = 0;
+      if (np == 0) pc[0] = q;
+      if (np == 1) pc[1] = q;
+      if (np == 2) pc[2] = q;
+      np++;
+      atoms += q.count;
+      img |= ix | iy | iz;
     }
-  S.group[9] = np;
-  S.npieces = np;
-  S.staged = dst;
-  // own cells cz0..cz1 lie in the image-free piece of the (0, 0) group
-  int s0 = 0, img = 0;
-  for (int k = 0; k < np; k++) {
-    const ClusterPiece& pc = S.piece[k];
-    if (k >= S.group[4] && k < S.group[5] && pc.iz == 0) s0 = pc.dst + (S.p0 - pc.src);
-    img |= pc.ix | pc.iy | pc.iz;
   }
-  S.self0 = s0;
-  S.img = img != 0;
-  atomicMax(&counters[0], dst);
+  int first = np, dst = atoms;  // inclusive, then exclusive, over the groups
+#pragma unroll
+  for (int o = 1; o < 16; o <<= 1) {
+    const int a = __shfl_up_sync(0xffffffffu, first, o), b = __shfl_up_sync(0xffffffffu, dst, o);
+    if (g >= o) {
+      first += a;
+      dst += b;
+    }
+  }
+  const int pieces = __shfl_sync(0xffffffffu, first, 8), staged = __shfl_sync(0xffffffffu, dst, 8);
+  first -= np;
+  dst -= atoms;
+  const bool any = __any_sync(0xffffffffu, img != 0);
+  const int p0 = start[cid(r, cx0, cy0, cz0)];
+  if (g < 9) {
+    S.group[g] = first;
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+      if (k < np) {
+        pc[k].dst += dst;
+        S.piece[first + k] = pc[k];
+        // own cells cz0..cz1 lie in the image-free piece of the (0, 0) group
+        if (g == 4 && pc[k].iz == 0) S.self0 = pc[k].dst + (p0 - pc[k].src);
+      }
+  }
+  if (g == 0) {
+    S.r = r;
+    S.p0 = p0;
+    S.p1 = start[cid(r, cx0, cy0, cz1) + 1];
+    S.group[9] = pieces;
+    S.npieces = pieces;
+    S.staged = staged;
+    S.img = any;
+    atomicMax(&counters[0], staged);
+  }
 }
 
 // ---- per-block segment context in shared memory ----
@@ -538,7 +589,7 @@ __device__ __forceinline__ void put_sentinel(float4* st, int staged) {
   if (threadIdx.x == 0) st[staged] = make_float4(1e18f, 1e18f, 1e18f, __int_as_float(SP_NG));
 }
 
-constexpr int kRowStep = 8;  // staged candidates tested per step of the row walk
+constexpr int kRowStep = 8;  // independent distance tests of the row walk
 
 // 4. compact rows from the build-time positions (MODE 0: count, 1: write,
 // 2: both, rows longer than cap truncated and reported through the counters)
@@ -565,48 +616,49 @@ __global__ void __launch_bounds__(256)
     int kept = 0;
     GroupWriter gw;
     if (live && !minimg) {
-      // the 9 column groups in row order, kRowStep independent distance
-      // tests per step; only the centre group holds the atom itself
+      // the 9 column groups in row order, 32 staged candidates at a time: their
+      // distance tests give a mask without a branch, then the kept ones (a
+      // tenth) are appended.  Only the centre group holds the atom itself.
       const int self = self_offset(sh, p);
       const float4 pi = st[self];
       const int zspan = sh.S.cz1 - sh.S.cz0 + 3;
       int w = 1;
       while (w < zspan - 2 && sh.off[4][w + 1] <= self) w++;
       const int u = w - 1;
-      auto near = [&](int q) {
-        const float4 pj = st[q];
-        const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-        return dx * dx + dy * dy + dz * dz < rv2;
-      };
-      auto take = [&](int q, bool in) {
-        if (in) {
-          if (MODE != 0) {
-            if (grouped)
-              gw.push(rows, ld, cap, p, (uint32_t)q << 4);
-            else if (kept < cap)
-              rows[(size_t)kept * ld + p] = (uint16_t)q;
-          }
-          kept++;
-        }
-      };
-      auto group = [&](int g, auto centre) {
+#pragma unroll 1
+      for (int g = 0; g < 9; g++) {
         const int qa = sh.off[g][u], qb = sh.off[g][u + 3];
-        int q = qa;
-        for (; q + kRowStep <= qb; q += kRowStep) {
-          bool in[kRowStep];
+#pragma unroll 1
+        for (int q = qa; q < qb; q += 32) {
+          uint32_t m = 0;
+          const int left = qb - q;
+#pragma unroll 1
+          for (int v = 0; v < 32 && v < left; v += kRowStep) {
+            uint32_t b = 0;
 #pragma unroll
-          for (int u = 0; u < kRowStep; u++)
-            in[u] = near(q + u) && (!decltype(centre)::value || q + u != self);
-#pragma unroll
-          for (int u = 0; u < kRowStep; u++) take(q + u, in[u]);
+            for (int x = 0; x < kRowStep; x++) {
+              const float4 pj = st[min(q + v + x, qb - 1)];
+              const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+              b |= (uint32_t)(dx * dx + dy * dy + dz * dz < rv2) << x;
+            }
+            m |= b << v;
+          }
+          if (left < 32) m &= (1u << left) - 1u;
+          if ((uint32_t)(self - q) < 32u) m &= ~(1u << (self - q));
+          if (MODE == 0) {
+            kept += __popc(m);
+          } else {
+            for (; m; m &= m - 1) {
+              const int k = q + __ffs(m) - 1;
+              if (grouped)
+                gw.push(rows, ld, cap, p, (uint32_t)k << 4);
+              else if (kept < cap)
+                rows[(size_t)kept * ld + p] = (uint16_t)k;
+              kept++;
+            }
+          }
         }
-        for (; q < qb; q++) take(q, near(q) && (!decltype(centre)::value || q != self));
-      };
-#pragma unroll 1
-      for (int g = 0; g < 4; g++) group(g, std::false_type());
-      group(4, std::true_type());
-#pragma unroll 1
-      for (int g = 5; g < 9; g++) group(g, std::false_type());
+      }
     } else if (live) {
       const int self = self_offset(sh, p);
       const float4 pi = st[self];
@@ -1893,17 +1945,22 @@ int cluster_build(ClusterList& cl, const std::vector<ClusterReplica>& reps_in, f
   if (n > 0) {
     k_cl_scatter<<<nb(n, T), T, 0, st>>>(cl.cell, n, cl.start, cl.fill, cl.unsorted);
     k_cl_rank<<<nb(n, T), T, 0, st>>>(cl.unsorted, cl.cell, cl.orig, n, cl.start, cl.perm);
-    // permute the state into cell order
-    k_gather<md_double4><<<nb(n, T), T, 0, st>>>(*pos, cl.pos_tmp, cl.perm, n);
-    std::swap(*pos, cl.pos_tmp);
+    Permute a{};
+    a.pos = *pos;
+    a.pos_out = cl.pos_tmp;
     for (int k = 0; k < 5; k++)
       if (v3[k] && *v3[k]) {
-        k_gather3<<<nb(n, T), T, 0, st>>>(*v3[k], cl.v3_tmp[k], cl.perm, n);
+        a.v3[k] = *v3[k];
+        a.v3_out[k] = cl.v3_tmp[k];
         std::swap(*v3[k], cl.v3_tmp[k]);
       }
-    k_gather<int><<<nb(n, T), T, 0, st>>>(cl.orig, cl.itmp, cl.perm, n);
+    a.orig = cl.orig;
+    a.orig_out = cl.itmp;
+    a.pb = cl.pos_build;
+    a.posf = posf;
+    k_cl_permute<<<nb(n, T), T, 0, st>>>(a, cl.perm, n);
+    std::swap(*pos, cl.pos_tmp);
     std::swap(cl.orig, cl.itmp);
-    k_cl_posf<<<nb(n, T), T, 0, st>>>(*pos, cl.pos_build, posf, n);
   }
   // segments: greedy cut of the columns (fill is free again and holds the flags)
   const int zmax = std::max(1, std::min(cl.Z, kClusterMaxZ));
@@ -1913,14 +1970,12 @@ int cluster_build(ClusterList& cl, const std::vector<ClusterReplica>& reps_in, f
   if ((e = scan_exclusive(cl.fill, cl.segidx, cl.ncells + 1, sc, st)) != cudaSuccess) return e;
   k_seg_emit<<<nb(cl.ncells, 256), 256, 0, st>>>(cl.rep, cl.nrep, cl.ncells, cl.fill, cl.segidx,
                                                  cl.seg);
-  k_cl_segments<<<nb(cl.ncells, 128), 128, 0, st>>>(cl.seg, cl.segidx + cl.ncells, cl.rep,
-                                                    cl.start, cl.counters);
-  int hc[8];
-  int status = 0, nseg = 0;
-  cudaMemcpyAsync(hc, cl.counters, sizeof(hc), cudaMemcpyDeviceToHost, st);
-  cudaMemcpyAsync(&status, d_status, sizeof(int), cudaMemcpyDeviceToHost, st);
-  cudaMemcpyAsync(&nseg, cl.segidx + cl.ncells, sizeof(int), cudaMemcpyDeviceToHost, st);
+  k_cl_segments<<<nb(cl.ncells, 4), 128, 0, st>>>(cl.seg, cl.segidx + cl.ncells, cl.rep,
+                                                  cl.start, cl.counters, d_status);
+  int* hc = sc.host;
+  cudaMemcpyAsync(hc, cl.counters, sizeof(int) * 8, cudaMemcpyDeviceToHost, st);
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
+  const int nseg = hc[5], status = hc[6];
   if (status & ST_NONFINITE) {
     err = "non-finite position at list build";
     return -1;
@@ -1994,7 +2049,7 @@ int cluster_build(ClusterList& cl, const std::vector<ClusterReplica>& reps_in, f
       k_cl_rows<0><<<cl.nseg, cl.block, smem, st>>>(cl.seg, cl.rep, cl.start, cl.pos_build, cl.rv2,
                                                nullptr, cl.len, cl.ld, 0, cl.counters, 0);
   }
-  cudaMemcpyAsync(hc, cl.counters, sizeof(hc), cudaMemcpyDeviceToHost, st);
+  cudaMemcpyAsync(hc, cl.counters, sizeof(int) * 8, cudaMemcpyDeviceToHost, st);
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
   cl.maxlen = hc[1];
   {

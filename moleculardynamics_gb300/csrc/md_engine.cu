@@ -518,25 +518,32 @@ void leave_cluster(md_ctx* c) {
 // readyList + buildList for the lists due at step t (Host.cpp:143-152)
 md_status rebuild(md_ctx* c, int t) {
   Timed tm(c, 4);
-  unsigned long long um[2];
+  // the largest squared speed and coordinate, the status and the skin flags of
+  // the list in use: one wait
+  const bool cl_due = c->cluster && c->cfg.use_lj && (c->lj_next == t || c->cfg.periodic);
+  const bool lj_due = !c->cluster && c->cfg.use_lj && (c->lj_next == t || c->cfg.periodic);
+  const int* skin = cl_due ? c->cl.skin : (lj_due ? c->lj.skin : nullptr);
+  int* const host = c->sc.host;
   launch_ready(c->pos, c->vel, c->n, c->sc.umax, c->status, c->st);
-  CK(cudaMemcpyAsync(um, c->sc.umax, sizeof(um), cudaMemcpyDeviceToHost, c->st), "ready");
-  int s = 0;
-  CK(cudaMemcpyAsync(&s, c->status, sizeof(int), cudaMemcpyDeviceToHost, c->st), "ready");
+  CK(cudaMemcpyAsync(host, c->sc.umax, 16, cudaMemcpyDeviceToHost, c->st), "ready");
+  CK(cudaMemcpyAsync(host + 4, c->status, sizeof(int), cudaMemcpyDeviceToHost, c->st), "ready");
+  if (skin)
+    CK(cudaMemcpyAsync(host + 8, skin, sizeof(int) * 5, cudaMemcpyDeviceToHost, c->st), "skin");
   CK(cudaStreamSynchronize(c->st), "ready");
   c->stats.launches += 1;
-  if (s & ST_NONFINITE) return fail(c, MD_NONFINITE, "non-finite position or velocity");
+  if (host[4] & ST_NONFINITE) return fail(c, MD_NONFINITE, "non-finite position or velocity");
   double vmax, maxabs;
-  memcpy(&vmax, &um[0], 8);
-  memcpy(&maxabs, &um[1], 8);
+  memcpy(&vmax, host, 8);
+  memcpy(&maxabs, host + 2, 8);
+  vmax = sqrt(vmax);  // rounded like each atom's root, which it is the largest of
+  int sk[5];
+  memcpy(sk, host + 8, sizeof(sk));
   const double box_list = maxabs * 2;
   const bool both = c->cfg.periodic != 0;
   const double dt = (double)c->cfg.dt;
   bool did_lj = false;
   if (c->cluster && c->cfg.use_lj && (c->lj_next == t || both)) {
     if (c->cl.skin) {
-      int sk[5];
-      CK(cudaMemcpy(sk, c->cl.skin, sizeof(sk), cudaMemcpyDeviceToHost), "skin");
       c->stats.list_trips += sk[4];
       if (sk[3]) c->cl.headroom *= 1.5f;  // a refreshed row did not fit: more room
       CK(cudaMemsetAsync(c->cl.skin + 4, 0, sizeof(int), c->st), "skin");
@@ -572,9 +579,7 @@ md_status rebuild(md_ctx* c, int t) {
     }
   }
   if (c->cfg.use_lj && (c->lj_next == t || both)) {
-    if (c->lj.skin) {
-      int sk[5];
-      CK(cudaMemcpy(sk, c->lj.skin, sizeof(sk), cudaMemcpyDeviceToHost), "skin");
+    if (c->lj.skin && skin == c->lj.skin) {
       c->stats.list_trips += sk[4];
       if (sk[3]) c->lj.headroom *= 1.5f;  // a refreshed row did not fit: more room
       CK(cudaMemsetAsync(c->lj.skin + 4, 0, sizeof(int), c->st), "skin");
@@ -1120,6 +1125,8 @@ md_status md_create(const md_config* cfg, md_ctx** out) {
   if ((e = cudaMemset(c->status, 0, sizeof(int) * kStatusInts)) != cudaSuccess) return bail(e, "flags");
   if ((e = cudaMalloc(&c->sc.dpart, sizeof(double) * (8 * 1024 + 64))) != cudaSuccess)
     return bail(e, "scratch");
+  if ((e = cudaMallocHost(&c->sc.host, sizeof(int) * 32)) != cudaSuccess)
+    return bail(e, "scratch");
   if ((e = cudaMalloc(&c->sc.umax, sizeof(unsigned long long) * 4)) != cudaSuccess)
     return bail(e, "scratch");
   if ((e = cudaMalloc(&c->sc.counts, sizeof(int) * 8)) != cudaSuccess) return bail(e, "scratch");
@@ -1152,6 +1159,7 @@ void md_destroy(md_ctx* c) {
                   c->sc.dpart, c->sc.umax, c->sc.counts, c->sc.block_sums};
   for (void* p : ptrs)
     if (p) cudaFree(p);
+  if (c->sc.host) cudaFreeHost(c->sc.host);
   for (auto& p : c->pending) {
     cudaEventDestroy(p.second.first);
     cudaEventDestroy(p.second.second);

@@ -138,14 +138,31 @@ __global__ void k_wall_accel(const md_double4* __restrict__ pos, double* __restr
   for (int d = 0; d < 3; d++) acc[3 * i + d] = xdiv(f3[3 * i + d], mass);
 }
 
-// cpu/common/Device.cpp:125-133
+// quotients by the three masses (div_mass)
+struct MassDiv {
+  double m[3];
+  uint64_t y[3];
+};
+static MassDiv mass_div(const Species& sp) {
+  MassDiv d;
+  for (int t = 0; t < 3; t++) {
+    d.m[t] = (double)sp.mass[t];
+    uint64_t b;
+    memcpy(&b, &d.m[t], sizeof(b));
+    d.y[t] = divisor_fraction(b);
+  }
+  return d;
+}
+
+// cpu/common/Device.cpp:125-133, a component per thread
 __global__ void k_accel(const md_double4* __restrict__ pos, double* __restrict__ acc,
-                        const double* __restrict__ f3, int n, Species sp) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double mass = mass_of((int)pos[i].w, sp);
-#pragma unroll
-  for (int d = 0; d < 3; d++) acc[3 * i + d] = xdiv(f3[3 * i + d], mass);
+                        const double* __restrict__ f3, int m, const __grid_constant__ MassDiv md) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= m) return;
+  const int type = (int)pos[k / 3].w;
+  const int t = type == SP_N ? 0 : (type == SP_O ? 1 : 2);
+  acc[k] = div_mass(f3[k], t == 0 ? md.m[0] : (t == 1 ? md.m[1] : md.m[2]),
+                    t == 0 ? md.y[0] : (t == 1 ? md.y[1] : md.y[2]));
 }
 
 __global__ void k_posf(const md_double4* __restrict__ pos, float4* __restrict__ posf, int n) {
@@ -164,31 +181,31 @@ __device__ __forceinline__ unsigned long long warp_umax(unsigned long long v) {
   return v;
 }
 
-// cpu/cpumd/Host.cpp:245-271 (max over atoms is exact in any order)
+// cpu/cpumd/Host.cpp:245-271: the largest squared speed (its root is the
+// largest speed: rounding keeps the order) and the largest coordinate, by the
+// bit patterns of non-negative numbers
 __global__ void k_ready(const md_double4* __restrict__ pos, const double* __restrict__ vel,
                         int n, unsigned long long* umax, int* status) {
+  constexpr unsigned long long kInf = 0x7FF0000000000000ull, kAbs = ~(1ull << 63);
   unsigned long long vm = 0, bm = 0;
-  bool bad = false;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const double vx = vel[3 * i], vy = vel[3 * i + 1], vz = vel[3 * i + 2];
-    double s = sqrt(norm2_exact(vx, vy, vz));
-    md_double4 p = pos[i];
-    double b = fmax(fabs(p.x), fmax(fabs(p.y), fabs(p.z)));
-    if (!(isfinite(s) && isfinite(b))) {
-      bad = true;
-      continue;
-    }
-    unsigned long long us = __double_as_longlong(s), ub = __double_as_longlong(b);
-    vm = us > vm ? us : vm;
-    bm = ub > bm ? ub : bm;
+    const double s = norm2_exact(vel[3 * i], vel[3 * i + 1], vel[3 * i + 2]);
+    const md_double4 p = pos[i];
+    const unsigned long long us = __double_as_longlong(s) & kAbs;
+    const unsigned long long x = __double_as_longlong(p.x) & kAbs,
+                             y = __double_as_longlong(p.y) & kAbs,
+                             z = __double_as_longlong(p.z) & kAbs;
+    const unsigned long long ub = max(x, max(y, z));
+    vm = max(vm, us);
+    bm = max(bm, ub);
   }
   vm = warp_umax(vm);
   bm = warp_umax(bm);
   if ((threadIdx.x & 31) == 0) {
     atomicMax(&umax[0], vm);
     atomicMax(&umax[1], bm);
+    if (vm >= kInf || bm >= kInf) atomicOr(status, ST_NONFINITE);
   }
-  if (bad) atomicOr(status, ST_NONFINITE);
 }
 
 constexpr int kRedBlocks = 1024;
@@ -787,11 +804,10 @@ void gear64_args(const GearArgs& a, md_double4* pos_next, bool predict, Gear64& 
   g.b = a.b;
   g.c = a.c;
   g.k = a.k;
+  const MassDiv d = mass_div(a.sp);
   for (int t = 0; t < 3; t++) {
-    g.mass[t] = (double)a.sp.mass[t];
-    uint64_t b;
-    memcpy(&b, &g.mass[t], sizeof(b));
-    g.ymass[t] = divisor_fraction(b);
+    g.mass[t] = d.m[t];
+    g.ymass[t] = d.y[t];
   }
   g.npos = a.npos;
   g.energy_loss = (double)a.energy_loss;
@@ -848,7 +864,8 @@ void launch_wall_redo(const GearArgs& a, const int* hit, int* hits, int* flag_ne
 }
 void launch_accel(const md_double4* pos, double* acc, const double* f3, int n, Species sp,
                   cudaStream_t st) {
-  if (n > 0) k_accel<<<nblk(n, 256), 256, 0, st>>>(pos, acc, f3, n, sp);
+  if (n > 0)  // kMaxAtoms x 3 fits an int
+    k_accel<<<nblk(3LL * n, 256), 256, 0, st>>>(pos, acc, f3, 3 * n, mass_div(sp));
 }
 void launch_posf(const md_double4* pos, float4* posf, int n, cudaStream_t st) {
   if (n > 0) k_posf<<<nblk(n, 256), 256, 0, st>>>(pos, posf, n);

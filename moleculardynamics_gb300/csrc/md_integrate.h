@@ -48,7 +48,7 @@ void gear64_args(const GearArgs& a, md_double4* pos_next, bool predict, Gear64& 
 void launch_accel(const md_double4* pos, double* acc, const double* f3, int n, Species sp,
                   cudaStream_t st);
 void launch_posf(const md_double4* pos, float4* posf, int n, cudaStream_t st);
-// max |v| and max |coordinate| (cpu/cpumd/Host.cpp:245-271) into umax[0..1]
+// max |v|^2 and max |coordinate| (cpu/cpumd/Host.cpp:245-271) into umax[0..1]
 // as the bit patterns of non-negative doubles; sets ST_NONFINITE.
 void launch_ready(const md_double4* pos, const double* vel, int n, unsigned long long* umax,
                   int* status, cudaStream_t st);

@@ -64,6 +64,7 @@ struct NeighborList {
 
 // Scratch shared by reductions.
 struct Scratch {
+  int* host = nullptr;      // 32 ints of page-locked memory for the builds' read-backs
   double* dpart = nullptr;  // per-block partial sums
   int dpart_cap = 0;
   unsigned long long* umax = nullptr;  // 4 max slots

@@ -410,6 +410,10 @@ cudaError_t scan_exclusive(const int* in, int* out, int n, Scratch& sc, cudaStre
     if (e != cudaSuccess) return e;
     sc.block_sums_cap = 2 * tiles + 2;
   }
+  if (tiles == 1) {
+    k_scan_tiles<<<1, kScanThreads, 0, st>>>(in, out, n, nullptr);
+    return cudaGetLastError();
+  }
   int* sums = sc.block_sums;
   int* pre = sc.block_sums + tiles + 1;
   k_scan_tiles<<<tiles, kScanThreads, 0, st>>>(in, out, n, sums);
