@@ -21,6 +21,7 @@
 #include <type_traits>
 
 #include "md_exact64.cuh"
+#include "md_fixed64.cuh"
 #include "md_forces.h"
 #include "md_gear64.cuh"
 #include "md_neighbor.cuh"
@@ -805,41 +806,54 @@ __device__ __forceinline__ void mb_angular(double c, double& g, double& gpre) {
 }
 
 // Neighbours of the block's atom i (up to 32 of its short list), in shared
-// memory: the vector r_i - r_s, the distance, its reciprocal, the unit vector
-// and the cutoff, and as the partner j of a bond the pair terms.
+// memory: the vector r_i - r_s, the unit vector, the distance, its reciprocal
+// and the cutoff; as the partner j of a bond the pair terms.
 struct Nb {
-  double d[3][32], u[3][32], r[32], ir[32], fc[32], dfc[32];
-  double E[32], va[32], dva[32], dv[32], v0[32];  // pair terms: E, Va, Va', Vr' + Vdw', Vr + Vdw
-  int id[32];
+  double d[3][32], u[3][32];
+  q56 qu[3][32], qr[32], qir[32], qfc[32], qdm[32];  // fixed point; qdm: -dfc
   // bit 6: not a third body of i's bonds (NG), 7: not a bond (NG, or beyond
-  // the pair cutoff); bits 0-2: in the cell below i's along x, y, z, 3-5: above
+  // the pair cutoff), 8: its distance is outside the fixed point's range;
+  // bits 0-2: in the cell below i's along x, y, z, 3-5: above
   int flag[32];
 };
-constexpr int kNbNoThird = 64, kNbNoBond = 128;
+// pair terms: E, Va, Va', Vr' + Vdw', Vr + Vdw
+struct NbPair {
+  double E[32], va[32], dva[32], dv[32], v0[32];
+};
+constexpr int kNbNoThird = 64, kNbNoBond = 128, kNbFar = 256;
 
-// one neighbour per thread (tid < 32)
-template <bool PAIR>
-__device__ __forceinline__ void mb_stage(Nb& N, int q, uint32_t e, double xi, double yi, double zi, int ti,
-                                         const md_double4* pos, const float4* posf, const Grid& g,
-                                         const int* cell3, int i) {
+// squared distances that the fixed-point terms take (0.5 .. 8 angstrom; 16 between
+// two neighbours)
+__device__ __forceinline__ bool mb_in_range(double r2, double most) { return r2 >= 0.25 && r2 < most; }
+
+// neighbour q by one thread
+__device__ __forceinline__ void mb_stage(Nb& N, int q, uint32_t e, double xi, double yi, double zi,
+                                         const md_double4* pos, const Grid& g, const int* cell3,
+                                         int i) {
   const int j = entry_index(e);
   double x, y, z;
   int tj;
-  PosT<double>::load(pos, posf, j, x, y, z, tj);
+  PosT<double>::load(pos, nullptr, j, x, y, z, tj);
   PosT<double>::image(x, y, z, e, g);
   const double dx = xi - x, dy = yi - y, dz = zi - z;
   const double r2 = dx * dx + dy * dy + dz * dz;
-  const double ir = rsqrt64(r2), r = r2 * ir;
-  double fc, dfc;
-  mb_cutoff(r, fc, dfc);
+  const double ir = rsqrt64(r2);
   N.d[0][q] = dx, N.d[1][q] = dy, N.d[2][q] = dz;
-  N.u[0][q] = dx * ir, N.u[1][q] = dy * ir, N.u[2][q] = dz * ir;
-  N.r[q] = r;
-  N.ir[q] = ir;
-  N.fc[q] = fc;
-  N.dfc[q] = dfc;
-  N.id[q] = j;
+  const double ux = dx * ir, uy = dy * ir, uz = dz * ir;
+  N.u[0][q] = ux, N.u[1][q] = uy, N.u[2][q] = uz;
   int flag = tj == SP_NG ? kNbNoThird | kNbNoBond : 0;
+  if (mb_in_range(r2, 64.0)) {
+    q56 fc, dm;
+    const q56 r = toq(r2 * ir);
+    N.qu[0][q] = toq(ux), N.qu[1][q] = toq(uy), N.qu[2][q] = toq(uz);
+    N.qr[q] = r;
+    N.qir[q] = toq(ir);
+    cutoffq(r, fc, dm);
+    N.qfc[q] = fc;
+    N.qdm[q] = dm;
+  } else {
+    flag |= kNbFar;
+  }
   if (r2 > (double)MD_CUTOFF_RIJSQ) flag |= kNbNoBond;
   if (cell3) {
     const int4 a = reinterpret_cast<const int4*>(cell3)[i],
@@ -853,24 +867,36 @@ __device__ __forceinline__ void mb_stage(Nb& N, int q, uint32_t e, double xi, do
     }
   }
   N.flag[q] = flag;
-  if (PAIR) {
-    // common/arvdwfc.cpp:17-48 with the powers of one exponential
-    const double de = get_de<double>(ti, tj), re = get_re<double>(ti, tj), beta = get_beta<double>(ti, tj);
-    const double x1 = exp64(-beta * (r - re)), x2 = x1 * x1, x4 = x2 * x2;
-    const double va = MD_S * de / (MD_S - 1.0f) * x1;
-    const double vr = de / (MD_S - 1.0f) * x2 + 7.0e-8f * (x4 * x4 * x2);
-    const double eplus = exp64(MD_ALFAV * (r - get_r0v<double>(ti, tj)));
-    const double gmexp = MD_GM * rcp64(eplus);
-    const double a = eplus + gmexp, b = MD_ALFAV * (eplus - gmexp), db = MD_ALFAVSQ * a;
-    const double v = 1.0f + 50.0f * MD_GM + MD_GMSQ + 10.0f * (MD_GM - 1.0f) * b;
-    const double ia = rcp64(a), ia2 = ia * ia;
-    const double dvdw = -1.0e-4f * ((10.0f * (MD_GM - 1.0f) * db * a - 2.0f * b * v) * (ia2 * ia));
-    N.E[q] = exp64((double)MD_LAMDA3 * (r - re));
-    N.va[q] = va;
-    N.dva[q] = beta * va;
-    N.dv[q] = beta * 2.0f * vr + dvdw;
-    N.v0[q] = vr + 1.0e-4f * v * ia2;
-  }
+}
+
+// its pair terms by a thread of another warp: common/arvdwfc.cpp:17-48 with the
+// powers of one exponential
+__device__ __forceinline__ void mb_stage_pair(NbPair& N, int q, uint32_t e, double xi, double yi,
+                                              double zi, int ti, const md_double4* pos,
+                                              const Grid& g) {
+  double x, y, z;
+  int tj;
+  PosT<double>::load(pos, nullptr, entry_index(e), x, y, z, tj);
+  PosT<double>::image(x, y, z, e, g);
+  const double dx = xi - x, dy = yi - y, dz = zi - z;
+  const double r2 = dx * dx + dy * dy + dz * dz;
+  const double r = r2 * rsqrt64(r2);
+  const double de = get_de<double>(ti, tj), re = get_re<double>(ti, tj),
+               beta = get_beta<double>(ti, tj);
+  const double x1 = exp64(-beta * (r - re)), x2 = x1 * x1, x4 = x2 * x2;
+  const double va = MD_S * de / (MD_S - 1.0f) * x1;
+  const double vr = de / (MD_S - 1.0f) * x2 + 7.0e-8f * (x4 * x4 * x2);
+  const double eplus = exp64(MD_ALFAV * (r - get_r0v<double>(ti, tj)));
+  const double gmexp = MD_GM * rcp64(eplus);
+  const double a = eplus + gmexp, b = MD_ALFAV * (eplus - gmexp), db = MD_ALFAVSQ * a;
+  const double v = 1.0f + 50.0f * MD_GM + MD_GMSQ + 10.0f * (MD_GM - 1.0f) * b;
+  const double ia = rcp64(a), ia2 = ia * ia;
+  const double dvdw = -1.0e-4f * ((10.0f * (MD_GM - 1.0f) * db * a - 2.0f * b * v) * (ia2 * ia));
+  N.E[q] = exp64((double)MD_LAMDA3 * (r - re));
+  N.va[q] = va;
+  N.dva[q] = beta * va;
+  N.dv[q] = beta * 2.0f * vr + dvdw;
+  N.v0[q] = vr + 1.0e-4f * v * ia2;
 }
 
 // What the angle terms of a bond i-j with the third body m give: the sums of
@@ -881,12 +907,15 @@ __device__ __forceinline__ void mb_stage(Nb& N, int q, uint32_t e, double xi, do
 struct Angle {
   double x, y, xj, yj, a, b, p, q;
 };
-__device__ __forceinline__ Angle mb_angle(const Nb& J, int j, const Nb& M, int m) {
+// in FP64, for distances outside the fixed point's range
+__device__ __noinline__ Angle mb_angle_far(const Nb& J, int j, const Nb& M, int m) {
   const double vx = M.d[0][m] - J.d[0][j], vy = M.d[1][m] - J.d[1][j], vz = M.d[2][m] - J.d[2][j];
-  const double rij = J.r[j], irij = J.ir[j], rim = M.r[m], irim = M.ir[m], fi = M.fc[m];
-  const double r2 = vx * vx + vy * vy + vz * vz;
-  const double irjm = rsqrt64(r2), rjm = r2 * irjm;
-  double fj, dfj, gi, pi, gj, pj;
+  const double r2 = vx * vx + vy * vy + vz * vz, irjm = rsqrt64(r2), rjm = r2 * irjm;
+  const double rij2 = J.d[0][j] * J.d[0][j] + J.d[1][j] * J.d[1][j] + J.d[2][j] * J.d[2][j];
+  const double rim2 = M.d[0][m] * M.d[0][m] + M.d[1][m] * M.d[1][m] + M.d[2][m] * M.d[2][m];
+  const double irij = rsqrt64(rij2), rij = rij2 * irij, irim = rsqrt64(rim2), rim = rim2 * irim;
+  double fi, dfi, fj, dfj, gi, pi, gj, pj;
+  mb_cutoff(rim, fi, dfi);
   mb_cutoff(rjm, fj, dfj);
   // cosines of the angles at i (unit vectors) and at j (projection)
   const double ci = J.u[0][j] * M.u[0][m] + J.u[1][j] * M.u[1][m] + J.u[2][j] * M.u[2][m];
@@ -899,14 +928,41 @@ __device__ __forceinline__ Angle mb_angle(const Nb& J, int j, const Nb& M, int m
   A.y = xi * fma(-ci, irij, irim);
   A.xj = fj * gj;
   A.yj = xj * fma(-cj, irij, irjm);
-  A.a = fma(xi, fma(-ci, irim, irij), M.dfc[m] * gi);
+  A.a = fma(xi, fma(-ci, irim, irij), dfi * gi);
   A.p = -xi * (irij * irim);
   A.b = -xj * (rim * irij) * irjm;
   A.q = fma(xj, fma(-cj, irjm, irij), dfj * gj) * irjm;
   return A;
 }
 
-constexpr int kMbPitch = 36;  // columns of a warp's coefficient table (bank-conflict-free)
+// the same in fixed point; the four sums stay there (sx, sy, sxj, syj)
+__device__ __forceinline__ void mb_angle_q(double r2, const Nb& J, int j, const Nb& M, int m,
+                                           bool sums, q56& sx, q56& sy, q56& sxj, q56& syj,
+                                           Angle& A) {
+  const q56 rij = J.qr[j], irij = J.qir[j], rim = M.qr[m], irim = M.qir[m], fi = M.qfc[m];
+  q56 rjm, irjm, fj, dj, gi, pi, gj, pj;
+  rsqrtq(r2, rjm, irjm);
+  cutoffq(rjm, fj, dj);
+  const q56 ci = dotq(J.qu[0][j], J.qu[1][j], J.qu[2][j], M.qu[0][m], M.qu[1][m], M.qu[2][m]);
+  const q56 cj = mulq(rij - mulq(rim, ci), irjm);
+  angularq(ci, gi, pi);
+  angularq(cj, gj, pj);
+  const q56 xi = mulq(fi, pi), xj = mulq(fj, pj);
+  if (sums) {
+    sx += mulq(fi, gi);
+    sy += mulq(xi, irim - mulq(ci, irij));
+    sxj += mulq(fj, gj);
+    syj += mulq(xj, irjm - mulq(cj, irij));
+  }
+  A.a = fromq(mulq(xi, irij - mulq(ci, irim)) - mulq(M.qdm[m], gi));
+  A.p = fromq(-mulq(xi, mulq(irij, irim)));
+  A.b = fromq(-mulq(mulq(xj, mulq(rim, irij)), irjm));
+  A.q = fromq(mulq(mulq(xj, irij - mulq(cj, irjm)) - mulq(dj, gj), irjm));
+}
+
+// columns of a warp's coefficient table: 34 keeps five blocks on an SM (36 would
+// store without bank conflicts, but only four blocks fit)
+constexpr int kMbPitch = 34;
 constexpr int kMbSlots = kMbSlotCount;  // third-body force slots per atom
 
 // Sum of 4 values over the warp, each value to a quarter of the lanes: value
@@ -935,12 +991,15 @@ __device__ __forceinline__ double quarter_sum(double v0, double v1, double v2, d
 // the bond's factors are known; then lane m adds over the eight bonds.  More
 // than 32 neighbours take the triplets twice, in tiles of 32.
 //
-// Bound by the FP64 pipe (77 operations per triplet; 86% busy).
+// The angle terms in FP64 (75 operations a triplet) kept the FP64 pipe 86% busy
+// and everything else idle: 568 us for 4,096 atoms; in 64-bit fixed point
+// (md_fixed64.cuh, 6 FP64 operations) 279 us, and with the pair terms
+// staged by a second warp and five blocks on an SM 265 us.
 // SLOTS: with the engine's own rows; caller-supplied rows may lack symmetry,
 // and k_mb_pass2 evaluates their third bodies.
 template <bool ENERGY, bool SLOTS>
-__global__ void __launch_bounds__(128)
-    k_mb_bonds(const md_double4* __restrict__ pos, const float4* __restrict__ posf,
+__global__ void __launch_bounds__(128, 5)
+    k_mb_bonds(const md_double4* __restrict__ pos,
                double* __restrict__ f3, int n, const uint32_t* __restrict__ sl, int pitch,
                const int* __restrict__ slen, Grid g, const int* __restrict__ cell3, int ljexist,
                double* __restrict__ wi_s, double* __restrict__ wj_s, double* __restrict__ fslot,
@@ -948,6 +1007,7 @@ __global__ void __launch_bounds__(128)
                double* __restrict__ eatom, const int* __restrict__ run_if) {
   if (!ENERGY && run_if && *run_if == 0) return;
   __shared__ Nb NA, NB;
+  __shared__ NbPair NP;
   __shared__ double table[4][4][8][kMbPitch];  // warp, coefficient, bond, m
   __shared__ double wsm[4][2][8];              // factors of the warp's bonds
   __shared__ double bsum[4][32];               // force of a bond, its energy
@@ -955,7 +1015,7 @@ __global__ void __launch_bounds__(128)
   const int jj = lane >> 2, quad = lane & 3;
   double xi, yi, zi;
   int ti;
-  PosT<double>::load(pos, posf, i, xi, yi, zi, ti);
+  PosT<double>::load(pos, nullptr, i, xi, yi, zi, ti);
   const int S = slen[i];
   const uint32_t* row = sl + (size_t)i * pitch;
   double fx = 0, fy = 0, fz = 0;
@@ -964,23 +1024,35 @@ __global__ void __launch_bounds__(128)
   const bool once = S <= 32;
   for (int j0 = 0; j0 < S; j0 += 32) {
     __syncthreads();
-    if (tid < 32 && j0 + tid < S)
-      mb_stage<true>(NA, tid, row[j0 + tid], xi, yi, zi, ti, pos, posf, g, cell3, i);
+    if (j0 + lane < S) {
+      if (warp == 0) mb_stage(NA, lane, row[j0 + lane], xi, yi, zi, pos, g, cell3, i);
+      if (warp == 1) mb_stage_pair(NP, lane, row[j0 + lane], xi, yi, zi, ti, pos, g);
+    }
     __syncthreads();
     const int j = 8 * warp + jj;  // bond of this lane in the tile
     const bool bond = j0 + j < S && !(NA.flag[j & 31] & kNbNoBond);
     double x = 0, y = 0, xj = 0, yj = 0;
+    q56 qx = 0, qy = 0, qxj = 0, qyj = 0;
     auto triplets = [&](const Nb& M, int m0, bool sums, bool store) {
       const int mn = min(32, S - m0);
       if (bond)
         for (int m = quad; m < mn; m += 4) {
           if (m0 + m == j0 + j) continue;
-          const Angle A = mb_angle(NA, j, M, m);
-          if (sums && !(M.flag[m] & kNbNoThird)) {
-            x += A.x;
-            y += A.y;
-            xj += A.xj;
-            yj += A.yj;
+          const double vx = M.d[0][m] - NA.d[0][j], vy = M.d[1][m] - NA.d[1][j],
+                       vz = M.d[2][m] - NA.d[2][j];
+          const double r2 = vx * vx + vy * vy + vz * vz;
+          const bool third = sums && !(M.flag[m] & kNbNoThird);
+          Angle A;
+          if (!((NA.flag[j] | M.flag[m]) & kNbFar) && mb_in_range(r2, 256.0)) {
+            mb_angle_q(r2, NA, j, M, m, third, qx, qy, qxj, qyj, A);
+          } else {
+            A = mb_angle_far(NA, j, M, m);
+            if (third) {
+              x += A.x;
+              y += A.y;
+              xj += A.xj;
+              yj += A.yj;
+            }
           }
           if (store) {
             table[warp][0][jj][m] = A.a;
@@ -995,11 +1067,16 @@ __global__ void __launch_bounds__(128)
       if (m0 == j0) return NA;
       __syncthreads();
       if (tid < 32 && m0 + tid < S)
-        mb_stage<false>(NB, tid, row[m0 + tid], xi, yi, zi, ti, pos, posf, g, cell3, i);
+        mb_stage(NB, tid, row[m0 + tid], xi, yi, zi, pos, g, cell3, i);
       __syncthreads();
       return NB;
     };
-    for (int m0 = 0; m0 < S; m0 += 32) triplets(tile(m0), m0, true, once);
+    for (int m0 = 0; m0 < S; m0 += 32) {
+      triplets(tile(m0), m0, true, once);
+      // a lane's eight triplets of a tile stay below the fixed point's range
+      x += fromq(qx), y += fromq(qy), xj += fromq(qxj), yj += fromq(qyj);
+      qx = qy = qxj = qyj = 0;
+    }
 #pragma unroll
     for (int o = 1; o < 4; o <<= 1) {
       x += __shfl_xor_sync(0xffffffffu, x, o);
@@ -1010,7 +1087,7 @@ __global__ void __launch_bounds__(128)
     if (quad == 0 && j0 + j < S) {
       double wi = (double)NAN, wj = (double)NAN;
       if (bond) {
-        const double E = NA.E[j], va = NA.va[j], lam = (double)MD_LAMDA3;
+        const double E = NP.E[j], va = NP.va[j], lam = (double)MD_LAMDA3;
         const double bi = rcp64(fma(E, x, 1.0)), bj = rcp64(fma(E, xj, 1.0));
         const double pi = bi * bi * E, pj = bj * bj * E;  // E / (1 + xi)^2
         const double bo = 0.5 * (bi + bj);
@@ -1018,11 +1095,11 @@ __global__ void __launch_bounds__(128)
         // what the third bodies need of this bond: va E / (4 (1 + xi)^2)
         wi = 0.25 * va * pi;
         wj = 0.25 * va * pj;
-        const double f = NA.dv[j] - bo * NA.dva[j] - va * db;
+        const double f = NP.dv[j] - bo * NP.dva[j] - va * db;
         bsum[0][j] = f * NA.u[0][j];
         bsum[1][j] = f * NA.u[1][j];
         bsum[2][j] = f * NA.u[2][j];
-        if (ENERGY) bsum[3][j] = 0.5 * (NA.v0[j] - bo * va);
+        if (ENERGY) bsum[3][j] = 0.5 * (NP.v0[j] - bo * va);
       } else {
         bsum[0][j] = bsum[1][j] = bsum[2][j] = bsum[3][j] = 0.0;
       }
@@ -1736,14 +1813,14 @@ static void launch_mb64(const MbArgs& a, cudaStream_t st) {
                                         a.rcutsq, a.sl, (size_t)a.pitch, 1, a.slen, gate);
   if (!a.ref_rows) {
     k_mb_bonds<ENERGY, true><<<a.n, 128, 0, st>>>(
-        a.pos, a.posf, a.f3, a.n, a.sl, a.pitch, a.slen, a.grid, a.cell3, a.ljexist, wi, wj, fs,
+        a.pos, a.f3, a.n, a.sl, a.pitch, a.slen, a.grid, a.cell3, a.ljexist, wi, wj, fs,
         a.missing, e1, ea, gate);
     k_mb_gather<ENERGY><<<B, 128, 0, st>>>(a.pos, a.posf, a.f3, a.n, a.sl, a.pitch,
                                                    a.slen, a.grid, a.cell3, a.rcutsq, wi, wj, fs,
                                                    a.missing, e2, gate);
   } else if constexpr (!ENERGY) {
     k_mb_bonds<false, false><<<a.n, 128, 0, st>>>(
-        a.pos, a.posf, a.f3, a.n, a.sl, a.pitch, a.slen, a.grid, nullptr, a.ljexist, wi, wj,
+        a.pos, a.f3, a.n, a.sl, a.pitch, a.slen, a.grid, nullptr, a.ljexist, wi, wj,
         nullptr, a.missing, nullptr, nullptr, gate);
     k_mb_pass2<<<B, 128, 0, st>>>(a.pos, a.f3, a.n, a.sl, a.pitch, a.slen, a.grid, a.ref_rows,
                                   a.ref_nls, a.ref_nlargest, a.rcutsq, wi, wj, a.missing);
