@@ -175,23 +175,13 @@ __global__ void k_pos_build(const md_double4* __restrict__ pos, int n, float4* _
   pb[i] = make_float4((float)p.x, (float)p.y, (float)p.z, __int_as_float((int)p.w));
 }
 
-// Rows, a warp per atom: 27 lanes look up the cells around the atom's own, a
-// warp scan joins them into one candidate sequence in the reference's order,
-// and the lanes test 32 candidates at a time (a ballot keeps the order).
-// MODE 0 counts (len[i] and maxima), 1 writes, 2 does both, with rows longer
-// than cap truncated and reported through the counters.  An entry k of atom i
-// goes to list[i * ri + k * rk].
-// A thread per atom walked its 600 candidates one dependent load after another:
-// 57 us (count) and 129 us (write) for 864 atoms, 177 and 380 for 108,000.
-template <int MODE>
-__global__ void __launch_bounds__(128)
-    k_rows(RowWalker w, const md_double4* __restrict__ pos, const float4* __restrict__ pb,
-           int compact, float rv2, float box_f, uint32_t* __restrict__ list,
-           int* __restrict__ len, size_t ri, size_t rk, int cap, int* __restrict__ counters) {
-  const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (i >= w.n) return;  // whole warp
-  const float4 pi = pb[i];
+// The candidates of row i by a warp, 32 at a time in the reference's order: 27
+// lanes look up the cells around the atom's own, and a warp scan joins them into
+// one sequence.  visit(valid, m, im) runs in all lanes; im holds the image's
+// three 2-bit fields.  Returns the number of candidates.
+template <typename F>
+__device__ __forceinline__ int warp_row(const RowWalker& w, const md_double4* __restrict__ pos,
+                                        int i, int lane, F&& visit) {
   const bool whole = w.g.periodic && w.g.cells == 1;  // minimum images of all atoms
   int first = 0, count = 0, img = 0;  // this lane's cell
   if (!whole && lane < 27) {
@@ -225,7 +215,7 @@ __global__ void __launch_bounds__(128)
   const int total = whole ? w.n : __shfl_sync(0xffffffffu, pre, 31);
   pre -= count;
   const md_double4 ei = whole ? pos[i] : md_double4{0, 0, 0, 0};
-  int kept = 0, self = 0;
+  int self = 0;
   for (int q0 = 0; q0 < total; q0 += 32) {
     const int q = q0 + lane;
     int m = q, im = 0;
@@ -241,13 +231,35 @@ __global__ void __launch_bounds__(128)
       im = __shfl_sync(0xffffffffu, img, c);
       if (q < total) m = w.sorted[f + q - p];
     }
-    bool keep = q < total && m != i;
+    const bool valid = q < total && m != i;
     if (q < total && m == i) self = 1;
-    if (keep && whole) {
+    if (valid && whole) {
       const md_double4 em = pos[m];
       im = (min_image(ei.x, em.x, w.g.box) & 3) | ((min_image(ei.y, em.y, w.g.box) & 3) << 2) |
            ((min_image(ei.z, em.z, w.g.box) & 3) << 4);
     }
+    visit(valid, m, im);
+  }
+  return total - (__any_sync(0xffffffffu, self) ? 1 : 0);
+}
+
+// Rows, a warp per atom; the lanes test 32 candidates at a time (a ballot keeps
+// the order).  MODE 0 counts (len[i] and maxima), 1 writes, 2 does both, with
+// rows longer than cap truncated and reported through the counters.  An entry k
+// of atom i goes to list[i * ri + k * rk].
+// A thread per atom walked its 600 candidates one dependent load after another:
+// 57 us (count) and 129 us (write) for 864 atoms, 177 and 380 for 108,000.
+template <int MODE>
+__global__ void __launch_bounds__(128)
+    k_rows(RowWalker w, const md_double4* __restrict__ pos, const float4* __restrict__ pb,
+           int compact, float rv2, float box_f, uint32_t* __restrict__ list,
+           int* __restrict__ len, size_t ri, size_t rk, int cap, int* __restrict__ counters) {
+  const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (i >= w.n) return;  // whole warp
+  const float4 pi = pb[i];
+  int kept = 0;
+  const int full = warp_row(w, pos, i, lane, [&](bool keep, int m, int im) {
     const uint32_t e = (uint32_t)m | ((uint32_t)im << kIndexBits);
     if (keep && compact) {
       const float4 pm = pb[m];
@@ -262,35 +274,41 @@ __global__ void __launch_bounds__(128)
       if (k < cap) list[(size_t)i * ri + (size_t)k * rk] = e;
     }
     kept += __popc(mask);
-  }
-  if (MODE != 1) {
-    const int full = total - (__any_sync(0xffffffffu, self) ? 1 : 0);
-    if (lane == 0) {
-      len[i] = kept;
-      atomicMax(&counters[1], full);
-      atomicMax(&counters[2], kept);
-      atomicAdd((unsigned long long*)(counters + 4), (unsigned long long)kept);
-    }
+  });
+  if (MODE != 1 && lane == 0) {
+    len[i] = kept;
+    atomicMax(&counters[1], full);
+    atomicMax(&counters[2], kept);
+    atomicAdd((unsigned long long*)(counters + 4), (unsigned long long)kept);
   }
 }
 
-__global__ void k_ref_rows(RowWalker w, const md_double4* __restrict__ pos, int nls,
-                           int* __restrict__ out, signed char* __restrict__ img) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= w.n) return;
+// Full rows in the reference's layout, a warp per atom (a thread per atom took
+// 89 us for 864 atoms, its stores a row apart; 10 us here).
+__global__ void __launch_bounds__(128)
+    k_ref_rows(RowWalker w, const md_double4* __restrict__ pos, int nls, int* __restrict__ out,
+               signed char* __restrict__ img) {
+  const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (i >= w.n) return;  // whole warp
   int* row = out + (size_t)i * nls;
-  signed char* im = img ? img + (size_t)i * nls : nullptr;
+  signed char* im_row = img ? img + (size_t)i * nls : nullptr;
   int count = 0;
-  walk_row(w, pos, i, [&](int m, int ix, int iy, int iz) {
-    if (count < nls) {
-      row[count] = m;
-      if (im) im[count] = (signed char)((ix + 1) * 9 + (iy + 1) * 3 + (iz + 1));
+  warp_row(w, pos, i, lane, [&](bool valid, int m, int im) {
+    const unsigned mask = __ballot_sync(0xffffffffu, valid);
+    const int k = count + __popc(mask & ((1u << lane) - 1u));
+    if (valid && k < nls) {
+      row[k] = m;
+      const uint32_t e = (uint32_t)im << kIndexBits;
+      if (im_row)
+        im_row[k] = (signed char)((entry_img(e, 0) + 1) * 9 + (entry_img(e, 1) + 1) * 3 +
+                                  (entry_img(e, 2) + 1));
     }
-    count++;
+    count += __popc(mask);
   });
-  for (int k = count; k < nls; k++) {
+  for (int k = count + lane; k < nls; k += 32) {
     row[k] = -1;
-    if (im) im[k] = 13;
+    if (im_row) im_row[k] = 13;
   }
 }
 
@@ -552,7 +570,7 @@ int list_reference_rows(const NeighborList& nl, const md_double4* pos, int* d_ou
                         signed char* d_img, cudaStream_t st) {
   if (nl.n <= 0 || nl.nlistsize <= 0) return 0;
   RowWalker w = make_walker(nl);
-  k_ref_rows<<<blocks(nl.n, 128), 128, 0, st>>>(w, pos, nl.nlistsize, d_out, d_img);
+  k_ref_rows<<<blocks(nl.n, 4), 128, 0, st>>>(w, pos, nl.nlistsize, d_out, d_img);
   return (int)cudaGetLastError();
 }
 

@@ -13,6 +13,7 @@
 #include "../../include/mdgb.h"
 #include "md_forces.h"
 #include "md_integrate.h"
+#include "md_lj64.cuh"
 #include "md_neighbor.cuh"
 #include "md_potential.cuh"
 
@@ -124,30 +125,81 @@ bool finish() {
     }                              \
   } while (0)
 
-// cpu/common/LennardJones.h:35-93 over rows in the reference layout
-__global__ void k_lj_rows(const md_double4* __restrict__ pos, double* __restrict__ f3, int n,
-                          int nlargest, int nls, const int* __restrict__ list, double rcutsq,
-                          Species sp) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// cpu/common/LennardJones.h:35-93 over rows in the reference layout.  A warp per
+// atom: 32 entries at a time, those that an FP32 screen leaves (conservative, as
+// k_lj_fp64's) queue in row order, then a pair per lane, and three lanes add the
+// components one after another, so the sums are the reference's to the bit.  A
+// thread per atom was one chain of FP64 divisions: 864 atoms took 400 us, and
+// take 22 us here (latency of the row reads and of the integer chains).
+constexpr int kRowsQueue = 96;
+__global__ void __launch_bounds__(128)
+    k_lj_rows(const md_double4* __restrict__ pos, double* __restrict__ f3, int n, int nlargest,
+              int nls, const int* __restrict__ list, double rcutsq,
+              const __grid_constant__ LjPairConst c) {
+  __shared__ int queue[4][kRowsQueue];
+  __shared__ double term[4][3][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i = blockIdx.x * 4 + warp;
   if (i >= n) return;
   const md_double4 pi = pos[i];
-  const int ti = (int)pi.w;
-  double fx = 0.0, fy = 0.0, fz = 0.0;
-  const int* row = list + (size_t)i * nls;
-  for (int j = 0; j < nlargest && row[j] != -1; j++) {
-    const md_double4 pj = pos[row[j]];
-    const double ijx = xsub(pi.x, pj.x), ijy = xsub(pi.y, pj.y), ijz = xsub(pi.z, pj.z);
-    const double r2 = norm2_exact(ijx, ijy, ijz);
-    if (r2 >= rcutsq) continue;
-    const int tj = (int)pj.w;
-    if (tj == SP_NG || ti == SP_NG) {
-      const int sel = lj_select(ti, tj);
-      lj_pair_exact(fx, fy, fz, __dsqrt_rn(r2), ijx, ijy, ijz, sp.sig[sel], sp.eps[sel]);
+  const int ti = species64(pi.w);
+  const float xf = trunc32(pi.x), yf = trunc32(pi.y), zf = trunc32(pi.z);
+  const float rc2 = (float)rcutsq * 1.000001f, rc = sqrtf(rc2);
+  const float off = (fmaxf(fabsf(xf), fmaxf(fabsf(yf), fabsf(zf))) + rc) * 0x1p-20f;
+  const float thr = rc2 + off * (8.0f * rc + 16.0f * off) + 1e-37f;  // for squares that underflow
+  const size_t row = (size_t)i * nls, end = (size_t)n * nls;
+  double acc = 0.0;  // lane < 3: component lane of the force
+  int* q = queue[warp];
+  for (int k0 = 0; k0 < nlargest;) {
+    int cnt = 0;
+    while (k0 < nlargest && cnt + 32 <= kRowsQueue) {
+      const int k = k0 + lane;
+      const int e = k < nlargest && row + k < end ? list[row + k] : -1;
+      const unsigned stop = __ballot_sync(0xffffffffu, e == -1);
+      bool keep = false;
+      if (!(stop & ((2u << lane) - 1u))) {  // no end of the row up to here
+        const md_double4 pj = pos[e];
+        const float dx = xf - trunc32(pj.x), dy = yf - trunc32(pj.y), dz = zf - trunc32(pj.z);
+        keep = !(dx * dx + dy * dy + dz * dz > thr);
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, keep);
+      if (keep) q[cnt + __popc(m & ((1u << lane) - 1u))] = e;
+      cnt += __popc(m);
+      k0 = stop ? nlargest : k0 + 32;
+    }
+    __syncwarp();
+    for (int s0 = 0; s0 < cnt; s0 += 32) {
+      double tx = 0.0, ty = 0.0, tz = 0.0;
+      bool in = s0 + lane < cnt;
+      if (in) {
+        const md_double4 pj = pos[q[s0 + lane]];
+        const double ijx = xsub(pi.x, pj.x), ijy = xsub(pi.y, pj.y), ijz = xsub(pi.z, pj.z);
+        const double r2 = xadd(xadd(sq64(ijx), sq64(ijy)), sq64(ijz));
+        const int tj = species64(pj.w);
+        in = below64(r2, rcutsq) && (tj == SP_NG || ti == SP_NG);
+        if (in) {
+          const int sel = lj_select(ti, tj);
+          const double sq = sel == 0 ? c.sq[0] : (sel == 1 ? c.sq[1] : c.sq[2]);
+          const double con = sel == 0 ? c.con[0] : (sel == 1 ? c.con[1] : c.con[2]);
+          const uint64_t yq = sel == 0 ? c.yq[0] : (sel == 1 ? c.yq[1] : c.yq[2]);
+          lj_terms(r2, ijx, ijy, ijz, sq, yq, con, tx, ty, tz);
+        }
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, in);
+      term[warp][0][lane] = tx;
+      term[warp][1][lane] = ty;
+      term[warp][2][lane] = tz;
+      __syncwarp();
+      if (lane < 3) {
+        const double* tv = term[warp][lane];
+#pragma unroll
+        for (int s = 0; s < 32; s++)
+          if ((m >> s) & 1u) acc = xadd(acc, tv[s]);
+      }
+      __syncwarp();
     }
   }
-  f3[3 * i] = fx;
-  f3[3 * i + 1] = fy;
-  f3[3 * i + 2] = fz;
+  if (lane < 3) f3[3 * (size_t)i + lane] = acc;
 }
 
 // reference rows -> ELL slot-major rows (candidate order kept)
@@ -251,9 +303,10 @@ void mdgb_lennard_jones_forces(const double* pos4, double* f3, int n, int nlarge
   SHIM_CK(grow(s.rows, s.rows_alloc, nrows), MD_OUT_OF_MEMORY);
   SHIM_CK(up(s.pos, pos4, 32 * (size_t)n), MD_CUDA_ERROR);
   if (nrows) SHIM_CK(up(s.rows, list, sizeof(int) * (size_t)nrows), MD_CUDA_ERROR);
-  k_lj_rows<<<(n + 127) / 128, 128, 0, s.st>>>(s.pos, s.v[4], n, nlistsize ? nlargestsize : 0,
-                                               nlistsize, s.rows, rcutsq,
-                                               shim_species(s.species));
+  k_lj_rows<<<n / 4 + (n % 4 != 0), 128, 0, s.st>>>(
+      s.pos, s.v[4], n, nlistsize ? nlargestsize : 0, nlistsize, s.rows,
+      rcutsq <= 0.0 ? 0.0 : rcutsq,  // nothing is below either; the kernel compares bits
+      lj_pair_const(shim_species(s.species), rcutsq));
   SHIM_CK(down(f3, s.v[4], 24 * (size_t)n) && finish(), MD_CUDA_ERROR);
 }
 

@@ -100,3 +100,21 @@ def test_tripped_skin_refreshes_rows(eng, oracle):
             out.append(e.download() + (e.stats()["list_trips"],))
     assert out[0][2] >= 0
     assert np.allclose(out[0][0], out[1][0], rtol=0, atol=1e-10)
+
+
+@pytest.mark.parametrize("n,a", [(1, 5.26), (2, 5.26), (33, 5.26), (129, 5.26), (500, 2.9),
+                                 (864, 5.26)])
+def test_rows_of_the_caller(eng, oracle, n, a):
+    # rows that end inside, at and after a chunk of 32; longer than the queue
+    pos, vel, _ = lat.make_system("fcc", 6, 94.4, seed=n, natoms=n, noise=0.05, a=a)
+    sh = eng.Shim(species=eng.SPECIES_ARGON)
+    nl = oracle.build_list(pos.copy(), RS, 40.0)
+    rcsq = oracle.settings(RS, RC)[2]
+    rows, nls, nlargest = sh.build_neighbor_list(pos, RS, RC, 40.0)
+    assert nls == nl.nlistsize and nlargest == nl.nlargest
+    if nls:
+        assert np.array_equal(rows, nl.rows)
+    f = sh.lennard_jones_forces(pos, rows, nlargest, rcsq)
+    assert np.array_equal(f, oracle.lj_forces(pos, nl, rcsq, eng.SPECIES_ARGON))
+    assert not sh.lennard_jones_forces(pos, rows, nlargest, -1.0).any()
+    oracle.free_list(nl)
