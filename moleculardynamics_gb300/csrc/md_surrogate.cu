@@ -14,6 +14,7 @@
 #include <algorithm>
 
 #include "../../include/mdgb.h"
+#include "md_exact64.cuh"
 #include "md_neighbor.cuh"
 #include "md_surrogate.h"
 #include "md_tc.cuh"
@@ -81,6 +82,7 @@ constexpr int oW1 = 0, oB1 = oW1 + kHid * kDesc, oW2 = oB1 + kHid, oB2 = oW2 + k
 DescParams default_desc(float rc) {
   DescParams P;
   P.rc = rc;
+  P.fca = 3.14159265358979f / rc;
   const float d = (rc - 0.8f) / (kRad - 1);
   P.eta_r = 0.5f / (d * d);
   for (int k = 0; k < kRad; k++) P.rs[k] = 0.8f + d * k;
@@ -96,42 +98,12 @@ DescParams default_desc(float rc) {
   return P;
 }
 
-__device__ __forceinline__ void fcut(float r, float rc, float& fc, float& dfc) {
-  const float a = 3.14159265358979f / rc;
+// a = pi / rc
+__device__ __forceinline__ void fcut(float r, float a, float& fc, float& dfc) {
   float s, c;
   __sincosf(a * r, &s, &c);
   fc = 0.5f * (c + 1.f);
   dfc = -0.5f * a * s;
-}
-
-// Angular factors of one neighbour pair for the 16 functions f = 8 e + 4 l + z
-// of default_desc's table (eta index e, lambda index l for +1 / -1, zeta index
-// z for 1, 2, 4, 16): powers of both bases by squaring and one exponential
-// per eta, instead of 16 of each.
-struct AngPair {
-  float b[2];        // 1 + lambda cos
-  float pz[2][4];    // b ^ zeta
-  float pz1[2][4];   // b ^ (zeta - 1)
-  float ex[2];       // exp(-eta q)
-};
-
-__device__ __forceinline__ void ang_pair(float c, float q, const DescParams& P, AngPair& A) {
-#pragma unroll
-  for (int l = 0; l < 2; l++) {
-    const float b = l ? 1.f - c : 1.f + c;
-    const float p2 = b * b, p4 = p2 * p2, p8 = p4 * p4;
-    A.b[l] = b;
-    A.pz[l][0] = b;
-    A.pz[l][1] = p2;
-    A.pz[l][2] = p4;
-    A.pz[l][3] = p8 * p8;
-    A.pz1[l][0] = 1.f;
-    A.pz1[l][1] = b;
-    A.pz1[l][2] = p2 * b;
-    A.pz1[l][3] = p8 * p4 * p2 * b;
-  }
-  A.ex[0] = __expf(-P.eta_a[0] * q);
-  A.ex[1] = __expf(-P.eta_a[8] * q);
 }
 
 // neighbours of i within rc (from the bond-order candidate rows: the 27
@@ -224,82 +196,162 @@ __global__ void __launch_bounds__(128)
 }
 
 // ---- warp-per-atom descriptor and force kernels (4 atoms per block) ----
-struct NbrSm {
-  float dx[kSgMax], dy[kSgMax], dz[kSgMax], r[kSgMax], ir[kSgMax], fc[kSgMax], dfc[kSgMax];
-  int idx[kSgMax];
-};
+// A lane takes a neighbour, then a neighbour pair after another: with S
+// neighbours, step d = 1 .. S / 2 gives lane a the pair (a, a + d mod S), which
+// is every pair once, with distinct a and distinct a + d in a step.  So a lane
+// keeps its own neighbour in registers, the other comes in 16-byte loads
+// without bank conflicts, no index is computed, and force sums need no atomics.
+// 22 neighbours within 3 angstrom of 32,768 atoms: forces 162 -> 73 us, descriptors
+// 73 -> 38, residual transform 126 -> 59 against 32 pairs at a time in index
+// order (shared-memory atomics and the index arithmetic bounded them).
 
-// neighbours of atom i into the warp's shared arrays; returns their count
-__device__ __forceinline__ int warp_load_nbrs(int i, const md_double4* pos, const uint32_t* sl,
-                                              const int* slen, double box, float rc,
-                                              NbrSm& N) {
+// x as the sum of two FP32 numbers, by moving the fields (conversions and
+// differences in FP64 take the narrow FP64 pipe)
+__device__ __forceinline__ float2 split64(double x) {
+  const float h = trunc32(x);
+  const uint32_t e = ((uint32_t)__double2hiint(x) >> 20) & 0x7FFu;
+  // the low 29 bits of the mantissa, worth 2^(e - 1075) each
+  const float u = __uint_as_float(e > 948u && e < 1151u ? (e - 948u) << 23 : 0u);
+  const float l = (float)((uint32_t)__double2loint(x) & 0x1FFFFFFFu) * u;
+  return make_float2(h, __double2hiint(x) < 0 ? -l : l);
+}
+
+// x_j + img box - x_i to FP32 accuracy
+__device__ __forceinline__ float diff32(float2 xj, float2 xi, int img, float2 box) {
+  float s = xj.x, l = xj.y - xi.y;
+  if (img) {
+    const float bh = img > 0 ? box.x : -box.x;
+    s = __fadd_rn(xj.x, bh);
+    const float t = __fsub_rn(s, xj.x);  // two-sum: s + rest is x_j + bh
+    const float rest = __fadd_rn(__fsub_rn(xj.x, __fsub_rn(s, t)), __fsub_rn(bh, t));
+    l = __fadd_rn(l, __fadd_rn(rest, img > 0 ? box.y : -box.y));
+  }
+  return __fadd_rn(__fsub_rn(s, xi.x), l);
+}
+
+// visit(s, S, j, ux, uy, uz, r, 1/r, fc, dfc) for neighbour s of atom i's S, a lane
+// each; returns S
+template <typename F>
+__device__ __forceinline__ int warp_nbrs(int i, const md_double4* pos, const uint32_t* sl,
+                                         const int* slen, double box, float fca, F&& visit) {
   const int lane = threadIdx.x & 31;
   const md_double4 pi = pos[i];
   const int S = slen[i];
+  const float2 xi = split64(pi.x), yi = split64(pi.y), zi = split64(pi.z), bx = split64(box);
   for (int s = lane; s < S; s += 32) {
     const uint32_t e = sl[(size_t)i * kSgMax + s];
     const int j = entry_index(e);
     const md_double4 pj = pos[j];
-    const float dx = (float)(pj.x + entry_img(e, 0) * box - pi.x);
-    const float dy = (float)(pj.y + entry_img(e, 1) * box - pi.y);
-    const float dz = (float)(pj.z + entry_img(e, 2) * box - pi.z);
-    const float r = sqrtf(dx * dx + dy * dy + dz * dz);
+    const float dx = diff32(split64(pj.x), xi, entry_img(e, 0), bx);
+    const float dy = diff32(split64(pj.y), yi, entry_img(e, 1), bx);
+    const float dz = diff32(split64(pj.z), zi, entry_img(e, 2), bx);
+    // root and reciprocal from one seed, a correction each (about half a unit off)
+    const float r2 = dx * dx + dy * dy + dz * dz, y = rsqrtf(r2), x = r2 * y;
+    const float r = r2 > 0.f ? fmaf(0.5f * y, fmaf(-x, x, r2), x) : r2;
+    const float ir = r2 > 0.f ? fmaf(y, fmaf(-r, y, 1.f), y) : y;
     float fc, dfc;
-    fcut(r, rc, fc, dfc);
-    N.dx[s] = dx;
-    N.dy[s] = dy;
-    N.dz[s] = dz;
-    N.r[s] = r;
-    N.ir[s] = 1.f / r;  // the pair terms multiply by it instead of dividing
-    N.fc[s] = fc;
-    N.dfc[s] = dfc;
-    N.idx[s] = j;
+    fcut(r, fca, fc, dfc);
+    visit(s, S, j, dx * ir, dy * ir, dz * ir, r, ir, fc, dfc);
   }
   __syncwarp();
   return S;
 }
 
-// k-th pair (a < b) of S neighbours in row-major order
-__device__ __forceinline__ void pair_of(int k, int S, int& a, int& b) {
-  const int m = 2 * S - 1;
-  int aa = (int)(0.5f * ((float)m - sqrtf((float)(m * m - 8 * k))));
-  aa = max(0, min(aa, S - 2));
-  auto off = [&](int x) { return x * (2 * S - x - 1) / 2; };
-  while (aa > 0 && off(aa) > k) aa--;
-  while (aa + 1 <= S - 2 && off(aa + 1) <= k) aa++;
-  a = aa;
-  b = k - off(aa) + aa + 1;
+// visit(d, on) for the steps of a lane's own neighbour a; on is whether it has a
+// pair in this step.  The neighbours lie twice in a row in shared memory (s and
+// s + S), so the other one is d places on.
+template <typename F>
+__device__ __forceinline__ void lane_pairs(int a, int S, F&& visit) {
+#pragma unroll 4
+  for (int d = 1; 2 * d < S; d++) visit(d, true);
+  if (S > 0 && !(S & 1)) visit(S / 2, 2 * a < S);
+}
+constexpr int kSgRow = 2 * kSgMax;
+
+template <typename T>
+__device__ __forceinline__ void put_twice(T* row, int s, int S, T v) {
+  row[s] = v;
+  row[s + S] = v;
 }
 
-// k-th pair (a < b) of S neighbours in diagonal order: pairs (a, a + d) for
-// d = 1, 2, ... in turn, so consecutive k have distinct a and distinct b
-// (lanes of a warp update distinct neighbours' force sums)
-__device__ __forceinline__ void pair_of_diag(int k, int S, int& a, int& b) {
-  // offset of diagonal d: (d - 1) S - (d - 1) d / 2
-  auto off = [&](int d) { return (d - 1) * S - (d - 1) * d / 2; };
-  const float m = (float)(2 * S - 1);
-  int d = 1 + (int)(0.5f * (m - sqrtf(fmaxf(m * m - 8.f * (float)k, 0.f))));
-  d = max(1, min(d, S - 1));
-  while (d > 1 && off(d) > k) d--;
-  while (d + 1 <= S - 1 && off(d + 1) <= k) d++;
-  a = k - off(d);
-  b = a + d;
+// two FP32 numbers in one operation (the issue slots bound the pair loops)
+struct F2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ F2 f2(float x, float y) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float2 f2_get(F2 a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
 }
 
-// sum over the warp of 32 per-lane vectors: lane f ends with component f
-__device__ __forceinline__ float warp_reduce_scatter32(float (&v)[32]) {
-  const int lane = threadIdx.x & 31;
+// The angular functions of default_desc's table, f = 8 e + 4 l + z (eta index e,
+// lambda index l for +1 / -1, zeta index z for 1, 2, 4, 16): a base
+// b = 1 + lambda cos, clipped at 0, serves four powers; the two bases are a pair.
+__device__ __forceinline__ float2 ang_bases(float c) {
+  return make_float2(fmaxf(1.f + c, 0.f), fmaxf(1.f - c, 0.f));
+}
+
+// 2^x, results below 2^-126 as 0
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+constexpr float kLog2e = 1.44269504088896f;
+
+// per-neighbour factors of the two angular exponents (the products over a pair
+// are exp(-eta (ra^2 + rb^2)) fca fcb and its derivatives along a and b)
+struct AngNbr {
+  float w[2], d[2];
+};
+__device__ __forceinline__ AngNbr ang_nbr(float r, float fc, float dfc, const DescParams& P) {
+  AngNbr A;
 #pragma unroll
-  for (int o = 16, h = 16; o > 0; o >>= 1, h >>= 1) {
+  for (int e = 0; e < 2; e++) {
+    const float eta = P.eta_a[8 * e], ex = ex2(-eta * kLog2e * r * r);
+    A.w[e] = ex * fc;
+    A.d[e] = ex * fmaf(-2.f * eta * r, fc, dfc);
+  }
+  return A;
+}
+
+// sums over the warp of the lanes' 16 angular terms (p[e][z], over l), times
+// their prefactors: lane 16 + f ends with function f
+__device__ __forceinline__ float angular_sum(const F2 (&p)[2][4], const DescParams& P) {
+  const int lane = threadIdx.x & 31;
+  float v[kAng];
+#pragma unroll
+  for (int f = 0; f < 8; f++) {
+    const float2 q = f2_get(p[f >> 2][f & 3]);
+    v[8 * (f >> 2) + (f & 3)] = q.x;
+    v[8 * (f >> 2) + 4 + (f & 3)] = q.y;
+  }
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) {
     const bool up = (lane & o) != 0;
 #pragma unroll
-    for (int k = 0; k < h; k++) {
-      const float send = up ? v[k] : v[k + h];
-      const float keep = up ? v[k + h] : v[k];
+    for (int k = 0; k < o; k++) {
+      const float send = up ? v[k] : v[k + o];
+      const float keep = up ? v[k + o] : v[k];
       v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
     }
   }
-  return v[0];
+  return (v[0] + __shfl_xor_sync(0xffffffffu, v[0], 16)) * P.pref[lane & 15];
 }
 
 // descriptors of atom i (one warp); out: normalised (G - mean) * istd, or raw G
@@ -308,56 +360,79 @@ __global__ void __launch_bounds__(128)
               const int* __restrict__ slen, double box, DescParams P,
               const float* __restrict__ mean, const float* __restrict__ istd,
               float* __restrict__ out) {
-  __shared__ NbrSm nb[4];
+  __shared__ float4 nu[4][kSgRow];  // unit vector
+  __shared__ float2 nw[4][kSgRow];  // w
+  __shared__ float2 nr[4][kSgMax];  // r, fc
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int i = blockIdx.x * 4 + warp;
   if (i >= n) return;  // whole warp
-  NbrSm& N = nb[warp];
-  const int S = warp_load_nbrs(i, pos, sl, slen, box, P.rc, N);
-  float v[32];
-#pragma unroll
-  for (int f = 0; f < 32; f++) v[f] = 0.f;
-  for (int s = lane; s < S; s += 32) {
-#pragma unroll
-    for (int k = 0; k < kRad; k++) {
-      const float t = N.r[s] - P.rs[k];
-      v[k] += __expf(-P.eta_r * t * t) * N.fc[s];
+  const int S = warp_nbrs(i, pos, sl, slen, box, P.fca,
+                          [&](int s, int S, int, float ux, float uy, float uz, float r, float,
+                              float fc, float dfc) {
+    const AngNbr A = ang_nbr(r, fc, dfc, P);
+    put_twice(nu[warp], s, S, make_float4(ux, uy, uz, 0.f));
+    put_twice(nw[warp], s, S, make_float2(A.w[0], A.w[1]));
+    nr[warp][s] = make_float2(r, fc);
+  });
+  // radial functions: lane k and lane k + 16 share function k
+  float radial = 0.f;
+  {
+    const float rs = P.rs[lane & 15], m = -P.eta_r * kLog2e;
+    for (int s = lane >> 4; s < S; s += 2) {
+      const float2 q = nr[warp][s];
+      const float t = q.x - rs;
+      radial = fmaf(ex2(t * m * t), q.y, radial);
     }
+    radial += __shfl_xor_sync(0xffffffffu, radial, 16);
   }
-  const int npair = S * (S - 1) / 2;
-  for (int k = lane; k < npair; k += 32) {
-    int a, b;
-    pair_of(k, S, a, b);
-    const float c = (N.dx[a] * N.dx[b] + N.dy[a] * N.dy[b] + N.dz[a] * N.dz[b]) * (N.ir[a] * N.ir[b]);
-    const float q = N.r[a] * N.r[a] + N.r[b] * N.r[b];
-    const float ff = N.fc[a] * N.fc[b];
-    AngPair T;
-    ang_pair(c, q, P, T);
+  F2 p[2][4];  // [e][z], over l
 #pragma unroll
-    for (int f = 0; f < kAng; f++) {
-      const int e = f >> 3, l = (f >> 2) & 1, z = f & 3;
-      const float pz = T.b[l] > 0.f ? T.pz[l][z] : 0.f;
-      v[kRad + f] += P.pref[f] * pz * T.ex[e] * ff;
-    }
+  for (int z = 0; z < 4; z++) p[0][z] = p[1][z] = f2(0.f, 0.f);
+  for (int a = lane; a - lane < S; a += 32) {
+    // lanes without a neighbour read the first one's, with weights 0
+    const float4* un = &nu[warp][a < S ? a : 0];
+    const float2* wn = &nw[warp][a < S ? a : 0];
+    const float4 ua = un[0];
+    const float2 wa = a < S ? wn[0] : make_float2(0.f, 0.f);
+    lane_pairs(a, S, [&](int d, bool on) {
+      const float4 ub = un[d];
+      const float2 wb = wn[d];
+      const float2 base = ang_bases(ua.x * ub.x + ua.y * ub.y + ua.z * ub.z);
+      const float w0 = on ? wa.x * wb.x : 0.f, w1 = on ? wa.y * wb.y : 0.f;
+      const F2 b1 = f2(base.x, base.y), b2 = f2_mul(b1, b1), b4 = f2_mul(b2, b2),
+               b8 = f2_mul(b4, b4);
+      const F2 pz[4] = {b1, b2, b4, f2_mul(b8, b8)}, w0p = f2(w0, w0), w1p = f2(w1, w1);
+#pragma unroll
+      for (int z = 0; z < 4; z++) {
+        p[0][z] = f2_fma(pz[z], w0p, p[0][z]);
+        p[1][z] = f2_fma(pz[z], w1p, p[1][z]);
+      }
+    });
   }
-  const float G = warp_reduce_scatter32(v);
+  const float angular = angular_sum(p, P);
+  const float G = lane < kRad ? radial : angular;
   out[(size_t)i * kDesc + lane] = mean ? (G - mean[lane]) * istd[lane] : G;
 }
 
-// forces from g_if = dE_i/dG_if (one warp per atom i; neighbour forces
-// gathered in shared memory, then one global atomic per neighbour)
+// forces from g_if = dE_i/dG_if, one warp per atom i, into F32 (n x 4, one
+// 16-byte reduction per neighbour).  A lane's own neighbour keeps its force in
+// registers; that of the pair's other one comes back to its lane by shuffles
+// (up to 32 neighbours) or through shared memory.
+// Per pair and base: sum_z g' b^zeta and its derivative by Horner's rule, with
+// the 32 coefficients of the atom in registers.
 __global__ void __launch_bounds__(128)
     k_sg_force(const md_double4* __restrict__ pos, int n, const uint32_t* __restrict__ sl,
                const int* __restrict__ slen, double box, DescParams P,
-               const float* __restrict__ gcoef, float* __restrict__ F32) {
-  __shared__ NbrSm nb[4];
+               const float* __restrict__ gcoef, float4* __restrict__ F32) {
+  __shared__ float4 nu[4][kSgRow];  // unit vector, 1/r
+  __shared__ float4 nw[4][kSgRow];  // w, d
+  __shared__ int idx[4][kSgMax];
   __shared__ float fn[4][3][kSgMax];
   __shared__ float gs[4][kDesc];
   __shared__ float gz[4][kAng];  // g_f pref_f zeta_f lambda_f of the angular functions
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int i = blockIdx.x * 4 + warp;
   if (i >= n) return;  // whole warp
-  NbrSm& N = nb[warp];
   {
     const float gv = gcoef[(size_t)i * kDesc + lane];
     // angular coefficients carry their prefactor 2^(1 - zeta)
@@ -365,100 +440,120 @@ __global__ void __launch_bounds__(128)
     gs[warp][lane] = f >= 0 ? gv * P.pref[f] : gv;
     if (f >= 0) gz[warp][f] = gv * P.pref[f] * (float)P.zeta[f] * P.lam[f];
   }
-  for (int s = lane; s < kSgMax; s += 32) fn[warp][0][s] = fn[warp][1][s] = fn[warp][2][s] = 0.f;
-  const int S = warp_load_nbrs(i, pos, sl, slen, box, P.rc, N);  // ends with __syncwarp
-  const float* g = gs[warp];
+  __syncwarp();
   float fix = 0.f, fiy = 0.f, fiz = 0.f;
-  for (int s = lane; s < S; s += 32) {
-    float sum = 0.f;  // sum_k g_k dphi_k/dr
+  const int S = warp_nbrs(i, pos, sl, slen, box, P.fca,
+                          [&](int s, int S, int j, float ux, float uy, float uz, float r,
+                              float ir, float fc, float dfc) {
+    const AngNbr A = ang_nbr(r, fc, dfc, P);
+    put_twice(nu[warp], s, S, make_float4(ux, uy, uz, ir));
+    put_twice(nw[warp], s, S, make_float4(A.w[0], A.w[1], A.d[0], A.d[1]));
+    idx[warp][s] = j;
+    // sum_k g_k dphi_k/dr = dfc sum_k g_k e_k - 2 eta fc sum_k g_k e_k t_k
+    float s0 = 0.f, s1 = 0.f;
+    const float m = -P.eta_r * kLog2e;
 #pragma unroll
     for (int k = 0; k < kRad; k++) {
-      const float t = N.r[s] - P.rs[k];
-      sum += g[k] * __expf(-P.eta_r * t * t) * (-2.f * P.eta_r * t * N.fc[s] + N.dfc[s]);
+      const float t = r - P.rs[k], e = gs[warp][k] * ex2(t * m * t);
+      s0 += e;
+      s1 = fmaf(e, t, s1);
     }
-    const float ir = N.ir[s];
-    const float gx = sum * N.dx[s] * ir, gy = sum * N.dy[s] * ir, gz = sum * N.dz[s] * ir;
+    const float sum = fmaf(-2.f * P.eta_r * fc, s1, dfc * s0);
     // dG/dr_j = +grad, dG/dr_i = -grad; F = -dE/dr
-    fn[warp][0][s] -= gx;
-    fn[warp][1][s] -= gy;
-    fn[warp][2][s] -= gz;
-    fix += gx;
-    fiy += gy;
-    fiz += gz;
+    fn[warp][0][s] = -sum * ux;
+    fn[warp][1][s] = -sum * uy;
+    fn[warp][2][s] = -sum * uz;
+  });
+  F2 g[2][4], h[2][4];  // [e][z], over l
+#pragma unroll
+  for (int f = 0; f < 8; f++) {
+    const int e = f >> 2, z = f & 3;
+    g[e][z] = f2(gs[warp][kRad + 8 * e + z], gs[warp][kRad + 8 * e + 4 + z]);
+    h[e][z] = f2(gz[warp][8 * e + z], gz[warp][8 * e + 4 + z]);
   }
-  __syncwarp();
-  const float* gzw = gz[warp];
-  const int npair = S * (S - 1) / 2;
-  for (int k = lane; k < npair; k += 32) {
-    int a, b;
-    pair_of_diag(k, S, a, b);
-    const float ra = N.r[a], rb = N.r[b];
-    const float ia = N.ir[a], ib = N.ir[b], irab = ia * ib;
-    const float c = (N.dx[a] * N.dx[b] + N.dy[a] * N.dy[b] + N.dz[a] * N.dz[b]) * irab;
-    const float q = ra * ra + rb * rb;
-    const float fca = N.fc[a], fcb = N.fc[b], dfa = N.dfc[a], dfb = N.dfc[b];
-    AngPair T;
-    ang_pair(c, q, P, T);
-    // the sums over f = 8 e + 4 l + z factor per eta index e:
-    //   A  = fca fcb sum_e ex_e sum_lz g' zeta lambda b^(zeta-1)
-    //   Ba = fcb sum_e ex_e (-2 eta_e ra fca + dfa) sum_lz g' b^zeta, Bb likewise
-    float A = 0.f, Ba = 0.f, Bb = 0.f;
+  // dE/dr_a = sum_b A (u_b - c u_a) / r_a + B u_a of the pairs; per lane the
+  // sums over its pairs of A u_b, A c and B
+  for (int a = lane; a - lane < S; a += 32) {
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    // lanes without a neighbour read the first one's, with weights 0
+    const int own = a < S ? a : 0;
+    const float4 *un = &nu[warp][own], *wn = &nw[warp][own];
+    const float4 ua = un[0], wa = a < S ? wn[0] : zero;
+    float vx = 0.f, vy = 0.f, vz = 0.f, vc = 0.f, vb = 0.f;
+    int from = lane;
+    lane_pairs(a, S, [&](int d, bool on) {
+      const float4 ub = un[d], wb = wn[d];
+      const float c = ua.x * ub.x + ua.y * ub.y + ua.z * ub.z;
+      const float2 base = ang_bases(c);
+      const float on0 = base.x > 0.f ? 1.f : 0.f, on1 = base.y > 0.f ? 1.f : 0.f;
+      const F2 b1 = f2(base.x, base.y), b2 = f2_mul(b1, b1), b4 = f2_mul(b2, b2),
+               b12 = f2_mul(f2_mul(b4, b4), b4);
+      float se[2], ae[2];
 #pragma unroll
-    for (int e = 0; e < 2; e++) {
-      float se = 0.f, ae = 0.f;
-#pragma unroll
-      for (int l = 0; l < 2; l++) {
-        const float on = T.b[l] > 0.f ? 1.f : 0.f;  // (1 + lambda cos) clipped at 0
-#pragma unroll
-        for (int z = 0; z < 4; z++) {
-          const int f = 8 * e + 4 * l + z;
-          se = fmaf(on * g[kRad + f], T.pz[l][z], se);
-          ae = fmaf(on * gzw[f], T.pz1[l][z], ae);
-        }
+      for (int e = 0; e < 2; e++) {
+        const float2 s =
+            f2_get(f2_fma(b1, f2_fma(b2, f2_fma(b12, g[e][3], g[e][2]), g[e][1]), g[e][0]));
+        const float2 q =
+            f2_get(f2_fma(b1, f2_fma(b2, f2_fma(b12, h[e][3], h[e][2]), h[e][1]), h[e][0]));
+        se[e] = fmaf(base.y, s.y, base.x * s.x);
+        ae[e] = fmaf(on1, q.y, on0 * q.x);
       }
-      const float eta = P.eta_a[8 * e];
-      A = fmaf(ae, T.ex[e], A);
-      se *= T.ex[e];
-      Ba = fmaf(se, fmaf(-2.f * eta * ra, fca, dfa), Ba);
-      Bb = fmaf(se, fmaf(-2.f * eta * rb, fcb, dfb), Bb);
+      // dE/dcos, and along a and b
+      float A = ae[0] * (wa.x * wb.x) + ae[1] * (wa.y * wb.y);
+      float Ba = se[0] * (wa.z * wb.x) + se[1] * (wa.w * wb.y);
+      float Bb = se[0] * (wa.x * wb.z) + se[1] * (wa.y * wb.w);
+      A = on ? A : 0.f;
+      Ba = on ? Ba : 0.f;
+      Bb = on ? Bb : 0.f;
+      const float Ac = A * c;
+      vx = fmaf(A, ub.x, vx);
+      vy = fmaf(A, ub.y, vy);
+      vz = fmaf(A, ub.z, vz);
+      vc += Ac;
+      vb += Ba;
+      if (S <= 32) {
+        // the pair that has this lane's neighbour as its b
+        from = from == 0 ? S - 1 : from - 1;
+        const float4 uo = un[S - d];
+        const float Ao = __shfl_sync(0xffffffffu, A, from);
+        vx = fmaf(Ao, uo.x, vx);
+        vy = fmaf(Ao, uo.y, vy);
+        vz = fmaf(Ao, uo.z, vz);
+        vc += __shfl_sync(0xffffffffu, Ac, from);
+        vb += __shfl_sync(0xffffffffu, Bb, from);
+      } else {
+        if (a < S) {  // distinct b
+          const int b = a + d < S ? a + d : a + d - S;
+          const float Ab = A * ub.w, Cb = fmaf(-Ac, ub.w, Bb);
+          fn[warp][0][b] -= fmaf(Ab, ua.x, Cb * ub.x);
+          fn[warp][1][b] -= fmaf(Ab, ua.y, Cb * ub.y);
+          fn[warp][2][b] -= fmaf(Ab, ua.z, Cb * ub.z);
+        }
+        __syncwarp();
+      }
+    });
+    if (a < S) {
+      const float Ca = fmaf(-vc, ua.w, vb);
+      fn[warp][0][a] -= fmaf(vx, ua.w, Ca * ua.x);
+      fn[warp][1][a] -= fmaf(vy, ua.w, Ca * ua.y);
+      fn[warp][2][a] -= fmaf(vz, ua.w, Ca * ua.z);
     }
-    A *= fca * fcb;
-    Ba *= fcb;
-    Bb *= fca;
-    // dc/dd_a = d_b / (ra rb) - c d_a / ra^2
-    const float gax = A * (N.dx[b] * irab - c * N.dx[a] * ia * ia) + Ba * N.dx[a] * ia;
-    const float gay = A * (N.dy[b] * irab - c * N.dy[a] * ia * ia) + Ba * N.dy[a] * ia;
-    const float gaz = A * (N.dz[b] * irab - c * N.dz[a] * ia * ia) + Ba * N.dz[a] * ia;
-    const float gbx = A * (N.dx[a] * irab - c * N.dx[b] * ib * ib) + Bb * N.dx[b] * ib;
-    const float gby = A * (N.dy[a] * irab - c * N.dy[b] * ib * ib) + Bb * N.dy[b] * ib;
-    const float gbz = A * (N.dz[a] * irab - c * N.dz[b] * ib * ib) + Bb * N.dz[b] * ib;
-    atomicAdd(&fn[warp][0][a], -gax);
-    atomicAdd(&fn[warp][1][a], -gay);
-    atomicAdd(&fn[warp][2][a], -gaz);
-    atomicAdd(&fn[warp][0][b], -gbx);
-    atomicAdd(&fn[warp][1][b], -gby);
-    atomicAdd(&fn[warp][2][b], -gbz);
-    fix += gax + gbx;
-    fiy += gay + gby;
-    fiz += gaz + gbz;
+    __syncwarp();
   }
-  __syncwarp();
+  for (int s = lane; s < S; s += 32) {
+    const float x = fn[warp][0][s], y = fn[warp][1][s], z = fn[warp][2][s];
+    atomicAdd(&F32[idx[warp][s]], make_float4(x, y, z, 0.f));
+    fix -= x;
+    fiy -= y;
+    fiz -= z;
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     fix += __shfl_xor_sync(0xffffffffu, fix, o);
     fiy += __shfl_xor_sync(0xffffffffu, fiy, o);
     fiz += __shfl_xor_sync(0xffffffffu, fiz, o);
   }
-  for (int s = lane; s < S; s += 32) {
-    atomicAdd(&F32[3 * N.idx[s]], fn[warp][0][s]);
-    atomicAdd(&F32[3 * N.idx[s] + 1], fn[warp][1][s]);
-    atomicAdd(&F32[3 * N.idx[s] + 2], fn[warp][2][s]);
-  }
-  if (lane == 0) {
-    atomicAdd(&F32[3 * i], fix);
-    atomicAdd(&F32[3 * i + 1], fiy);
-    atomicAdd(&F32[3 * i + 2], fiz);
-  }
+  if (lane == 0) atomicAdd(&F32[i], make_float4(fix, fiy, fiz, 0.f));
 }
 
 __global__ void k_sg_pos32(const md_double4* __restrict__ pos, int n, float4* __restrict__ out) {
@@ -470,7 +565,7 @@ __global__ void k_sg_pos32(const md_double4* __restrict__ pos, int n, float4* __
 
 // skip (optional, device): when set, the forces are not stored and
 // skipped (device, optional) counts the call once
-__global__ void k_sg_store(const float* __restrict__ F32, double* __restrict__ f3, int n,
+__global__ void k_sg_store(const float4* __restrict__ F32, double* __restrict__ f3, int n,
                            int accumulate, const int* __restrict__ skip,
                            int* __restrict__ skipped) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -479,7 +574,8 @@ __global__ void k_sg_store(const float* __restrict__ F32, double* __restrict__ f
     return;
   }
   if (k >= 3 * n) return;
-  f3[k] = accumulate ? f3[k] + (double)F32[k] : (double)F32[k];
+  const float v = ((const float*)F32)[k + k / 3];  // three of four
+  f3[k] = accumulate ? f3[k] + (double)v : (double)v;
 }
 
 // ---- the network: 32 -> 64 (tanh) -> 64 (tanh) -> 1, BF16 weights ----
@@ -805,91 +901,92 @@ __global__ void __launch_bounds__(128, 1)
 
 // q_if = sum_j (e_j - e_i) . dG_if/dd_j for the force residual e (n x 3),
 // written as v_if = scale * istd_f * q_if (the loss' sensitivity to dt/dx;
-// istd NULL: 1).  One warp per atom as k_sg_desc: lanes over neighbours,
-// then over neighbour pairs, each lane summing all 32 components, one
-// reduce-scatter at the end.  Per pair the 16 angular terms share
-//   K1 = fc_a fc_b (dc/dd_a . de_a + dc/dd_b . de_b) and, per eta index e,
-//   K2_e = fc_b (-2 eta_e r_a fc_a + dfc_a) u_a + fc_a (-2 eta_e r_b fc_b + dfc_b) u_b,
-// so q_f += pref_f ex_e (zeta_f lambda_f b^(zeta-1) K1 + b^zeta K2_e).
+// istd NULL: 1).  One warp per atom as k_sg_desc, each lane summing all 32
+// components, one reduce-scatter at the end.  With de_a = e_a - e_i and
+// s_a = u_a . de_a, the 16 angular terms of a pair share, per eta index e,
+//   K1_e = w_a w_b (u_b . de_a / r_a + u_a . de_b / r_b - c (s_a / r_a + s_b / r_b)),
+//   K2_e = w_b d_a s_a + w_a d_b s_b,
+// so q_f += pref_f (zeta_f lambda_f b^(zeta-1) K1_e + b^zeta K2_e).
 __global__ void __launch_bounds__(128)
     k_sg_ctrans(const md_double4* __restrict__ pos, int n, const uint32_t* __restrict__ sl,
                 const int* __restrict__ slen, double box, DescParams P,
                 const float* __restrict__ e3, float scale, const float* __restrict__ istd,
                 float* __restrict__ V) {
-  __shared__ NbrSm nb[4];
-  __shared__ float dex[4][kSgMax], dey[4][kSgMax], dez[4][kSgMax];
+  __shared__ float4 nu[4][kSgRow];  // unit vector, s / r
+  __shared__ float4 ne[4][kSgRow];  // de / r
+  __shared__ float4 nw[4][kSgRow];  // w, d s
+  __shared__ float4 nr[4][kSgMax];  // r and the radial terms' two factors
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int i = blockIdx.x * 4 + warp;
   if (i >= n) return;  // whole warp
-  NbrSm& N = nb[warp];
-  const int S = warp_load_nbrs(i, pos, sl, slen, box, P.rc, N);  // ends with __syncwarp
   const float eix = e3[3 * i], eiy = e3[3 * i + 1], eiz = e3[3 * i + 2];
-  float v[32];
-#pragma unroll
-  for (int f = 0; f < 32; f++) v[f] = 0.f;
-  for (int s = lane; s < S; s += 32) {
-    const int j = N.idx[s];
+  const int S = warp_nbrs(i, pos, sl, slen, box, P.fca,
+                          [&](int s, int S, int j, float ux, float uy, float uz, float r,
+                              float ir, float fc, float dfc) {
+    const AngNbr A = ang_nbr(r, fc, dfc, P);
     const float ex = e3[3 * j] - eix, ey = e3[3 * j + 1] - eiy, ez = e3[3 * j + 2] - eiz;
-    dex[warp][s] = ex;
-    dey[warp][s] = ey;
-    dez[warp][s] = ez;
-    const float ud = (N.dx[s] * ex + N.dy[s] * ey + N.dz[s] * ez) * N.ir[s];  // u . de
-#pragma unroll
-    for (int k = 0; k < kRad; k++) {
-      const float t = N.r[s] - P.rs[k];
-      v[k] += __expf(-P.eta_r * t * t) * (-2.f * P.eta_r * t * N.fc[s] + N.dfc[s]) * ud;
+    const float ud = ux * ex + uy * ey + uz * ez;
+    put_twice(nu[warp], s, S, make_float4(ux, uy, uz, ud * ir));
+    put_twice(ne[warp], s, S, make_float4(ex * ir, ey * ir, ez * ir, 0.f));
+    put_twice(nw[warp], s, S, make_float4(A.w[0], A.w[1], A.d[0] * ud, A.d[1] * ud));
+    nr[warp][s] = make_float4(r, -2.f * P.eta_r * fc * ud, dfc * ud, 0.f);
+  });
+  // radial functions: lane k and lane k + 16 share function k
+  float radial = 0.f;
+  {
+    const float rs = P.rs[lane & 15], m = -P.eta_r * kLog2e;
+    for (int s = lane >> 4; s < S; s += 2) {
+      const float4 q = nr[warp][s];
+      const float t = q.x - rs;
+      radial = fmaf(ex2(t * m * t), fmaf(q.y, t, q.z), radial);
     }
+    radial += __shfl_xor_sync(0xffffffffu, radial, 16);
   }
-  __syncwarp();
-  const int npair = S * (S - 1) / 2;
-  for (int k = lane; k < npair; k += 32) {
-    int a, b;
-    pair_of(k, S, a, b);
-    const float ra = N.r[a], rb = N.r[b];
-    const float ia = N.ir[a], ib = N.ir[b], irab = ia * ib;
-    const float dax = N.dx[a], day = N.dy[a], daz = N.dz[a];
-    const float dbx = N.dx[b], dby = N.dy[b], dbz = N.dz[b];
-    const float eax = dex[warp][a], eay = dey[warp][a], eaz = dez[warp][a];
-    const float ebx = dex[warp][b], eby = dey[warp][b], ebz = dez[warp][b];
-    const float c = (dax * dbx + day * dby + daz * dbz) * irab;
-    const float q2 = ra * ra + rb * rb;
-    const float pa = dax * eax + day * eay + daz * eaz;  // d_a . de_a
-    const float pb = dbx * ebx + dby * eby + dbz * ebz;
-    const float dca = (dbx * eax + dby * eay + dbz * eaz) * irab - c * pa * ia * ia;
-    const float dcb = (dax * ebx + day * eby + daz * ebz) * irab - c * pb * ib * ib;
-    const float ua = pa * ia, ub = pb * ib;
-    const float fca = N.fc[a], fcb = N.fc[b], dfa = N.dfc[a], dfb = N.dfc[b];
-    AngPair T;
-    ang_pair(c, q2, P, T);
-    const float K1 = fca * fcb * (dca + dcb);
+  F2 p[2][4];  // [e][z], over l
 #pragma unroll
-    for (int e = 0; e < 2; e++) {
-      const float eta = P.eta_a[8 * e];
-      const float K2 = fcb * fmaf(-2.f * eta * ra, fca, dfa) * ua +
-                       fca * fmaf(-2.f * eta * rb, fcb, dfb) * ub;
+  for (int z = 0; z < 4; z++) p[0][z] = p[1][z] = f2(0.f, 0.f);
+  for (int a = lane; a - lane < S; a += 32) {
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    // lanes without a neighbour read the first one's, with weights 0
+    const int own = a < S ? a : 0;
+    const float4 *un = &nu[warp][own], *en = &ne[warp][own], *wn = &nw[warp][own];
+    const float4 ua = un[0], ea = en[0], wa = a < S ? wn[0] : zero;
+    lane_pairs(a, S, [&](int d, bool on) {
+      const float4 ub = un[d], eb = en[d], wb = wn[d];
+      const float c = ua.x * ub.x + ua.y * ub.y + ua.z * ub.z;
+      float dc = (ub.x * ea.x + ub.y * ea.y + ub.z * ea.z) - c * ua.w +
+                 ((ua.x * eb.x + ua.y * eb.y + ua.z * eb.z) - c * ub.w);
+      const float2 base = ang_bases(c);
+      const F2 b1 = f2(base.x, base.y), b2 = f2_mul(b1, b1), b3 = f2_mul(b2, b1),
+               b4 = f2_mul(b2, b2), b8 = f2_mul(b4, b4), b12 = f2_mul(b8, b4);
+      const F2 pz[4] = {b1, b2, b4, f2_mul(b8, b8)};
+      // zeta lambda b^(zeta - 1)
+      const F2 dz[4] = {f2(base.x > 0.f ? 1.f : 0.f, base.y > 0.f ? -1.f : 0.f),
+                        f2_mul(b1, f2(2.f, -2.f)), f2_mul(b3, f2(4.f, -4.f)),
+                        f2_mul(f2_mul(b12, b3), f2(16.f, -16.f))};
 #pragma unroll
-      for (int l = 0; l < 2; l++) {
-        const float on = T.b[l] > 0.f ? T.ex[e] : 0.f;  // (1 + lambda cos) clipped at 0
+      for (int e = 0; e < 2; e++) {
+        const float wab = e ? wa.y * wb.y : wa.x * wb.x;
+        const float k1 = on ? wab * dc : 0.f;
+        const float k2 = on ? (e ? wa.w * wb.y + wa.y * wb.w : wa.z * wb.x + wa.x * wb.z) : 0.f;
+        const F2 K1 = f2(k1, k1), K2 = f2(k2, k2);
 #pragma unroll
-        for (int z = 0; z < 4; z++) {
-          const int f = 8 * e + 4 * l + z;
-          const float zl = (float)P.zeta[f] * P.lam[f];
-          v[kRad + f] += P.pref[f] * on * fmaf(zl * T.pz1[l][z], K1, T.pz[l][z] * K2);
-        }
+        for (int z = 0; z < 4; z++) p[e][z] = f2_fma(dz[z], K1, f2_fma(pz[z], K2, p[e][z]));
       }
-    }
+    });
   }
-  const float q = warp_reduce_scatter32(v);
+  const float angular = angular_sum(p, P);
+  const float q = lane < kRad ? radial : angular;
   V[(size_t)i * kDesc + lane] = scale * (istd ? istd[lane] : 1.f) * q;
 }
 
 // e = F_pred - F_exact (FP32) and sum e^2 into acc[0]
-__global__ void k_fm_resid(const float* __restrict__ F32, const double* __restrict__ fx, int n3,
+__global__ void k_fm_resid(const float4* __restrict__ F32, const double* __restrict__ fx, int n3,
                            float* __restrict__ e3, double* __restrict__ acc) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   double s = 0.0;
   if (k < n3) {
-    const float e = F32[k] - (float)fx[k];
+    const float e = ((const float*)F32)[k + k / 3] - (float)fx[k];  // three of four
     e3[k] = e;
     s = (double)e * e;
   }
@@ -1404,9 +1501,9 @@ __global__ void k_fh_probe(float* __restrict__ gcoef, long long n32, const float
 }
 
 // acc[0] += sum_k F[k]^2
-__global__ void k_sumsq(const float* __restrict__ F, int n3, double* __restrict__ acc) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  double s = k < n3 ? (double)F[k] * F[k] : 0.0;
+__global__ void k_sumsq(const float* __restrict__ F, long long m, double* __restrict__ acc) {
+  const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  double s = k < m ? (double)F[k] * F[k] : 0.0;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if ((threadIdx.x & 31) == 0) atomicAdd(acc, s);
@@ -1679,7 +1776,7 @@ int sur_descriptors(Surrogate& s, const md_double4* pos, int n, const RowWalker&
     h = 0;
     if ((e = sur_grow(s.t, h, n)) != cudaSuccess) return e;
     h = 0;
-    if ((e = sur_grow(s.F32, h, 3LL * n)) != cudaSuccess) return e;
+    if ((e = sur_grow(s.F32, h, n)) != cudaSuccess) return e;
     h = 0;
     if ((e = sur_grow(s.eatom, h, n)) != cudaSuccess) return e;
     h = 0;
@@ -1895,7 +1992,7 @@ int sur_forces(Surrogate& s, const md_double4* pos, int n, const RowWalker& w, d
     // models forces only, so the energy it reports is NaN
     k_fh_gscale<<<1, 32, 0, st>>>(s.istd_d, (float)fh_out_scale(s), s.fh_gs);
     fh_forward(s, s.X, n, s.gcoef, false, st);
-    cudaMemsetAsync(s.F32, 0, sizeof(float) * 3 * (size_t)n, st);
+    cudaMemsetAsync(s.F32, 0, sizeof(float4) * (size_t)n, st);
     k_sg_force<<<sblocks(n, 4), 128, 0, st>>>(pos, n, s.sl, s.slen, w.g.box, s.P, s.gcoef, s.F32);
     k_sg_store<<<sblocks(3LL * n, 256), 256, 0, st>>>(s.F32, f3, n, accumulate, skip,
                                                       declined_count);
@@ -1905,7 +2002,7 @@ int sur_forces(Surrogate& s, const md_double4* pos, int n, const RowWalker& w, d
   k_net_infer<<<(n + 127) / 128, 128, kSmInfer, st>>>(s.X, n, net_of(s), s.t, s.dtdx, s.status_d);
   k_sg_scale<<<sblocks(n, 256), 256, 0, st>>>(s.t, s.dtdx, n, s.mu, s.sigma, s.istd_d, s.gcoef,
                                               s.eatom);
-  cudaMemsetAsync(s.F32, 0, sizeof(float) * 3 * (size_t)n, st);
+  cudaMemsetAsync(s.F32, 0, sizeof(float4) * (size_t)n, st);
   k_sg_force<<<sblocks(n, 4), 128, 0, st>>>(pos, n, s.sl, s.slen, w.g.box, s.P, s.gcoef, s.F32);
   k_sg_store<<<sblocks(3LL * n, 256), 256, 0, st>>>(s.F32, f3, n, accumulate, skip,
                                                     declined_count);
@@ -2002,11 +2099,11 @@ int train_fh(Surrogate& s, int steps, float lr, int nmax, double* loss_e, double
     const SurConfig& c = s.cfgs[0];
     k_fh_probe<<<sblocks(32LL * c.n, 256), 256, 0, st>>>(s.gcoef, 32LL * c.n, s.istd_d,
                                                          s.seed);
-    cudaMemsetAsync(s.F32, 0, sizeof(float) * 3 * (size_t)c.n, st);
+    cudaMemsetAsync(s.F32, 0, sizeof(float4) * (size_t)c.n, st);
     k_sg_force<<<sblocks(c.n, 4), 128, 0, st>>>(c.pos, c.n, c.sl, c.slen, c.box, s.P, s.gcoef,
                                                 s.F32);
     cudaMemsetAsync(s.scratch, 0, sizeof(double), st);
-    k_sumsq<<<sblocks(3LL * c.n, 256), 256, 0, st>>>(s.F32, 3 * c.n, s.scratch);
+    k_sumsq<<<sblocks(4LL * c.n, 256), 256, 0, st>>>((const float*)s.F32, 4LL * c.n, s.scratch);
     double sq = 0;
     cudaMemcpyAsync(&sq, s.scratch, sizeof(double), cudaMemcpyDeviceToHost, st);
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
@@ -2021,7 +2118,7 @@ int train_fh(Surrogate& s, int steps, float lr, int nmax, double* loss_e, double
     const SurConfig& c = s.cfgs[(it * 7919 + (int)(s.seed % 101)) % ncfg];
     const int n = c.n;
     fh_forward(s, c.X, n, s.gcoef, true, st);
-    cudaMemsetAsync(s.F32, 0, sizeof(float) * 3 * (size_t)n, st);
+    cudaMemsetAsync(s.F32, 0, sizeof(float4) * (size_t)n, st);
     k_sg_force<<<sblocks(n, 4), 128, 0, st>>>(c.pos, n, c.sl, c.slen, c.box, s.P, s.gcoef,
                                                 s.F32);
     cudaMemsetAsync(s.scratch, 0, sizeof(double) * 2, st);
@@ -2148,7 +2245,7 @@ int sur_train_fm(Surrogate& s, int steps, float lr, double* loss_e, double* loss
     h = 0;
     if ((e = sur_grow(s.t, h, nmax)) != cudaSuccess) return e;
     h = 0;
-    if ((e = sur_grow(s.F32, h, 3LL * nmax)) != cudaSuccess) return e;
+    if ((e = sur_grow(s.F32, h, nmax)) != cudaSuccess) return e;
     h = 0;
     if ((e = sur_grow(s.eatom, h, nmax)) != cudaSuccess) return e;
     h = 0;
@@ -2192,7 +2289,7 @@ int sur_train_fm(Surrogate& s, int steps, float lr, double* loss_e, double* loss
     k_net_infer<<<tiles, 128, kSmInfer, st>>>(c.X, n, w, s.t, s.dtdx, s.status_d);
     k_sg_scale<<<sblocks(n, 256), 256, 0, st>>>(s.t, s.dtdx, n, s.mu, s.sigma, s.istd_d,
                                                 s.gcoef, s.eatom);
-    cudaMemsetAsync(s.F32, 0, sizeof(float) * 3 * (size_t)n, st);
+    cudaMemsetAsync(s.F32, 0, sizeof(float4) * (size_t)n, st);
     k_sg_force<<<sblocks(n, 4), 128, 0, st>>>(c.pos, n, c.sl, c.slen, c.box, s.P, s.gcoef,
                                                 s.F32);
     cudaMemsetAsync(s.scratch, 0, sizeof(double) * 2, st);

@@ -15,7 +15,7 @@ constexpr int kSurDesc = 32;  // 16 radial + 16 angular symmetry functions
 // G4_f = pref_f sum_{j<k} (1 + lam_f cos) ^ zeta_f exp(-eta_f (rj^2 + rk^2))
 // fc(rj) fc(rk), fc(r) = (cos(pi r / rc) + 1) / 2 for r < rc.
 struct DescParams {
-  float rc;
+  float rc, fca;  // cutoff, pi / rc
   float eta_r;
   float rs[16];
   float eta_a[16], lam[16], pref[16];
@@ -57,7 +57,8 @@ struct md_surrogate {
   long long n_sl = 0;
   uint32_t* sl = nullptr;
   int* slen = nullptr;
-  float *X = nullptr, *t = nullptr, *dtdx = nullptr, *gcoef = nullptr, *F32 = nullptr;
+  float *X = nullptr, *t = nullptr, *dtdx = nullptr, *gcoef = nullptr;
+  float4* F32 = nullptr;           // forces, x y z 0
   float4* pos32 = nullptr;         // FP32 positions for the neighbour search
   double* eatom = nullptr;
   // training samples: raw descriptors and exact per-atom energies
