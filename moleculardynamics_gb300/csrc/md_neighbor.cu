@@ -175,74 +175,6 @@ __global__ void k_pos_build(const md_double4* __restrict__ pos, int n, float4* _
   pb[i] = make_float4((float)p.x, (float)p.y, (float)p.z, __int_as_float((int)p.w));
 }
 
-// The candidates of row i by a warp, 32 at a time in the reference's order: 27
-// lanes look up the cells around the atom's own, and a warp scan joins them into
-// one sequence.  visit(valid, m, im) runs in all lanes; im holds the image's
-// three 2-bit fields.  Returns the number of candidates.
-template <typename F>
-__device__ __forceinline__ int warp_row(const RowWalker& w, const md_double4* __restrict__ pos,
-                                        int i, int lane, F&& visit) {
-  const bool whole = w.g.periodic && w.g.cells == 1;  // minimum images of all atoms
-  int first = 0, count = 0, img = 0;  // this lane's cell
-  if (!whole && lane < 27) {
-    const int4 c4 = reinterpret_cast<const int4*>(w.cell3)[i];
-    int nc[3] = {c4.x + lane / 9 - 1, c4.y + lane / 3 % 3 - 1, c4.z + lane % 3 - 1};
-    bool out = false;
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-      if (!w.g.periodic) {
-        out |= nc[d] >= w.g.cells || nc[d] < 0;
-      } else if (nc[d] < 0) {
-        nc[d] += w.g.cells;
-        img |= 3 << (2 * d);
-      } else if (nc[d] >= w.g.cells) {
-        nc[d] -= w.g.cells;
-        img |= 1 << (2 * d);
-      }
-    }
-    const int s = out ? -1 : table_find(w.keys, w.cap, cell_key(nc[0], nc[1], nc[2]));
-    if (s >= 0) {
-      first = w.start[s];
-      count = w.count[s];
-    }
-  }
-  int pre = count;  // inclusive, then exclusive
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, pre, o);
-    if (lane >= o) pre += y;
-  }
-  const int total = whole ? w.n : __shfl_sync(0xffffffffu, pre, 31);
-  pre -= count;
-  const md_double4 ei = whole ? pos[i] : md_double4{0, 0, 0, 0};
-  int self = 0;
-  for (int q0 = 0; q0 < total; q0 += 32) {
-    const int q = q0 + lane;
-    int m = q, im = 0;
-    if (!whole) {
-      // the last cell that starts at or before q
-      int c = 0;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const int p = __shfl_sync(0xffffffffu, pre, (c + o) & 31);
-        if (c + o < 27 && p <= q) c += o;
-      }
-      const int p = __shfl_sync(0xffffffffu, pre, c), f = __shfl_sync(0xffffffffu, first, c);
-      im = __shfl_sync(0xffffffffu, img, c);
-      if (q < total) m = w.sorted[f + q - p];
-    }
-    const bool valid = q < total && m != i;
-    if (q < total && m == i) self = 1;
-    if (valid && whole) {
-      const md_double4 em = pos[m];
-      im = (min_image(ei.x, em.x, w.g.box) & 3) | ((min_image(ei.y, em.y, w.g.box) & 3) << 2) |
-           ((min_image(ei.z, em.z, w.g.box) & 3) << 4);
-    }
-    visit(valid, m, im);
-  }
-  return total - (__any_sync(0xffffffffu, self) ? 1 : 0);
-}
-
 // Rows, a warp per atom; the lanes test 32 candidates at a time (a ballot keeps
 // the order).  MODE 0 counts (len[i] and maxima), 1 writes, 2 does both, with
 // rows longer than cap truncated and reported through the counters.  An entry k
@@ -259,7 +191,7 @@ __global__ void __launch_bounds__(128)
   if (i >= w.n) return;  // whole warp
   const float4 pi = pb[i];
   int kept = 0;
-  const int full = warp_row(w, pos, i, lane, [&](bool keep, int m, int im) {
+  const int full = warp_row<true>(w, pos, i, lane, [&](bool keep, int m, int im) {
     const uint32_t e = (uint32_t)m | ((uint32_t)im << kIndexBits);
     if (keep && compact) {
       const float4 pm = pb[m];
@@ -294,7 +226,7 @@ __global__ void __launch_bounds__(128)
   int* row = out + (size_t)i * nls;
   signed char* im_row = img ? img + (size_t)i * nls : nullptr;
   int count = 0;
-  warp_row(w, pos, i, lane, [&](bool valid, int m, int im) {
+  warp_row<true>(w, pos, i, lane, [&](bool valid, int m, int im) {
     const unsigned mask = __ballot_sync(0xffffffffu, valid);
     const int k = count + __popc(mask & ((1u << lane) - 1u));
     if (valid && k < nls) {

@@ -79,6 +79,81 @@ __device__ __forceinline__ void walk_row(const RowWalker& w, const md_double4* p
       }
 }
 
+// The candidates of row i by a warp of a block of 128 threads, 32 at a time in
+// the reference's order: 27 lanes look up the cells around the atom's own, a warp
+// scan joins the occupied ones into one sequence, and per 32 candidates the cells
+// that start among them are a mask from which each lane counts its own (a binary
+// search by shuffles took @R@).
+// visit(valid, m, im) runs in all lanes; im holds the image's three 2-bit fields.
+// Returns the number of candidates.  MIN_IMAGE: a periodic box of one cell takes
+// the minimum images of all atoms, as walk_row does.
+template <bool MIN_IMAGE, typename F>
+__device__ __forceinline__ int warp_row(const RowWalker& w, const md_double4* __restrict__ pos,
+                                        int i, int lane, F&& visit) {
+  __shared__ int2 cell[4][27];  // of the occupied cells: first atom - start, image
+  int2* cw = cell[threadIdx.x >> 5];
+  const bool whole = MIN_IMAGE && w.g.periodic && w.g.cells == 1;
+  int first = 0, count = 0, img = 0;  // this lane's cell
+  if (!whole && lane < 27) {
+    const int4 c4 = reinterpret_cast<const int4*>(w.cell3)[i];
+    int nc[3] = {c4.x + lane / 9 - 1, c4.y + lane / 3 % 3 - 1, c4.z + lane % 3 - 1};
+    bool out = false;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      if (!w.g.periodic) {
+        out |= nc[d] >= w.g.cells || nc[d] < 0;
+      } else if (nc[d] < 0) {
+        nc[d] += w.g.cells;
+        img |= 3 << (2 * d);
+      } else if (nc[d] >= w.g.cells) {
+        nc[d] -= w.g.cells;
+        img |= 1 << (2 * d);
+      }
+    }
+    const int s = out ? -1 : table_find(w.keys, w.cap, cell_key(nc[0], nc[1], nc[2]));
+    if (s >= 0) {
+      first = w.start[s];
+      count = w.count[s];
+    }
+  }
+  int pre = count;  // inclusive, then exclusive
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, pre, o);
+    if (lane >= o) pre += y;
+  }
+  const int total = whole ? w.n : __shfl_sync(0xffffffffu, pre, 31);
+  pre -= count;
+  const unsigned used = __ballot_sync(0xffffffffu, count > 0);
+  if (count > 0) cw[__popc(used & ((1u << lane) - 1u))] = make_int2(first - pre, img);
+  __syncwarp();
+  md_double4 ei = md_double4{0, 0, 0, 0};
+  if (MIN_IMAGE && whole) ei = pos[i];
+  int self = 0, before = -1;
+  for (int q0 = 0; q0 < total; q0 += 32) {
+    const int q = q0 + lane;
+    int m = q, im = 0;
+    if (!whole) {
+      const unsigned at = (unsigned)(pre - q0);
+      const unsigned starts =
+          __reduce_or_sync(0xffffffffu, count > 0 && at < 32u ? 1u << at : 0u);
+      const int2 c = cw[before + __popc(starts & (0xffffffffu >> (31 - lane)))];
+      before += __popc(starts);
+      im = c.y;
+      if (q < total) m = w.sorted[c.x + q];
+    }
+    const bool valid = q < total && m != i;
+    if (q < total && m == i) self = 1;
+    if (MIN_IMAGE && valid && whole) {
+      const md_double4 em = pos[m];
+      im = (min_image(ei.x, em.x, w.g.box) & 3) | ((min_image(ei.y, em.y, w.g.box) & 3) << 2) |
+           ((min_image(ei.z, em.z, w.g.box) & 3) << 4);
+    }
+    visit(valid, m, im);
+  }
+  return total - (__any_sync(0xffffffffu, self) ? 1 : 0);
+}
+
 // Is j in the full candidate row of k (27-cell adjacency of build-time
 // cells)?  img receives the periodic image of j in k's row, as walk_row
 // produces it.  Periodic boxes need at least 3 cells per axis here.
