@@ -83,7 +83,7 @@ __device__ __forceinline__ void walk_row(const RowWalker& w, const md_double4* p
 // the reference's order: 27 lanes look up the cells around the atom's own, a warp
 // scan joins the occupied ones into one sequence, and per 32 candidates the cells
 // that start among them are a mask from which each lane counts its own (a binary
-// search by shuffles took @R@).
+// search by shuffles took 15% more instructions).
 // visit(valid, m, im) runs in all lanes; im holds the image's three 2-bit fields.
 // Returns the number of candidates.  MIN_IMAGE: a periodic box of one cell takes
 // the minimum images of all atoms, as walk_row does.

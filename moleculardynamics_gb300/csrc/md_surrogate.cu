@@ -526,65 +526,92 @@ __global__ void k_sg_store(const float4* __restrict__ F32, double* __restrict__ 
 }
 
 // ---- the network: 32 -> 64 (tanh) -> 64 (tanh) -> 1, BF16 weights ----
-// Device weight copies for the tensor cores, K-major B operands:
-// W1 [64 out][32 in], W1T [32 in][64 out], W2 [64 out][64 in], W2T [64 in][64 out].
+// Device weight copies for the tensor cores: W1 [64 out][32 in], W2 [64 out][64 in].
+// A tile serves as K-major operand and, read across its rows, as the transposed
+// one (tc_product), so the backward products and the sums over rows need no
+// transposed copies: those were written two bytes at a time with four-way bank
+// conflicts and kept a block's shared memory at 104 and 180 KB.
 struct NetDev {
-  const __nv_bfloat16 *W1, *W1T, *W2, *W2T;
+  const __nv_bfloat16 *W1, *W2;
   const float* P;  // FP32 master parameters (biases and w3 used from here)
 };
 
-// shared-memory plan of the network kernels (bytes)
-constexpr int kSmA = 0;                  // 128 x 64 BF16 operand (16 KB)
-constexpr int kSmB = kSmA + 16384;       // 128 x 64 BF16 operand (16 KB)
-constexpr int kSmW1 = kSmB + 16384;      // 64 x 32 (4 KB)
-constexpr int kSmW1T = kSmW1 + 4096;     // 32 x 64 (4 KB)
-constexpr int kSmW2 = kSmW1T + 4096;     // 64 x 64 (8 KB)
-constexpr int kSmW2T = kSmW2 + 8192;     // 64 x 64 (8 KB)
-constexpr int kSmAT = kSmW2T + 8192;     // training: 128 x 128 BF16 (32 KB)
-constexpr int kSmBT = kSmAT + 32768;     // training: 64 x 128 BF16 (16 KB)
-constexpr int kSmTrain = kSmBT + 16384;  // 104 KB
-constexpr int kSmALo = kSmAT;            // inference: low BF16 parts of A / B operands
-constexpr int kSmBLo = kSmALo + 16384;
-constexpr int kSmInfer = kSmBLo + 16384; // 88 KB
+constexpr int kTileX = 8192, kTileH = 16384;    // 128 x 32 and 128 x 64 BF16
+constexpr int kTileW1 = 4096, kTileW2 = 8192;   // 64 x 32 and 64 x 64
+constexpr int kSmTail = 2048;                   // read behind the last transposed tile
+// shared-memory plans (bytes): weights first, then the operands
+constexpr int kSmOps = kTileW1 + kTileW2;
+constexpr int kSmInfer = kSmOps + 4 * kTileH;
+constexpr int kSmTrain = kSmOps + kTileX + 2 * kTileH + kSmTail;
+constexpr int kSmForce = kSmOps + 2 * kTileX + 4 * kTileH + kSmTail;
 
-__device__ __forceinline__ void put_bf16(unsigned char* base, int r, int k, int K, float v) {
-  *(__nv_bfloat16*)(base + tc_offset(r, k, K)) = __float2bfloat16_rn(v);
+__device__ __forceinline__ uint32_t bf16_pair(float a, float b) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+  return *(const uint32_t*)&v;
 }
 
-// weights (row-major BF16 R x K in global) into the K-major tile layout
+// eight values of a row from column k (a multiple of 8), one 16-byte store
+__device__ __forceinline__ void put8(unsigned char* tile, int r, int k, int K, const float* v) {
+  *(uint4*)(tile + tc_offset(r, k, K)) =
+      make_uint4(bf16_pair(v[0], v[1]), bf16_pair(v[2], v[3]), bf16_pair(v[4], v[5]),
+                 bf16_pair(v[6], v[7]));
+}
+
+// weights (row-major BF16 R x K in global) into the tile layout
 __device__ __forceinline__ void load_tile(unsigned char* dst, const __nv_bfloat16* src, int R,
                                           int K) {
-  for (int e = threadIdx.x; e < R * K; e += blockDim.x)
-    *(__nv_bfloat16*)(dst + tc_offset(e / K, e % K, K)) = src[e];
+  for (int e = threadIdx.x; e < R * K / 8; e += blockDim.x)
+    *(uint4*)(dst + tc_offset(e / (K / 8), e % (K / 8) * 8, K)) = ((const uint4*)src)[e];
+}
+
+// this thread's row of 32 values (zeros where it has none)
+__device__ __forceinline__ void load_row(float (&x)[kDesc], const float* X, size_t row,
+                                         bool live) {
+#pragma unroll
+  for (int q = 0; q < kDesc / 4; q++) {
+    const float4 v = live ? ((const float4*)(X + row * kDesc))[q] : make_float4(0.f, 0.f, 0.f, 0.f);
+    x[4 * q] = v.x, x[4 * q + 1] = v.y, x[4 * q + 2] = v.z, x[4 * q + 3] = v.w;
+  }
+}
+
+// biases and output weights in shared memory: b1, b2, w3, b3
+struct NetBias {
+  float b1[kHid], b2[kHid], w3[kHid], b3;
+};
+__device__ __forceinline__ void load_bias(NetBias& b, const float* P) {
+  const int t = threadIdx.x;
+  if (t < kHid) {
+    b.b1[t] = P[oB1 + t];
+    b.b2[t] = P[oB2 + t];
+    b.w3[t] = P[oW3 + t];
+  }
+  if (t == 0) b.b3 = P[oB3];
 }
 
 // a value as the sum of two BF16 numbers (hi = round(v), lo = round(v - hi)):
 // products of hi and lo parts with BF16 weights keep the network input and
 // hidden activations to about 16 significant bits, so the energy is a smooth
 // function of the positions and the forces are its gradient
-__device__ __forceinline__ void put_split(unsigned char* hi, unsigned char* lo, int r, int k,
-                                          int K, float v) {
-  const __nv_bfloat16 h = __float2bfloat16_rn(v);
-  *(__nv_bfloat16*)(hi + tc_offset(r, k, K)) = h;
-  *(__nv_bfloat16*)(lo + tc_offset(r, k, K)) = __float2bfloat16_rn(v - __bfloat162float(h));
+__device__ __forceinline__ void put8_split(unsigned char* hi, unsigned char* lo, int r, int k,
+                                           int K, const float* v) {
+  float rest[8];
+#pragma unroll
+  for (int q = 0; q < 8; q++) rest[q] = v[q] - __bfloat162float(__float2bfloat16_rn(v[q]));
+  put8(hi, r, k, K, v);
+  put8(lo, r, k, K, rest);
 }
 
 // operands written by threads -> visible to the tensor core; then one thread
-// issues the product (A + Alo when given) and all wait for its completion
-__device__ __forceinline__ bool tc_run(uint32_t d, const unsigned char* A, const unsigned char* B,
-                                       int N, int K, uint64_t* bar, uint32_t& phase,
-                                       int* status, const unsigned char* Alo = nullptr) {
+// issues products and all wait for their completion
+template <typename F>
+__device__ __forceinline__ bool tc_run(uint64_t* bar, uint32_t& phase, int* status, F&& issue) {
   fence_proxy_async();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   if (threadIdx.x == 0) {
-    if (Alo) {
-      tc_gemm_issue(d, A, B, N, K, nullptr);
-      tc_gemm_issue(d, Alo, B, N, K, bar, true);
-    } else {
-      tc_gemm_issue(d, A, B, N, K, bar);
-    }
+    issue();
+    tc_commit(bar);
   }
   const bool ok = mbar_wait(bar, phase, status);
   phase ^= 1u;
@@ -599,27 +626,29 @@ __device__ __forceinline__ float tanh_fast(float x) {
 
 // Inference on 128 atoms per CTA: t_i = net(x_i) and dt/dx_i (4 tensor-core
 // products: two forward, two for the input gradient; every A operand as a
-// pair of BF16 parts).
-__global__ void __launch_bounds__(128, 1)
+// pair of BF16 parts).  Latency of the chain of products, tensor-memory reads and
+// operand stores bounds it: 43 us for 32,768 atoms with two-byte stores and
+// loads a row apart, 31 now.
+__global__ void __launch_bounds__(128)
     k_net_infer(const float* __restrict__ X, int n, NetDev w, float* __restrict__ t_out,
                 float* __restrict__ dtdx, int* status) {
   extern __shared__ __align__(1024) unsigned char sm[];
   __shared__ __align__(8) uint64_t bar;
   __shared__ uint32_t s_taddr;
+  __shared__ NetBias bias;
   const int tid = threadIdx.x, warp = tid >> 5;
   const int row = 32 * warp + (tid & 31);
   const int i = blockIdx.x * 128 + row;
   const bool live = i < n;
-  unsigned char* A = sm + kSmA;
-  unsigned char* B = sm + kSmB;
-  unsigned char* Al = sm + kSmALo;
-  unsigned char* Bl = sm + kSmBLo;
-  load_tile(sm + kSmW1, w.W1, kHid, kDesc);
-  load_tile(sm + kSmW1T, w.W1T, kDesc, kHid);
-  load_tile(sm + kSmW2, w.W2, kHid, kHid);
-  load_tile(sm + kSmW2T, w.W2T, kHid, kHid);
-  for (int f = 0; f < kDesc; f++)
-    put_split(A, Al, row, f, kDesc, live ? X[(size_t)i * kDesc + f] : 0.f);
+  unsigned char *W1 = sm, *W2 = W1 + kTileW1;
+  unsigned char *A = W2 + kTileW2, *Al = A + kTileH, *B = Al + kTileH, *Bl = B + kTileH;
+  float x[kDesc];
+  load_row(x, X, i, live);
+  load_tile(W1, w.W1, kHid, kDesc);
+  load_tile(W2, w.W2, kHid, kHid);
+  load_bias(bias, w.P);
+#pragma unroll
+  for (int f = 0; f < kDesc; f += 8) put8_split(A, Al, row, f, kDesc, x + f);
   if (warp == 0) tc_alloc(&s_taddr, 128);
   if (tid == 0) {
     mbar_init(&bar, 1);
@@ -628,47 +657,63 @@ __global__ void __launch_bounds__(128, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tm = s_taddr + ((uint32_t)(32 * warp) << 16);
+  const uint32_t T = s_taddr, tm = T + ((uint32_t)(32 * warp) << 16);
   uint32_t phase = 0;
-  bool ok = tc_run(s_taddr, A, sm + kSmW1, kHid, kDesc, &bar, phase, status, Al);
+  bool ok = tc_run(&bar, phase, status, [&] {
+    tc_product<false, false>(T, A, kDesc, W1, kDesc, kHid, kDesc);
+    tc_product<false, false>(T, Al, kDesc, W1, kDesc, kHid, kDesc, true);
+  });
   float h1[kHid];
   if (ok) {
+#pragma unroll
     for (int c0 = 0; c0 < kHid; c0 += 16) {
       float v[16];
       tc_ld16(tm + c0, v);
 #pragma unroll
-      for (int k = 0; k < 16; k++) {
-        h1[c0 + k] = tanh_fast(v[k] + w.P[oB1 + c0 + k]);
-        put_split(B, Bl, row, c0 + k, kHid, h1[c0 + k]);
-      }
+      for (int k = 0; k < 16; k++) h1[c0 + k] = tanh_fast(v[k] + bias.b1[c0 + k]);
+      put8_split(B, Bl, row, c0, kHid, h1 + c0);
+      put8_split(B, Bl, row, c0 + 8, kHid, h1 + c0 + 8);
     }
-    ok = tc_run(s_taddr + 64, B, sm + kSmW2, kHid, kHid, &bar, phase, status, Bl);
+    ok = tc_run(&bar, phase, status, [&] {
+      tc_product<false, false>(T + 64, B, kHid, W2, kHid, kHid, kHid);
+      tc_product<false, false>(T + 64, Bl, kHid, W2, kHid, kHid, kHid, true);
+    });
   }
   if (ok) {
-    float t = w.P[oB3];
+    float t = bias.b3;
+#pragma unroll
     for (int c0 = 0; c0 < kHid; c0 += 16) {
       float v[16];
       tc_ld16(tm + 64 + c0, v);
 #pragma unroll
       for (int k = 0; k < 16; k++) {
-        const float h2 = tanh_fast(v[k] + w.P[oB2 + c0 + k]);
-        const float w3 = w.P[oW3 + c0 + k];
+        const float h2 = tanh_fast(v[k] + bias.b2[c0 + k]), w3 = bias.w3[c0 + k];
         t = fmaf(w3, h2, t);
-        put_split(A, Al, row, c0 + k, kHid, w3 * (1.f - h2 * h2));  // delta2
+        v[k] = w3 * (1.f - h2 * h2);  // delta2
       }
+      put8_split(A, Al, row, c0, kHid, v);
+      put8_split(A, Al, row, c0 + 8, kHid, v + 8);
     }
     if (live) t_out[i] = t;
-    ok = tc_run(s_taddr, A, sm + kSmW2T, kHid, kHid, &bar, phase, status, Al);
+    ok = tc_run(&bar, phase, status, [&] {  // delta2 W2
+      tc_product<false, true>(T, A, kHid, W2, kHid, kHid, kHid);
+      tc_product<false, true>(T, Al, kHid, W2, kHid, kHid, kHid, true);
+    });
   }
   if (ok) {
+#pragma unroll
     for (int c0 = 0; c0 < kHid; c0 += 16) {
       float v[16];
       tc_ld16(tm + c0, v);
 #pragma unroll
-      for (int k = 0; k < 16; k++)
-        put_split(B, Bl, row, c0 + k, kHid, v[k] * (1.f - h1[c0 + k] * h1[c0 + k]));  // delta1
+      for (int k = 0; k < 16; k++) v[k] *= 1.f - h1[c0 + k] * h1[c0 + k];  // delta1
+      put8_split(B, Bl, row, c0, kHid, v);
+      put8_split(B, Bl, row, c0 + 8, kHid, v + 8);
     }
-    ok = tc_run(s_taddr + 64, B, sm + kSmW1T, kDesc, kHid, &bar, phase, status, Bl);
+    ok = tc_run(&bar, phase, status, [&] {  // delta1 W1
+      tc_product<false, true>(T + 64, B, kHid, W1, kDesc, kDesc, kHid);
+      tc_product<false, true>(T + 64, Bl, kHid, W1, kDesc, kDesc, kHid, true);
+    });
   }
   if (ok) {  // every lane reads (tcgen05.ld is warp-collective); live rows store
     for (int c0 = 0; c0 < kDesc; c0 += 16) {
@@ -676,13 +721,15 @@ __global__ void __launch_bounds__(128, 1)
       tc_ld16(tm + 64 + c0, v);
       if (live) {
 #pragma unroll
-        for (int k = 0; k < 16; k++) dtdx[(size_t)i * kDesc + c0 + k] = v[k];
+        for (int k = 0; k < 16; k += 4)
+          *(float4*)&dtdx[(size_t)i * kDesc + c0 + k] =
+              make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
       }
     }
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tc_dealloc(s_taddr, 128);
+  if (warp == 0) tc_dealloc(T, 128);
 }
 
 // 64-bit mix of (seed, k) for batch sampling
@@ -699,11 +746,45 @@ __device__ __forceinline__ float col_sum(float v) {
   return v;
 }
 
+// sums of 16 columns over the warp's rows, added to out[0..15]: a column per lane
+// (80 shuffles one column after another, 16 this way)
+__device__ __forceinline__ void add_cols16(float (&v)[16], float* out) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int k = 0; k < o; k++) {
+      const float send = up ? v[k] : v[k + o];
+      const float keep = up ? v[k + o] : v[k];
+      v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  const float s = v[0] + __shfl_xor_sync(0xffffffffu, v[0], 16);
+  if (lane < 16) atomicAdd(&out[lane], s);
+}
+
+// rows 0..63 of a weight gradient from tensor memory (warps 0 and 1), added to
+// out (row-major, `cols` wide) 16 bytes at a time
+__device__ __forceinline__ void add_weights(uint32_t taddr, int row, int cols, float* out) {
+  for (int c0 = 0; c0 < cols; c0 += 16) {
+    float v[16];
+    tc_ld16(taddr + c0, v);
+#pragma unroll
+    for (int q = 0; q < 16; q += 4)
+      atomicAdd((float4*)&out[row * cols + c0 + q],
+                make_float4(v[q], v[q + 1], v[q + 2], v[q + 3]));
+  }
+}
+
 // One training pass over 128 samples per CTA: forward, squared loss on the
 // normalised per-atom energy, backward; gradients are accumulated into grad
 // (FP32, same layout as the parameters) and loss into loss[0].
 // Samples: rows sel(k) of X/T, sel = explicit list, or hashed from seed.
-__global__ void __launch_bounds__(128, 1)
+// Latency bounds it; three blocks fit on an SM (one shared-memory transposed
+// copy of each operand, a chain of shuffles and an atomic for each of 192
+// columns took 127 us for 32,768 rows, now 48).
+__global__ void __launch_bounds__(128)
     k_net_train(const float* __restrict__ X, const float* __restrict__ T, int nsamples,
                 const int* __restrict__ rows, int nrows, unsigned long long seed, NetDev w,
                 float inv_batch, float* __restrict__ grad, double* __restrict__ loss,
@@ -711,26 +792,26 @@ __global__ void __launch_bounds__(128, 1)
   extern __shared__ __align__(1024) unsigned char sm[];
   __shared__ __align__(8) uint64_t bar;
   __shared__ uint32_t s_taddr;
+  __shared__ NetBias bias;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int row = 32 * warp + lane;
   const int k = blockIdx.x * 128 + row;
   const bool live = k < nrows;
   int src = 0;
   if (live) src = rows ? rows[k] : (int)(mix2(seed, (unsigned long long)k) % (unsigned long long)nsamples);
-  unsigned char* A = sm + kSmA;
-  unsigned char* B = sm + kSmB;
-  unsigned char* AT = sm + kSmAT;
-  unsigned char* BT = sm + kSmBT;
-  load_tile(sm + kSmW1, w.W1, kHid, kDesc);
-  load_tile(sm + kSmW2, w.W2, kHid, kHid);
-  load_tile(sm + kSmW2T, w.W2T, kHid, kHid);
-  for (int e = tid; e < 32768 / 16; e += blockDim.x) ((uint4*)AT)[e] = make_uint4(0, 0, 0, 0);
-  float x[kDesc];
-  for (int f = 0; f < kDesc; f++) {
-    x[f] = live ? X[(size_t)src * kDesc + f] : 0.f;
-    put_bf16(A, row, f, kDesc, x[f]);
+  unsigned char *W1 = sm, *W2 = W1 + kTileW1;
+  // inputs, hidden activations, deltas (the transposed operands read behind D)
+  unsigned char *XS = W2 + kTileW2, *H = XS + kTileX, *D = H + kTileH;
+  {
+    float x[kDesc];
+    load_row(x, X, src, live);
+#pragma unroll
+    for (int f = 0; f < kDesc; f += 8) put8(XS, row, f, kDesc, x + f);
   }
-  if (warp == 0) tc_alloc(&s_taddr, 256);
+  load_tile(W1, w.W1, kHid, kDesc);
+  load_tile(W2, w.W2, kHid, kHid);
+  load_bias(bias, w.P);
+  if (warp == 0) tc_alloc(&s_taddr, 128);
   if (tid == 0) {
     mbar_init(&bar, 1);
     fence_mbar_init();
@@ -738,112 +819,86 @@ __global__ void __launch_bounds__(128, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tm = s_taddr + ((uint32_t)(32 * warp) << 16);
+  const uint32_t T0 = s_taddr, tm = T0 + ((uint32_t)(32 * warp) << 16);
   uint32_t phase = 0;
   float h1[kHid];
-  bool ok = tc_run(s_taddr, A, sm + kSmW1, kHid, kDesc, &bar, phase, status);
+  bool ok = tc_run(&bar, phase, status, [&] {
+    tc_product<false, false>(T0, XS, kDesc, W1, kDesc, kHid, kDesc);
+  });
   if (ok) {
+#pragma unroll
     for (int c0 = 0; c0 < kHid; c0 += 16) {
       float v[16];
       tc_ld16(tm + c0, v);
 #pragma unroll
-      for (int q = 0; q < 16; q++) {
-        const int c = c0 + q;
-        h1[c] = tanh_fast(v[q] + w.P[oB1 + c]);
-        put_bf16(B, row, c, kHid, h1[c]);
-        put_bf16(BT, c, row, 128, h1[c]);  // H1^T: B operand of the W2 gradient
-      }
+      for (int q = 0; q < 16; q++) h1[c0 + q] = tanh_fast(v[q] + bias.b1[c0 + q]);
+      put8(H, row, c0, kHid, h1 + c0);
+      put8(H, row, c0 + 8, kHid, h1 + c0 + 8);
     }
-    ok = tc_run(s_taddr + 64, B, sm + kSmW2, kHid, kHid, &bar, phase, status);
+    ok = tc_run(&bar, phase, status, [&] {
+      tc_product<false, false>(T0 + 64, H, kHid, W2, kHid, kHid, kHid);
+    });
   }
-  float d3 = 0.f;
   if (ok) {
     float h2[kHid];
-    float t = w.P[oB3];
+    float t = bias.b3;
+#pragma unroll
     for (int c0 = 0; c0 < kHid; c0 += 16) {
       float v[16];
       tc_ld16(tm + 64 + c0, v);
 #pragma unroll
       for (int q = 0; q < 16; q++) {
-        h2[c0 + q] = tanh_fast(v[q] + w.P[oB2 + c0 + q]);
-        t = fmaf(w.P[oW3 + c0 + q], h2[c0 + q], t);
+        h2[c0 + q] = tanh_fast(v[q] + bias.b2[c0 + q]);
+        t = fmaf(bias.w3[c0 + q], h2[c0 + q], t);
       }
     }
     const float res = live ? t - T[src] : 0.f;
-    d3 = 2.f * res * inv_batch;
+    const float d3 = 2.f * res * inv_batch;
     const double l = (double)res * res * inv_batch;
     const double lw = (double)col_sum((float)l);
     if (lane == 0) atomicAdd(loss, lw);
     const float gb3 = col_sum(d3);
     if (lane == 0) atomicAdd(&grad[oB3], gb3);
-    for (int c = 0; c < kHid; c++) {
-      const float gw3 = col_sum(d3 * h2[c]);
-      const float d2 = d3 * w.P[oW3 + c] * (1.f - h2[c] * h2[c]);
-      const float gb2 = col_sum(d2);
-      if (lane == 0) {
-        atomicAdd(&grad[oW3 + c], gw3);
-        atomicAdd(&grad[oB2 + c], gb2);
+#pragma unroll
+    for (int c0 = 0; c0 < kHid; c0 += 16) {
+      float g[16], d2[16];
+#pragma unroll
+      for (int q = 0; q < 16; q++) {
+        const float h = h2[c0 + q];
+        g[q] = d3 * h;
+        d2[q] = d3 * bias.w3[c0 + q] * (1.f - h * h);
       }
-      put_bf16(A, row, c, kHid, d2);   // delta2 for dH1 = delta2 W2
-      put_bf16(AT, c, row, 128, d2);   // delta2^T for the W2 gradient
+      put8(D, row, c0, kHid, d2);  // delta2
+      put8(D, row, c0 + 8, kHid, d2 + 8);
+      add_cols16(g, grad + oW3 + c0);
+      add_cols16(d2, grad + oB2 + c0);
     }
-    // W2 gradient (rows out, cols in) and dH1, one commit for both
-    fence_proxy_async();
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    if (tid == 0) {
-      const uint32_t a0 = smem_addr(AT), b0 = smem_addr(BT);
-      const uint32_t idesc = tc_idesc_bf16(128, kHid);
-      for (int j = 0; j < 128 / 16; j++)
-        tc_mma(s_taddr + 128, tc_desc(a0 + j * 256u, 128u, 128u * 16u),
-               tc_desc(b0 + j * 256u, 128u, 128u * 16u), idesc, j > 0);
-      const uint32_t a1 = smem_addr(A), b1 = smem_addr(sm + kSmW2T);
-      for (int j = 0; j < kHid / 16; j++)
-        tc_mma(s_taddr, tc_desc(a1 + j * 256u, 128u, kHid * 16u),
-               tc_desc(b1 + j * 256u, 128u, kHid * 16u), idesc, j > 0);
-      tc_commit(&bar);
-    }
-    const bool got = mbar_wait(&bar, phase, status);
-    phase ^= 1u;
-    tc_fence_after();
-    ok = __syncthreads_and(got);
+    // W2 gradient delta2^T h1 (rows out, cols in) and dH1 = delta2 W2
+    ok = tc_run(&bar, phase, status, [&] {
+      tc_product<true, true>(T0 + 64, D, kHid, H, kHid, kHid, 128);
+      tc_product<false, true>(T0, D, kHid, W2, kHid, kHid, kHid);
+    });
   }
   if (ok) {
-    if (warp < 2) {  // rows 0..63 of the W2 gradient
-      for (int c0 = 0; c0 < kHid; c0 += 16) {
-        float v[16];
-        tc_ld16(tm + 128 + c0, v);
+    if (warp < 2) add_weights(tm + 64, row, kHid, grad + oW2);
 #pragma unroll
-        for (int q = 0; q < 16; q++) atomicAdd(&grad[oW2 + row * kHid + c0 + q], v[q]);
-      }
-    }
     for (int c0 = 0; c0 < kHid; c0 += 16) {
       float v[16];
       tc_ld16(tm + c0, v);
 #pragma unroll
-      for (int q = 0; q < 16; q++) {
-        const int c = c0 + q;
-        const float d1 = v[q] * (1.f - h1[c] * h1[c]);
-        const float gb1 = col_sum(d1);
-        if (lane == 0) atomicAdd(&grad[oB1 + c], gb1);
-        put_bf16(AT, c, row, 128, d1);  // delta1^T
-      }
+      for (int q = 0; q < 16; q++) v[q] *= 1.f - h1[c0 + q] * h1[c0 + q];
+      put8(D, row, c0, kHid, v);  // delta1
+      put8(D, row, c0 + 8, kHid, v + 8);
+      add_cols16(v, grad + oB1 + c0);
     }
-    for (int f = 0; f < kDesc; f++) put_bf16(BT, f, row, 128, x[f]);  // X^T
-    ok = tc_run(s_taddr + 192, AT, BT, kDesc, 128, &bar, phase, status);
+    ok = tc_run(&bar, phase, status, [&] {  // W1 gradient delta1^T x
+      tc_product<true, true>(T0, D, kHid, XS, kDesc, kDesc, 128);
+    });
   }
-  if (ok && warp < 2) {  // rows 0..63 of the W1 gradient
-    for (int c0 = 0; c0 < kDesc; c0 += 16) {
-      float v[16];
-      tc_ld16(tm + 192 + c0, v);
-#pragma unroll
-      for (int q = 0; q < 16; q++) atomicAdd(&grad[oW1 + row * kDesc + c0 + q], v[q]);
-    }
-  }
+  if (ok && warp < 2) add_weights(tm, row, kDesc, grad + oW1);
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tc_dealloc(s_taddr, 256);
+  if (warp == 0) tc_dealloc(T0, 128);
 }
 
 // q_if = sum_j (e_j - e_i) . dG_if/dd_j for the force residual e (n x 3),
@@ -942,37 +997,38 @@ __global__ void k_fm_resid(const float4* __restrict__ F32, const double* __restr
   if ((threadIdx.x & 31) == 0) atomicAdd(acc, s);
 }
 
-// shared-memory plan of the force-term training kernel (bytes)
-constexpr int kFA = 0, kFA2 = 16384, kFB = 32768, kFB2 = 49152;
-constexpr int kFW1 = 65536, kFW2 = kFW1 + 4096, kFW2T = kFW2 + 8192;
-constexpr int kFAT = kFW2T + 8192, kFAT2 = kFAT + 32768;
-constexpr int kFBT = kFAT2 + 32768, kFBT2 = kFBT + 16384;
-constexpr int kSmForce = kFBT2 + 16384;  // 180 KB
-
 // Parameter gradient of sum_i v_i . dt/dx(x_i) (the force-matching term),
 // accumulated into grad: the network's tangent along v (forward) and the
-// adjoint of that tangent, eight tensor-core products per 128 rows.
-__global__ void __launch_bounds__(128, 1)
+// adjoint of that tangent, ten tensor-core products per 128 rows.  As
+// k_net_train: two blocks fit on an SM (one before), 153 us for 32,768 rows
+// before, 55 now.
+__global__ void __launch_bounds__(128)
     k_net_train_force(const float* __restrict__ X, const float* __restrict__ V, int n, NetDev w,
                       float* __restrict__ grad, int* status) {
   extern __shared__ __align__(1024) unsigned char sm[];
   __shared__ __align__(8) uint64_t bar;
   __shared__ uint32_t s_taddr;
+  __shared__ NetBias bias;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int row = 32 * warp + lane;
   const int i = blockIdx.x * 128 + row;
   const bool live = i < n;
-  unsigned char *A = sm + kFA, *A2 = sm + kFA2, *B = sm + kFB, *B2 = sm + kFB2;
-  unsigned char *AT = sm + kFAT, *AT2 = sm + kFAT2, *BT = sm + kFBT, *BT2 = sm + kFBT2;
-  load_tile(sm + kFW1, w.W1, kHid, kDesc);
-  load_tile(sm + kFW2, w.W2, kHid, kHid);
-  load_tile(sm + kFW2T, w.W2T, kHid, kHid);
-  for (int e = tid; e < 2 * 32768 / 16; e += blockDim.x) ((uint4*)AT)[e] = make_uint4(0, 0, 0, 0);
-  for (int f = 0; f < kDesc; f++) {
-    put_bf16(A, row, f, kDesc, live ? X[(size_t)i * kDesc + f] : 0.f);
-    put_bf16(A2, row, f, kDesc, live ? V[(size_t)i * kDesc + f] : 0.f);
+  unsigned char *W1 = sm, *W2 = W1 + kTileW1;
+  unsigned char *XS = W2 + kTileW2, *VS = XS + kTileX, *H = VS + kTileX, *HD = H + kTileH,
+                *A = HD + kTileH, *A2 = A + kTileH;
+  {
+    float x[kDesc];
+    load_row(x, X, i, live);
+#pragma unroll
+    for (int f = 0; f < kDesc; f += 8) put8(XS, row, f, kDesc, x + f);
+    load_row(x, V, i, live);
+#pragma unroll
+    for (int f = 0; f < kDesc; f += 8) put8(VS, row, f, kDesc, x + f);
   }
-  if (warp == 0) tc_alloc(&s_taddr, 512);
+  load_tile(W1, w.W1, kHid, kDesc);
+  load_tile(W2, w.W2, kHid, kHid);
+  load_bias(bias, w.P);
+  if (warp == 0) tc_alloc(&s_taddr, 256);
   if (tid == 0) {
     mbar_init(&bar, 1);
     fence_mbar_init();
@@ -980,30 +1036,16 @@ __global__ void __launch_bounds__(128, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t T0 = s_taddr;
-  const uint32_t tm = s_taddr + ((uint32_t)(32 * warp) << 16);
+  const uint32_t T0 = s_taddr, tm = T0 + ((uint32_t)(32 * warp) << 16);
   uint32_t phase = 0;
-  auto sync_issue = [&](auto&& issue) {
-    fence_proxy_async();
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    if (tid == 0) {
-      issue();
-      tc_commit(&bar);
-    }
-    const bool got = mbar_wait(&bar, phase, status);
-    phase ^= 1u;
-    tc_fence_after();
-    return __syncthreads_and(got);
-  };
   // z1 = x W1^T and its tangent zd1 = v W1^T
-  bool ok = sync_issue([&] {
-    tc_gemm_issue(T0, A, sm + kFW1, kHid, kDesc, nullptr);
-    tc_gemm_issue(T0 + 64, A2, sm + kFW1, kHid, kDesc, nullptr);
+  bool ok = tc_run(&bar, phase, status, [&] {
+    tc_product<false, false>(T0, XS, kDesc, W1, kDesc, kHid, kDesc);
+    tc_product<false, false>(T0 + 64, VS, kDesc, W1, kDesc, kHid, kDesc);
   });
   float h1[kHid], zd1[kHid];
   if (ok) {
+#pragma unroll
     for (int c0 = 0; c0 < kHid; c0 += 16) {
       float z[16], zd[16];
       tc_ld16(tm + c0, z);
@@ -1011,62 +1053,56 @@ __global__ void __launch_bounds__(128, 1)
 #pragma unroll
       for (int q = 0; q < 16; q++) {
         const int c = c0 + q;
-        h1[c] = tanh_fast(z[q] + w.P[oB1 + c]);
+        h1[c] = tanh_fast(z[q] + bias.b1[c]);
         zd1[c] = zd[q];
-        const float hd = (1.f - h1[c] * h1[c]) * zd[q];
-        put_bf16(B, row, c, kHid, h1[c]);
-        put_bf16(B2, row, c, kHid, hd);
-        put_bf16(BT, c, row, 128, h1[c]);
-        put_bf16(BT2, c, row, 128, hd);
+        zd[q] *= 1.f - h1[c] * h1[c];
+      }
+#pragma unroll
+      for (int q = 0; q < 16; q += 8) {
+        put8(H, row, c0 + q, kHid, h1 + c0 + q);
+        put8(HD, row, c0 + q, kHid, zd + q);
       }
     }
-    ok = sync_issue([&] {
-      tc_gemm_issue(T0 + 128, B, sm + kFW2, kHid, kHid, nullptr);
-      tc_gemm_issue(T0 + 192, B2, sm + kFW2, kHid, kHid, nullptr);
+    ok = tc_run(&bar, phase, status, [&] {
+      tc_product<false, false>(T0 + 128, H, kHid, W2, kHid, kHid, kHid);
+      tc_product<false, false>(T0 + 192, HD, kHid, W2, kHid, kHid, kHid);
     });
   }
   if (ok) {
+#pragma unroll
     for (int c0 = 0; c0 < kHid; c0 += 16) {
-      float z[16], zd[16];
+      float z[16], zd[16], g[16];
       tc_ld16(tm + 128 + c0, z);
       tc_ld16(tm + 192 + c0, zd);
 #pragma unroll
       for (int q = 0; q < 16; q++) {
         const int c = c0 + q;
-        const float h2 = tanh_fast(z[q] + w.P[oB2 + c]);
+        const float h2 = tanh_fast(z[q] + bias.b2[c]);
         const float s2 = 1.f - h2 * h2;
-        const float w3 = w.P[oW3 + c];
-        const float hd2 = s2 * zd[q];
-        const float a_zd2 = live ? w3 * s2 : 0.f;
-        const float a_z2 = w3 * (-2.f * h2 * zd[q]) * s2;
-        const float gw3 = col_sum(hd2), gb2 = col_sum(a_z2);
-        if (lane == 0) {
-          atomicAdd(&grad[oW3 + c], gw3);
-          atomicAdd(&grad[oB2 + c], gb2);
-        }
-        put_bf16(A, row, c, kHid, a_z2);
-        put_bf16(A2, row, c, kHid, a_zd2);
-        put_bf16(AT, c, row, 128, a_z2);
-        put_bf16(AT2, c, row, 128, a_zd2);
+        const float w3 = bias.w3[c];
+        g[q] = s2 * zd[q];                         // hd2
+        z[q] = w3 * (-2.f * h2 * zd[q]) * s2;      // a_z2
+        zd[q] = live ? w3 * s2 : 0.f;              // a_zd2
       }
+#pragma unroll
+      for (int q = 0; q < 16; q += 8) {
+        put8(A, row, c0 + q, kHid, z + q);
+        put8(A2, row, c0 + q, kHid, zd + q);
+      }
+      add_cols16(g, grad + oW3 + c0);
+      add_cols16(z, grad + oB2 + c0);
     }
     // W2 gradient a_z2^T h1 + a_zd2^T hd1; a_h1 = a_z2 W2; a_hd1 = a_zd2 W2
-    ok = sync_issue([&] {
-      tc_gemm_issue(T0 + 256, AT, BT, kHid, 128, nullptr);
-      tc_gemm_issue(T0 + 256, AT2, BT2, kHid, 128, nullptr, true);
-      tc_gemm_issue(T0, A, sm + kFW2T, kHid, kHid, nullptr);
-      tc_gemm_issue(T0 + 64, A2, sm + kFW2T, kHid, kHid, nullptr);
+    ok = tc_run(&bar, phase, status, [&] {
+      tc_product<true, true>(T0 + 128, A, kHid, H, kHid, kHid, 128);
+      tc_product<true, true>(T0 + 128, A2, kHid, HD, kHid, kHid, 128, true);
+      tc_product<false, true>(T0, A, kHid, W2, kHid, kHid, kHid);
+      tc_product<false, true>(T0 + 64, A2, kHid, W2, kHid, kHid, kHid);
     });
   }
   if (ok) {
-    if (warp < 2) {
-      for (int c0 = 0; c0 < kHid; c0 += 16) {
-        float g[16];
-        tc_ld16(tm + 256 + c0, g);
+    if (warp < 2) add_weights(tm + 128, row, kHid, grad + oW2);
 #pragma unroll
-        for (int q = 0; q < 16; q++) atomicAdd(&grad[oW2 + row * kHid + c0 + q], g[q]);
-      }
-    }
     for (int c0 = 0; c0 < kHid; c0 += 16) {
       float ah[16], ahd[16];
       tc_ld16(tm + c0, ah);
@@ -1075,35 +1111,26 @@ __global__ void __launch_bounds__(128, 1)
       for (int q = 0; q < 16; q++) {
         const int c = c0 + q;
         const float s1 = 1.f - h1[c] * h1[c];
-        const float a_zd1 = ahd[q] * s1;
-        const float a_z1 = (ah[q] + ahd[q] * (-2.f * h1[c] * zd1[c])) * s1;
-        const float gb1 = col_sum(a_z1);
-        if (lane == 0) atomicAdd(&grad[oB1 + c], gb1);
-        put_bf16(AT, c, row, 128, a_z1);
-        put_bf16(AT2, c, row, 128, a_zd1);
+        ah[q] = (ah[q] + ahd[q] * (-2.f * h1[c] * zd1[c])) * s1;  // a_z1
+        ahd[q] *= s1;                                             // a_zd1
       }
-    }
-    for (int f = 0; f < kDesc; f++) {
-      put_bf16(BT, f, row, 128, live ? X[(size_t)i * kDesc + f] : 0.f);
-      put_bf16(BT2, f, row, 128, live ? V[(size_t)i * kDesc + f] : 0.f);
+#pragma unroll
+      for (int q = 0; q < 16; q += 8) {
+        put8(A, row, c0 + q, kHid, ah + q);
+        put8(A2, row, c0 + q, kHid, ahd + q);
+      }
+      add_cols16(ah, grad + oB1 + c0);
     }
     // W1 gradient a_z1^T x + a_zd1^T v
-    ok = sync_issue([&] {
-      tc_gemm_issue(T0 + 320, AT, BT, kDesc, 128, nullptr);
-      tc_gemm_issue(T0 + 320, AT2, BT2, kDesc, 128, nullptr, true);
+    ok = tc_run(&bar, phase, status, [&] {
+      tc_product<true, true>(T0 + 192, A, kHid, XS, kDesc, kDesc, 128);
+      tc_product<true, true>(T0 + 192, A2, kHid, VS, kDesc, kDesc, 128, true);
     });
   }
-  if (ok && warp < 2) {
-    for (int c0 = 0; c0 < kDesc; c0 += 16) {
-      float g[16];
-      tc_ld16(tm + 320 + c0, g);
-#pragma unroll
-      for (int q = 0; q < 16; q++) atomicAdd(&grad[oW1 + row * kDesc + c0 + q], g[q]);
-    }
-  }
+  if (ok && warp < 2) add_weights(tm + 192, row, kDesc, grad + oW1);
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tc_dealloc(s_taddr, 512);
+  if (warp == 0) tc_dealloc(T0, 256);
 }
 
 // Adam (Kingma & Ba): m = b1 m + (1-b1) g; v = b2 v + (1-b2) g^2;
@@ -1123,32 +1150,25 @@ __global__ void k_adam(float* __restrict__ P, float* __restrict__ M, float* __re
   P[k] -= lr * mh / (sqrtf(vh) + eps);
 }
 
-__global__ void k_net_cast(const float* __restrict__ P, __nv_bfloat16* W1, __nv_bfloat16* W1T,
-                           __nv_bfloat16* W2, __nv_bfloat16* W2T) {
+__global__ void k_net_cast(const float* __restrict__ P, __nv_bfloat16* W1, __nv_bfloat16* W2) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < kHid * kDesc) {
-    const int o = k / kDesc, in = k % kDesc;
-    const __nv_bfloat16 b = __float2bfloat16_rn(P[oW1 + k]);
-    W1[k] = b;
-    W1T[in * kHid + o] = b;
-  }
-  if (k < kHid * kHid) {
-    const int o = k / kHid, in = k % kHid;
-    const __nv_bfloat16 b = __float2bfloat16_rn(P[oW2 + k]);
-    W2[k] = b;
-    W2T[in * kHid + o] = b;
-  }
+  if (k < kHid * kDesc) W1[k] = __float2bfloat16_rn(P[oW1 + k]);
+  if (k < kHid * kHid) W2[k] = __float2bfloat16_rn(P[oW2 + k]);
 }
 
-// energy E_i = mu + sigma t_i; gcoef = sigma * dt/dx * istd; block sums of E
-__global__ void k_sg_scale(const float* __restrict__ t, const float* __restrict__ dtdx, int n,
-                           double mu, double sigma, const float* __restrict__ istd,
-                           float* __restrict__ gcoef, double* __restrict__ eatom) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  if (eatom) eatom[i] = mu + sigma * (double)t[i];
-  for (int f = 0; f < kDesc; f++)
-    gcoef[(size_t)i * kDesc + f] = (float)sigma * dtdx[(size_t)i * kDesc + f] * istd[f];
+// energy E_i = mu + sigma t_i; gcoef = sigma * dt/dx * istd, four values a thread
+// (a thread per atom took 12 us for 32,768 atoms, its rows 128 bytes apart)
+__global__ void k_sg_scale(const float* __restrict__ t, const float4* __restrict__ dtdx, int n,
+                           double mu, double sigma, const float4* __restrict__ istd,
+                           float4* __restrict__ gcoef, double* __restrict__ eatom) {
+  const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  constexpr int kQ = kDesc / 4;
+  if (k >= (long long)n * kQ) return;
+  const int q = (int)(k % kQ);
+  if (eatom && q == 0) eatom[k / kQ] = mu + sigma * (double)t[k / kQ];
+  const float s = (float)sigma;
+  const float4 d = dtdx[k], w = istd[q];
+  gcoef[k] = make_float4(s * d.x * w.x, s * d.y * w.y, s * d.z * w.z, s * d.w * w.w);
 }
 
 __global__ void k_sum_d(const double* __restrict__ v, int n, double* __restrict__ out) {
@@ -1206,9 +1226,7 @@ cudaError_t sur_grow(T*& p, long long& have, long long need) {
 NetDev net_of(const Surrogate& s) {
   NetDev w;
   w.W1 = s.W1;
-  w.W1T = s.W1T;
   w.W2 = s.W2;
-  w.W2T = s.W2T;
   w.P = s.P_d;
   return w;
 }
@@ -1632,7 +1650,7 @@ int sur_init(Surrogate& s, unsigned long long seed, cudaStream_t st) {
     h = 0;
     if ((e = sur_grow(*p, h, kParams)) != cudaSuccess) return e;
   }
-  for (__nv_bfloat16** p : {&s.W1, &s.W1T, &s.W2, &s.W2T}) {
+  for (__nv_bfloat16** p : {&s.W1, &s.W2}) {
     h = 0;
     if ((e = sur_grow(*p, h, kHid * kHid)) != cudaSuccess) return e;
   }
@@ -1671,7 +1689,7 @@ int sur_set_params(Surrogate& s, const float* P, cudaStream_t st) {
   cudaMemsetAsync(s.M_d, 0, sizeof(float) * kParams, st);
   cudaMemsetAsync(s.V_d, 0, sizeof(float) * kParams, st);
   s.adam_step = 0;
-  k_net_cast<<<sblocks(kHid * kHid, 256), 256, 0, st>>>(s.P_d, s.W1, s.W1T, s.W2, s.W2T);
+  k_net_cast<<<sblocks(kHid * kHid, 256), 256, 0, st>>>(s.P_d, s.W1, s.W2);
   return cudaStreamSynchronize(st);
 }
 
@@ -1838,7 +1856,7 @@ int sur_train(Surrogate& s, int steps, int batch, float lr, double* loss_out, cu
     s.adam_step++;
     k_adam<<<sblocks(kParams, 256), 256, 0, st>>>(s.P_d, s.M_d, s.V_d, s.G_d, s.adam_step, lr,
                                                  0.9f, 0.999f, 1e-8f);
-    k_net_cast<<<sblocks(kHid * kHid, 256), 256, 0, st>>>(s.P_d, s.W1, s.W1T, s.W2, s.W2T);
+    k_net_cast<<<sblocks(kHid * kHid, 256), 256, 0, st>>>(s.P_d, s.W1, s.W2);
     if (it >= steps - 16) {  // mean loss of the last steps
       double l = 0;
       cudaMemcpyAsync(&l, s.loss_d, sizeof(double), cudaMemcpyDeviceToHost, st);
@@ -1889,10 +1907,10 @@ int sur_net_eval(Surrogate& s, const float* X, int n, float* t, float* dtdx, cud
   if ((e = sur_grow(s.Tg, h, (long long)n * (kDesc + 1))) != cudaSuccess) return e;
   s.nxg = n;
   cudaMemcpyAsync(s.Xg, X, sizeof(float) * kDesc * n, cudaMemcpyHostToDevice, st);
-  k_net_infer<<<(n + 127) / 128, 128, kSmInfer, st>>>(s.Xg, n, net_of(s), s.Tg, s.Tg + n,
-                                                     s.status_d);
-  cudaMemcpyAsync(t, s.Tg, sizeof(float) * n, cudaMemcpyDeviceToHost, st);
-  cudaMemcpyAsync(dtdx, s.Tg + n, sizeof(float) * kDesc * n, cudaMemcpyDeviceToHost, st);
+  float* t_d = s.Tg + (size_t)kDesc * n;  // behind the gradients, whose rows are 16-byte aligned
+  k_net_infer<<<(n + 127) / 128, 128, kSmInfer, st>>>(s.Xg, n, net_of(s), t_d, s.Tg, s.status_d);
+  cudaMemcpyAsync(t, t_d, sizeof(float) * n, cudaMemcpyDeviceToHost, st);
+  cudaMemcpyAsync(dtdx, s.Tg, sizeof(float) * kDesc * n, cudaMemcpyDeviceToHost, st);
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
   return (int)cudaGetLastError();
 }
@@ -1947,8 +1965,9 @@ int sur_forces(Surrogate& s, const md_double4* pos, int n, const RowWalker& w, d
     return (int)cudaGetLastError();
   }
   k_net_infer<<<(n + 127) / 128, 128, kSmInfer, st>>>(s.X, n, net_of(s), s.t, s.dtdx, s.status_d);
-  k_sg_scale<<<sblocks(n, 256), 256, 0, st>>>(s.t, s.dtdx, n, s.mu, s.sigma, s.istd_d, s.gcoef,
-                                              s.eatom);
+  k_sg_scale<<<sblocks(8LL * n, 256), 256, 0, st>>>(
+        s.t, (const float4*)s.dtdx, n, s.mu, s.sigma, (const float4*)s.istd_d, (float4*)s.gcoef,
+        s.eatom);
   cudaMemsetAsync(s.F32, 0, sizeof(float4) * (size_t)n, st);
   k_sg_force<<<sblocks(n, 4), 128, 0, st>>>(pos, n, s.sl, s.slen, w.g.box, s.P, s.gcoef, s.F32);
   k_sg_store<<<sblocks(3LL * n, 256), 256, 0, st>>>(s.F32, f3, n, accumulate, skip,
@@ -2234,8 +2253,9 @@ int sur_train_fm(Surrogate& s, int steps, float lr, double* loss_e, double* loss
     const int tiles = (n + 127) / 128;
     // forces of the current network on this configuration
     k_net_infer<<<tiles, 128, kSmInfer, st>>>(c.X, n, w, s.t, s.dtdx, s.status_d);
-    k_sg_scale<<<sblocks(n, 256), 256, 0, st>>>(s.t, s.dtdx, n, s.mu, s.sigma, s.istd_d,
-                                                s.gcoef, s.eatom);
+    k_sg_scale<<<sblocks(8LL * n, 256), 256, 0, st>>>(
+        s.t, (const float4*)s.dtdx, n, s.mu, s.sigma, (const float4*)s.istd_d, (float4*)s.gcoef,
+        s.eatom);
     cudaMemsetAsync(s.F32, 0, sizeof(float4) * (size_t)n, st);
     k_sg_force<<<sblocks(n, 4), 128, 0, st>>>(c.pos, n, c.sl, c.slen, c.box, s.P, s.gcoef,
                                                 s.F32);
@@ -2256,7 +2276,7 @@ int sur_train_fm(Surrogate& s, int steps, float lr, double* loss_e, double* loss
     s.adam_step++;
     k_adam<<<sblocks(kParams, 256), 256, 0, st>>>(s.P_d, s.M_d, s.V_d, s.G_d, s.adam_step, lr,
                                                  0.9f, 0.999f, 1e-8f);
-    k_net_cast<<<sblocks(kHid * kHid, 256), 256, 0, st>>>(s.P_d, s.W1, s.W1T, s.W2, s.W2T);
+    k_net_cast<<<sblocks(kHid * kHid, 256), 256, 0, st>>>(s.P_d, s.W1, s.W2);
     if (it >= steps - std::min(steps, 2 * ncfg)) {  // losses over the last pass
       double le = 0, lf[2];
       cudaMemcpyAsync(&le, s.loss_d, sizeof(double), cudaMemcpyDeviceToHost, st);
@@ -2313,7 +2333,7 @@ int sur_rel_err(const double* a, const double* b, int n, double* scratch, double
 }  // namespace mdgb
 
 md_surrogate::~md_surrogate() {
-  void* ptrs[] = {P_d, M_d,   V_d, G_d,   W1,    W1T,     W2,     W2T,    mean_d, istd_d,
+  void* ptrs[] = {P_d, M_d,   V_d, G_d,   W1,    W2,     mean_d, istd_d,
                   sl,  slen,  X,   t,     dtdx,  gcoef,   F32,    eatom,  SG,     SE,
                   SX,  ST,    loss_d, scratch, rows_d, Xg, Tg, status_d};
   for (void* p : ptrs)

@@ -46,7 +46,7 @@ struct md_surrogate {
   mdgb::DescParams P{};
   // network parameters (FP32 master), Adam moments, gradients, BF16 copies
   float *P_d = nullptr, *M_d = nullptr, *V_d = nullptr, *G_d = nullptr;
-  __nv_bfloat16 *W1 = nullptr, *W1T = nullptr, *W2 = nullptr, *W2T = nullptr;
+  __nv_bfloat16 *W1 = nullptr, *W2 = nullptr;
   int adam_step = 0;
   // input and target normalisation (fixed at the first training)
   float *mean_d = nullptr, *istd_d = nullptr;

@@ -35,10 +35,12 @@ __device__ __forceinline__ uint64_t tc_desc(uint32_t saddr, uint32_t lbo, uint32
   return d;
 }
 
-// instruction descriptor of kind::f16: BF16 A and B (K-major), FP32 D, M x N
-__host__ __device__ constexpr uint32_t tc_idesc_bf16(int M, int N) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) |
-         ((uint32_t)(M >> 4) << 24);
+// instruction descriptor of kind::f16: BF16 A and B (K-major, or MN-major where
+// at / bt is set), FP32 D, M x N
+__host__ __device__ constexpr uint32_t tc_idesc_bf16(int M, int N, bool at = false,
+                                                     bool bt = false) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)at << 15) | ((uint32_t)bt << 16) |
+         ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
 __device__ __forceinline__ void tc_alloc(uint32_t* smem_dst, uint32_t ncols) {
@@ -94,20 +96,31 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&v)[16]) {
   for (int k = 0; k < 16; k++) v[k] = __uint_as_float(r[k]);
 }
 
-// D[128 x N] (+)= A[128 x K] * B[N x K]^T with A and B in shared memory
-// (layout above); issued by the calling thread; with bar, completion of all
-// earlier products of this thread is signalled there
+// D[128 x N] (+)= A * B over K, A and B in shared memory (layout above), issued by
+// the calling thread.  AT false: A is a 128 x wa tile (wa = K); true: a K x wa
+// tile, read across its rows (MN-major: the same core matrices, their strides
+// exchanged, so a tile that was written row by row is the transposed operand
+// too).  BT likewise: N x wb or K x wb.  With AT and wa < 128 the upper rows of D
+// are the products of what follows the tile: up to 2 KB behind it are read.
+template <bool AT, bool BT>
+__device__ __forceinline__ void tc_product(uint32_t d_tmem, const void* A, int wa, const void* B,
+                                           int wb, int N, int K, bool accumulate = false) {
+  const uint32_t a0 = smem_addr(A), b0 = smem_addr(B), sa = wa * 16u, sb = wb * 16u;
+  const uint32_t idesc = tc_idesc_bf16(128, N, AT, BT);
+  for (int j = 0; j < K / 16; j++) {
+    // K = 16 per instruction: two core matrices along K
+    const uint32_t a = a0 + j * (AT ? 2 * sa : 256u), b = b0 + j * (BT ? 2 * sb : 256u);
+    tc_mma(d_tmem, AT ? tc_desc(a, sa, 128u) : tc_desc(a, 128u, sa),
+           BT ? tc_desc(b, sb, 128u) : tc_desc(b, 128u, sb), idesc, accumulate || j > 0);
+  }
+}
+
+// D[128 x N] (+)= A[128 x K] * B[N x K]^T; with bar, completion of all earlier
+// products of this thread is signalled there
 __device__ __forceinline__ void tc_gemm_issue(uint32_t d_tmem, const void* A, const void* B,
                                               int N, int K, uint64_t* bar,
                                               bool accumulate = false) {
-  const uint32_t a0 = smem_addr(A), b0 = smem_addr(B);
-  const uint32_t sbo = (uint32_t)K * 16u;
-  const uint32_t idesc = tc_idesc_bf16(128, N);
-  for (int j = 0; j < K / 16; j++) {
-    // K = 16 per instruction: two core matrices along K
-    tc_mma(d_tmem, tc_desc(a0 + j * 256u, 128u, sbo), tc_desc(b0 + j * 256u, 128u, sbo), idesc,
-           accumulate || j > 0);
-  }
+  tc_product<false, false>(d_tmem, A, K, B, K, N, K, accumulate);
   if (bar) tc_commit(bar);
 }
 

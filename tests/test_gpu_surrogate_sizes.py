@@ -53,3 +53,26 @@ def test_neighbour_counts(eng, n, a, L):
     terms = coef * qr
     assert abs((coef * q).sum() - terms.sum()) <= 1e-4 * np.abs(terms).sum() + 1e-12
     assert abs((f * e3).sum() + terms.sum()) <= 1e-4 * np.abs(terms).sum() + 1e-12
+
+
+@pytest.mark.parametrize("n", [1, 127, 128, 129])
+def test_network_row_counts(eng, n):
+    # the ends of the tensor-core tiles of 128 rows; odd counts (the gradient rows
+    # leave in 16-byte stores); bars as for the whole tiles
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((n, 32)).astype(np.float32)
+    y = rng.standard_normal(n).astype(np.float32)
+    v = rng.standard_normal((n, 32)).astype(np.float32) * 0.1
+    with eng.Surrogate(cutoff=3.0) as s:
+        p = s.params(rng.standard_normal(s.nparams).astype(np.float32) * 0.3)
+        t, d = s.net(x)
+        loss, g = s.loss_grad(x, y)
+        gf = s.force_grad(x, v)
+    tr, dr = sref.net(p, x)
+    assert np.abs(t - tr).max() <= 2e-3 * np.abs(tr).max()
+    assert np.abs(d - dr).max() <= 2e-3 * np.abs(dr).max()
+    lr, gr = sref.loss_grad(p, x, y)
+    assert abs(loss - lr) <= 1e-4 * lr
+    for got, ref in ((g, gr), (gf, sref.force_grad(p, x, v))):
+        for a, b in ((0, 2048), (2048, 2112), (2112, 6208), (6208, 6272), (6272, 6336)):
+            assert np.abs(got[a:b] - ref[a:b]).max() <= 5e-3 * np.abs(ref[a:b]).max() + 1e-30
