@@ -1262,56 +1262,123 @@ bool attrs_set = false;
 // Nothing makes gcoef a gradient, so the forces need not be conservative,
 // as the reference's bond-order forces are not.  FP32 on the CUDA cores: the
 // outputs multiply the descriptor derivatives directly, so BF16 weights would
-// bound the force error near 1e-3; at 8-33 K parameters and one thread per
-// atom the layers take tens of microseconds per 32,768 atoms.
+// bound the force error near 1e-3; at 8-33 K parameters the layers take tens of
+// microseconds per 32,768 atoms.
 // Parameters: W1 [H][32], b1 [H], W2 [H][H], b2 [H], W3 [32][H], b3 [32].
 __host__ __device__ constexpr int fh_params(int H) { return H * 32 + H + H * H + H + 32 * H + 32; }
 
-// forward, one thread per atom (weights in shared memory, read as broadcasts):
-// gcoef (atom-major) and, for training, the input and hidden activations
-// feature-major (xT[d n + i], h1T[j n + i], h2T[j n + i])
-template <int H>
-__global__ void __launch_bounds__(128)
+// forward: an atom or two per lane and a quarter of each layer's outputs per warp;
+// weights (read as broadcasts) and hidden activations in shared memory, two
+// products per instruction.  The weights' reads bound it.  gcoef (atom-major) and, for training, the
+// input and hidden activations feature-major (xT[d n + i], h1T[j n + i],
+// h2T[j n + i]).  A thread per atom left two warps to a scheduler: 42 us for
+// 32,768 atoms and H = 64, now 32 with an atom per lane and 25 with two, which
+// share the reads; 34 -> 11 for 4,096 atoms, where two would leave SMs idle.
+// Wide heads share their weights' copy among four such groups (111 -> 75 us).
+__host__ __device__ constexpr int fh_groups(int H) { return H > 64 ? 4 : 1; }
+
+// acc[u][o] += the pairwise products of row o of W (K columns) with the activations
+// h[k / 4] of this lane's atom u (four per entry, entries `ld` apart, atoms 32)
+template <int A, int O, int K>
+__device__ __forceinline__ void fh_layer(F2 (&acc)[A][O], const float* W, const float4* h,
+                                         int ld) {
+#pragma unroll 2
+  for (int k = 0; k < K / 4; k++) {
+    F2 lo[A], hi[A];
+#pragma unroll
+    for (int u = 0; u < A; u++) {
+      const float4 v = h[k * ld + 32 * u];
+      lo[u] = f2(v.x, v.y);
+      hi[u] = f2(v.z, v.w);
+    }
+#pragma unroll
+    for (int o = 0; o < O; o++) {
+      const float4 q = *(const float4*)(W + o * K + 4 * k);
+      const F2 ql = f2(q.x, q.y), qh = f2(q.z, q.w);
+#pragma unroll
+      for (int u = 0; u < A; u++) acc[u][o] = f2_fma(qh, hi[u], f2_fma(ql, lo[u], acc[u][o]));
+    }
+  }
+}
+
+template <int H, int A>
+__global__ void __launch_bounds__(128 * fh_groups(H))
     k_fh_forward(const float* __restrict__ X, int n, const float* __restrict__ P,
                  const float* __restrict__ gscale, float* __restrict__ gcoef,
                  float* __restrict__ xT, float* __restrict__ h1T, float* __restrict__ h2T) {
-  extern __shared__ float wsm[];
-  for (int k = threadIdx.x; k < fh_params(H); k += blockDim.x) wsm[k] = P[k];
+  extern __shared__ float4 wsm4[];
+  constexpr int kA = 32 * A * fh_groups(H), O = H / 4;  // atoms of the block, outputs of a warp
+  float* wsm = (float*)wsm4;
+  float4* hs = wsm4 + fh_params(H) / 4;  // [unit / 4][atom]
+  const int tid = threadIdx.x, lane = tid & 31, part = tid >> 5 & 3;
+  for (int k = tid; k < fh_params(H) / 4; k += blockDim.x) wsm4[k] = ((const float4*)P)[k];
+  const int a = 32 * A * (tid >> 7) + lane;  // the lane's first atom; the others 32 apart
+  const long long i0 = (long long)blockIdx.x * kA + a;
+  // the input, a quarter of it per warp
+#pragma unroll
+  for (int u = 0; u < A; u++) {
+    const long long i = i0 + 32 * u;
+#pragma unroll
+    for (int q = 2 * part; q < 2 * part + 2; q++) {
+      const float4 v = i < n ? ((const float4*)(X + i * 32))[q] : make_float4(0.f, 0.f, 0.f, 0.f);
+      hs[q * kA + a + 32 * u] = v;
+      if (xT && i < n) {
+        const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int d = 0; d < 4; d++) xT[(size_t)(4 * q + d) * n + i] = x[d];
+      }
+    }
+  }
   __syncthreads();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
   const float *W1 = wsm, *b1 = W1 + H * 32, *W2 = b1 + H, *b2 = W2 + H * H, *W3 = b2 + H,
               *b3 = W3 + 32 * H;
-  float x[32];
+  auto start = [&](auto& acc, const float* b) {
 #pragma unroll
-  for (int d = 0; d < 32; d++) {
-    x[d] = X[(size_t)i * 32 + d];
-    if (xT) xT[(size_t)d * n + i] = x[d];
+    for (int u = 0; u < A; u++)
+#pragma unroll
+      for (int o = 0; o < (int)(sizeof(acc[0]) / sizeof(F2)); o++) acc[u][o] = f2(b[o], 0.f);
+  };
+  auto hidden = [&](F2 (&acc)[A][O], float* hT) {
+    __syncthreads();  // the layer's inputs are read
+#pragma unroll
+    for (int u = 0; u < A; u++)
+#pragma unroll
+      for (int o = 0; o < O; o += 4) {
+        float h[4];
+#pragma unroll
+        for (int d = 0; d < 4; d++) {
+          const float2 v = f2_get(acc[u][o + d]);
+          h[d] = tanhf(v.x + v.y);
+          if (hT && i0 + 32 * u < n) hT[(size_t)(O * part + o + d) * n + i0 + 32 * u] = h[d];
+        }
+        hs[(O * part + o) / 4 * kA + a + 32 * u] = make_float4(h[0], h[1], h[2], h[3]);
+      }
+    __syncthreads();
+  };
+  F2 acc[A][O];
+  start(acc, b1 + O * part);
+  fh_layer<A, O, 32>(acc, W1 + O * part * 32, hs + a, kA);
+  hidden(acc, h1T);
+  start(acc, b2 + O * part);
+  fh_layer<A, O, H>(acc, W2 + O * part * H, hs + a, kA);
+  hidden(acc, h2T);
+  F2 out[A][8];
+  start(out, b3 + 8 * part);
+  fh_layer<A, 8, H>(out, W3 + 8 * part * H, hs + a, kA);
+#pragma unroll
+  for (int u = 0; u < A; u++) {
+    const long long i = i0 + 32 * u;
+    if (i >= n) return;
+    float w[8];
+#pragma unroll
+    for (int o = 0; o < 8; o++) {
+      const float2 v = f2_get(out[u][o]);
+      w[o] = (v.x + v.y) * (gscale ? gscale[8 * part + o] : 1.f);
+    }
+    float4* g = (float4*)(gcoef + i * 32 + 8 * part);
+    g[0] = make_float4(w[0], w[1], w[2], w[3]);
+    g[1] = make_float4(w[4], w[5], w[6], w[7]);
   }
-  float h1[H];
-#pragma unroll
-  for (int j = 0; j < H; j++) {
-    float a = b1[j];
-#pragma unroll
-    for (int d = 0; d < 32; d++) a = fmaf(W1[j * 32 + d], x[d], a);
-    h1[j] = tanhf(a);
-    if (h1T) h1T[(size_t)j * n + i] = h1[j];
-  }
-  float w[32];
-#pragma unroll
-  for (int d = 0; d < 32; d++) w[d] = b3[d];
-#pragma unroll 1
-  for (int j = 0; j < H; j++) {
-    float a = b2[j];
-#pragma unroll
-    for (int k = 0; k < H; k++) a = fmaf(W2[j * H + k], h1[k], a);
-    const float h = tanhf(a);
-    if (h2T) h2T[(size_t)j * n + i] = h;
-#pragma unroll
-    for (int d = 0; d < 32; d++) w[d] = fmaf(W3[d * H + j], h, w[d]);
-  }
-#pragma unroll
-  for (int d = 0; d < 32; d++) gcoef[(size_t)i * 32 + d] = gscale ? w[d] * gscale[d] : w[d];
 }
 
 // backward of sum_i v_i . w_i (v = dL/dw, atom-major): the output and hidden
@@ -1474,13 +1541,18 @@ __global__ void k_sumsq(const float* __restrict__ F, long long m, double* __rest
   if ((threadIdx.x & 31) == 0) atomicAdd(acc, s);
 }
 
+// shared memory of k_fh_forward: weights, and the activations of a block's atoms
+constexpr int fh_smem(int H, int A) { return 4 * (fh_params(H) + 32 * A * fh_groups(H) * H); }
+
 void set_attrs() {
   if (attrs_set) return;
   cudaFuncSetAttribute(k_net_infer, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmInfer);
   cudaFuncSetAttribute(k_net_train, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmTrain);
   cudaFuncSetAttribute(k_net_train_force, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmForce);
-  cudaFuncSetAttribute(k_fh_forward<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)sizeof(float) * fh_params(128));
+  cudaFuncSetAttribute(k_fh_forward<64, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       fh_smem(64, 2));
+  cudaFuncSetAttribute(k_fh_forward<128, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       fh_smem(128, 1));
   cudaFuncSetAttribute(k_fh_backward<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)sizeof(float) * fh_params(128));
   attrs_set = true;
@@ -1494,18 +1566,22 @@ double fh_out_scale(const Surrogate& s) {
 // the direct-force head's launches for its width
 void fh_forward(const Surrogate& s, const float* X, int n, float* gcoef, bool keep,
                 cudaStream_t st) {
-  const int B = (n + 127) / 128;
-  const size_t sm = sizeof(float) * fh_params(s.fh_hidden);
   float* xT = keep ? s.fh_xT : nullptr;
   float* h1 = keep ? s.fh_h1T : nullptr;
   float* h2 = keep ? s.fh_h2T : nullptr;
   const float* gs = s.fh_gs;
+  auto run = [&](auto kernel, int H, int A) {
+    const int g = fh_groups(H);
+    kernel<<<sblocks(n, 32 * A * g), 128 * g, fh_smem(H, A), st>>>(X, n, s.FP_d, gs, gcoef, xT, h1,
+                                                                   h2);
+  };
+  const bool two = n > 64 * 152;  // blocks of 64 atoms for every SM
   if (s.fh_hidden == 32)
-    k_fh_forward<32><<<B, 128, sm, st>>>(X, n, s.FP_d, gs, gcoef, xT, h1, h2);
+    two ? run(k_fh_forward<32, 2>, 32, 2) : run(k_fh_forward<32, 1>, 32, 1);
   else if (s.fh_hidden == 64)
-    k_fh_forward<64><<<B, 128, sm, st>>>(X, n, s.FP_d, gs, gcoef, xT, h1, h2);
+    two ? run(k_fh_forward<64, 2>, 64, 2) : run(k_fh_forward<64, 1>, 64, 1);
   else
-    k_fh_forward<128><<<B, 128, sm, st>>>(X, n, s.FP_d, gs, gcoef, xT, h1, h2);
+    run(k_fh_forward<128, 1>, 128, 1);
 }
 
 // FG += d(sum_i v_i . w_i)/dparams for the activations of the last kept forward

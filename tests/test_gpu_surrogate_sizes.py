@@ -76,3 +76,19 @@ def test_network_row_counts(eng, n):
     for got, ref in ((g, gr), (gf, sref.force_grad(p, x, v))):
         for a, b in ((0, 2048), (2048, 2112), (2112, 6208), (6208, 6272), (6272, 6336)):
             assert np.abs(got[a:b] - ref[a:b]).max() <= 5e-3 * np.abs(ref[a:b]).max() + 1e-30
+
+
+@pytest.mark.parametrize("hidden", [32, 64, 128])
+@pytest.mark.parametrize("n", [1, 33, 129])
+def test_head_row_counts(eng, n, hidden):
+    # the direct head's gradient comes from the activations its forward keeps (FP32)
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((n, 32)).astype(np.float32)
+    v = rng.standard_normal((n, 32)).astype(np.float32)
+    with eng.Surrogate(seed=4, cutoff=3.0) as s:
+        s.set_model(1, hidden)
+        p = s.head_params()
+        p = s.head_params(p + rng.standard_normal(len(p)).astype(np.float32) * 0.05)
+        g = s.head_grad(x, v)
+    gr = sref.head_grad(p, x, v, hidden)
+    assert np.abs(g - gr).max() < 1e-4 * np.abs(gr).max()
