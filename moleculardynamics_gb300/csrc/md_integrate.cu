@@ -15,6 +15,7 @@
 #include "md_gear64.cuh"
 #include "md_integrate.h"
 #include "md_potential.cuh"
+#include "md_tma.cuh"
 
 namespace mdgb {
 
@@ -110,6 +111,8 @@ __global__ void __launch_bounds__(128)
              const int* __restrict__ hit, int* hits, int* flag_next) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int i = t >> 2, d = t & 3;
+  grid_wait();
+  grid_launch_dependents();
   const bool gate = MODE != GEAR64_REDO || *hit != 0;
   if (MODE == GEAR64_REDO && t == 0) {
     if (gate) atomicAdd(hits, 1);
@@ -829,7 +832,8 @@ static void launch_gear64(const GearArgs& a, bool predict, const int* hit, int* 
   Gear64 g;
   gear64_args(a, a.pos, predict, g);
   const int T = a.n <= 8 * 152 ? 32 : 128;
-  k_gear64<MODE><<<nblk(4LL * a.n, T), T, 0, st>>>(g, a.f3, a.n, hit, hits, flag_next);
+  launch_dependent(true, k_gear64<MODE>, nblk(4LL * a.n, T), T, st, g, (const double*)a.f3, a.n, hit, hits,
+                   flag_next);
 }
 
 void launch_predict(const GearArgs& a, cudaStream_t st) {
