@@ -1618,15 +1618,18 @@ inline int nblk(long long n, int t) { return (int)((n + t - 1) / t); }
 
 }  // namespace
 
-// Lanes per atom of the FP64 LJ kernel: the most that keep the launch within
-// four warps per scheduler (n G / 32 <= 16 x 152), as every doubling costs
-// throughput (the ordered sums keep three lanes of each group) and gains
-// latency.  Measured, us per launch with 4 / 8 / 16 / 32 lanes: 864 atoms
-// - / - / 18 / 17 (205 with a thread per atom), 8,000 atoms
-// 44 / 35 / 38 / 53 (207), 108,000 atoms 255 / 270 / - / - (1010).
+// Lanes per atom of the FP64 LJ kernel.  More lanes shorten an atom's chain of
+// pairs, but its ordered sums keep three of them and its last batch leaves the
+// others idle, so the lines lie where more warps stop helping: at 5 (32 lanes),
+// 8.5 (16) and 21 warps (8) an SM.  Measured, ms per 100 steps in a periodic box
+// (640, 1,700, 2,432 atoms: within walls) with 32 / 16 / 8 / 4 lanes:
+//    640 atoms  2.39 2.54 3.29 4.91     2,432  4.12 3.53 3.55 5.05
+//    864        2.46 2.37 3.17 4.91     2,916  4.17 3.77 3.75 5.04
+//  1,372        3.08 2.95 3.29 4.94     6,912  7.97 5.67 4.65 6.02
+//  1,700        4.55 4.30 4.62 6.31    13,500  13.9 9.59 6.95 6.83
+// (a thread per atom with the FP64 instructions: 20.5 at 864 to 8,000 atoms).
 static int lj64_lanes(int n) {
-  const long long room = 16LL * 152 * 32;
-  return n * 32LL <= room ? 32 : (n * 16LL <= room ? 16 : (n * 8LL <= room ? 8 : 4));
+  return n <= 5 * 152 ? 32 : (n <= 17 * 152 ? 16 : (n <= 85 * 152 ? 8 : 4));
 }
 
 template <int G>

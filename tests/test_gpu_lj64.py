@@ -32,7 +32,8 @@ def _check(eng, oracle, pos, vel, L, periodic, table="argon", rs=RS, rc=RC, nlj=
     return en
 
 
-@pytest.mark.parametrize("n", [1, 2, 31, 33, 2432, 2433, 4864, 4865, 9728, 9729])
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 760, 761, 2432, 2433, 2584, 2585, 4864, 4865, 9728,
+                               9729, 12920, 12921])
 def test_lane_counts(eng, oracle, n):
     cells = max(6, int(np.ceil((n / 4.0) ** (1.0 / 3.0))))
     pos, vel, L = lat.make_system("fcc", cells, 94.4, seed=n, natoms=n, noise=0.1)
