@@ -301,7 +301,7 @@ __device__ __forceinline__ float angular_sum(const F2 (&p)[2][4], const DescPara
   return (v[0] + __shfl_xor_sync(0xffffffffu, v[0], 16)) * P.pref[lane & 15];
 }
 
-// descriptors of atom i (one warp); out: normalised (G - mean) * istd, or raw G
+// descriptors of atom i (one warp), normalised: (G - mean) * istd
 __global__ void __launch_bounds__(128)
     k_sg_desc(const md_double4* __restrict__ pos, int n, const uint32_t* __restrict__ sl,
               const int* __restrict__ slen, double box, DescParams P,
@@ -358,7 +358,150 @@ __global__ void __launch_bounds__(128)
   }
   const float angular = angular_sum(p, P);
   const float G = lane < kRad ? radial : angular;
-  out[(size_t)i * kDesc + lane] = mean ? (G - mean[lane]) * istd[lane] : G;
+  out[(size_t)i * kDesc + lane] = (G - mean[lane]) * istd[lane];
+}
+
+// ---- raw descriptors, the features of training ----
+// Features are scaled to unit variance and rounded to BF16 for the tensor cores,
+// and Adam's first steps move a weight by the learning rate whatever its
+// gradient's size: a last bit of a feature decides the sign of a gradient that is
+// nearly zero.  With k_sg_desc's order of sums one training in thirty of 10 to 20
+// steps ended with a weight a whole step off; with this order and these roundings
+// trainings differ by 1e-6, as two runs on the same features do.  So this kernel
+// keeps them (73 us for 32,768 atoms against 38, once per configuration).
+
+// Angular factors of one neighbour pair for the 16 functions f = 8 e + 4 l + z
+// of default_desc's table (eta index e, lambda index l for +1 / -1, zeta index
+// z for 1, 2, 4, 16): powers of both bases by squaring and one exponential
+// per eta, instead of 16 of each.
+struct AngPair {
+  float b[2];        // 1 + lambda cos
+  float pz[2][4];    // b ^ zeta
+  float pz1[2][4];   // b ^ (zeta - 1)
+  float ex[2];       // exp(-eta q)
+};
+
+__device__ __forceinline__ void ang_pair(float c, float q, const DescParams& P, AngPair& A) {
+#pragma unroll
+  for (int l = 0; l < 2; l++) {
+    const float b = l ? 1.f - c : 1.f + c;
+    const float p2 = b * b, p4 = p2 * p2, p8 = p4 * p4;
+    A.b[l] = b;
+    A.pz[l][0] = b;
+    A.pz[l][1] = p2;
+    A.pz[l][2] = p4;
+    A.pz[l][3] = p8 * p8;
+    A.pz1[l][0] = 1.f;
+    A.pz1[l][1] = b;
+    A.pz1[l][2] = p2 * b;
+    A.pz1[l][3] = p8 * p4 * p2 * b;
+  }
+  A.ex[0] = __expf(-P.eta_a[0] * q);
+  A.ex[1] = __expf(-P.eta_a[8] * q);
+}
+
+struct NbrSm {
+  float dx[kSgMax], dy[kSgMax], dz[kSgMax], r[kSgMax], ir[kSgMax], fc[kSgMax], dfc[kSgMax];
+  int idx[kSgMax];
+};
+
+// neighbours of atom i into the warp's shared arrays; returns their count
+__device__ __forceinline__ int warp_load_nbrs(int i, const md_double4* pos, const uint32_t* sl,
+                                              const int* slen, double box, float fca,
+                                              NbrSm& N) {
+  const int lane = threadIdx.x & 31;
+  const md_double4 pi = pos[i];
+  const int S = slen[i];
+  for (int s = lane; s < S; s += 32) {
+    const uint32_t e = sl[(size_t)i * kSgMax + s];
+    const int j = entry_index(e);
+    const md_double4 pj = pos[j];
+    const float dx = (float)(pj.x + entry_img(e, 0) * box - pi.x);
+    const float dy = (float)(pj.y + entry_img(e, 1) * box - pi.y);
+    const float dz = (float)(pj.z + entry_img(e, 2) * box - pi.z);
+    const float r = sqrtf(dx * dx + dy * dy + dz * dz);
+    float fc, dfc;
+    fcut(r, fca, fc, dfc);
+    N.dx[s] = dx;
+    N.dy[s] = dy;
+    N.dz[s] = dz;
+    N.r[s] = r;
+    N.ir[s] = 1.f / r;  // the pair terms multiply by it instead of dividing
+    N.fc[s] = fc;
+    N.dfc[s] = dfc;
+    N.idx[s] = j;
+  }
+  __syncwarp();
+  return S;
+}
+
+// k-th pair (a < b) of S neighbours in row-major order
+__device__ __forceinline__ void pair_of(int k, int S, int& a, int& b) {
+  const int m = 2 * S - 1;
+  int aa = (int)(0.5f * ((float)m - sqrtf((float)(m * m - 8 * k))));
+  aa = max(0, min(aa, S - 2));
+  auto off = [&](int x) { return x * (2 * S - x - 1) / 2; };
+  while (aa > 0 && off(aa) > k) aa--;
+  while (aa + 1 <= S - 2 && off(aa + 1) <= k) aa++;
+  a = aa;
+  b = k - off(aa) + aa + 1;
+}
+
+// sum over the warp of 32 per-lane vectors: lane f ends with component f
+__device__ __forceinline__ float warp_reduce_scatter32(float (&v)[32]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 16, h = 16; o > 0; o >>= 1, h >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int k = 0; k < h; k++) {
+      const float send = up ? v[k] : v[k + h];
+      const float keep = up ? v[k + h] : v[k];
+      v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  return v[0];
+}
+
+// raw descriptors of atom i (one warp)
+__global__ void __launch_bounds__(128)
+    k_sg_desc_raw(const md_double4* __restrict__ pos, int n, const uint32_t* __restrict__ sl,
+                  const int* __restrict__ slen, double box, DescParams P,
+                  float* __restrict__ out) {
+  __shared__ NbrSm nb[4];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int i = blockIdx.x * 4 + warp;
+  if (i >= n) return;  // whole warp
+  NbrSm& N = nb[warp];
+  const int S = warp_load_nbrs(i, pos, sl, slen, box, P.fca, N);
+  float v[32];
+#pragma unroll
+  for (int f = 0; f < 32; f++) v[f] = 0.f;
+  for (int s = lane; s < S; s += 32) {
+#pragma unroll
+    for (int k = 0; k < kRad; k++) {
+      const float t = N.r[s] - P.rs[k];
+      v[k] += __expf(-P.eta_r * t * t) * N.fc[s];
+    }
+  }
+  const int npair = S * (S - 1) / 2;
+  for (int k = lane; k < npair; k += 32) {
+    int a, b;
+    pair_of(k, S, a, b);
+    const float c = (N.dx[a] * N.dx[b] + N.dy[a] * N.dy[b] + N.dz[a] * N.dz[b]) * (N.ir[a] * N.ir[b]);
+    const float q = N.r[a] * N.r[a] + N.r[b] * N.r[b];
+    const float ff = N.fc[a] * N.fc[b];
+    AngPair T;
+    ang_pair(c, q, P, T);
+#pragma unroll
+    for (int f = 0; f < kAng; f++) {
+      const int e = f >> 3, l = (f >> 2) & 1, z = f & 3;
+      const float pz = T.b[l] > 0.f ? T.pz[l][z] : 0.f;
+      v[kRad + f] += P.pref[f] * pz * T.ex[e] * ff;
+    }
+  }
+  const float G = warp_reduce_scatter32(v);
+  out[(size_t)i * kDesc + lane] = G;
 }
 
 // forces from g_if = dE_i/dG_if, one warp per atom i, into F32 (n x 4, one
@@ -1829,9 +1972,11 @@ int sur_descriptors(Surrogate& s, const md_double4* pos, int n, const RowWalker&
   if (n == 0) return 0;
   k_sg_pos32<<<sblocks(n, 256), 256, 0, st>>>(pos, n, s.pos32);
   k_sg_short<<<sblocks(n, 4), 128, 0, st>>>(s.pos32, w, s.rc, s.sl, s.slen, d_status);
-  k_sg_desc<<<sblocks(n, 4), 128, 0, st>>>(pos, n, s.sl, s.slen, w.g.box, s.P,
-                                             normalised ? s.mean_d : nullptr,
-                                             normalised ? s.istd_d : nullptr, s.X);
+  if (normalised)
+    k_sg_desc<<<sblocks(n, 4), 128, 0, st>>>(pos, n, s.sl, s.slen, w.g.box, s.P, s.mean_d, s.istd_d,
+                                             s.X);
+  else
+    k_sg_desc_raw<<<sblocks(n, 4), 128, 0, st>>>(pos, n, s.sl, s.slen, w.g.box, s.P, s.X);
   return (int)cudaGetLastError();
 }
 
