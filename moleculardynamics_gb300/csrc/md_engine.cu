@@ -349,6 +349,7 @@ MbArgs mb_args(md_ctx* c, double* f3, int ljexist) {
   a.xsi = c->xsi;
   a.xsj = c->xsj;
   a.missing = c->missing;
+  a.early = true;
   a.epart1 = nullptr;
   a.epart2 = nullptr;
   return a;

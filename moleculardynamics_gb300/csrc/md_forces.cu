@@ -1730,19 +1730,17 @@ static void launch_mb64(const MbArgs& a, cudaStream_t st) {
   double *e1 = ENERGY ? a.epart1 : nullptr, *e2 = ENERGY ? a.epart2 : nullptr;
   double* ea = ENERGY ? a.eatom : nullptr;
   const int B = nblk(a.n, 4);
-  launch_dependent(true, k_mb_short<double>, B, 128, st, a.pos, a.posf, a.n, a.list, a.ri, a.rk, a.len, a.grid,
-                                        a.rcutsq, a.sl, (size_t)a.pitch, 1, a.slen, gate);
+  launch_dependent(a.early, k_mb_short<double>, B, 128, st, a.pos, a.posf, a.n, a.list, a.ri, a.rk,
+                   a.len, a.grid, a.rcutsq, a.sl, (size_t)a.pitch, 1, a.slen, gate);
   if (!a.ref_rows) {
-    launch_dependent(
-        true, k_mb_bonds<ENERGY, true>, a.n, 128, st, a.pos, a.f3, a.n, a.sl, a.pitch, a.slen, a.grid, a.cell3, a.ljexist, wi, wj, fs,
-        a.missing, e1, ea, gate);
-    launch_dependent(true, k_mb_gather<ENERGY>, B, 128, st, a.pos, a.posf, a.f3, a.n, a.sl, a.pitch,
-                                                   a.slen, a.grid, a.cell3, a.rcutsq, wi, wj, fs,
-                                                   a.missing, e2, gate);
+    launch_dependent(a.early, k_mb_bonds<ENERGY, true>, a.n, 128, st, a.pos, a.f3, a.n, a.sl, a.pitch,
+                     a.slen, a.grid, a.cell3, a.ljexist, wi, wj, fs, a.missing, e1, ea, gate);
+    launch_dependent(a.early, k_mb_gather<ENERGY>, B, 128, st, a.pos, a.posf, a.f3, a.n, a.sl,
+                     a.pitch, a.slen, a.grid, a.cell3, a.rcutsq, wi, wj, fs, a.missing, e2, gate);
   } else if constexpr (!ENERGY) {
-    launch_dependent(
-        true, k_mb_bonds<false, false>, a.n, 128, st, a.pos, a.f3, a.n, a.sl, a.pitch, a.slen, a.grid, nullptr, a.ljexist, wi, wj,
-        nullptr, a.missing, nullptr, nullptr, gate);
+    launch_dependent(a.early, k_mb_bonds<false, false>, a.n, 128, st, a.pos, a.f3, a.n, a.sl, a.pitch,
+                     a.slen, a.grid, nullptr, a.ljexist, wi, wj, nullptr, a.missing, nullptr, nullptr,
+                     gate);
     k_mb_pass2<<<B, 128, 0, st>>>(a.pos, a.f3, a.n, a.sl, a.pitch, a.slen, a.grid, a.ref_rows,
                                   a.ref_nls, a.ref_nlargest, a.rcutsq, wi, wj, a.missing);
   }
