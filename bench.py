@@ -194,14 +194,14 @@ def fp32_roofline(entries: int, launch_s: float, arith: dict) -> dict:
 
 def fp64_lj_roofline(entries: int, launch_s: float, arith: dict) -> dict:
     """The plain FP64 LJ kernel (k_lj_fp64) against the FP64 rate measured
-    on this device.  Operations of the reference's formula as the kernel
-    evaluates it (no FMA contraction, for bit-exact parity;
-    cpu/common/LennardJones.h:12-30): per row entry 3 differences, r^2 (3
+    on this device.  Operations of the reference's formula (no FMA
+    contraction, for bit-exact parity; cpu/common/LennardJones.h:12-30): per row entry 3 differences, r^2 (3
     products, 2 sums) and the cutoff test = 8; per pair inside the cutoff
     a square root, 4 divisions, 10 products and sums and 3 FMA-free updates
-    of the sums (6) = 21, each counted as one flop.  Divisions and square
-    roots take many FP64 pipe slots each, so this count sits well below
-    the pipe's occupancy."""
+    of the sums (6) = 21, each counted as one flop.  The kernel takes the
+    root, the quotients and most products in integer instructions, and its
+    launch includes the step's Gear update, so the fraction compares the
+    formula's work with the FP64 rate; it is not the pipe's occupancy."""
     inside = entries * (2.5 / 2.8) ** 3
     flops = 8.0 * entries + 21.0 * inside
     achieved = flops / launch_s / 1e12
@@ -212,15 +212,15 @@ def fp64_lj_roofline(entries: int, launch_s: float, arith: dict) -> dict:
             "divisions_and_sqrt_per_launch": 5.0 * inside}
 
 
-# FP32 flops of the bond-order force evaluation (k_mb_short + k_mb_pass1 +
-# k_mb_pass2), counted from the kernels' FP32 expressions with FMA = 2 and a
+# FP32 flops of the bond-order force evaluation (k_mb_short + k_mb_pass1_32 +
+# k_mb_pass2_32), counted from the kernels' FP32 expressions with FMA = 2 and a
 # reciprocal, square root, exponential or tanh = 1: per pair within the cutoff
 # (attractive, repulsive and van der Waals terms, the pair cutoff, the bond
 # order from xi, the force) 75; per pass-1 triplet (i, j, m), both sides of
 # the angle term with their derivatives, 110; per pass-2 triplet (k, i, j)
-# 130.  The FP64 instantiation evaluates the reference's own expressions
-# (more operations, divisions in place of products); the same counts are used
-# for it, so its fraction is a lower bound.
+# 130.  The FP64 form evaluates a triplet once for both passes, its angle terms
+# in fixed point; the same counts are used for it, so its fraction compares the
+# two passes' work with the FP64 rate.
 MB_FLOPS_PAIR, MB_FLOPS_TRIPLET1, MB_FLOPS_TRIPLET2 = 75.0, 110.0, 130.0
 
 
@@ -245,7 +245,8 @@ def bond_order_roofline(counts: dict, launch_s: float, arith: dict, fp64: bool) 
              + MB_FLOPS_TRIPLET2 * counts["triplets_pass2"])
     achieved = flops / launch_s / 1e12
     peak = (arith["fp64_gflops"] if fp64 else arith["fp32_gflops"]) / 1e3
-    return {"kernel": "k_mb_short + k_mb_pass1 + k_mb_pass2" + ("<double>" if fp64 else "<float>"),
+    return {"kernel": "k_mb_short + k_mb_bonds + k_mb_gather" if fp64
+            else "k_mb_short + k_mb_pass1_32 + k_mb_pass2_32",
             "bound": "fp64" if fp64 else "fp32", "achieved": achieved, "peak": peak,
             "unit": "TFLOP/s", "frac": achieved / peak,
             "peak_source": "measured (FMA chains on this device)",
