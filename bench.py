@@ -218,10 +218,11 @@ def fp64_lj_roofline(entries: int, launch_s: float, arith: dict) -> dict:
 # (attractive, repulsive and van der Waals terms, the pair cutoff, the bond
 # order from xi, the force) 75; per pass-1 triplet (i, j, m), both sides of
 # the angle term with their derivatives, 110; per pass-2 triplet (k, i, j)
-# 130.  The FP64 form evaluates a triplet once for both passes, its angle terms
-# in fixed point; the same counts are used for it, so its fraction compares the
-# two passes' work with the FP64 rate.
+# 130.  The FP64 form evaluates a triplet once, 110 and 30 for the force on its
+# third body; its angle terms are in fixed point, so its fraction compares that
+# work with the FP64 rate and is not the pipe's occupancy.
 MB_FLOPS_PAIR, MB_FLOPS_TRIPLET1, MB_FLOPS_TRIPLET2 = 75.0, 110.0, 130.0
+MB_FLOPS_TRIPLET64 = 140.0
 
 
 def bond_order_counts(pos: np.ndarray, L: float, rcut: float = 3.0) -> dict:
@@ -241,8 +242,9 @@ def bond_order_counts(pos: np.ndarray, L: float, rcut: float = 3.0) -> dict:
 
 
 def bond_order_roofline(counts: dict, launch_s: float, arith: dict, fp64: bool) -> dict:
-    flops = (MB_FLOPS_PAIR * counts["pairs"] + MB_FLOPS_TRIPLET1 * counts["triplets_pass1"]
-             + MB_FLOPS_TRIPLET2 * counts["triplets_pass2"])
+    flops = MB_FLOPS_PAIR * counts["pairs"] + (
+        MB_FLOPS_TRIPLET64 * counts["triplets_pass1"] if fp64 else
+        MB_FLOPS_TRIPLET1 * counts["triplets_pass1"] + MB_FLOPS_TRIPLET2 * counts["triplets_pass2"])
     achieved = flops / launch_s / 1e12
     peak = (arith["fp64_gflops"] if fp64 else arith["fp32_gflops"]) / 1e3
     return {"kernel": "k_mb_short + k_mb_bonds + k_mb_gather" if fp64
