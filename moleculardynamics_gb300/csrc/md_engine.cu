@@ -17,7 +17,6 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -1692,8 +1691,8 @@ static void copy_parts(void* const (&dst)[2], const void* const (&src)[2],
   int started = 0;
   try {
     for (; started + 1 < parts; started++) t[started] = std::thread(piece, started, parts);
-  } catch (const std::system_error&) {
-    // no more threads: the rest is copied here
+  } catch (...) {
+    // no more threads (or memory for one): the rest is copied here
   }
   for (int p = started; p < parts; p++) piece(p, parts);
   for (int p = 0; p < started; p++) t[p].join();
