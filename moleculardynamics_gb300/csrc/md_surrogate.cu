@@ -115,6 +115,8 @@ __device__ __forceinline__ void fcut(float r, float a, float& fc, float& dfc) {
 __global__ void __launch_bounds__(128)
     k_sg_short(const float4* __restrict__ pos, RowWalker w, float rc,
                uint32_t* __restrict__ sl, int* __restrict__ slen, int* __restrict__ status) {
+  grid_wait();
+  grid_launch_dependents();
   const int lane = threadIdx.x & 31;
   const int i = blockIdx.x * 4 + (threadIdx.x >> 5);
   if (i >= w.n) return;  // whole warp
@@ -307,6 +309,8 @@ __global__ void __launch_bounds__(128)
               const int* __restrict__ slen, double box, DescParams P,
               const float* __restrict__ mean, const float* __restrict__ istd,
               float* __restrict__ out) {
+  grid_wait();
+  grid_launch_dependents();
   __shared__ float4 nu[4][kSgRow];  // unit vector
   __shared__ float2 nw[4][kSgRow];  // w
   __shared__ float2 nr[4][kSgMax];  // r, fc
@@ -514,6 +518,8 @@ __global__ void __launch_bounds__(128)
     k_sg_force(const md_double4* __restrict__ pos, int n, const uint32_t* __restrict__ sl,
                const int* __restrict__ slen, double box, DescParams P,
                const float* __restrict__ gcoef, float4* __restrict__ F32) {
+  grid_wait();
+  grid_launch_dependents();
   __shared__ float4 nu[4][kSgRow];  // unit vector, 1/r
   __shared__ float4 nw[4][kSgRow];  // w, d
   __shared__ int idx[4][kSgMax];
@@ -647,6 +653,8 @@ __global__ void __launch_bounds__(128)
 }
 
 __global__ void k_sg_pos32(const md_double4* __restrict__ pos, int n, float4* __restrict__ out) {
+  grid_wait();
+  grid_launch_dependents();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const md_double4 p = pos[i];
@@ -658,6 +666,8 @@ __global__ void k_sg_pos32(const md_double4* __restrict__ pos, int n, float4* __
 __global__ void k_sg_store(const float4* __restrict__ F32, double* __restrict__ f3, int n,
                            int accumulate, const int* __restrict__ skip,
                            int* __restrict__ skipped) {
+  grid_wait();
+  grid_launch_dependents();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (skip && *skip) {
     if (k == 0 && skipped) atomicAdd(skipped, 1);
@@ -775,6 +785,8 @@ __device__ __forceinline__ float tanh_fast(float x) {
 __global__ void __launch_bounds__(128)
     k_net_infer(const float* __restrict__ X, int n, NetDev w, float* __restrict__ t_out,
                 float* __restrict__ dtdx, int* status) {
+  grid_wait();
+  grid_launch_dependents();
   extern __shared__ __align__(1024) unsigned char sm[];
   __shared__ __align__(8) uint64_t bar;
   __shared__ uint32_t s_taddr;
@@ -932,6 +944,8 @@ __global__ void __launch_bounds__(128)
                 const int* __restrict__ rows, int nrows, unsigned long long seed, NetDev w,
                 float inv_batch, float* __restrict__ grad, double* __restrict__ loss,
                 int* status) {
+  grid_wait();
+  grid_launch_dependents();
   extern __shared__ __align__(1024) unsigned char sm[];
   __shared__ __align__(8) uint64_t bar;
   __shared__ uint32_t s_taddr;
@@ -1057,6 +1071,8 @@ __global__ void __launch_bounds__(128)
                 const int* __restrict__ slen, double box, DescParams P,
                 const float* __restrict__ e3, float scale, const float* __restrict__ istd,
                 float* __restrict__ V) {
+  grid_wait();
+  grid_launch_dependents();
   __shared__ float4 nu[4][kSgRow];  // unit vector, s / r
   __shared__ float4 ne[4][kSgRow];  // de / r
   __shared__ float4 nw[4][kSgRow];  // w, d s
@@ -1128,6 +1144,8 @@ __global__ void __launch_bounds__(128)
 // e = F_pred - F_exact (FP32) and sum e^2 into acc[0]
 __global__ void k_fm_resid(const float4* __restrict__ F32, const double* __restrict__ fx, int n3,
                            float* __restrict__ e3, double* __restrict__ acc) {
+  grid_wait();
+  grid_launch_dependents();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   double s = 0.0;
   if (k < n3) {
@@ -1148,6 +1166,8 @@ __global__ void k_fm_resid(const float4* __restrict__ F32, const double* __restr
 __global__ void __launch_bounds__(128)
     k_net_train_force(const float* __restrict__ X, const float* __restrict__ V, int n, NetDev w,
                       float* __restrict__ grad, int* status) {
+  grid_wait();
+  grid_launch_dependents();
   extern __shared__ __align__(1024) unsigned char sm[];
   __shared__ __align__(8) uint64_t bar;
   __shared__ uint32_t s_taddr;
@@ -1281,6 +1301,8 @@ __global__ void __launch_bounds__(128)
 __global__ void k_adam(float* __restrict__ P, float* __restrict__ M, float* __restrict__ V,
                        const float* __restrict__ G, int step, float lr, float b1, float b2,
                        float eps) {
+  grid_wait();
+  grid_launch_dependents();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= kParams) return;
   const float g = G[k];
@@ -1294,6 +1316,8 @@ __global__ void k_adam(float* __restrict__ P, float* __restrict__ M, float* __re
 }
 
 __global__ void k_net_cast(const float* __restrict__ P, __nv_bfloat16* W1, __nv_bfloat16* W2) {
+  grid_wait();
+  grid_launch_dependents();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k < kHid * kDesc) W1[k] = __float2bfloat16_rn(P[oW1 + k]);
   if (k < kHid * kHid) W2[k] = __float2bfloat16_rn(P[oW2 + k]);
@@ -1304,6 +1328,8 @@ __global__ void k_net_cast(const float* __restrict__ P, __nv_bfloat16* W1, __nv_
 __global__ void k_sg_scale(const float* __restrict__ t, const float4* __restrict__ dtdx, int n,
                            double mu, double sigma, const float4* __restrict__ istd,
                            float4* __restrict__ gcoef, double* __restrict__ eatom) {
+  grid_wait();
+  grid_launch_dependents();
   const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   constexpr int kQ = kDesc / 4;
   if (k >= (long long)n * kQ) return;
@@ -1449,6 +1475,8 @@ __global__ void __launch_bounds__(128 * fh_groups(H))
     k_fh_forward(const float* __restrict__ X, int n, const float* __restrict__ P,
                  const float* __restrict__ gscale, float* __restrict__ gcoef,
                  float* __restrict__ xT, float* __restrict__ h1T, float* __restrict__ h2T) {
+  grid_wait();
+  grid_launch_dependents();
   extern __shared__ float4 wsm4[];
   constexpr int kA = 32 * A * fh_groups(H), O = H / 4;  // atoms of the block, outputs of a warp
   float* wsm = (float*)wsm4;
@@ -1715,8 +1743,8 @@ void fh_forward(const Surrogate& s, const float* X, int n, float* gcoef, bool ke
   const float* gs = s.fh_gs;
   auto run = [&](auto kernel, int H, int A) {
     const int g = fh_groups(H);
-    kernel<<<sblocks(n, 32 * A * g), 128 * g, fh_smem(H, A), st>>>(X, n, s.FP_d, gs, gcoef, xT, h1,
-                                                                   h2);
+    launch_dependent_smem(true, fh_smem(H, A), kernel, sblocks(n, 32 * A * g), 128 * g, st, X, n,
+                          s.FP_d, gs, gcoef, xT, h1, h2);
   };
   const bool two = n > 64 * 152;  // blocks of 64 atoms for every SM
   if (s.fh_hidden == 32)
@@ -1908,7 +1936,7 @@ int sur_set_params(Surrogate& s, const float* P, cudaStream_t st) {
   cudaMemsetAsync(s.M_d, 0, sizeof(float) * kParams, st);
   cudaMemsetAsync(s.V_d, 0, sizeof(float) * kParams, st);
   s.adam_step = 0;
-  k_net_cast<<<sblocks(kHid * kHid, 256), 256, 0, st>>>(s.P_d, s.W1, s.W2);
+  launch_dependent(true, k_net_cast, sblocks(kHid * kHid, 256), 256, st, s.P_d, s.W1, s.W2);
   return cudaStreamSynchronize(st);
 }
 
@@ -1935,8 +1963,8 @@ int sur_directional(Surrogate& s, const md_double4* pos, int n, double box, cons
     e = cudaMemcpyAsync(de, he.data(), sizeof(float) * he.size(), cudaMemcpyHostToDevice, st);
   std::vector<float> hv(kDesc * (size_t)n);
   if (e == cudaSuccess) {
-    k_sg_ctrans<<<sblocks(n, 4), 128, 0, st>>>(pos, n, s.sl, s.slen, box, s.P, de, 1.f, nullptr,
-                                               dv);
+    launch_dependent(true, k_sg_ctrans, sblocks(n, 4), 128, st, pos, n, s.sl, s.slen, box, s.P,
+                     de, 1.f, nullptr, dv);
     e = cudaMemcpyAsync(hv.data(), dv, sizeof(float) * hv.size(), cudaMemcpyDeviceToHost, st);
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -1970,11 +1998,12 @@ int sur_descriptors(Surrogate& s, const md_double4* pos, int n, const RowWalker&
     s.n_alloc = n;
   }
   if (n == 0) return 0;
-  k_sg_pos32<<<sblocks(n, 256), 256, 0, st>>>(pos, n, s.pos32);
-  k_sg_short<<<sblocks(n, 4), 128, 0, st>>>(s.pos32, w, s.rc, s.sl, s.slen, d_status);
+  launch_dependent(true, k_sg_pos32, sblocks(n, 256), 256, st, pos, n, s.pos32);
+  launch_dependent(true, k_sg_short, sblocks(n, 4), 128, st, s.pos32, w, s.rc, s.sl, s.slen,
+                   d_status);
   if (normalised)
-    k_sg_desc<<<sblocks(n, 4), 128, 0, st>>>(pos, n, s.sl, s.slen, w.g.box, s.P, s.mean_d, s.istd_d,
-                                             s.X);
+    launch_dependent(true, k_sg_desc, sblocks(n, 4), 128, st, pos, n, s.sl, s.slen, w.g.box, s.P,
+                     s.mean_d, s.istd_d, s.X);
   else
     k_sg_desc_raw<<<sblocks(n, 4), 128, 0, st>>>(pos, n, s.sl, s.slen, w.g.box, s.P, s.X);
   return (int)cudaGetLastError();
@@ -2071,13 +2100,13 @@ int sur_train(Surrogate& s, int steps, int batch, float lr, double* loss_out, cu
   for (int it = 0; it < steps; it++) {
     cudaMemsetAsync(s.G_d, 0, sizeof(float) * kParams, st);
     cudaMemsetAsync(s.loss_d, 0, sizeof(double), st);
-    k_net_train<<<tiles, 128, kSmTrain, st>>>(s.SX, s.ST, s.ns, nullptr, tiles * 128,
-                                              s.seed + 0x9E37ULL * (unsigned long long)(s.adam_step + 1),
-                                              net_of(s), inv, s.G_d, s.loss_d, s.status_d);
+    launch_dependent_smem(true, kSmTrain, k_net_train, tiles, 128, st, s.SX, s.ST, s.ns, nullptr,
+                          tiles * 128, s.seed + 0x9E37ULL * (unsigned long long)(s.adam_step + 1),
+                          net_of(s), inv, s.G_d, s.loss_d, s.status_d);
     s.adam_step++;
-    k_adam<<<sblocks(kParams, 256), 256, 0, st>>>(s.P_d, s.M_d, s.V_d, s.G_d, s.adam_step, lr,
-                                                 0.9f, 0.999f, 1e-8f);
-    k_net_cast<<<sblocks(kHid * kHid, 256), 256, 0, st>>>(s.P_d, s.W1, s.W2);
+    launch_dependent(true, k_adam, sblocks(kParams, 256), 256, st, s.P_d, s.M_d, s.V_d, s.G_d,
+                     s.adam_step, lr, 0.9f, 0.999f, 1e-8f);
+    launch_dependent(true, k_net_cast, sblocks(kHid * kHid, 256), 256, st, s.P_d, s.W1, s.W2);
     if (it >= steps - 16) {  // mean loss of the last steps
       double l = 0;
       cudaMemcpyAsync(&l, s.loss_d, sizeof(double), cudaMemcpyDeviceToHost, st);
@@ -2109,9 +2138,9 @@ int sur_loss_grad(Surrogate& s, const float* X, const float* T, int n, float* gr
   cudaMemcpyAsync(s.rows_d, rows.data(), sizeof(int) * n, cudaMemcpyHostToDevice, st);
   cudaMemsetAsync(s.G_d, 0, sizeof(float) * kParams, st);
   cudaMemsetAsync(s.loss_d, 0, sizeof(double), st);
-  k_net_train<<<(n + 127) / 128, 128, kSmTrain, st>>>(s.Xg, s.Tg, n, s.rows_d, n, 0ULL,
-                                                      net_of(s), 1.f / (float)n, s.G_d,
-                                                      s.loss_d, s.status_d);
+  launch_dependent_smem(true, kSmTrain, k_net_train, (n + 127) / 128, 128, st, s.Xg, s.Tg, n,
+                        s.rows_d, n, 0ULL, net_of(s), 1.f / (float)n, s.G_d, s.loss_d,
+                        s.status_d);
   cudaMemcpyAsync(grad, s.G_d, sizeof(float) * kParams, cudaMemcpyDeviceToHost, st);
   cudaMemcpyAsync(loss, s.loss_d, sizeof(double), cudaMemcpyDeviceToHost, st);
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
@@ -2129,7 +2158,8 @@ int sur_net_eval(Surrogate& s, const float* X, int n, float* t, float* dtdx, cud
   s.nxg = n;
   cudaMemcpyAsync(s.Xg, X, sizeof(float) * kDesc * n, cudaMemcpyHostToDevice, st);
   float* t_d = s.Tg + (size_t)kDesc * n;  // behind the gradients, whose rows are 16-byte aligned
-  k_net_infer<<<(n + 127) / 128, 128, kSmInfer, st>>>(s.Xg, n, net_of(s), t_d, s.Tg, s.status_d);
+  launch_dependent_smem(true, kSmInfer, k_net_infer, (n + 127) / 128, 128, st, s.Xg, n, net_of(s),
+                        t_d, s.Tg, s.status_d);
   cudaMemcpyAsync(t, t_d, sizeof(float) * n, cudaMemcpyDeviceToHost, st);
   cudaMemcpyAsync(dtdx, s.Tg, sizeof(float) * kDesc * n, cudaMemcpyDeviceToHost, st);
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
@@ -2179,20 +2209,22 @@ int sur_forces(Surrogate& s, const md_double4* pos, int n, const RowWalker& w, d
     k_fh_gscale<<<1, 32, 0, st>>>(s.istd_d, (float)fh_out_scale(s), s.fh_gs);
     fh_forward(s, s.X, n, s.gcoef, false, st);
     cudaMemsetAsync(s.F32, 0, sizeof(float4) * (size_t)n, st);
-    k_sg_force<<<sblocks(n, 4), 128, 0, st>>>(pos, n, s.sl, s.slen, w.g.box, s.P, s.gcoef, s.F32);
-    k_sg_store<<<sblocks(3LL * n, 256), 256, 0, st>>>(s.F32, f3, n, accumulate, skip,
-                                                      declined_count);
+    launch_dependent(true, k_sg_force, sblocks(n, 4), 128, st, pos, n, s.sl, s.slen, w.g.box, s.P,
+                     s.gcoef, s.F32);
+    launch_dependent(true, k_sg_store, sblocks(3LL * n, 256), 256, st, s.F32, f3, n, accumulate,
+                     skip, declined_count);
     if (energy_dev) k_fill_nan<<<1, 1, 0, st>>>(energy_dev);
     return (int)cudaGetLastError();
   }
-  k_net_infer<<<(n + 127) / 128, 128, kSmInfer, st>>>(s.X, n, net_of(s), s.t, s.dtdx, s.status_d);
-  k_sg_scale<<<sblocks(8LL * n, 256), 256, 0, st>>>(
-        s.t, (const float4*)s.dtdx, n, s.mu, s.sigma, (const float4*)s.istd_d, (float4*)s.gcoef,
-        s.eatom);
+  launch_dependent_smem(true, kSmInfer, k_net_infer, (n + 127) / 128, 128, st, s.X, n, net_of(s),
+                        s.t, s.dtdx, s.status_d);
+  launch_dependent(true, k_sg_scale, sblocks(8LL * n, 256), 256, st, s.t, (const float4*)s.dtdx,
+                   n, s.mu, s.sigma, (const float4*)s.istd_d, (float4*)s.gcoef, s.eatom);
   cudaMemsetAsync(s.F32, 0, sizeof(float4) * (size_t)n, st);
-  k_sg_force<<<sblocks(n, 4), 128, 0, st>>>(pos, n, s.sl, s.slen, w.g.box, s.P, s.gcoef, s.F32);
-  k_sg_store<<<sblocks(3LL * n, 256), 256, 0, st>>>(s.F32, f3, n, accumulate, skip,
-                                                    declined_count);
+  launch_dependent(true, k_sg_force, sblocks(n, 4), 128, st, pos, n, s.sl, s.slen, w.g.box, s.P,
+                   s.gcoef, s.F32);
+  launch_dependent(true, k_sg_store, sblocks(3LL * n, 256), 256, st, s.F32, f3, n, accumulate,
+                   skip, declined_count);
   if (energy_dev) k_sum_d<<<1, 256, 0, st>>>(s.eatom, n, energy_dev);
   return (int)cudaGetLastError();
 }
@@ -2287,8 +2319,8 @@ int train_fh(Surrogate& s, int steps, float lr, int nmax, double* loss_e, double
     k_fh_probe<<<sblocks(32LL * c.n, 256), 256, 0, st>>>(s.gcoef, 32LL * c.n, s.istd_d,
                                                          s.seed);
     cudaMemsetAsync(s.F32, 0, sizeof(float4) * (size_t)c.n, st);
-    k_sg_force<<<sblocks(c.n, 4), 128, 0, st>>>(c.pos, c.n, c.sl, c.slen, c.box, s.P, s.gcoef,
-                                                s.F32);
+    launch_dependent(true, k_sg_force, sblocks(c.n, 4), 128, st, c.pos, c.n, c.sl, c.slen, c.box,
+                     s.P, s.gcoef, s.F32);
     cudaMemsetAsync(s.scratch, 0, sizeof(double), st);
     k_sumsq<<<sblocks(4LL * c.n, 256), 256, 0, st>>>((const float*)s.F32, 4LL * c.n, s.scratch);
     double sq = 0;
@@ -2306,13 +2338,14 @@ int train_fh(Surrogate& s, int steps, float lr, int nmax, double* loss_e, double
     const int n = c.n;
     fh_forward(s, c.X, n, s.gcoef, true, st);
     cudaMemsetAsync(s.F32, 0, sizeof(float4) * (size_t)n, st);
-    k_sg_force<<<sblocks(n, 4), 128, 0, st>>>(c.pos, n, c.sl, c.slen, c.box, s.P, s.gcoef,
-                                                s.F32);
+    launch_dependent(true, k_sg_force, sblocks(n, 4), 128, st, c.pos, n, c.sl, c.slen, c.box, s.P,
+                     s.gcoef, s.F32);
     cudaMemsetAsync(s.scratch, 0, sizeof(double) * 2, st);
-    k_fm_resid<<<sblocks(3LL * n, 256), 256, 0, st>>>(s.F32, c.fx, 3 * n, s.E3, s.scratch);
+    launch_dependent(true, k_fm_resid, sblocks(3LL * n, 256), 256, st, s.F32, c.fx, 3 * n, s.E3,
+                     s.scratch);
     const float kappa = (float)(s.w_force / (3.0 * n * s.force_var));
-    k_sg_ctrans<<<sblocks(n, 4), 128, 0, st>>>(c.pos, n, c.sl, c.slen, c.box, s.P, s.E3,
-                                                 -2.f * kappa * gsc, s.istd_d, s.V);
+    launch_dependent(true, k_sg_ctrans, sblocks(n, 4), 128, st, c.pos, n, c.sl, c.slen, c.box,
+                     s.P, s.E3, -2.f * kappa * gsc, s.istd_d, s.V);
     cudaMemsetAsync(s.FG_d, 0, sizeof(float) * s.fh_np, st);
     fh_backward(s, s.V, n, st);
     s.fh_step++;
@@ -2473,31 +2506,32 @@ int sur_train_fm(Surrogate& s, int steps, float lr, double* loss_e, double* loss
     const int n = c.n;
     const int tiles = (n + 127) / 128;
     // forces of the current network on this configuration
-    k_net_infer<<<tiles, 128, kSmInfer, st>>>(c.X, n, w, s.t, s.dtdx, s.status_d);
-    k_sg_scale<<<sblocks(8LL * n, 256), 256, 0, st>>>(
-        s.t, (const float4*)s.dtdx, n, s.mu, s.sigma, (const float4*)s.istd_d, (float4*)s.gcoef,
-        s.eatom);
+    launch_dependent_smem(true, kSmInfer, k_net_infer, tiles, 128, st, c.X, n, w, s.t, s.dtdx,
+                          s.status_d);
+    launch_dependent(true, k_sg_scale, sblocks(8LL * n, 256), 256, st, s.t, (const float4*)s.dtdx,
+                     n, s.mu, s.sigma, (const float4*)s.istd_d, (float4*)s.gcoef, s.eatom);
     cudaMemsetAsync(s.F32, 0, sizeof(float4) * (size_t)n, st);
-    k_sg_force<<<sblocks(n, 4), 128, 0, st>>>(c.pos, n, c.sl, c.slen, c.box, s.P, s.gcoef,
-                                                s.F32);
+    launch_dependent(true, k_sg_force, sblocks(n, 4), 128, st, c.pos, n, c.sl, c.slen, c.box, s.P,
+                     s.gcoef, s.F32);
     cudaMemsetAsync(s.scratch, 0, sizeof(double) * 2, st);
-    k_fm_resid<<<sblocks(3LL * n, 256), 256, 0, st>>>(s.F32, c.fx, 3 * n, s.E3, s.scratch);
+    launch_dependent(true, k_fm_resid, sblocks(3LL * n, 256), 256, st, s.F32, c.fx, 3 * n, s.E3,
+                     s.scratch);
     // dL_F/d(dt/dx) = -2 kappa sigma istd q with kappa = w_force / (3 n var_F)
     const float kappa = (float)(s.w_force / (3.0 * n * s.force_var));
-    k_sg_ctrans<<<sblocks(n, 4), 128, 0, st>>>(c.pos, n, c.sl, c.slen, c.box, s.P, s.E3,
-                                                 (float)(-2.0 * kappa * s.sigma), s.istd_d, s.V);
+    launch_dependent(true, k_sg_ctrans, sblocks(n, 4), 128, st, c.pos, n, c.sl, c.slen, c.box,
+                     s.P, s.E3, (float)(-2.0 * kappa * s.sigma), s.istd_d, s.V);
     cudaMemsetAsync(s.G_d, 0, sizeof(float) * kParams, st);
     cudaMemsetAsync(s.loss_d, 0, sizeof(double), st);
     if (s.w_energy > 0.f)
-      k_net_train<<<tiles, 128, kSmTrain, st>>>(c.X, c.T, n, s.iota_d, n, 0ULL, w,
-                                                s.w_energy / (float)n, s.G_d, s.loss_d,
-                                                s.status_d);
+      launch_dependent_smem(true, kSmTrain, k_net_train, tiles, 128, st, c.X, c.T, n, s.iota_d, n,
+                            0ULL, w, s.w_energy / (float)n, s.G_d, s.loss_d, s.status_d);
     if (s.w_force > 0.f)
-      k_net_train_force<<<tiles, 128, kSmForce, st>>>(c.X, s.V, n, w, s.G_d, s.status_d);
+      launch_dependent_smem(true, kSmForce, k_net_train_force, tiles, 128, st, c.X, s.V, n, w,
+                            s.G_d, s.status_d);
     s.adam_step++;
-    k_adam<<<sblocks(kParams, 256), 256, 0, st>>>(s.P_d, s.M_d, s.V_d, s.G_d, s.adam_step, lr,
-                                                 0.9f, 0.999f, 1e-8f);
-    k_net_cast<<<sblocks(kHid * kHid, 256), 256, 0, st>>>(s.P_d, s.W1, s.W2);
+    launch_dependent(true, k_adam, sblocks(kParams, 256), 256, st, s.P_d, s.M_d, s.V_d, s.G_d,
+                     s.adam_step, lr, 0.9f, 0.999f, 1e-8f);
+    launch_dependent(true, k_net_cast, sblocks(kHid * kHid, 256), 256, st, s.P_d, s.W1, s.W2);
     if (it >= steps - std::min(steps, 2 * ncfg)) {  // losses over the last pass
       double le = 0, lf[2];
       cudaMemcpyAsync(&le, s.loss_d, sizeof(double), cudaMemcpyDeviceToHost, st);
@@ -2529,8 +2563,8 @@ int sur_force_grad(Surrogate& s, const float* X, const float* V, int n, float* g
   cudaMemcpyAsync(dX, X, sizeof(float) * kDesc * n, cudaMemcpyHostToDevice, st);
   cudaMemcpyAsync(dV, V, sizeof(float) * kDesc * n, cudaMemcpyHostToDevice, st);
   cudaMemsetAsync(s.G_d, 0, sizeof(float) * kParams, st);
-  k_net_train_force<<<(n + 127) / 128, 128, kSmForce, st>>>(dX, dV, n, net_of(s), s.G_d,
-                                                           s.status_d);
+  launch_dependent_smem(true, kSmForce, k_net_train_force, (n + 127) / 128, 128, st, dX, dV, n,
+                        net_of(s), s.G_d, s.status_d);
   cudaMemcpyAsync(grad, s.G_d, sizeof(float) * kParams, cudaMemcpyDeviceToHost, st);
   e = cudaStreamSynchronize(st);
   cudaFree(dX);
