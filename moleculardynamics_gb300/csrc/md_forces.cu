@@ -1367,6 +1367,8 @@ __global__ void __launch_bounds__(128, 8)
                const int* __restrict__ slen, Grid g, int ljexist, float* __restrict__ xsi_s,
                float* __restrict__ xsj_s, double* __restrict__ epart,
                double* __restrict__ eatom, const int* __restrict__ run_if) {
+  grid_wait();
+  grid_launch_dependents();
   if (!ENERGY && run_if && *run_if == 0) return;
   const int warps = blockDim.x >> 5;
   const int i = blockIdx.x * warps + (threadIdx.x >> 5);
@@ -1577,6 +1579,8 @@ __global__ void __launch_bounds__(128, 12)
                const float* __restrict__ wi_s, const float* __restrict__ wj_s,
                int* __restrict__ missing, double* __restrict__ epart,
                const int* __restrict__ run_if) {
+  grid_wait();
+  grid_launch_dependents();
   if (!ENERGY && run_if && *run_if == 0) return;
   using T = float;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1751,14 +1755,14 @@ static void launch_mb32(const MbArgs& a, cudaStream_t st) {
   const int* gate = ENERGY ? nullptr : a.run_if;
   float *wi = (float*)a.xsi, *wj = (float*)a.xsj;
   const int B = nblk(a.n, 4);
-  k_mb_short<float><<<B, 128, 0, st>>>(a.pos, a.posf, a.n, a.list, a.ri, a.rk, a.len, a.grid,
-                                       a.rcutsq, a.sl, 1, (size_t)a.n, a.slen, gate);
-  k_mb_pass1_32<ENERGY><<<B, 128, 0, st>>>(a.pos, a.posf, a.f3, a.n, a.sl, a.slen, a.grid,
-                                           a.ljexist, wi, wj, ENERGY ? a.epart1 : nullptr,
-                                           ENERGY ? a.eatom : nullptr, gate);
-  k_mb_pass2_32<ENERGY><<<B, 128, 0, st>>>(a.pos, a.posf, a.f3, a.n, a.sl, a.slen, a.grid,
-                                           a.cell3, a.ref_rows, a.ref_nls, a.ref_nlargest, a.rcutsq,
-                                           wi, wj, a.missing, ENERGY ? a.epart2 : nullptr, gate);
+  launch_dependent(a.early, k_mb_short<float>, B, 128, st, a.pos, a.posf, a.n, a.list, a.ri, a.rk,
+                   a.len, a.grid, a.rcutsq, a.sl, 1, (size_t)a.n, a.slen, gate);
+  launch_dependent(a.early, k_mb_pass1_32<ENERGY>, B, 128, st, a.pos, a.posf, a.f3, a.n, a.sl, a.slen,
+                   a.grid, a.ljexist, wi, wj, ENERGY ? a.epart1 : nullptr, ENERGY ? a.eatom : nullptr,
+                   gate);
+  launch_dependent(a.early, k_mb_pass2_32<ENERGY>, B, 128, st, a.pos, a.posf, a.f3, a.n, a.sl, a.slen,
+                   a.grid, a.cell3, a.ref_rows, a.ref_nls, a.ref_nlargest, a.rcutsq, wi, wj, a.missing,
+                   ENERGY ? a.epart2 : nullptr, gate);
 }
 
 void launch_mb(const MbArgs& a, bool fp32, bool energy, cudaStream_t st) {

@@ -65,7 +65,7 @@ struct MbArgs {
   void* fslot = nullptr;  // FP64: forces on third bodies, 4 for each of an atom's kMbSlotCount
                           // first slots (not needed with ref_rows)
   int* missing;
-  bool early = false;   // FP64: launches may start early (streams of this library only)
+  bool early = false;   // launches may start early (streams of this library only)
   const int* run_if = nullptr;  // force launches only: return at once unless *run_if != 0
   double* epart1;       // energy launches: 2 doubles per entry of mb_blocks (bonds)
   double* epart2;       // and 1 (third bodies)

@@ -54,6 +54,8 @@ enum { G_PREDICT = 0, G_CORRECT = 1, G_CORRECT_PREDICT = 2 };
 // form: FP64 state, products fused into FMAs, F/m as F * (1/m).
 template <int MODE>
 __global__ void __launch_bounds__(256) k_gear(GearArgs a) {
+  grid_wait();
+  grid_launch_dependents();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n) return;
   const GearCoef k = a.k;
@@ -841,21 +843,21 @@ void launch_predict(const GearArgs& a, cudaStream_t st) {
   if (a.exact)
     launch_gear64<GEAR64_PREDICT>(a, true, nullptr, nullptr, nullptr, st);
   else
-    k_gear<G_PREDICT><<<nblk(a.n, 256), 256, 0, st>>>(a);
+    launch_dependent(true, k_gear<G_PREDICT>, nblk(a.n, 256), 256, st, a);
 }
 void launch_correct(const GearArgs& a, cudaStream_t st) {
   if (a.n <= 0) return;
   if (a.exact)
     launch_gear64<GEAR64_CORRECT>(a, false, nullptr, nullptr, nullptr, st);
   else
-    k_gear<G_CORRECT><<<nblk(a.n, 256), 256, 0, st>>>(a);
+    launch_dependent(true, k_gear<G_CORRECT>, nblk(a.n, 256), 256, st, a);
 }
 void launch_correct_predict(const GearArgs& a, cudaStream_t st) {
   if (a.n <= 0) return;
   if (a.exact)
     launch_gear64<GEAR64_CORRECT>(a, true, nullptr, nullptr, nullptr, st);
   else
-    k_gear<G_CORRECT_PREDICT><<<nblk(a.n, 256), 256, 0, st>>>(a);
+    launch_dependent(true, k_gear<G_CORRECT_PREDICT>, nblk(a.n, 256), 256, st, a);
 }
 void launch_wall_redo(const GearArgs& a, const int* hit, int* hits, int* flag_next, bool predict,
                       cudaStream_t st) {
