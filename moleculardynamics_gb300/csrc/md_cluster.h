@@ -87,9 +87,12 @@ struct ClusterList {
   long long entries = 0;
   int Z = kClusterMaxZ;                           // cells per segment (upper bound)
   int block = 128;                                // threads per segment block (<= 224)
-  int stage_cap = kClusterMaxStaged;              // staged atoms per segment (soft cap)
-  int row_loads = 2;                              // 1 block TMA tiles, 2 register prefetch,
-                                                  // 3 per-warp TMA tiles
+  // asked for: staged atoms per segment (soft cap) and row scheme (1 block TMA
+  // tiles, 2 register prefetch, 3 per-warp TMA tiles, 4 three block tiles in
+  // flight); 0: the build chooses, by all_ng (atoms of one species) and the sizes
+  int stage_cap = 0, row_loads = 0;
+  bool all_ng = false;
+  int built_loads = 1;                            // scheme of the rows in place: launches go by it
   int grouped = 0;                                // rows grouped by eight slots with byte
                                                   // offsets (the register-prefetch scheme):
                                                   // rows[((k / 8) ld + p) 8 + k % 8] = 16 q

@@ -126,7 +126,6 @@ struct md_ctx {
   // due): two slots, since a correct-only step swaps the position buffers
   // once and windows then start from either buffer order
   bool graphs = false;
-  bool tuned = false;  // md_autotune picked the tiles
   cudaGraphExec_t gexec[2] = {nullptr, nullptr};
   std::vector<unsigned char> gsig[2];
   int glast = 0;  // slot replayed last
@@ -849,7 +848,7 @@ md_status run_window(md_ctx* c) {
   sig.cap = c->cl.cap;
   sig.ld = c->cl.ld;
   sig.wait_limit = c->wait_limit;
-  sig.row_loads = c->cl.row_loads;
+  sig.row_loads = c->cl.built_loads;
   sig.grouped = c->cl.grouped;
   sig.trip2 = gear_args(c, c->t + 1).trip2;
   const void* ptrs[14] = {c->pos, c->pos_alt, c->posf, c->posf_alt, c->vel, c->acc, c->b, c->c,
@@ -1236,18 +1235,6 @@ md_status get_array(md_ctx* c, double* dst, const double* src, int width) {
   return MD_OK;
 }
 
-// Tiles of the cluster kernel where neither the configuration nor the autotuner
-// chose them.  One species: register-prefetch rows, the lean kernel's (33.6 ->
-// 23.1 us per step for 4,000 atoms, 91 -> 69 us for 256,000); block tiles for
-// mixed species.  Up to 65,536 atoms segments are cut at 1,152 staged atoms, so
-// that more blocks share the chip (23.1 -> 21.2 us for 4,000 atoms, 27.1 ->
-// 25.4 us for 32,000); from 87,808 atoms on the blocks fill it anyway (36.1 us
-// against 39 us with the cut).
-void cluster_defaults(md_ctx* c) {
-  if (c->cfg.cluster_row_loads == 0) c->cl.row_loads = c->all_ng ? 2 : 1;
-  if (c->cfg.cluster_stage_cap == 0) c->cl.stage_cap = c->n <= 65536 ? 1152 : kClusterMaxStaged;
-}
-
 md_status md_upload_state(md_ctx* c, const double* pos4, const double* vel3, const double* a3,
                           const double* b3, const double* c3) {
   if (!c) return MD_BAD_ARGUMENT;
@@ -1268,7 +1255,7 @@ md_status md_upload_state(md_ctx* c, const double* pos4, const double* vel3, con
   CK(cudaStreamSynchronize(c->st), "upload");
   if (pos4) {
     c->all_ng = flag == 0;
-    if (c->cluster && !c->tuned) cluster_defaults(c);
+    c->cl.all_ng = c->all_ng;  // for the next build; the rows in place stay as they are
   }
   return MD_OK;
 }
@@ -1608,7 +1595,6 @@ md_status md_autotune(md_ctx* c, int evals, md_tune_result* out) {
   }
   if (s != MD_OK) return s;
   if ((s = build(best_t, best_c, best_l)) != MD_OK) return s;
-  c->tuned = true;
   c->stats.cluster_segments = c->cl.nseg;
   c->stats.cluster_max_staged = c->cl.max_staged;
   if (out) {
