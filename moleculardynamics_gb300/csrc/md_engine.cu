@@ -1254,6 +1254,10 @@ md_status md_upload_state(md_ctx* c, const double* pos4, const double* vel3, con
   if (pos4) CK(cudaMemcpyAsync(&flag, other, sizeof(int), cudaMemcpyDeviceToHost, c->st), "upload");
   CK(cudaStreamSynchronize(c->st), "upload");
   if (pos4) {
+    // the step counters of the one-species launches (ClusterList::sched) hold from
+    // step to step only: steps of other species between would leave them standing
+    if (c->cl.sched && (flag == 0) != (c->all_ng != 0))
+      CK(cudaMemsetAsync(c->cl.sched, 0, sizeof(int) * 8, c->st), "upload");
     c->all_ng = flag == 0;
     c->cl.all_ng = c->all_ng;  // for the next build; the rows in place stay as they are
   }

@@ -66,3 +66,25 @@ def test_upload_changes_the_species(eng, first):
         f2 = e.compute_forces()[0]
     assert rel_rms(f, _fp64_forces(eng, p, v, L, species=0)) < 1e-4
     assert rel_rms(f2, _fp64_forces(eng, p2, v2, L, species=0)) < 1e-4
+
+
+def test_species_changed_twice_between_steps(eng):
+    # The launches of one species hand out segments by counters that each step's
+    # launch clears for the next one; the steps of three species between do not.
+    # Blocks of one warp, more segments than can be resident (32 an SM): a counter
+    # left behind would leave atoms out.  Every tiling gives the same bits.
+    pos, vel, L = argon_fcc(36, noise=0.1)
+    out = []
+    for kw in (dict(cluster_row_loads=1), dict(cluster_threads=32, cluster_row_loads=2)):
+        with _engine(eng, len(pos), L, species=0, **kw) as e:
+            e.upload(pos, vel)
+            e.begin(0.0)
+            for one in (True, False, True, False, True):
+                p, v = e.download()
+                p[:, 3] = pos[:, 3] if one else _types(pos)[:, 3]
+                e.upload(p, v)
+                e.step(2)
+            st = e.stats()
+            out.append(e.download())
+    assert st["cluster_segments"] > 32 * 152 and st["list_builds"] == 1
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
