@@ -2086,11 +2086,8 @@ int sur_train(Surrogate& s, int steps, int batch, float lr, double* loss_out, cu
     int r = sur_normalise(s, st);
     if (r) return r;
   }
-  long long h = s.nsx;
-  if ((e = sur_grow(s.SX, h, (long long)s.ns * kDesc)) != cudaSuccess) return e;
-  h = s.nsx;
-  if ((e = sur_grow(s.ST, h, s.ns)) != cudaSuccess) return e;
-  s.nsx = s.ns;
+  if ((e = sur_grow(s.SX, s.n_sx, (long long)s.ns * kDesc)) != cudaSuccess) return e;
+  if ((e = sur_grow(s.ST, s.n_st, s.ns)) != cudaSuccess) return e;
   k_normalise<<<sblocks(s.ns, 256), 256, 0, st>>>(s.SG, s.SE, s.ns, s.mean_d, s.istd_d, s.mu,
                                                   s.sigma, s.SX, s.ST);
   const int tiles = (batch + 127) / 128;
@@ -2124,13 +2121,9 @@ int sur_loss_grad(Surrogate& s, const float* X, const float* T, int n, float* gr
                   double* loss, cudaStream_t st) {
   cudaError_t e;
   set_attrs();
-  long long h = s.nxg;
-  if ((e = sur_grow(s.Xg, h, (long long)n * kDesc)) != cudaSuccess) return e;
-  h = s.nxg;
-  if ((e = sur_grow(s.Tg, h, n)) != cudaSuccess) return e;
-  h = s.nxg;
-  if ((e = sur_grow(s.rows_d, h, n)) != cudaSuccess) return e;
-  s.nxg = n;
+  if ((e = sur_grow(s.Xg, s.n_xg, (long long)n * kDesc)) != cudaSuccess) return e;
+  if ((e = sur_grow(s.Tg, s.n_tg, n)) != cudaSuccess) return e;
+  if ((e = sur_grow(s.rows_d, s.n_rows, n)) != cudaSuccess) return e;
   std::vector<int> rows(n);
   for (int k = 0; k < n; k++) rows[k] = k;
   cudaMemcpyAsync(s.Xg, X, sizeof(float) * kDesc * n, cudaMemcpyHostToDevice, st);
@@ -2151,11 +2144,8 @@ int sur_loss_grad(Surrogate& s, const float* X, const float* T, int n, float* gr
 int sur_net_eval(Surrogate& s, const float* X, int n, float* t, float* dtdx, cudaStream_t st) {
   cudaError_t e;
   set_attrs();
-  long long h = s.nxg;
-  if ((e = sur_grow(s.Xg, h, (long long)n * kDesc)) != cudaSuccess) return e;
-  h = s.nxg;
-  if ((e = sur_grow(s.Tg, h, (long long)n * (kDesc + 1))) != cudaSuccess) return e;
-  s.nxg = n;
+  if ((e = sur_grow(s.Xg, s.n_xg, (long long)n * kDesc)) != cudaSuccess) return e;
+  if ((e = sur_grow(s.Tg, s.n_tg, (long long)n * (kDesc + 1))) != cudaSuccess) return e;
   cudaMemcpyAsync(s.Xg, X, sizeof(float) * kDesc * n, cudaMemcpyHostToDevice, st);
   float* t_d = s.Tg + (size_t)kDesc * n;  // behind the gradients, whose rows are 16-byte aligned
   launch_dependent_smem(true, kSmInfer, k_net_infer, (n + 127) / 128, 128, st, s.Xg, n, net_of(s),

@@ -65,13 +65,13 @@ struct md_surrogate {
   int ns = 0, ns_cap = 0;
   float* SG = nullptr;
   double* SE = nullptr;
-  long long nsx = 0;
   float *SX = nullptr, *ST = nullptr;
+  long long n_sx = 0, n_st = 0;        // elements allocated
   // scratch
   double *loss_d = nullptr, *scratch = nullptr;
   int* rows_d = nullptr;
   float *Xg = nullptr, *Tg = nullptr;
-  long long nxg = 0;
+  long long n_rows = 0, n_xg = 0, n_tg = 0;  // elements allocated
   int* status_d = nullptr;
   cudaStream_t stream = nullptr;   // stream of the calls that take no context
   // force matching: stored configurations, loss weights, force scale
