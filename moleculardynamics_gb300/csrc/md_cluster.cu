@@ -1859,16 +1859,29 @@ void allow_smem(K kern) {
 
 int cluster_blocks(const ClusterList& cl) { return cl.nseg; }
 
-// Tiles of a list where neither the configuration nor the autotuner chose them.
-// One species: register-prefetch rows, the lean kernel's (33.6 -> 23.1 us per step
-// for 4,000 atoms, 91 -> 69 us for 256,000); block tiles for mixed species.  Up to
-// 65,536 atoms segments are cut at 1,152 staged atoms, so that more blocks share
-// the chip (23.1 -> 21.2 us for 4,000 atoms, 27.1 -> 25.4 us for 32,000); from
-// 87,808 atoms on the blocks fill it anyway (36.1 us against 39 us with the cut).
+// Tiles of a list where neither the configuration nor the autotuner chose them
+// (figures: us per step, atoms of argon at 0.0213 per cubic angstrom).
+// Row scheme.  One species: register-prefetch rows, the lean kernel's (4,000 atoms
+// 15.2 against 19.5 with block tiles, 256,000 72.8 against 84.0, 64 replicas of
+// 2,000 38.9 against 48.3); block tiles for mixed species.  Replicas of one cell
+// (minimum images, up to 500 atoms) cost the lean kernel an out-of-line call per
+// pair: 16 of 500 atoms 86 against 65, 256 of 500 176 against 102, 64 of 256 to
+// 32,000 (396,000 in all) 187 against 165.  So they take block tiles, unless the
+// other atoms outweigh them: 820,000 in all 295 against 304, 1,690,000 512 against
+// 563, and with a 32nd of the atoms in one-cell replicas (916,000) 325 against 324.
 static int choose_row_loads(const ClusterList& cl) {
   if (cl.row_loads) return cl.row_loads;
-  return cl.all_ng ? 2 : 1;
+  if (!cl.all_ng) return 1;
+  long long one_cell = 0;
+  for (const ClusterReplica& r : cl.h_rep)
+    if (r.G == 1) one_cell += r.n;
+  return one_cell == 0 || (cl.natoms >= 786432 && one_cell <= cl.natoms / 32) ? 2 : 1;
 }
+// Segments.  Up to 65,536 atoms they are cut at 1,152 staged atoms, so that more
+// blocks share the chip: one species 2,048 atoms 13.9 against 16.3, 32,000 20.9
+// against 22.0, 55,296 26.9 against 29.7 (62,500: 32.5 against 30.5); mixed species
+// 4,000 20.9 against 22.1, 32,000 26.6 against 27.2, 62,500 the same.  Beyond, the
+// blocks fill the chip anyway: 87,808 40.2 with the cut, 32.1 without.
 static int choose_stage_cap(const ClusterList& cl) {
   const int cap = cl.stage_cap ? cl.stage_cap : (cl.natoms <= 65536 ? 1152 : kClusterMaxStaged);
   return std::min(cap, kClusterMaxStaged);
