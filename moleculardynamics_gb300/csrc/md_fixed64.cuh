@@ -3,9 +3,15 @@
 // GB300's FP64 pipe takes 64 cycles of a scheduler for a warp-wide operation; a
 // 64-bit fixed-point product is four 32 x 32 -> 64 multiply-adds and about
 // twelve simpler instructions.  The angle terms of a triplet are 75 FP64
-// operations on quantities of known size (cosines, cutoffs in 0 .. 1, distances
-// and their reciprocals), so they are evaluated here with 56 bits after the
-// point, |v| < 64: a step of 1.4e-17, against FP64's 1.1e-16 for values about 1.
+// operations on quantities of known size (cosines, distances and their
+// reciprocals), so they are evaluated here with 56 bits after the point,
+// |v| < 64: a step of 1.4e-17, against FP64's 1.1e-16 for values about 1.
+// The one quantity that runs over many sizes, the cutoff function (e^-4 per
+// angstrom), carries a power of two beside its fixed-point number, as do the sums
+// and the coefficients that it multiplies: a term of 1e-10 has as many bits as
+// one of 1.  (Without it the force on an atom 4 angstrom from a bonded pair had an
+// error of 8e-14 of its size, 7 angstrom away 6e-11; 3e-15 with it at either.  The
+// reference's (1 - tanh) / 2 in FP64: 9e-15 and 2e-11.)
 // The caller keeps distances within 0.5 .. 16 angstrom.
 //
 // Plain integer code but for the two seeds; compiled for the host as well.
@@ -21,12 +27,13 @@ namespace mdgb {
 typedef long long q56;
 constexpr q56 kQOne = 1ll << 56;
 
-// a b, rounded down; |a|, |b| and the product below 64.  Limbs of 31 bits keep
+// a b, rounded; |a|, |b| and the product below 64.  Limbs of 31 bits keep
 // every partial product a signed 32 x 32 one.
 __host__ __device__ __forceinline__ q56 mulq(q56 a, q56 b) {
   const int32_t ah = (int32_t)(a >> 31), bh = (int32_t)(b >> 31);
   const int32_t al = (int32_t)a & 0x7FFFFFFF, bl = (int32_t)b & 0x7FFFFFFF;
-  const int64_t mid = (int64_t)ah * bl + (int64_t)al * bh + (((int64_t)al * bl) >> 31);
+  const int64_t mid =
+      (int64_t)ah * bl + (int64_t)al * bh + (((int64_t)al * bl + (1ll << 55)) >> 31);
   return (((int64_t)ah * bh) << 6) + (mid >> 25);
 }
 
@@ -48,7 +55,8 @@ __host__ __device__ __forceinline__ q56 toq(double v) {
   return (u >> 63) ? -(q56)r : (q56)r;
 }
 
-__host__ __device__ __forceinline__ double fromq(q56 v) {
+// v 2^-n
+__host__ __device__ __forceinline__ double fromq(q56 v, int n = 0) {
   const uint64_t a = v < 0 ? (uint64_t)-v : (uint64_t)v;
 #ifdef __CUDA_ARCH__
   const int lz = __clzll((long long)a);
@@ -59,7 +67,7 @@ __host__ __device__ __forceinline__ double fromq(q56 v) {
   const uint64_t m = (top >> 11) + ((top >> 10) & 1);
   // v = m 2^(11 - lz - 56); m may have carried into 2^53
   const uint64_t u = a == 0 ? 0
-                            : pack64(1023 + 7 - lz, m) |
+                            : pack64(1023 + 7 - lz - n, m) |
                                   ((uint64_t)v & 0x8000000000000000ull);
 #ifdef __CUDA_ARCH__
   return __longlong_as_double((long long)u);
@@ -136,11 +144,14 @@ static const
     0x85aac367cc487bll, 0x84f1f656379c1all, 0x843a28c3acde40ll, 0x8383594eefb6eell, 0x82cd8698ac2ba2ll, 0x8218af4373fc26ll,
     0x8164d1f3bc0307ll, 0x80b1ed4fd999abll, 0x80000000000000ll};
 
-// exp(-a), a >= 0: 2^-n 2^-(k / 128) e^-t, |t| <= ln 2 / 256, the last by its
-// series to t^5 (the next term is 5e-19)
-__host__ __device__ __forceinline__ q56 expnegq(q56 a) {
-  const q56 w = mulq(a, 0x171547652b82fe1ll);  // a / ln 2
-  const int n = (int)(w >> 56);
+// exp(-a) = v 2^-n, a >= 0, v in (0.49, 1]: 2^-n 2^-(k / 128) e^-t, |t| <=
+// ln 2 / 256, the last by its series to t^5 (the next term is 5e-19)
+__host__ __device__ __forceinline__ q56 expnegq(q56 a, int& n) {
+  // a / ln 2 (the second constant: 2^31 times what the first one rounds off, up to
+  // 27 units for a = 58)
+  const q56 w = mulq(a, 0x171547652b82fe1ll) +
+                (((int64_t)(int32_t)(a >> 31) * 1002342399) >> 56);
+  n = (int)(w >> 56);
   const q56 f = w & (kQOne - 1);
   const int k = (int)((f + (1ll << 48)) >> 49);
   const q56 t = mulq(f - ((q56)k << 49), 0xb17217f7d1cf7all);
@@ -152,45 +163,97 @@ __host__ __device__ __forceinline__ q56 expnegq(q56 a) {
   const int64_t h = (1ll << 39) - (((int64_t)t39 * p) >> 31);
   const q56 e = kQOne - t + mulq(mulq(t, t), h << 16);
 #ifdef __CUDA_ARCH__
-  const q56 v = mulq(__ldg(&kExpTableQ[k]), e);
+  return mulq(__ldg(&kExpTableQ[k]), e);
 #else
-  const q56 v = mulq(kExpTableQ[k], e);
+  return mulq(kExpTableQ[k], e);
 #endif
+}
+__host__ __device__ __forceinline__ q56 expnegq(q56 a) {
+  int n;
+  const q56 v = expnegq(a, n);
   return n > 62 ? 0 : v >> n;
 }
 
-#ifdef __CUDACC__
-__device__ __forceinline__ q56 rcpq(q56 den) {
-  const uint32_t f = 0x3F800000u + (uint32_t)((uint64_t)(den - kQOne) >> 33);
+// the fractions of the two seeds, from an argument in [1, 2) and [1, 4) as FP32
+// bits; correctly rounded on the host
+__host__ __device__ __forceinline__ uint32_t rcp_seed(uint32_t f) {
   float s;
+#ifdef __CUDA_ARCH__
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(__uint_as_float(f)));
-  return rcpq_seeded(den, seed_fraction(__float_as_uint(s)));
+  return seed_fraction(__float_as_uint(s));
+#else
+  __builtin_memcpy(&s, &f, 4);
+  s = (float)(1.0 / (double)s);
+  __builtin_memcpy(&f, &s, 4);
+  return seed_fraction(f);
+#endif
 }
-
-__device__ __forceinline__ void rsqrtq(double x, q56& r, q56& ir) {
-  const uint64_t b = (uint64_t)__double_as_longlong(x);
-  const uint32_t f = ((b >> 52) & 1 ? 0x3F800000u : 0x40000000u) | (uint32_t)((b >> 29) & 0x7FFFFFu);
+__host__ __device__ __forceinline__ uint32_t rsqrt_seed(uint32_t f) {
   float s;
+#ifdef __CUDA_ARCH__
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(__uint_as_float(f)));
-  rsqrtq_seeded(b, seed_fraction(__float_as_uint(s)), r, ir);
+  return seed_fraction(__float_as_uint(s));
+#else
+  __builtin_memcpy(&s, &f, 4);
+  s = (float)(1.0 / __builtin_sqrt((double)s));
+  __builtin_memcpy(&f, &s, 4);
+  return seed_fraction(f);
+#endif
 }
 
-// the cutoff 1 / (1 + e^x), x = 4 (r - R0), and minus its derivative 4 fc (1 - fc)
-__device__ __forceinline__ void cutoffq(q56 r, q56& fc, q56& dfc) {
+__host__ __device__ __forceinline__ q56 rcpq(q56 den) {
+  return rcpq_seeded(den, rcp_seed(0x3F800000u + (uint32_t)((uint64_t)(den - kQOne) >> 33)));
+}
+
+__host__ __device__ __forceinline__ void rsqrtq(double x, q56& r, q56& ir) {
+#ifdef __CUDA_ARCH__
+  const uint64_t b = (uint64_t)__double_as_longlong(x);
+#else
+  uint64_t b;
+  __builtin_memcpy(&b, &x, 8);
+#endif
+  const uint32_t f = ((b >> 52) & 1 ? 0x3F800000u : 0x40000000u) | (uint32_t)((b >> 29) & 0x7FFFFFu);
+  rsqrtq_seeded(b, rsqrt_seed(f), r, ir);
+}
+
+// the cutoff fc = 1 / (1 + e^x) = f 2^-n, x = 4 (r - R0), f in (0.24, 1], and
+// h = 4 (1 - fc), with which its derivative is -h fc
+__host__ __device__ __forceinline__ void cutoffq(q56 r, q56& f, int& n, q56& h) {
   const q56 x = (r - 0x14ccccc00000000ll) << 2;
-  const q56 s = expnegq(x < 0 ? -x : x);
+  const q56 v = expnegq(x < 0 ? -x : x, n);
+  const q56 s = n > 62 ? 0 : v >> n;
   const q56 d = rcpq(kQOne + s);
-  fc = x < 0 ? d : mulq(s, d);
-  dfc = mulq(fc, kQOne - fc) << 2;
+  if (x < 0) {
+    f = d;
+    h = (mulq(v << 2, d) + ((1ll << n) >> 1)) >> n;  // n at most 4
+    n = 0;
+  } else {
+    f = mulq(v, d);
+    h = d << 2;
+  }
 }
 
 // the angular function K - C / (D + c^2) and its prefactor 2 C c / (D + c^2)^2
-__device__ __forceinline__ void angularq(q56 c, q56& g, q56& gpre) {
+__host__ __device__ __forceinline__ void angularq(q56 c, q56& g, q56& gpre) {
   const q56 iq = rcpq((0x40aacd800000000ll + mulq(c, c)) >> 2) >> 2;
   const q56 h = 25 * iq;
   g = 0x72f7e0000000000ll - h;
   gpre = mulq(mulq(h, iq), c) << 1;
 }
-#endif
+
+// two sums of terms that share a power of two: (x, y) 2^-n, n that of the
+// largest term so far (smaller terms lose the bits below its last, as in FP64)
+struct SumQ {
+  q56 x = 0, y = 0;
+  int n = 127;
+};
+__host__ __device__ __forceinline__ void addq(SumQ& s, q56 x, q56 y, int n) {
+  const int d = n - s.n;
+  const int down = d > 0 ? (d < 63 ? d : 63) : 0;  // of the term
+  const int sum = d < 0 ? (d > -63 ? -d : 63) : 0;
+  s.x = (s.x >> sum) + (x >> down);
+  s.y = (s.y >> sum) + (y >> down);
+  s.n = n < s.n ? n : s.n;
+}
 
 }  // namespace mdgb

@@ -738,8 +738,8 @@ __device__ __forceinline__ void mb_angular(double c, double& g, double& gpre) {
 // and the cutoff; as the partner j of a bond the pair terms.
 struct Nb {
   double d[3][32], u[3][32];
-  q56 qu[3][32], qr[32], qir[32], qfc[32], qdm[32];  // fixed point; qdm: -dfc
-  // bit 6: not a third body of i's bonds (NG), 7: not a bond (NG, or beyond
+  q56 qu[3][32], qr[32], qir[32], qf[32], qh[32];  // fixed point (cutoffq's f and h)
+  // bits 16 and up: cutoffq's n; bit 6: not a third body of i's bonds (NG), 7: not a bond (NG, or beyond
   // the pair cutoff), 8: its distance is outside the fixed point's range;
   // bits 0-2: in the cell below i's along x, y, z, 3-5: above
   int flag[32];
@@ -771,14 +771,16 @@ __device__ __forceinline__ void mb_stage(Nb& N, int q, uint32_t e, double xi, do
   N.u[0][q] = ux, N.u[1][q] = uy, N.u[2][q] = uz;
   int flag = tj == SP_NG ? kNbNoThird | kNbNoBond : 0;
   if (mb_in_range(r2, 64.0)) {
-    q56 fc, dm;
-    const q56 r = toq(r2 * ir);
+    q56 r, irq, f, h;
+    int n;
+    rsqrtq(r2, r, irq);
     N.qu[0][q] = toq(ux), N.qu[1][q] = toq(uy), N.qu[2][q] = toq(uz);
     N.qr[q] = r;
-    N.qir[q] = toq(ir);
-    cutoffq(r, fc, dm);
-    N.qfc[q] = fc;
-    N.qdm[q] = dm;
+    N.qir[q] = irq;
+    cutoffq(r, f, n, h);
+    N.qf[q] = f;
+    N.qh[q] = h;
+    flag |= n << 16;
   } else {
     flag |= kNbFar;
   }
@@ -863,29 +865,29 @@ __device__ __noinline__ Angle mb_angle_far(const Nb& J, int j, const Nb& M, int 
   return A;
 }
 
-// the same in fixed point; the four sums stay there (sx, sy, sxj, syj)
+// the same in fixed point; the sums stay there, (x, y) in si and (xj, yj) in sj.
+// The cutoffs multiply last, so that each result keeps their power of two.
 __device__ __forceinline__ void mb_angle_q(double r2, const Nb& J, int j, const Nb& M, int m,
-                                           bool sums, q56& sx, q56& sy, q56& sxj, q56& syj,
-                                           Angle& A) {
-  const q56 rij = J.qr[j], irij = J.qir[j], rim = M.qr[m], irim = M.qir[m], fi = M.qfc[m];
-  q56 rjm, irjm, fj, dj, gi, pi, gj, pj;
+                                           bool sums, SumQ& si, SumQ& sj, Angle& A) {
+  const q56 rij = J.qr[j], irij = J.qir[j], rim = M.qr[m], irim = M.qir[m];
+  const q56 fi = M.qf[m], hi = M.qh[m];
+  const int ni = M.flag[m] >> 16;
+  q56 rjm, irjm, fj, hj, gi, pi, gj, pj;
+  int nj;
   rsqrtq(r2, rjm, irjm);
-  cutoffq(rjm, fj, dj);
+  cutoffq(rjm, fj, nj, hj);
   const q56 ci = dotq(J.qu[0][j], J.qu[1][j], J.qu[2][j], M.qu[0][m], M.qu[1][m], M.qu[2][m]);
   const q56 cj = mulq(rij - mulq(rim, ci), irjm);
   angularq(ci, gi, pi);
   angularq(cj, gj, pj);
-  const q56 xi = mulq(fi, pi), xj = mulq(fj, pj);
   if (sums) {
-    sx += mulq(fi, gi);
-    sy += mulq(xi, irim - mulq(ci, irij));
-    sxj += mulq(fj, gj);
-    syj += mulq(xj, irjm - mulq(cj, irij));
+    addq(si, mulq(fi, gi), mulq(fi, mulq(pi, irim - mulq(ci, irij))), ni);
+    addq(sj, mulq(fj, gj), mulq(fj, mulq(pj, irjm - mulq(cj, irij))), nj);
   }
-  A.a = fromq(mulq(xi, irij - mulq(ci, irim)) - mulq(M.qdm[m], gi));
-  A.p = fromq(-mulq(xi, mulq(irij, irim)));
-  A.b = fromq(-mulq(mulq(xj, mulq(rim, irij)), irjm));
-  A.q = fromq(mulq(mulq(xj, irij - mulq(cj, irjm)) - mulq(dj, gj), irjm));
+  A.a = fromq(mulq(fi, mulq(pi, irij - mulq(ci, irim)) - mulq(hi, gi)), ni);
+  A.p = fromq(-mulq(fi, mulq(pi, mulq(irij, irim))), ni);
+  A.b = fromq(-mulq(fj, mulq(mulq(pj, mulq(rim, irij)), irjm)), nj);
+  A.q = fromq(mulq(fj, mulq(mulq(pj, irij - mulq(cj, irjm)) - mulq(hj, gj), irjm)), nj);
 }
 
 // columns of a warp's coefficient table: 34 keeps five blocks on an SM (36 would
@@ -962,7 +964,7 @@ __global__ void __launch_bounds__(128, 5)
     const int j = 8 * warp + jj;  // bond of this lane in the tile
     const bool bond = j0 + j < S && !(NA.flag[j & 31] & kNbNoBond);
     double x = 0, y = 0, xj = 0, yj = 0;
-    q56 qx = 0, qy = 0, qxj = 0, qyj = 0;
+    SumQ si, sj;
     auto triplets = [&](const Nb& M, int m0, bool sums, bool store) {
       const int mn = min(32, S - m0);
       if (bond)
@@ -974,7 +976,7 @@ __global__ void __launch_bounds__(128, 5)
           const bool third = sums && !(M.flag[m] & kNbNoThird);
           Angle A;
           if (!((NA.flag[j] | M.flag[m]) & kNbFar) && mb_in_range(r2, 256.0)) {
-            mb_angle_q(r2, NA, j, M, m, third, qx, qy, qxj, qyj, A);
+            mb_angle_q(r2, NA, j, M, m, third, si, sj, A);
           } else {
             A = mb_angle_far(NA, j, M, m);
             if (third) {
@@ -1004,8 +1006,9 @@ __global__ void __launch_bounds__(128, 5)
     for (int m0 = 0; m0 < S; m0 += 32) {
       triplets(tile(m0), m0, true, once);
       // a lane's eight triplets of a tile stay below the fixed point's range
-      x += fromq(qx), y += fromq(qy), xj += fromq(qxj), yj += fromq(qyj);
-      qx = qy = qxj = qyj = 0;
+      x += fromq(si.x, si.n), y += fromq(si.y, si.n);
+      xj += fromq(sj.x, sj.n), yj += fromq(sj.y, sj.n);
+      si = sj = SumQ();
     }
 #pragma unroll
     for (int o = 1; o < 4; o <<= 1) {
