@@ -349,6 +349,10 @@ md_status mdgb_tc_selftest(const float* a, const float* b, float* c, int ncols, 
  * result (wide_ref, narrow_ref), for count values on the device. */
 md_status mdgb_conv_selftest(const float* f, const double* d, int count, double* wide,
                              double* wide_ref, float* narrow, float* narrow_ref);
+/* Self-test of the FP64 reciprocal, inverse root, root (of x, positive and normal)
+ * and exponential (of y) of the plain bond order, for count values on the device. */
+md_status mdgb_fp64_selftest(const double* x, const double* y, int count, double* rcp,
+                             double* rsqrt, double* root, double* expo);
 
 /* Wait for all work of the context; returns the first deferred error. */
 md_status md_synchronize(md_ctx* ctx);

@@ -810,7 +810,7 @@ __device__ __forceinline__ void mb_stage_pair(NbPair& N, int q, uint32_t e, doub
   PosT<double>::image(x, y, z, e, g);
   const double dx = xi - x, dy = yi - y, dz = zi - z;
   const double r2 = dx * dx + dy * dy + dz * dz;
-  const double r = r2 * rsqrt64(r2);
+  const double r = root64(r2, rsqrt64(r2));
   const double de = get_de<double>(ti, tj), re = get_re<double>(ti, tj),
                beta = get_beta<double>(ti, tj);
   const double x1 = exp64(-beta * (r - re)), x2 = x1 * x1, x4 = x2 * x2;
@@ -840,10 +840,11 @@ struct Angle {
 // in FP64, for distances outside the fixed point's range
 __device__ __noinline__ Angle mb_angle_far(const Nb& J, int j, const Nb& M, int m) {
   const double vx = M.d[0][m] - J.d[0][j], vy = M.d[1][m] - J.d[1][j], vz = M.d[2][m] - J.d[2][j];
-  const double r2 = vx * vx + vy * vy + vz * vz, irjm = rsqrt64(r2), rjm = r2 * irjm;
+  const double r2 = vx * vx + vy * vy + vz * vz, irjm = rsqrt64(r2), rjm = root64(r2, irjm);
   const double rij2 = J.d[0][j] * J.d[0][j] + J.d[1][j] * J.d[1][j] + J.d[2][j] * J.d[2][j];
   const double rim2 = M.d[0][m] * M.d[0][m] + M.d[1][m] * M.d[1][m] + M.d[2][m] * M.d[2][m];
-  const double irij = rsqrt64(rij2), rij = rij2 * irij, irim = rsqrt64(rim2), rim = rim2 * irim;
+  const double irij = rsqrt64(rij2), rij = root64(rij2, irij);
+  const double irim = rsqrt64(rim2), rim = root64(rim2, irim);
   double fi, dfi, fj, dfj, gi, pi, gj, pj;
   mb_cutoff(rim, fi, dfi);
   mb_cutoff(rjm, fj, dfj);

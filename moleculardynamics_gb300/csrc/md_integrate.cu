@@ -1005,7 +1005,38 @@ __global__ void k_conv_selftest(const float* f, const double* d, int n, double* 
   nrr[i] = __double2float_rn(d[i]);
 }
 
+__global__ void k_fp64_selftest(const double* in, int n, double* out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double x = in[i], ir = mdgb::rsqrt64(x);
+  out[i] = mdgb::rcp64(x);
+  out[(size_t)n + i] = ir;
+  out[2 * (size_t)n + i] = mdgb::root64(x, ir);
+  out[3 * (size_t)n + i] = mdgb::exp64(in[(size_t)n + i]);
+}
+
 }  // namespace
+
+extern "C" md_status mdgb_fp64_selftest(const double* x, const double* y, int count, double* rcp,
+                                        double* rsqrt, double* root, double* expo) {
+  if (count <= 0 || !x || !y || !rcp || !rsqrt || !root || !expo) return MD_BAD_ARGUMENT;
+  const size_t n = (size_t)count, B = n * sizeof(double);
+  double* d = nullptr;
+  if (cudaMalloc(&d, 6 * B) != cudaSuccess) return MD_CUDA_ERROR;
+  md_status r = MD_OK;
+  if (cudaMemcpy(d, x, B, cudaMemcpyHostToDevice) != cudaSuccess ||
+      cudaMemcpy(d + n, y, B, cudaMemcpyHostToDevice) != cudaSuccess)
+    r = MD_CUDA_ERROR;
+  if (r == MD_OK) {
+    k_fp64_selftest<<<(count + 255) / 256, 256>>>(d, count, d + 2 * n);
+    double* const out[4] = {rcp, rsqrt, root, expo};
+    for (int k = 0; k < 4 && r == MD_OK; k++)
+      if (cudaMemcpy(out[k], d + (2 + k) * n, B, cudaMemcpyDeviceToHost) != cudaSuccess)
+        r = MD_CUDA_ERROR;
+  }
+  cudaFree(d);
+  return r;
+}
 
 extern "C" md_status mdgb_conv_selftest(const float* f, const double* d, int count, double* wide,
                                         double* wide_ref, float* narrow, float* narrow_ref) {

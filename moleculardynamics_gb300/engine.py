@@ -104,6 +104,7 @@ EXPORTS = ["md_create", "md_destroy", "md_status_string", "md_last_error", "md_u
            "md_set_equilibration",
            "mdgb_many_body_forces_static", "md_autotune", "md_set_graphs", "md_batch_create",
            "md_batch_size", "md_batch_records", "mdgb_tc_selftest", "mdgb_conv_selftest",
+           "mdgb_fp64_selftest",
            "md_surrogate_create",
            "md_surrogate_destroy", "md_surrogate_param_count", "md_surrogate_collect",
            "md_surrogate_samples", "md_surrogate_train", "md_surrogate_attach",
@@ -156,6 +157,7 @@ def load(path: str | None = None) -> C.CDLL:
     L.md_device_sm_count.argtypes = [C.c_int, P(C.c_int)]
     L.mdgb_tc_selftest.argtypes = [_fp, _fp, _fp, C.c_int, C.c_int]
     L.mdgb_conv_selftest.argtypes = [_fp, _dp, C.c_int, _dp, _dp, _fp, _fp]
+    L.mdgb_fp64_selftest.argtypes = [_dp, _dp, C.c_int, _dp, _dp, _dp, _dp]
     L.md_surrogate_create.argtypes = [C.c_int, C.c_ulonglong, C.c_float, P(C.c_void_p)]
     L.md_surrogate_destroy.argtypes = [C.c_void_p]
     L.md_surrogate_param_count.restype = C.c_int
@@ -711,6 +713,22 @@ def conv_selftest(f: np.ndarray, d: np.ndarray):
     if s != 0:
         raise EngineError(s, "mdgb_conv_selftest")
     return w, wr, nr, nrr
+
+
+def fp64_selftest(x: np.ndarray, y: np.ndarray):
+    """The plain bond order's FP64 functions on the device: (1 / x, x^(-1/2),
+    x^(1/2), exp(y)); x positive and normal, x and y of equal length."""
+    L = load()
+    x = np.ascontiguousarray(x, np.float64)
+    y = np.ascontiguousarray(y, np.float64)
+    n = len(x)
+    if len(y) != n:
+        raise ValueError("x and y differ in length")
+    out = [np.zeros(n) for _ in range(4)]
+    s = L.mdgb_fp64_selftest(x, y, n, *out)
+    if s != 0:
+        raise EngineError(s, "mdgb_fp64_selftest")
+    return tuple(out)
 
 
 def pinned(shape, dtype=np.float64):
