@@ -1061,7 +1061,8 @@ __global__ void __launch_bounds__(128, 5)
           // j and m on opposite sides of i's cell are no candidates of each other
           const bool seen = SLOTS && !(NA.flag[jb] & opposite);
           if (NA.flag[jb] & kNbNoBond) {
-            miss += seen && NA.flag[jb] & kNbNoThird;
+            // a third body beyond the slots counts its own (k_mb_gather)
+            miss += seen && m0 + m < kMbSlots && NA.flag[jb] & kNbNoThird;
             continue;
           }
           const double wi = wsm[warp][0][b], wj = wsm[warp][1][b];
