@@ -150,6 +150,7 @@ struct md_ctx {
   int* mb_slen = nullptr;
   void *xsi = nullptr, *xsj = nullptr, *mb_fslot = nullptr;
   long long mb_elems = 0;
+  int mb_slots = 0;  // of mb_fslot, per atom
   // flags and reductions
   int* status = nullptr;
   int wait_limit = 1 << 20;  // polls of a bounded mbarrier wait (md_set_wait_limit)
@@ -282,19 +283,29 @@ int mb_pitch(const md_ctx* c) { return std::max(c->mb.cap, 4); }
 md_status ensure_mb_scratch(md_ctx* c) {
   const size_t nmb = (size_t)std::max(c->cfg.n_mb, 1);
   const size_t es = c->mixed() ? sizeof(float) : sizeof(double);
-  if (!c->mixed() && !c->mb_fslot)
-    CK(cudaMalloc(&c->mb_fslot, 4 * es * kMbSlotCount * nmb), "mb third-body forces");
   const long long need = (long long)mb_pitch(c) * (long long)nmb;
-  if (need <= c->mb_elems && c->mb_sl) return MD_OK;
-  for (void** p : {(void**)&c->mb_sl, &c->xsi, &c->xsj})
-    if (*p) {
-      cudaFree(*p);
-      *p = nullptr;
+  if (need > c->mb_elems || !c->mb_sl) {
+    void** const bufs[4] = {(void**)&c->mb_sl, &c->xsi, &c->xsj, &c->mb_fslot};
+    for (void** p : bufs)
+      if (*p) {
+        cudaFree(*p);
+        *p = nullptr;
+      }
+    CK(cudaMalloc(&c->mb_sl, sizeof(uint32_t) * (size_t)need), "mb short list");
+    CK(cudaMalloc(&c->xsi, es * (size_t)need), "mb xi");
+    CK(cudaMalloc(&c->xsj, es * (size_t)need), "mb xi");
+    c->mb_elems = need;
+    c->mb_slots = 0;
+    size_t free_bytes = 0, total = 0;
+    if (!c->mixed() && cudaMemGetInfo(&free_bytes, &total) == cudaSuccess)
+      c->mb_slots = mb_slot_count((long long)nmb, mb_pitch(c), free_bytes);
+    if (c->mb_slots &&
+        cudaMalloc(&c->mb_fslot, 3 * es * (size_t)c->mb_slots * nmb) != cudaSuccess) {
+      cudaGetLastError();  // none, then
+      c->mb_fslot = nullptr;
+      c->mb_slots = 0;
     }
-  CK(cudaMalloc(&c->mb_sl, sizeof(uint32_t) * (size_t)need), "mb short list");
-  CK(cudaMalloc(&c->xsi, es * (size_t)need), "mb xi");
-  CK(cudaMalloc(&c->xsj, es * (size_t)need), "mb xi");
-  c->mb_elems = need;
+  }
   return MD_OK;
 }
 
@@ -343,6 +354,7 @@ MbArgs mb_args(md_ctx* c, double* f3, int ljexist) {
   a.sl = c->mb_sl;
   a.pitch = mb_pitch(c);
   a.fslot = c->mb_fslot;
+  a.slots = c->mb_slots;
   a.slen = c->mb_slen;
   a.xsi = c->xsi;
   a.xsj = c->xsj;

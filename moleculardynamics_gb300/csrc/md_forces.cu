@@ -894,7 +894,6 @@ __device__ __forceinline__ void mb_angle_q(double r2, const Nb& J, int j, const 
 // columns of a warp's coefficient table: 34 keeps five blocks on an SM (36 would
 // store without bank conflicts, but only four blocks fit)
 constexpr int kMbPitch = 34;
-constexpr int kMbSlots = kMbSlotCount;  // third-body force slots per atom
 
 // Sum of 4 values over the warp, each value to a quarter of the lanes: value
 // ((lane >> 3) & 3) of every lane's v comes back in all lanes of that quarter
@@ -934,7 +933,7 @@ __global__ void __launch_bounds__(128, 5)
                double* __restrict__ f3, int n, const uint32_t* __restrict__ sl, int pitch,
                const int* __restrict__ slen, Grid g, const int* __restrict__ cell3, int ljexist,
                double* __restrict__ wi_s, double* __restrict__ wj_s, double* __restrict__ fslot,
-               int* __restrict__ missing, double* __restrict__ epart,
+               int slots, int* __restrict__ missing, double* __restrict__ epart,
                double* __restrict__ eatom, const int* __restrict__ run_if) {
   grid_wait();
   grid_launch_dependents();
@@ -1062,7 +1061,7 @@ __global__ void __launch_bounds__(128, 5)
           const bool seen = SLOTS && !(NA.flag[jb] & opposite);
           if (NA.flag[jb] & kNbNoBond) {
             // a third body beyond the slots counts its own (k_mb_gather)
-            miss += seen && m0 + m < kMbSlots && NA.flag[jb] & kNbNoThird;
+            miss += seen && m0 + m < slots && NA.flag[jb] & kNbNoThird;
             continue;
           }
           const double wi = wsm[warp][0][b], wj = wsm[warp][1][b];
@@ -1105,8 +1104,8 @@ __global__ void __launch_bounds__(128, 5)
           fy = fma(w, M.u[1][m], fy);
           fz = fma(w, M.u[2][m], fz);
         }
-        if (SLOTS && m0 + m < kMbSlots) {
-          double* o = fslot + 4 * ((size_t)i * kMbSlots + m0 + m);
+        if (SLOTS && m0 + m < slots) {
+          double* o = fslot + 3 * ((size_t)i * slots + m0 + m);
           const double ox = fma(v[3], M.u[0][m], v[0]), oy = fma(v[3], M.u[1][m], v[1]),
                   oz = fma(v[3], M.u[2][m], v[2]);
           o[0] = j0 ? o[0] + ox : ox;
@@ -1294,7 +1293,7 @@ __global__ void __launch_bounds__(128)
                 double* __restrict__ f3, int n, const uint32_t* __restrict__ sl, int pitch,
                 const int* __restrict__ slen, Grid g, const int* __restrict__ cell3,
                 double rcutsq, const double* __restrict__ wi_s, const double* __restrict__ wj_s,
-                const double* __restrict__ fslot, int* __restrict__ missing,
+                const double* __restrict__ fslot, int slots, int* __restrict__ missing,
                 double* __restrict__ epart, const int* __restrict__ run_if) {
   grid_wait();
   grid_launch_dependents();
@@ -1308,7 +1307,7 @@ __global__ void __launch_bounds__(128)
   for (int s = lane; s < Sk; s += 32) {
     const uint32_t e = sl[(size_t)k * pitch + s];
     const int i = entry_index(e);
-    const int Si = slen[i], lim = min(Si, kMbSlots);
+    const int Si = slen[i], lim = min(Si, slots);
     const uint4* row = reinterpret_cast<const uint4*>(sl + (size_t)i * pitch);
     int q = -1;
     for (int q0 = 0; q0 < lim && q < 0; q0 += 4) {  // pitch is a multiple of 4
@@ -1319,7 +1318,7 @@ __global__ void __launch_bounds__(128)
       if (entry_index(w.x) == k) q = q0;
     }
     if (q >= 0 && q < lim) {
-      const double* o = fslot + 4 * ((size_t)i * kMbSlots + q);
+      const double* o = fslot + 3 * ((size_t)i * slots + q);
       fx += o[0];
       fy += o[1];
       fz += o[2];
@@ -1743,12 +1742,12 @@ static void launch_mb64(const MbArgs& a, cudaStream_t st) {
                    a.len, a.grid, a.rcutsq, a.sl, (size_t)a.pitch, 1, a.slen, gate);
   if (!a.ref_rows) {
     launch_dependent(a.early, k_mb_bonds<ENERGY, true>, a.n, 128, st, a.pos, a.f3, a.n, a.sl, a.pitch,
-                     a.slen, a.grid, a.cell3, a.ljexist, wi, wj, fs, a.missing, e1, ea, gate);
+                     a.slen, a.grid, a.cell3, a.ljexist, wi, wj, fs, a.slots, a.missing, e1, ea, gate);
     launch_dependent(a.early, k_mb_gather<ENERGY>, B, 128, st, a.pos, a.posf, a.f3, a.n, a.sl,
-                     a.pitch, a.slen, a.grid, a.cell3, a.rcutsq, wi, wj, fs, a.missing, e2, gate);
+                     a.pitch, a.slen, a.grid, a.cell3, a.rcutsq, wi, wj, fs, a.slots, a.missing, e2, gate);
   } else if constexpr (!ENERGY) {
     launch_dependent(a.early, k_mb_bonds<false, false>, a.n, 128, st, a.pos, a.f3, a.n, a.sl, a.pitch,
-                     a.slen, a.grid, nullptr, a.ljexist, wi, wj, nullptr, a.missing, nullptr, nullptr,
+                     a.slen, a.grid, nullptr, a.ljexist, wi, wj, nullptr, 0, a.missing, nullptr, nullptr,
                      gate);
     k_mb_pass2<<<B, 128, 0, st>>>(a.pos, a.f3, a.n, a.sl, a.pitch, a.slen, a.grid, a.ref_rows,
                                   a.ref_nls, a.ref_nlargest, a.rcutsq, wi, wj, a.missing);

@@ -62,8 +62,8 @@ struct MbArgs {
   int* slen;
   void* xsi;            // per (i, slot), T: the bond's factor va E / (4 (1 + xi_ij)^2)
   void* xsj;            // and va E / (4 (1 + xi_ji)^2), NaN where there is no bond
-  void* fslot = nullptr;  // FP64: forces on third bodies, 4 for each of an atom's kMbSlotCount
-                          // first slots (not needed with ref_rows)
+  void* fslot = nullptr;  // FP64: forces on third bodies, 3 for each of an atom's first
+  int slots = 0;          // `slots` slots (not needed with ref_rows)
   int* missing;
   bool early = false;   // launches may start early (streams of this library only)
   const int* run_if = nullptr;  // force launches only: return at once unless *run_if != 0
@@ -81,6 +81,16 @@ void launch_lj_redo64(const ForceArgs& a, cudaStream_t st);
 void launch_mb(const MbArgs& a, bool fp32, bool energy, cudaStream_t st);
 int lj_blocks(int n, bool fp32);  // blocks of an energy launch of launch_lj
 int mb_blocks(int n, bool fp32);  // entries of an energy launch in epart1, epart2
-constexpr int kMbSlotCount = 64;
+// Force slots for each of n atoms with short lists of up to `pitch`: 64 (usual
+// lattices use 28), fewer where those would take more than a quarter of the free
+// memory.  Third bodies beyond them are evaluated by k_mb_gather, so any number will
+// do; with 64 of them an atom takes 1.5 KB more.
+inline int mb_slot_count(long long n, int pitch, unsigned long long free_bytes) {
+  int slots = pitch < 64 ? pitch : 64;
+  while (slots && 3ull * sizeof(double) * (unsigned long long)slots * (unsigned long long)n >
+                      free_bytes / 4)
+    slots /= 2;
+  return slots;
+}
 
 }  // namespace mdgb
