@@ -150,6 +150,30 @@ inline uint64_t divisor_fraction(uint64_t b) {
   return q >> 64 ? ~0ull : (uint64_t)q;
 }
 
+// x truncated to FP32 by moving the fields (a conversion instruction takes the
+// FP64 pipe): tiny values to 0; NaN beyond FP32's range
+__host__ __device__ __forceinline__ float trunc32(double x) {
+#ifdef __CUDA_ARCH__
+  const uint64_t u = (uint64_t)__double_as_longlong(x);
+#else
+  uint64_t u;
+  __builtin_memcpy(&u, &x, 8);
+#endif
+  const uint32_t hi = (uint32_t)(u >> 32), lo = (uint32_t)u;
+  const uint32_t e = (hi >> 20) & 0x7FFu;
+  const uint32_t m = ((hi & 0xFFFFFu) << 3) | (lo >> 29);
+  const uint32_t v = e >= 1151u  ? 0x7FC00000u
+                     : e < 897u ? 0u
+                                : (hi & 0x80000000u) | ((e - 896u) << 23) | m;
+#ifdef __CUDA_ARCH__
+  return __uint_as_float(v);
+#else
+  float f;
+  __builtin_memcpy(&f, &v, 4);
+  return f;
+#endif
+}
+
 #ifdef __CUDACC__
 __device__ __forceinline__ uint64_t ircp64(uint64_t b) {
   const uint32_t f = 0x3F800000u | (uint32_t)((b >> 29) & 0x7FFFFFu);
@@ -242,16 +266,6 @@ static __device__ const double2 kExp2Table[64] = {
     {0x1.dfc97337b9b5fp+0, -0x1.1a5cd4f184b5cp-54}, {0x1.e502ee78b3ff6p+0, 0x1.39e8980a9cc8fp-55},
     {0x1.ea4afa2a490dap+0, -0x1.e9c23179c2893p-54}, {0x1.efa1bee615a27p+0, 0x1.dc7f486a4b6b0p-54},
     {0x1.f50765b6e4540p+0, 0x1.9d3e12dd8a18bp-54}, {0x1.fa7c1819e90d8p+0, 0x1.74853f3a5931ep-55}};
-
-// x truncated to FP32 by moving the fields (a conversion instruction takes the
-// FP64 pipe): tiny values to 0; NaN beyond FP32's range
-__device__ __forceinline__ float trunc32(double x) {
-  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
-  const uint32_t e = (hi >> 20) & 0x7FFu;
-  if (e >= 1151u) return __int_as_float(0x7FC00000);
-  const uint32_t m = ((hi & 0xFFFFFu) << 3) | (lo >> 29);
-  return __uint_as_float(e < 897u ? 0u : (hi & 0x80000000u) | ((e - 896u) << 23) | m);
-}
 
 // exp(x) by the table-driven method of P. T. P. Tang (ACM TOMS 15, 1989): x =
 // (64 q + k) ln 2 / 64 + r, exp(x) = 2^q 2^(k/64) (1 + r + r^2/2 + ... + r^6/720),

@@ -14,8 +14,8 @@
 #include <algorithm>
 
 #include "../../include/mdgb.h"
-#include "md_exact64.cuh"
 #include "md_neighbor.cuh"
+#include "md_split32.cuh"
 #include "md_surrogate.h"
 #include "md_tc.cuh"
 
@@ -153,30 +153,6 @@ __global__ void __launch_bounds__(128)
 // 22 neighbours within 3 angstrom of 32,768 atoms: forces 162 -> 73 us, descriptors
 // 73 -> 38, residual transform 126 -> 59 against 32 pairs at a time in index
 // order (shared-memory atomics and the index arithmetic bounded them).
-
-// x as the sum of two FP32 numbers, by moving the fields (conversions and
-// differences in FP64 take the narrow FP64 pipe)
-__device__ __forceinline__ float2 split64(double x) {
-  const float h = trunc32(x);
-  const uint32_t e = ((uint32_t)__double2hiint(x) >> 20) & 0x7FFu;
-  // the low 29 bits of the mantissa, worth 2^(e - 1075) each
-  const float u = __uint_as_float(e > 948u && e < 1151u ? (e - 948u) << 23 : 0u);
-  const float l = (float)((uint32_t)__double2loint(x) & 0x1FFFFFFFu) * u;
-  return make_float2(h, __double2hiint(x) < 0 ? -l : l);
-}
-
-// x_j + img box - x_i to FP32 accuracy
-__device__ __forceinline__ float diff32(float2 xj, float2 xi, int img, float2 box) {
-  float s = xj.x, l = xj.y - xi.y;
-  if (img) {
-    const float bh = img > 0 ? box.x : -box.x;
-    s = __fadd_rn(xj.x, bh);
-    const float t = __fsub_rn(s, xj.x);  // two-sum: s + rest is x_j + bh
-    const float rest = __fadd_rn(__fsub_rn(xj.x, __fsub_rn(s, t)), __fsub_rn(bh, t));
-    l = __fadd_rn(l, __fadd_rn(rest, img > 0 ? box.y : -box.y));
-  }
-  return __fadd_rn(__fsub_rn(s, xi.x), l);
-}
 
 // visit(s, S, j, ux, uy, uz, r, 1/r, fc, dfc) for neighbour s of atom i's S, a lane
 // each; returns S
