@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(128, 8) k_lj_fp64(const __grid_constant__ Lj64
       lj64_refresh<ENERGY>(first + tid, a.pos, sums + 3 * tid, a.ld, a.list, a.len, a.w, a.skin,
                            a.cap, a.rv2, a.pos_build, a.rcutsq, a.c, ev);
     if (t == 0) atomicAdd(&a.skin[4], 1);
-    __syncthreads();  // gate and trip are the same for the whole launch
+    __syncthreads();  // the whole block is here: it read the flag once (s_trip)
     if (live && gl < 3) acc = sums[3 * (warp * kAtoms + group) + gl];
     if (live) ti = species64(a.pos[i].w);
   } else {
@@ -1346,12 +1346,13 @@ __global__ void __launch_bounds__(128)
 }
 
 // ---- the precision form: pass 1 and pass 2 ----
-// The order and the roundings of these FP32 sums are part of the form's
-// results: the bond order jumps where a pair passes the cutoff, so two runs
-// that differ in the last FP32 bit part by 1e-2 of a velocity once a pair
-// crosses it a step earlier.  Measured: k_mb_bonds<float> took 228 us per
-// evaluation of 32,768 atoms against 420 here, but its runs of 50 steps left
-// the present ones' tolerance for 45% of the seeds.
+// The order and the roundings of these FP32 sums are part of the form's results:
+// the bond order jumps by 1e-3 of a force where a pair passes the cutoff, so two
+// runs that differ in the last FP32 bit part once a pair crosses it a step earlier
+// in one of them.  k_mb_bonds in FP32 took 228 us per evaluation of 32,768 atoms
+// against 420 here, but after 50 steps at 900 K its velocities differed from the
+// present ones by up to 1e-2 of their size for 45% of the seeds, by 1e-6 for the
+// others; so the passes and their bits stay.
 
 // Third bodies m of the warp's atom i (pass 1): what depends on i and m
 // only, computed once per warp instead of once per pair i-j.
