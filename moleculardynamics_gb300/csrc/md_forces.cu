@@ -1760,12 +1760,20 @@ static void launch_mb32(const MbArgs& a, cudaStream_t st) {
   const int* gate = ENERGY ? nullptr : a.run_if;
   float *wi = (float*)a.xsi, *wj = (float*)a.xsj;
   const int B = nblk(a.n, 4);
-  launch_dependent(a.early, k_mb_short<float>, B, 128, st, a.pos, a.posf, a.n, a.list, a.ri, a.rk,
+  // Blocks that wait early keep their places, and a grid of up to a wave (8 blocks
+  // an SM) then lies unevenly on the SMs: us per step in a periodic box with early
+  // launches and without 1,000 atoms 76.9 and 74.4, 2,744 101.8 and 80.2, 4,096 105.8
+  // and 90.1; below and beyond 512 71.0 and 72.3, 5,832 110.5 and 112.7, 32,768 406.6
+  // and 410.5.  Gated launches, which mostly return at once, start early at any size
+  // (walls: 1,728 atoms 88.0 and 94.7); energy launches for a block per SM at most
+  // (records of 64 atoms 100.8 and 105.2, of 2,744 163.2 and 141.9, of 32,768 the same).
+  const bool early = a.early && (ENERGY ? B <= 152 : gate || B <= 152 || B > 8 * 152);
+  launch_dependent(early, k_mb_short<float>, B, 128, st, a.pos, a.posf, a.n, a.list, a.ri, a.rk,
                    a.len, a.grid, a.rcutsq, a.sl, 1, (size_t)a.n, a.slen, gate);
-  launch_dependent(a.early, k_mb_pass1_32<ENERGY>, B, 128, st, a.pos, a.posf, a.f3, a.n, a.sl, a.slen,
+  launch_dependent(early, k_mb_pass1_32<ENERGY>, B, 128, st, a.pos, a.posf, a.f3, a.n, a.sl, a.slen,
                    a.grid, a.ljexist, wi, wj, ENERGY ? a.epart1 : nullptr, ENERGY ? a.eatom : nullptr,
                    gate);
-  launch_dependent(a.early, k_mb_pass2_32<ENERGY>, B, 128, st, a.pos, a.posf, a.f3, a.n, a.sl, a.slen,
+  launch_dependent(early, k_mb_pass2_32<ENERGY>, B, 128, st, a.pos, a.posf, a.f3, a.n, a.sl, a.slen,
                    a.grid, a.cell3, a.ref_rows, a.ref_nls, a.ref_nlargest, a.rcutsq, wi, wj, a.missing,
                    ENERGY ? a.epart2 : nullptr, gate);
 }
