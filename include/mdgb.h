@@ -78,11 +78,13 @@ typedef struct md_config {
   int lj_kernel;           /* MD_LJ_AUTO, MD_LJ_ROWS or MD_LJ_CLUSTER (precision form) */
   int cluster_cells;       /* cells per segment of the cluster kernel (0: default) */
   int cluster_threads;     /* threads per segment block (0: default; multiple of 32, <= 224) */
-  int cluster_row_loads;   /* rows of the cluster kernel: 0 default / autotuned, 1 TMA tiles of
+  int cluster_row_loads;   /* rows of the cluster kernel: 0 autotuned, or picked at each list
+                              build (2 for one species, 1 for several and for replicas of
+                              one cell); 1 TMA tiles of
                               the block in shared memory (two in flight), 2 per-lane register
                               prefetch, 3 TMA tiles of each warp, 4 as 1 with three in flight */
-  int cluster_stage_cap;   /* staged atoms per segment of the cluster kernel (0: default /
-                              autotuned; otherwise 64 .. 11264) */
+  int cluster_stage_cap;   /* staged atoms per segment of the cluster kernel (0: autotuned,
+                              or picked at each list build; otherwise 64 .. 11264) */
 } md_config;
 
 /* LJ kernel of the precision form.  ROWS: compact rows of packed atom

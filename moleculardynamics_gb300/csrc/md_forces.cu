@@ -923,8 +923,10 @@ __device__ __forceinline__ double quarter_sum(double v0, double v1, double v2, d
 //
 // The angle terms in FP64 (75 operations a triplet) kept the FP64 pipe 86% busy
 // and everything else idle: 568 us for 4,096 atoms; in 64-bit fixed point
-// (md_fixed64.cuh, 6 FP64 operations) 279 us, and with the pair terms
-// staged by a second warp and five blocks on an SM 265 us.
+// (md_fixed64.cuh, 6 FP64 operations) 279 us, with the pair terms staged by a
+// second warp and five blocks on an SM 265 us, and with the power of two that keeps
+// small terms' bits, rounded products and exponentials to half a unit 293 us (FP64
+// pipe 54%, issue 46%).
 // SLOTS: with the engine's own rows; caller-supplied rows may lack symmetry,
 // and k_mb_pass2 evaluates their third bodies.
 template <bool ENERGY, bool SLOTS>
