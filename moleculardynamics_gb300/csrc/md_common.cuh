@@ -14,6 +14,9 @@ namespace mdgb {
 // 32-byte aligned so that one atom is one 256-bit load.
 typedef double4_32a md_double4;
 
+// SMs of a GB300; rules that choose lanes or launches by size count in them
+constexpr int kSms = 152;
+
 // species indices, common/Constants.h:13-15
 constexpr int SP_N = 0, SP_O = 1, SP_NG = 2;
 

@@ -1640,7 +1640,7 @@ inline int nblk(long long n, int t) { return (int)((n + t - 1) / t); }
 //  1,700        4.55 4.30 4.62 6.31    13,500  13.9 9.59 6.95 6.83
 // (a thread per atom with the FP64 instructions: 20.5 at 864 to 8,000 atoms).
 static int lj64_lanes(int n) {
-  return n <= 5 * 152 ? 32 : (n <= 17 * 152 ? 16 : (n <= 85 * 152 ? 8 : 4));
+  return n <= 5 * kSms ? 32 : (n <= 17 * kSms ? 16 : (n <= 85 * kSms ? 8 : 4));
 }
 
 template <int G>
@@ -1650,13 +1650,13 @@ static void launch_lj64_g(const Lj64Args& k, int mode, bool energy, cudaStream_t
   // lies unevenly on the SMs: 100 steps of 8,000 atoms within walls took 6.2 ms
   // with early launches and 5.1 without; at 172 atoms they save a sixth.
   if (mode == LJ64_STEP)
-    launch_dependent(B <= 2 * 152, k_lj_fp64<G, LJ64_STEP, false>, B, 128, st, k);
+    launch_dependent(B <= 2 * kSms, k_lj_fp64<G, LJ64_STEP, false>, B, 128, st, k);
   else if (mode == LJ64_REDO)
-    launch_dependent(B <= 2 * 152, k_lj_fp64<G, LJ64_REDO, false>, B, 128, st, k);
+    launch_dependent(B <= 2 * kSms, k_lj_fp64<G, LJ64_REDO, false>, B, 128, st, k);
   else if (energy)
-    launch_dependent(B <= 2 * 152, k_lj_fp64<G, LJ64_FORCE, true>, B, 128, st, k);
+    launch_dependent(B <= 2 * kSms, k_lj_fp64<G, LJ64_FORCE, true>, B, 128, st, k);
   else
-    launch_dependent(B <= 2 * 152, k_lj_fp64<G, LJ64_FORCE, false>, B, 128, st, k);
+    launch_dependent(B <= 2 * kSms, k_lj_fp64<G, LJ64_FORCE, false>, B, 128, st, k);
 }
 
 static void launch_lj64(const ForceArgs& a, int mode, bool energy, cudaStream_t st) {
@@ -1769,7 +1769,7 @@ static void launch_mb32(const MbArgs& a, cudaStream_t st) {
   // and 410.5.  Gated launches, which mostly return at once, start early at any size
   // (walls: 1,728 atoms 88.0 and 94.7); energy launches for a block per SM at most
   // (records of 64 atoms 100.8 and 105.2, of 2,744 163.2 and 141.9, of 32,768 the same).
-  const bool early = a.early && (ENERGY ? B <= 152 : gate || B <= 152 || B > 8 * 152);
+  const bool early = a.early && (ENERGY ? B <= kSms : gate || B <= kSms || B > 8 * kSms);
   launch_dependent(early, k_mb_short<float>, B, 128, st, a.pos, a.posf, a.n, a.list, a.ri, a.rk,
                    a.len, a.grid, a.rcutsq, a.sl, 1, (size_t)a.n, a.slen, gate);
   launch_dependent(early, k_mb_pass1_32<ENERGY>, B, 128, st, a.pos, a.posf, a.f3, a.n, a.sl, a.slen,

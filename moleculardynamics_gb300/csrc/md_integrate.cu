@@ -833,7 +833,7 @@ static void launch_gear64(const GearArgs& a, bool predict, const int* hit, int* 
   if (a.n <= 0) return;
   Gear64 g;
   gear64_args(a, a.pos, predict, g);
-  const int T = a.n <= 8 * 152 ? 32 : 128;
+  const int T = a.n <= 8 * kSms ? 32 : 128;
   launch_dependent(true, k_gear64<MODE>, nblk(4LL * a.n, T), T, st, g, (const double*)a.f3, a.n, hit, hits,
                    flag_next);
 }

@@ -1722,7 +1722,7 @@ void fh_forward(const Surrogate& s, const float* X, int n, float* gcoef, bool ke
     launch_dependent_smem(true, fh_smem(H, A), kernel, sblocks(n, 32 * A * g), 128 * g, st, X, n,
                           s.FP_d, gs, gcoef, xT, h1, h2);
   };
-  const bool two = n > 64 * 152;  // blocks of 64 atoms for every SM
+  const bool two = n > 64 * kSms;  // blocks of 64 atoms for every SM
   if (s.fh_hidden == 32)
     two ? run(k_fh_forward<32, 2>, 32, 2) : run(k_fh_forward<32, 1>, 32, 1);
   else if (s.fh_hidden == 64)
